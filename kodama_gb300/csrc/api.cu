@@ -1604,8 +1604,8 @@ void matrix_from_device_graph(Ctx& ctx, const float* d_x, int n, int d, int* d_g
     tail.gi.assign(static_cast<size_t>(n) * K, 0);
     tail.gd.assign(static_cast<size_t>(n) * K, 0.0f);
     if (o->apply_dissimilarity) {
-      int* d_lbs = ctx.alloc<int>(static_cast<size_t>(M) * n);
-      ck_launch(kgb::transpose_runs(d_res, M, n, d_lbs, st), "transpose");
+      int* d_lbs = ctx.alloc<int>(static_cast<size_t>(kgb::label_stride(M)) * n);
+      ck_launch(kgb::transpose_runs(d_res, M, n, kgb::label_stride(M), d_lbs, st), "transpose");
       int* d_oidx = ctx.alloc<int>(static_cast<size_t>(n) * K);
       float* d_odist = ctx.alloc<float>(static_cast<size_t>(n) * K);
       kgb::DissimArgs a{};
@@ -1617,6 +1617,7 @@ void matrix_from_device_graph(Ctx& ctx, const float* d_x, int n, int d, int* d_g
       a.idx = d_gidx;
       a.dist = d_gdist;
       a.lbs = d_lbs;
+      a.stride = kgb::label_stride(M);
       a.out_idx = d_oidx;
       a.out_dist = d_odist;
       ck_launch(kgb::dissimilarity(a, st), "dissimilarity");
@@ -2636,8 +2637,8 @@ int kgb_dissimilarity_inplace(int32_t* gidx, float* gdist, int32_t samples, int3
     int* d_idx = ctx.upload(gidx, total);
     float* d_dist = ctx.upload(gdist, total);
     const int* d_res = ctx.upload(res, static_cast<size_t>(runs) * samples);
-    int* d_lbs = ctx.alloc<int>(static_cast<size_t>(runs) * samples);
-    ck_launch(kgb::transpose_runs(d_res, runs, samples, d_lbs, st), "transpose");
+    int* d_lbs = ctx.alloc<int>(static_cast<size_t>(kgb::label_stride(runs)) * samples);
+    ck_launch(kgb::transpose_runs(d_res, runs, samples, kgb::label_stride(runs), d_lbs, st), "transpose");
     int* d_oidx = ctx.alloc<int>(total);
     float* d_odist = ctx.alloc<float>(total);
     kgb::DissimArgs a{};
@@ -2649,6 +2650,7 @@ int kgb_dissimilarity_inplace(int32_t* gidx, float* gdist, int32_t samples, int3
     a.idx = d_idx;
     a.dist = d_dist;
     a.lbs = d_lbs;
+    a.stride = kgb::label_stride(runs);
     a.out_idx = d_oidx;
     a.out_dist = d_odist;
     ck_launch(kgb::dissimilarity(a, st), "dissimilarity");

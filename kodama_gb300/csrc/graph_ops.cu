@@ -23,6 +23,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 namespace kgb {
 
 namespace {
@@ -301,29 +303,58 @@ __global__ void fnv_rows_kernel(const int* __restrict__ data, int rows, int n, u
 }
 
 // 32 x 32 tiles; a CTA walks the run tiles blockIdx.y, blockIdx.y + gridDim.y,
-// ... so any number of runs fits the grid's y limit.
-__global__ void transpose_kernel(const int* __restrict__ res, int runs, int n, int* __restrict__ out) {
+// ... so any number of runs fits the grid's y limit.  Sample rows of `out` are
+// `stride` ints apart; the padding past the runs is written as label 0 (no
+// label), so that dissimilarity_kernel can load whole 16-byte vectors.
+// idx != nullptr: the CTAs past the last sample tile check a one-based graph
+// instead, flagging any stored index outside {negative (missing)} U [1, n].
+__global__ void transpose_kernel(const int* __restrict__ res, int runs, int n, int stride, int* __restrict__ out,
+                                 const int* __restrict__ idx, size_t total, int* bad) {
   __shared__ int tile[32][33];
+  const int sample_tiles = (n + 31) / 32;
+  if (static_cast<int>(blockIdx.x) >= sample_tiles) {
+    const size_t step = static_cast<size_t>(gridDim.x - sample_tiles) * gridDim.y * 256;
+    size_t e = (static_cast<size_t>(blockIdx.x - sample_tiles) * gridDim.y + blockIdx.y) * 256 + threadIdx.y * 32 +
+               threadIdx.x;
+    for (; e < total; e += step) {
+      const int v = idx[e];
+      if (v >= 0 && (v < 1 || v > n)) atomicExch(bad, 1);
+    }
+    return;
+  }
   const int s0 = blockIdx.x * 32;
-  const int run_tiles = (runs + 31) / 32;
+  const int run_tiles = (stride + 31) / 32;
   for (int rt = blockIdx.y; rt < run_tiles; rt += gridDim.y) {
     const int r0 = rt * 32;
     for (int k = threadIdx.y; k < 32; k += blockDim.y) {
       const int r = r0 + k, s = s0 + threadIdx.x;
-      if (r < runs && s < n) tile[k][threadIdx.x] = res[static_cast<size_t>(r) * n + s];
+      tile[k][threadIdx.x] = r < runs && s < n ? res[static_cast<size_t>(r) * n + s] : 0;
     }
     __syncthreads();
     for (int k = threadIdx.y; k < 32; k += blockDim.y) {
       const int s = s0 + k, r = r0 + threadIdx.x;
-      if (r < runs && s < n) out[static_cast<size_t>(s) * runs + r] = tile[threadIdx.x][k];
+      if (r < stride && s < n) out[static_cast<size_t>(s) * stride + r] = tile[threadIdx.x][k];
     }
     __syncthreads();
   }
 }
 
-// One warp per row; lanes cooperate over runs for each neighbour, then a
-// rank sort of the row in shared memory.
-__global__ void dissimilarity_kernel(DissimArgs a) {
+// Co-label proximity of one graph row per warp, then a rank sort of the row in
+// shared memory.  Eight lanes share a neighbour (four neighbours per step, two
+// steps in flight) and read its labels and the row's own as vectors of VEC
+// ints.  The counts of 32 neighbours end up one per lane, so the two double
+// divisions of each neighbour run on all lanes: double division is a long
+// serial sequence here, and one lane forming it for each neighbour in turn was
+// most of the earlier kernel's time (20000 rows x 30 neighbours x 100 runs,
+// whole in-place call: 879 us; with this split 129 us).  What remains is the
+// gather of the neighbours' labels from L2 (rows x neighbours x runs x 4
+// bytes).
+// A warp reads its whole row before it writes any of it and no other warp
+// touches that row, so the outputs may be the inputs.  Nothing is written when
+// a.bad is set (an index check in front of the kernel failed).
+template <int VEC>
+__global__ void __launch_bounds__(256) dissimilarity_kernel(DissimArgs a) {
+  using Vec = typename std::conditional<VEC == 4, int4, int>::type;
   extern __shared__ unsigned char dsm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wpb = blockDim.x >> 5;
@@ -331,39 +362,81 @@ __global__ void dissimilarity_kernel(DissimArgs a) {
   int* ki = reinterpret_cast<int*>(reinterpret_cast<float*>(dsm) + static_cast<size_t>(wpb) * a.K) +
             static_cast<size_t>(warp) * a.K;
   const int i = blockIdx.x * wpb + warp;
-  if (i >= a.n) return;
-  const int* li = a.lbs + static_cast<size_t>(i) * a.runs;
-  for (int j = 0; j < a.K; ++j) {
+  if (i >= a.n || (a.bad != nullptr && *a.bad != 0)) return;
+  const int sub = lane & 7, grp = lane >> 3;
+  const int nvec = a.stride / VEC;
+  const Vec* lbs = reinterpret_cast<const Vec*>(a.lbs);
+  const Vec* li = lbs + static_cast<size_t>(i) * nvec;
+  for (int j0 = 0; j0 < a.K; j0 += 32) {
+    const int j = j0 + lane;
     const size_t off = static_cast<size_t>(i) * a.K + j;
-    const int stored = a.idx[off];
+    const int stored = j < a.K ? a.idx[off] : -1;
+    float d = j < a.K ? a.dist[off] : INFINITY;
     const int nb = (stored >= 0 && a.in_one_based) ? stored - 1 : stored;
-    float d = a.dist[off];
-    if (nb < 0 || nb >= a.n || !isfinite(d)) {
-      if (lane == 0) {
-        kd[j] = INFINITY;
-        ki[j] = stored;
+    const bool live = nb >= 0 && nb < a.n && isfinite(d);
+    int my_same = 0, my_valid = 0;
+    for (int s = 0; s < 8 && j0 + 4 * s < a.K; s += 2) {
+      int same[2] = {0, 0}, valid[2] = {0, 0};
+      const Vec* lj[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int q = __shfl_sync(kFull, live ? nb : -1, (4 * (s + u) + grp) & 31);
+        lj[u] = q >= 0 ? lbs + static_cast<size_t>(q) * nvec : nullptr;
       }
-      continue;
+#pragma unroll 2
+      for (int v = sub; v < nvec; v += 8) {
+        const Vec x = li[v];
+        Vec y[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          if (lj[u] != nullptr) y[u] = lj[u][v];
+          else y[u] = Vec{};
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          if constexpr (VEC == 4) {
+            const int px = (x.x != 0) & (y[u].x != 0), py = (x.y != 0) & (y[u].y != 0),
+                      pz = (x.z != 0) & (y[u].z != 0), pw = (x.w != 0) & (y[u].w != 0);
+            valid[u] += px + py + pz + pw;
+            same[u] += (px & (x.x == y[u].x)) + (py & (x.y == y[u].y)) + (pz & (x.z == y[u].z)) +
+                       (pw & (x.w == y[u].w));
+          } else {
+            const int p = (x != 0) & (y[u] != 0);
+            valid[u] += p;
+            same[u] += p & (x == y[u]);
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+          same[u] += __shfl_xor_sync(kFull, same[u], o);
+          valid[u] += __shfl_xor_sync(kFull, valid[u], o);
+        }
+        // group g holds the counts of neighbour 4 (s + u) + g of this batch
+        const int gs = __shfl_sync(kFull, same[u], (lane & 3) * 8), gv = __shfl_sync(kFull, valid[u], (lane & 3) * 8);
+        if ((lane >> 2) == s + u) {
+          my_same = gs;
+          my_valid = gv;
+        }
+      }
     }
-    const int* lj = a.lbs + static_cast<size_t>(nb) * a.runs;
-    int same = 0, valid = 0;
-    for (int r = lane; r < a.runs; r += 32) {
-      const int x = li[r], y = lj[r];
-      const int pv = (x != 0) & (y != 0);
-      valid += pv;
-      same += pv & (x == y);
-    }
-    same = __reduce_add_sync(kFull, same);
-    valid = __reduce_add_sync(kFull, valid);
-    if (lane == 0) {
-      if (same == 0 || valid == 0) {
+    if (j < a.K) {
+      int id = stored;
+      if (!live) {
         d = INFINITY;
       } else {
-        const double agr = __ddiv_rn(static_cast<double>(same), static_cast<double>(valid));
-        d = static_cast<float>(__ddiv_rn(__dadd_rn(1.0, static_cast<double>(d)), __dmul_rn(agr, agr)));
+        id = a.out_one_based ? nb + 1 : nb;
+        if (my_same == 0 || my_valid == 0) {
+          d = INFINITY;
+        } else {
+          const double agr = __ddiv_rn(static_cast<double>(my_same), static_cast<double>(my_valid));
+          d = static_cast<float>(__ddiv_rn(__dadd_rn(1.0, static_cast<double>(d)), __dmul_rn(agr, agr)));
+        }
       }
       kd[j] = d;
-      ki[j] = a.out_one_based ? nb + 1 : nb;
+      ki[j] = id;
     }
   }
   __syncwarp();
@@ -458,26 +531,41 @@ int fnv_rows(const int* data, int rows, int n, uint64_t* out, cudaStream_t st) {
   return static_cast<int>(cudaGetLastError());
 }
 
-int transpose_runs(const int* res, int runs, int n, int* out, cudaStream_t st) {
-  const int run_tiles = (runs + 31) / 32;
+int transpose_runs(const int* res, int runs, int n, int stride, int* out, cudaStream_t st, const int* idx,
+                   size_t total, int* bad) {
+  const int run_tiles = (stride + 31) / 32, sample_tiles = (n + 31) / 32;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((n + 31) / 32, run_tiles < 65535 ? run_tiles : 65535);
+  cfg.gridDim = dim3(sample_tiles, run_tiles < 65535 ? run_tiles : 65535);
+  if (idx != nullptr) {
+    // about 1024 CTAs' worth of index checks at most
+    const size_t want = (total + 255) / 256;
+    cfg.gridDim.x += static_cast<unsigned>(((want < 1024 ? want : 1024) + cfg.gridDim.y - 1) / cfg.gridDim.y);
+  }
   cfg.blockDim = dim3(32, 8);
   cfg.stream = st;
   // the launch's own status (not an error left over from earlier work)
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, transpose_kernel, res, runs, n, out);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, transpose_kernel, res, runs, n, stride, out, idx, total, bad);
   count_launch();
   return static_cast<int>(e);
 }
 
 int dissimilarity(const DissimArgs& a, cudaStream_t st) {
   const int wpb = 8;
-  const size_t smem = static_cast<size_t>(wpb) * a.K * (sizeof(float) + sizeof(int));
-  if (smem > 48 * 1024) cudaFuncSetAttribute(dissimilarity_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            static_cast<int>(smem));
-  dissimilarity_kernel<<<(a.n + wpb - 1) / wpb, wpb * 32, smem, st>>>(a);
+  // rows of whole 16-byte vectors, or any row length
+  const auto kernel = a.stride % 4 == 0 ? dissimilarity_kernel<4> : dissimilarity_kernel<1>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>((a.n + wpb - 1) / wpb));
+  cfg.blockDim = dim3(wpb * 32);
+  cfg.dynamicSmemBytes = static_cast<size_t>(wpb) * a.K * (sizeof(float) + sizeof(int));
+  cfg.stream = st;
+  if (cfg.dynamicSmemBytes > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(cfg.dynamicSmemBytes));
+    if (e != cudaSuccess) return static_cast<int>(e);
+  }
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a);
   count_launch();
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(e);
 }
 
 }  // namespace kgb

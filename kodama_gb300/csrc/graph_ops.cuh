@@ -50,9 +50,11 @@ struct DissimArgs {
   int in_one_based, out_one_based;
   const int* idx;         // n x K
   const float* dist;      // n x K
-  const int* lbs;         // n x runs labels (transposed result matrix)
-  int* out_idx;
-  float* out_dist;
+  const int* lbs;         // n x stride labels (transposed result matrix, padding 0), 16-byte aligned
+  int stride;             // >= runs; a multiple of 4 lets the kernel load 16-byte vectors
+  int* out_idx;           // may be idx
+  float* out_dist;        // may be dist
+  const int* bad;         // nullptr, or a device flag: non-zero = write nothing
 };
 
 int graph_minmax(const int* idx, size_t total, int* mm, cudaStream_t st);
@@ -66,7 +68,12 @@ int build_reverse_tables(const ReverseArgs& a, cudaStream_t st);
 int project_labels(const ProjectArgs& a, cudaStream_t st);
 int code_labels(const CodingArgs& a, cudaStream_t st);
 int fnv_rows(const int* data, int rows, int n, uint64_t* out, cudaStream_t st);
-int transpose_runs(const int* res, int runs, int n, int* out, cudaStream_t st);
+// res (runs x n) -> out (n x stride, zero padding); with idx also checks the
+// `total` one-based indices of a graph and sets *bad (cleared by the caller)
+int transpose_runs(const int* res, int runs, int n, int stride, int* out, cudaStream_t st, const int* idx = nullptr,
+                   size_t total = 0, int* bad = nullptr);
+// label row stride of `runs` runs: whole 16-byte vectors
+inline int label_stride(int runs) { return (runs + 3) / 4 * 4; }
 int dissimilarity(const DissimArgs& a, cudaStream_t st);
 
 }  // namespace kgb

@@ -14,8 +14,10 @@
 // Scratch layout (kScratchBytes = 16 MiB, 256-byte aligned):
 //   [0, 256)           header; int at offset 0 = "bad graph index seen" flag,
 //                      cleared at the start of every call
-//   [256, 16 MiB)      labels transposed to samples x runs (int32), which
-//                      bounds samples * runs to kMaxLabelCells.
+//   [256, 16 MiB)      labels transposed to samples x stride (int32), which
+//                      bounds samples * runs to kMaxLabelCells.  The stride is
+//                      the runs rounded up to whole 16-byte vectors where that
+//                      fits, else the runs themselves.
 //
 // The scratch is shared by every call on a device.  Two calls that overlap
 // in time on one device (two host threads, or work still queued on another
@@ -41,89 +43,9 @@ constexpr size_t kScratchBytes = size_t(16) << 20;
 constexpr size_t kHeaderBytes = 256;
 constexpr size_t kMaxLabelCells = (kScratchBytes - kHeaderBytes) / sizeof(int);
 constexpr int kMaxNeighbors = 2048;  // 8 warps x K x 8 bytes of shared memory <= 128 KB
-constexpr unsigned kFullMask = 0xffffffffu;
 
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
-
-// Flags any stored index outside {negative (missing)} U [1, n].
-__global__ void check_one_based_kernel(const int* __restrict__ idx, size_t total, int n, int* bad) {
-  for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const int v = idx[e];
-    if (v >= 0 && (v < 1 || v > n)) atomicExch(bad, 1);
-  }
-}
-
-// One warp per graph row.  The warp reads its whole row (neighbour id and
-// distance) before any lane writes, and no other warp touches that row, so
-// the sorted row can be written back over the input.  Nothing is written
-// when the check kernel flagged a bad index, so a rejected call leaves the
-// graph as it was.  Arithmetic and ordering are those of the out-of-place
-// kernel: d' = (1 + d) / agr^2 in double with agr = same / valid over runs
-// where both labels are non-zero, +inf when nothing agrees, then a stable
-// sort by (d', id).
-__global__ void dissimilarity_inplace_kernel(int* __restrict__ idx, float* __restrict__ dist, int n, int K, int runs,
-                                             const int* __restrict__ lbs, const int* __restrict__ bad) {
-  if (*bad != 0) return;
-  extern __shared__ unsigned char dsm[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wpb = blockDim.x >> 5;
-  float* kd = reinterpret_cast<float*>(dsm) + static_cast<size_t>(warp) * K;
-  int* ki = reinterpret_cast<int*>(reinterpret_cast<float*>(dsm) + static_cast<size_t>(wpb) * K) +
-            static_cast<size_t>(warp) * K;
-  const int i = blockIdx.x * wpb + warp;
-  if (i >= n) return;
-  const int* li = lbs + static_cast<size_t>(i) * runs;
-  for (int j = 0; j < K; ++j) {
-    const size_t off = static_cast<size_t>(i) * K + j;
-    const int stored = idx[off];
-    const int nb = stored >= 0 ? stored - 1 : stored;
-    float d = dist[off];
-    if (nb < 0 || nb >= n || !isfinite(d)) {
-      if (lane == 0) {
-        kd[j] = INFINITY;
-        ki[j] = stored;
-      }
-      continue;
-    }
-    const int* lj = lbs + static_cast<size_t>(nb) * runs;
-    int same = 0, valid = 0;
-    for (int r = lane; r < runs; r += 32) {
-      const int x = li[r], y = lj[r];
-      const int pv = (x != 0) & (y != 0);
-      valid += pv;
-      same += pv & (x == y);
-    }
-    same = __reduce_add_sync(kFullMask, same);
-    valid = __reduce_add_sync(kFullMask, valid);
-    if (lane == 0) {
-      if (same == 0 || valid == 0) {
-        d = INFINITY;
-      } else {
-        const double agr = __ddiv_rn(static_cast<double>(same), static_cast<double>(valid));
-        d = static_cast<float>(__ddiv_rn(__dadd_rn(1.0, static_cast<double>(d)), __dmul_rn(agr, agr)));
-      }
-      kd[j] = d;
-      ki[j] = nb + 1;
-    }
-  }
-  __syncwarp();
-  for (int j = lane; j < K; j += 32) {
-    const float dj = kd[j];
-    const int ij = ki[j];
-    int rank = 0;
-    for (int q = 0; q < K; ++q) {
-      const float dq = kd[q];
-      const int iq = ki[q];
-      const bool less = dq < dj || (!(dj < dq) && iq < ij);
-      const bool equal_before = !(dq < dj) && !(dj < dq) && iq == ij && q < j;
-      rank += less || equal_before;
-    }
-    idx[static_cast<size_t>(i) * K + rank] = ij;
-    dist[static_cast<size_t>(i) * K + rank] = dj;
-  }
-}
 
 struct Fail {
   int code;
@@ -186,33 +108,26 @@ void run(int32_t* gidx, float* gdist, int32_t samples, int32_t gk, const int32_t
   const size_t total = static_cast<size_t>(samples) * gk;
 
   ck(cudaMemsetAsync(scratch, 0, kHeaderBytes, st), "clear scratch header");
-  const size_t want = (total + 255) / 256;
-  // each launch through cudaLaunchKernelEx, so its own status is checked and
-  // an error left on the thread by earlier, unrelated work is left alone
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(want < 1024 ? want : 1024));
-  cfg.blockDim = dim3(256);
-  cfg.stream = st;
-  ck(cudaLaunchKernelEx(&cfg, check_one_based_kernel, static_cast<const int*>(gidx), total, static_cast<int>(samples),
-                        bad),
-     "check indices");
-  kgb::count_launch();
-  ck(static_cast<cudaError_t>(kgb::transpose_runs(res, runs, samples, lbs, st)), "transpose");
-  const int wpb = 8;
-  const size_t smem = static_cast<size_t>(wpb) * gk * (sizeof(float) + sizeof(int));
-  if (smem > 48 * 1024) {
-    ck(cudaFuncSetAttribute(dissimilarity_inplace_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            static_cast<int>(smem)),
-       "shared memory size");
-  }
-  cfg.gridDim = dim3(static_cast<unsigned>((samples + wpb - 1) / wpb));
-  cfg.blockDim = dim3(wpb * 32);
-  cfg.dynamicSmemBytes = smem;
-  ck(cudaLaunchKernelEx(&cfg, dissimilarity_inplace_kernel, static_cast<int*>(gidx), static_cast<float*>(gdist),
-                        static_cast<int>(samples), static_cast<int>(gk), static_cast<int>(runs),
-                        static_cast<const int*>(lbs), static_cast<const int*>(bad)),
-     "dissimilarity");
-  kgb::count_launch();
+  const int padded = kgb::label_stride(runs);
+  const int stride = static_cast<size_t>(samples) * padded <= kMaxLabelCells ? padded : runs;
+  // both launches report their own status, so an error left on the thread by
+  // earlier, unrelated work is left alone
+  ck(static_cast<cudaError_t>(kgb::transpose_runs(res, runs, samples, stride, lbs, st, gidx, total, bad)),
+     "transpose and check indices");
+  kgb::DissimArgs a{};
+  a.n = samples;
+  a.K = gk;
+  a.runs = runs;
+  a.in_one_based = 1;
+  a.out_one_based = 1;
+  a.idx = gidx;
+  a.dist = gdist;
+  a.lbs = lbs;
+  a.stride = stride;
+  a.out_idx = gidx;
+  a.out_dist = gdist;
+  a.bad = bad;
+  ck(static_cast<cudaError_t>(kgb::dissimilarity(a, st)), "dissimilarity");
   int h_bad = 0;
   ck(cudaMemcpyAsync(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, st), "read index check");
   ck(cudaStreamSynchronize(st), "synchronize");
