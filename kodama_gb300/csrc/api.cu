@@ -1741,37 +1741,35 @@ void matrix_finalize(Ctx* ctx, MatrixTail& t, kgb_matrix_result* out, Clock& clk
 void exact_graph(Ctx& ctx, const float* d_x, int n, int d, int K, int method, int metric, int* d_idx, float* d_dist,
                  int* fallback_rows) {
   const int segments = 4;
-  if (metric != KGB_METRIC_EUCLIDEAN) {
-    if (method == KGB_KNN_TENSOR) fail(KGB_EINVAL, "the tensor-core kNN search is for the Euclidean metric");
-    const float* xs = d_x;
-    if (metric == KGB_METRIC_COSINE) {
-      float* xn = ctx.alloc<float>(static_cast<size_t>(n) * d);
-      ck_launch(kgb::normalize_rows(d_x, n, d, 2, xn, ctx.stream()), "cosine rows");
-      xs = xn;
-    }
-    void* scratch = ctx.alloc<unsigned char>(kgb::knn_bruteforce_scratch(n, K, segments));
-    ck_launch(kgb::knn_bruteforce_inner(xs, n, d, K, metric, segments, scratch, d_idx, d_dist, ctx.stream()),
-              "kNN graph");
-    if (fallback_rows != nullptr) *fallback_rows = n;
-    return;
+  if (method == KGB_KNN_TENSOR && metric != KGB_METRIC_EUCLIDEAN)
+    fail(KGB_EINVAL, "the tensor-core kNN search is for the Euclidean metric");
+  if (method == KGB_KNN_TENSOR && !kgb::knn_tc_explicit(n, d, K))
+    fail(KGB_EINVAL, "the tensor-core kNN search needs d <= 256, K <= 96 and n > 2 * (K + 16) + 64");
+  const float* xs = d_x;
+  if (metric == KGB_METRIC_COSINE) {
+    float* xn = ctx.alloc<float>(static_cast<size_t>(n) * d);
+    ck_launch(kgb::normalize_rows(d_x, n, d, 2, xn, ctx.stream()), "cosine rows");
+    xs = xn;
   }
   const bool tc = method == KGB_KNN_TENSOR || (method == KGB_KNN_AUTO && kgb::knn_tc_supported(n, d, K));
-  if (method == KGB_KNN_TENSOR && !kgb::knn_tc_supported(n, d, K))
-    fail(KGB_EINVAL, "the tensor-core kNN search needs d <= 256, K <= 96 and n > 2 * (K + 16) + 64");
   if (tc) {
-    void* scratch = ctx.alloc<unsigned char>(kgb::knn_tc_scratch(n, d, K, segments));
-    ck_launch(kgb::knn_tc_graph(d_x, n, d, K, segments, scratch, d_idx, d_dist, ctx.stream()), "kNN graph");
+    void* scratch = ctx.alloc<unsigned char>(kgb::knn_tc_scratch(n, d, K, segments, ctx.sms()));
+    ck_launch(kgb::knn_tc_graph(xs, n, d, K, metric, segments, ctx.sms(), scratch, d_idx, d_dist, ctx.stream()),
+              "kNN graph");
     if (fallback_rows != nullptr) {
       int count = 0;
-      ck_launch(kgb::knn_tc_fallback_count(scratch, n, d, K, segments, &count, ctx.stream()), "kNN graph");
+      ck_launch(kgb::knn_tc_fallback_count(scratch, n, d, K, segments, ctx.sms(), &count, ctx.stream()), "kNN graph");
       ctx.sync();
       *fallback_rows = count;
     }
-  } else {
-    void* scratch = ctx.alloc<unsigned char>(kgb::knn_bruteforce_scratch(n, K, segments));
-    ck_launch(kgb::knn_bruteforce(d_x, n, d, K, segments, scratch, d_idx, d_dist, ctx.stream()), "kNN graph");
-    if (fallback_rows != nullptr) *fallback_rows = n;
+    return;
   }
+  void* scratch = ctx.alloc<unsigned char>(kgb::knn_bruteforce_scratch(n, K, segments));
+  ck_launch(metric == KGB_METRIC_EUCLIDEAN
+                ? kgb::knn_bruteforce(xs, n, d, K, segments, scratch, d_idx, d_dist, ctx.stream())
+                : kgb::knn_bruteforce_inner(xs, n, d, K, metric, segments, scratch, d_idx, d_dist, ctx.stream()),
+            "kNN graph");
+  if (fallback_rows != nullptr) *fallback_rows = n;
 }
 
 // The exact graph a KODAMA.matrix call works on: under the cosine and
@@ -2385,6 +2383,28 @@ void check_training_rows(const std::vector<int>& folds) {
   for (int f : folds) size[f]++;
   for (const auto& kv : size)
     if (kv.second == static_cast<int>(folds.size())) fail(KGB_EINTERNAL, "KNN fold has no training samples.");
+}
+
+// The fold-wise exact search of KNNCV and CoreKNN into idx / dist (n x K): the
+// tensor-core candidate search where it applies, else the brute force.
+void fold_search(Ctx& ctx, const float* xs, int n, int d, int K, int metric, const std::vector<int>& folds,
+                 const int* d_folds, int* d_idx, float* d_dist) {
+  const int segments = 4;
+  const bool inner = metric != KGB_METRIC_EUCLIDEAN;
+  if (kgb::knn_tc_supported(n, d, K)) {
+    const kgb::KnnFoldPlan fp = kgb::knn_fold_plan(folds);
+    const int* d_perm = ctx.upload(fp.perm.data(), fp.perm.size());
+    const int* d_off = ctx.upload(fp.off.data(), fp.off.size());
+    const int* d_skip = ctx.upload(fp.skip.data(), fp.skip.size());
+    void* scratch = ctx.alloc<unsigned char>(kgb::knn_tc_scratch(n, d, K, segments, ctx.sms(), &fp));
+    ck_launch(kgb::knn_tc_fold_search(xs, n, d, K, inner, d_folds, fp, d_perm, d_off, d_skip, segments, ctx.sms(),
+                                      scratch, d_idx, d_dist, ctx.stream()),
+              "fold-wise kNN");
+    return;
+  }
+  void* scratch = ctx.alloc<unsigned char>(kgb::knn_bruteforce_scratch(n, K, segments));
+  ck_launch(kgb::knn_fold_search(xs, n, d, K, inner, d_folds, segments, scratch, d_idx, d_dist, ctx.stream()),
+            "fold-wise kNN");
 }
 
 // The search matrix of a metric on the device: cosine rows normalised
@@ -3063,11 +3083,7 @@ int kgb_knncv(const float* x, int32_t n, int32_t d, const int32_t* labels, const
     const int* d_folds = ctx.upload(folds.data(), folds.size());
     int* d_idx = ctx.alloc<int>(static_cast<size_t>(n) * K);
     float* d_dist = ctx.alloc<float>(static_cast<size_t>(n) * K);
-    const int segments = 4;
-    void* scratch = ctx.alloc<unsigned char>(kgb::knn_bruteforce_scratch(n, K, segments));
-    ck_launch(kgb::knn_fold_search(xs, n, d, K, opt->metric != KGB_METRIC_EUCLIDEAN, d_folds, segments, scratch,
-                                   d_idx, d_dist, st),
-              "fold-wise kNN");
+    fold_search(ctx, xs, n, d, K, opt->metric, folds, d_folds, d_idx, d_dist);
     int* d_pred = ctx.alloc<int>(static_cast<size_t>(n));
     ck_launch(kgb::knn_vote(d_idx, d_dist, n, K, ctx.upload(labels, static_cast<size_t>(n)), d_pred, st), "vote");
     ctx.download(predicted, d_pred, static_cast<size_t>(n));
@@ -3103,11 +3119,7 @@ int kgb_core_knn(const float* x, int32_t n, int32_t d, int32_t metric, const int
                    const int* d_folds = ctx.upload(folds[0].data(), folds[0].size());
                    int* d_idx = ctx.alloc<int>(static_cast<size_t>(n) * w);
                    float* d_dist = ctx.alloc<float>(static_cast<size_t>(n) * w);
-                   const int segments = 4;
-                   void* scratch = ctx.alloc<unsigned char>(kgb::knn_bruteforce_scratch(n, w, segments));
-                   ck_launch(kgb::knn_fold_search(xs, n, d, w, metric != KGB_METRIC_EUCLIDEAN, d_folds, segments,
-                                                  scratch, d_idx, d_dist, st),
-                             "fold-wise kNN");
+                   fold_search(ctx, xs, n, d, w, metric, folds[0], d_folds, d_idx, d_dist);
                    ck_launch(kgb::knn_fold_tables(d_idx, d_dist, n, w, w, d_nb, d_sc, st), "vote tables");
                  });
   });

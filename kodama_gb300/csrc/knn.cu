@@ -197,18 +197,6 @@ __global__ void __launch_bounds__(kQ) knn_segment_generic_kernel(const float* __
   }
 }
 
-// Reported distance of an internal one (native_knn_output_distance,
-// native_knn.cpp:1157-1164): sqrt for Euclidean, max(0, 1 + v) for cosine,
-// 1 + v for inner product; kOutRaw keeps the internal value.
-enum OutMode { kOutSqrt = 0, kOutRaw = 1, kOutCosine = 2, kOutInner = 3 };
-
-__device__ __forceinline__ float output_distance(float v, int mode) {
-  if (mode == kOutSqrt) return __fsqrt_rn(v);
-  if (mode == kOutRaw) return v;
-  const float o = __fadd_rn(1.0f, v);
-  return mode == kOutCosine ? ((0.0f < o) ? o : 0.0f) : o;
-}
-
 __global__ void knn_merge_kernel(int n, int K, int segs, const float* __restrict__ pd, const int* __restrict__ pi,
                                  const int* __restrict__ qrows, const int* __restrict__ nq, int mode,
                                  int* __restrict__ idx, float* __restrict__ dist) {
@@ -241,7 +229,7 @@ __global__ void knn_merge_kernel(int n, int K, int segs, const float* __restrict
     }
     ++head[bs];
     idx[out] = biv;
-    dist[out] = output_distance(bdv, mode);
+    dist[out] = knn_output_distance(bdv, mode);
   }
 }
 
@@ -369,20 +357,22 @@ int knn_bruteforce(const float* x, int n, int d, int K, int segments, void* scra
   int* pi = reinterpret_cast<int*>(pd + static_cast<size_t>(segments) * n * K);
   const int e = launch_segments<false, false>(x, n, d, K, segments, nullptr, nullptr, nullptr, pd, pi, st);
   if (e != 0) return e;
-  knn_merge_kernel<<<(n + 127) / 128, 128, 0, st>>>(n, K, segments, pd, pi, nullptr, nullptr, kOutSqrt, idx, dist);
+  knn_merge_kernel<<<(n + 127) / 128, 128, 0, st>>>(n, K, segments, pd, pi, nullptr, nullptr, kKnnOutSqrt, idx, dist);
   count_launch();
   return static_cast<int>(cudaGetLastError());
 }
 
-int knn_bruteforce_rows(const float* x, int n, int d, int K, int segments, const int* rows, const int* nrows,
-                        void* scratch, int* idx, float* dist, cudaStream_t st) {
+int knn_bruteforce_rows(const float* x, int n, int d, int K, bool inner, const int* folds, int mode, int segments,
+                        const int* rows, const int* nrows, void* scratch, int* idx, float* dist, cudaStream_t st) {
   if (segments < 1) segments = 1;
   if (segments > kMaxSegments) segments = kMaxSegments;
   float* pd = static_cast<float*>(scratch);
   int* pi = reinterpret_cast<int*>(pd + static_cast<size_t>(segments) * n * K);
-  const int e = launch_segments<false, false>(x, n, d, K, segments, nullptr, rows, nrows, pd, pi, st);
+  const auto run = folds != nullptr ? (inner ? launch_segments<true, true> : launch_segments<false, true>)
+                                    : (inner ? launch_segments<true, false> : launch_segments<false, false>);
+  const int e = run(x, n, d, K, segments, folds, rows, nrows, pd, pi, st);
   if (e != 0) return e;
-  knn_merge_kernel<<<(n + 127) / 128, 128, 0, st>>>(n, K, segments, pd, pi, rows, nrows, kOutSqrt, idx, dist);
+  knn_merge_kernel<<<(n + 127) / 128, 128, 0, st>>>(n, K, segments, pd, pi, rows, nrows, mode, idx, dist);
   count_launch();
   return static_cast<int>(cudaGetLastError());
 }
@@ -396,7 +386,7 @@ int knn_fold_search(const float* x, int n, int d, int K, bool inner, const int* 
   const int e = inner ? launch_segments<true, true>(x, n, d, K, segments, folds, nullptr, nullptr, pd, pi, st)
                       : launch_segments<false, true>(x, n, d, K, segments, folds, nullptr, nullptr, pd, pi, st);
   if (e != 0) return e;
-  knn_merge_kernel<<<(n + 127) / 128, 128, 0, st>>>(n, K, segments, pd, pi, nullptr, nullptr, kOutRaw, idx, dist);
+  knn_merge_kernel<<<(n + 127) / 128, 128, 0, st>>>(n, K, segments, pd, pi, nullptr, nullptr, kKnnOutRaw, idx, dist);
   count_launch();
   return static_cast<int>(cudaGetLastError());
 }
@@ -410,7 +400,7 @@ int knn_bruteforce_inner(const float* x, int n, int d, int K, int metric, int se
   const int e = launch_segments<true, false>(x, n, d, K, segments, nullptr, nullptr, nullptr, pd, pi, st);
   if (e != 0) return e;
   knn_merge_kernel<<<(n + 127) / 128, 128, 0, st>>>(n, K, segments, pd, pi, nullptr, nullptr,
-                                                   metric == 0 ? kOutCosine : kOutInner, idx, dist);
+                                                   metric == 0 ? kKnnOutCosine : kKnnOutInner, idx, dist);
   count_launch();
   return static_cast<int>(cudaGetLastError());
 }

@@ -5,6 +5,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <vector>
+
 namespace kgb {
 
 constexpr int kMaxSegments = 16;
@@ -13,21 +15,57 @@ size_t knn_bruteforce_scratch(int n, int K, int segments);
 int knn_bruteforce(const float* x, int n, int d, int K, int segments, void* scratch, int* idx, float* dist,
                    cudaStream_t st);
 
-// knn_bruteforce restricted to the *nrows rows listed in rows (read on the
-// device): their results are written, the other rows' left untouched.
-int knn_bruteforce_rows(const float* x, int n, int d, int K, int segments, const int* rows, const int* nrows,
-                        void* scratch, int* idx, float* dist, cudaStream_t st);
+// Reported distance of an internal one (native_knn_output_distance,
+// native_knn.cpp:1157-1164): sqrt for Euclidean, max(0, 1 + v) for cosine,
+// 1 + v for inner product; kKnnOutRaw keeps the internal value.
+enum KnnOut { kKnnOutSqrt = 0, kKnnOutRaw = 1, kKnnOutCosine = 2, kKnnOutInner = 3 };
 
-// The same exact graph as knn_bruteforce through a tensor-core candidate
-// search with an exact re-rank and a per-row certificate (knn_tc.cu); rows
-// whose certificate fails are recomputed by knn_bruteforce_rows.
+#ifdef __CUDACC__
+__device__ __forceinline__ float knn_output_distance(float v, int mode) {
+  if (mode == kKnnOutSqrt) return __fsqrt_rn(v);
+  if (mode == kKnnOutRaw) return v;
+  const float o = __fadd_rn(1.0f, v);
+  return mode == kKnnOutCosine ? ((0.0f < o) ? o : 0.0f) : o;
+}
+#endif
+
+// The brute force (any of the searches below: inner products, candidates of
+// other folds, out mode) restricted to the *nrows rows listed in rows (read on
+// the device): their results are written, the other rows' left untouched.
+int knn_bruteforce_rows(const float* x, int n, int d, int K, bool inner, const int* folds, int mode, int segments,
+                        const int* rows, const int* nrows, void* scratch, int* idx, float* dist, cudaStream_t st);
+
+// The same exact graph as knn_bruteforce (metric 2) or knn_bruteforce_inner
+// (metrics 0 and 1) through a tensor-core candidate search with an exact
+// re-rank and a per-row certificate (knn_tc.cu); rows whose certificate fails
+// are recomputed by knn_bruteforce_rows.  sms: the device's SM count.
 bool knn_tc_supported(int n, int d, int K);
-size_t knn_tc_scratch(int n, int d, int K, int segments);
-int knn_tc_graph(const float* x, int n, int d, int K, int segments, void* scratch, int* idx, float* dist,
-                 cudaStream_t st);
+// the sizes a caller may force the tensor search for (KGB_KNN_TENSOR)
+bool knn_tc_explicit(int n, int d, int K);
+struct KnnFoldPlan;
+size_t knn_tc_scratch(int n, int d, int K, int segments, int sms, const KnnFoldPlan* fp = nullptr);
+int knn_tc_graph(const float* x, int n, int d, int K, int metric, int segments, int sms, void* scratch, int* idx,
+                 float* dist, cudaStream_t st);
 // Rows of the last knn_tc_graph on this scratch that went to the fallback
 // (asynchronous copy into host memory).
-int knn_tc_fallback_count(const void* scratch, int n, int d, int K, int segments, int* out, cudaStream_t st);
+int knn_tc_fallback_count(const void* scratch, int n, int d, int K, int segments, int sms, int* out,
+                          cudaStream_t st);
+
+// Row order of the fold-wise tensor search: every fold's rows together, padded
+// to whole candidate tiles, so that a query tile leaves out its own fold's
+// tiles.  perm: row of every position (-1 = padding); per query tile the first
+// (query tile, candidate tile) pair and the (first, count) of the tiles left
+// out.
+struct KnnFoldPlan {
+  int tiles = 0, pairs = 0;
+  std::vector<int> perm, off, skip;
+};
+KnnFoldPlan knn_fold_plan(const std::vector<int>& folds);
+// knn_fold_search through the tensor-core candidate search; d_perm, d_off and
+// d_skip are the plan's arrays on the device.
+int knn_tc_fold_search(const float* x, int n, int d, int K, bool inner, const int* d_folds, const KnnFoldPlan& fp,
+                       const int* d_perm, const int* d_off, const int* d_skip, int segments, int sms, void* scratch,
+                       int* idx, float* dist, cudaStream_t st);
 
 // Rows of x (n x d) split into bfloat16 hi + lo parts (x = hi + lo + r,
 // |r| <= 2^-16 |x|), dp = d rounded up to 16, coordinates permuted inside

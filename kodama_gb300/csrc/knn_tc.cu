@@ -1,82 +1,736 @@
-// Exact kNN graph through a tensor-core candidate search (knn.cuh).
+// Exact nearest neighbours through a tensor-core candidate search (knn.cuh).
 //
-// The canonical result (knn.cu: squared L2 as a float32 chain over the
-// coordinates in order, each term separately rounded, ties by index) is
-// found in three steps:
+// The canonical result (knn.cu: a float32 chain over the coordinates in order,
+// each term separately rounded, ties by row) is found in three steps, for the
+// squared L2 distance or minus the inner product, over all other rows or over
+// the rows of other folds:
 //
-//  1. candidates: every row is split once into bfloat16 hi + lo parts
-//     (x = hi + lo + r, |r| <= 2^-16 |x|); a warp computes the approximate
-//     distances a = |q|^2 + |c|^2 - 2 (hi.hi + hi.lo + lo.hi) of 16 queries
-//     to a 64-row candidate tile with mma.sync (bf16 in, f32 accumulate).
-//     The candidate tiles are dealt to S segments (grid.y) in a scattered
-//     order; per segment every query keeps the kp smallest approximate
-//     distances of each half of its columns in two max-heaps, one per lane
-//     (lanes r and r + 16 own query row r).  The lanes holding the
-//     accumulator fragments flag the values below their heap's threshold and
-//     publish per-row masks; each owner lane inserts only its flagged
-//     values, so the 32 heaps of a warp fill side by side;
-//  2. re-rank: one warp per query takes A_K, the K-th smallest approximate
-//     distance over its heaps, computes the canonical distances of the
-//     candidates with a <= A_K + 2 delta, and keeps the K smallest by
-//     (distance, index);
-//  3. certificate: every row left out of the heaps has a >= B, the smallest
-//     final heap threshold.  A row of the true top K (ties by index
-//     included) has e <= e_K <= A_K + delta, hence a <= A_K + 2 delta, so
-//     B > A_K + 2 delta proves it was kept and re-ranked.  Rows whose
-//     certificate fails are listed and recomputed by the brute-force kernels
-//     (knn.cu).  delta bounds |a - e| for every row (below).
+//  1. prep: every row is split once into bfloat16 hi + lo parts
+//     (x = hi + lo + r, |r| <= 2^-18 |x|), stored in blocks of 256 rows as
+//     [chunk of 8 coordinates][row], the layout the tensor core reads, so that
+//     a tile is one contiguous copy;
+//  2. candidates: a persistent CTA per SM multiplies 128 queries with tiles of
+//     256 candidates (hi.hi + hi.lo + lo.hi, tcgen05.mma into TMEM).  A thread
+//     owns one query row of the accumulator, so it compares a = |c|^2 - 2 q.c
+//     (|q|^2 dropped; -q.c for inner products) with the row's threshold without
+//     talking to other lanes and appends the few values below it to the row's
+//     list.  When a list grows past its trigger the warp cuts it back: tau =
+//     A + 2 delta, A an upper bound of the K-th smallest value of the list;
+//  3. re-rank: one warp per query joins the row's lists, bounds the K-th
+//     smallest value A_K again, computes the canonical distances of the values
+//     within A_K + 2 delta and keeps the K smallest by (distance, row).
 //
-// Error bound (u = 2^-24): with D the true squared distance and e its
-// canonical value, |e - D| <= (d + 4) u D <= 2 (d + 4) u (|q|^2 + |c|^2);
-// the split drops hi.hi residuals of at most ~3.1 * 2^-16 sum|q_i c_i|, the
-// f32 accumulation of 3 dp products adds at most 3 dp 2^-22 sum|q_i c_i|
-// (tensor-core accumulation allowed two ulps per add), and
-// sum|q_i c_i| <= (|q|^2 + |c|^2) / 2; the f32 norms and the final
-// combination add (d + 8) u (|q|^2 + |c|^2).  So
-// delta <= (|q|^2 + max |c|^2) * (1e-4 + 2e-6 dp), a safe over-estimate.
+// Certificate.  A value is only ever dropped at a threshold >= A_K + 2 delta,
+// with delta >= |a - (e - |q|^2)| for every row that matters: the K smallest
+// a's rows have e - |q|^2 <= A_K + delta, so a row of the true top K does too,
+// and its a is at most A_K + 2 delta.  Rows whose lists overflow, hold too few
+// values, or lie outside the value range below go to the brute force.
+//
+// Error bound (u = 2^-24), N = |q|^2 + |c|^2: the split drops at most
+// 3.01 * 2^-18 sum|q_i c_i|; 3 dp accumulated products, allowed two ulps each,
+// add 3 dp 2^-22 sum|q_i c_i|; twice their sum is at most N times that for L2
+// (sum|q_i c_i| <= |q||c|), and |q||c| times that for inner products.  The
+// canonical chain adds 2 (d + 4) u N, the float norms and the last fma
+// (d + 4) u N.  delta = N crel, crel = 1.5e-5 + 1e-6 dp, covers the sum
+// (1.2e-5 + 7.2e-7 dp + 1.8e-7 (d + 4)).  The rows that matter lie within
+// R = sqrt(A + |q|^2 + 2 delta_max) of the query, so |c| <= |q| + R replaces
+// the largest norm of the data there; delta falls with A, so an earlier
+// threshold is never below a later one.  Norms outside [1e-20, 1e36] (or
+// non-finite values) send every row to the brute force; kDeltaFloor covers
+// products lost to underflow.
 #include "knn.cuh"
 #include "launch_count.cuh"
 
 #include "bf16_split.cuh"
+#include "tcgen05.cuh"
 
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
 
+#include <map>
+
 namespace kgb {
 
 namespace {
 
-constexpr int kTcWarps = 4;            // warps per CTA, 16 queries each
-constexpr int kTcQ = 16 * kTcWarps;    // queries per CTA
-constexpr int kTcN = 64;               // candidates per tile
-constexpr int kTcRegKs = 8;            // k-steps whose query fragments (hi and lo) sit in registers
-constexpr int kTcMaxKs = 16;           // dp <= 256: above kTcRegKs the lo fragments come from shared memory
-constexpr size_t kTcSmemLimit = 227 * 1024;
-constexpr int kTileStride = kTcN + 8;  // floats per row of a warp's distance tile
+constexpr unsigned kFull = 0xffffffffu;
+constexpr int kBlockRows = 256;   // rows of an operand block = candidates per tile (mma N)
+constexpr int kQRows = 128;       // queries per tile (mma M = TMEM lanes)
+constexpr int kMaxDp = 256;
+constexpr int kThreads = 320;     // 8 epilogue warps, the copy warp, the mma warp
+constexpr int kMaxStages = 4;
+constexpr size_t kSmemLimit = 227 * 1024;
+constexpr float kDeltaFloor = 2e-35f;
+constexpr int kSurvivors = 512;   // joined list entries of a query in the re-rank
 
-__global__ void tc_prep_kernel(const float* __restrict__ x, int n, int d, int dp, uint16_t* __restrict__ xh,
-                               uint16_t* __restrict__ xl, float* __restrict__ nrm, unsigned* __restrict__ nrm_max,
-                               int* __restrict__ nonfinite) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n) return;
+// status words: [0] largest norm (float bits), [1] non-finite value seen,
+// [2] fallback rows, [3] a wait of the candidate kernel ran out
+enum { kStNorm = 0, kStBad = 1, kStFallback = 2, kStTimeout = 3 };
+
+// Rows perm[pos] (pos itself without perm; -1 = padding) of x split into the
+// operand blocks.  A warp's lanes take 32 rows of one chunk, so the 16-byte
+// stores of a chunk are contiguous; the block's warps share the chunks.
+// cn: the additive term of a candidate (|c|^2, or 0 for inner products; +inf
+// for padding), qn: |q|^2 (-1 for padding).  xp != nullptr also gets the rows
+// as floats padded to d4 (a multiple of 4), for the re-rank's vector loads.
+__global__ void __launch_bounds__(256) prep_kernel(const float* __restrict__ x, int n, int d, int chunks, int npos,
+                                                   const int* __restrict__ perm, int inner,
+                                                   uint16_t* __restrict__ xh, uint16_t* __restrict__ xl,
+                                                   float* __restrict__ cn, float* __restrict__ qn,
+                                                   float* __restrict__ xp, int d4, unsigned* __restrict__ status) {
+  __shared__ float part[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int pos = blockIdx.x * 32 + lane;  // npos is a multiple of 256
+  const int row = perm != nullptr ? perm[pos] : (pos < n ? pos : -1);
+  const size_t base = static_cast<size_t>(pos / kBlockRows) * chunks * kBlockRows + pos % kBlockRows;
   float s = 0.0f;
   bool fin = true;
-  for (int k = 0; k < dp; ++k) {
-    const float v = k < d ? x[static_cast<size_t>(r) * d + k] : 0.0f;
-    fin = fin && isfinite(v);
-    const uint32_t hb = bf16_bits(v);
-    const float h = __uint_as_float(hb << 16);
-    const uint32_t lb = bf16_bits(__fsub_rn(v, h));
-    const size_t o = static_cast<size_t>(r) * dp + perm16(k);
-    xh[o] = static_cast<uint16_t>(hb);
-    xl[o] = static_cast<uint16_t>(lb);
-    s = __fadd_rn(s, __fmul_rn(v, v));
+  for (int c = warp; c < chunks; c += 8) {
+    float v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int k = c * 8 + e;
+      v[e] = row >= 0 && k < d ? x[static_cast<size_t>(row) * d + k] : 0.0f;
+      fin = fin && isfinite(v[e]);
+      s = __fadd_rn(s, __fmul_rn(v[e], v[e]));
+    }
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const uint32_t h0 = bf16_bits(v[2 * e]), h1 = bf16_bits(v[2 * e + 1]);
+      h[e] = h0 | (h1 << 16);
+      l[e] = bf16_bits(__fsub_rn(v[2 * e], __uint_as_float(h0 << 16))) |
+             (bf16_bits(__fsub_rn(v[2 * e + 1], __uint_as_float(h1 << 16))) << 16);
+    }
+    reinterpret_cast<uint4*>(xh)[base + static_cast<size_t>(c) * kBlockRows] = make_uint4(h[0], h[1], h[2], h[3]);
+    reinterpret_cast<uint4*>(xl)[base + static_cast<size_t>(c) * kBlockRows] = make_uint4(l[0], l[1], l[2], l[3]);
+    if (xp != nullptr && row >= 0) {
+      float4* o = reinterpret_cast<float4*>(xp + static_cast<size_t>(row) * d4);
+      if (c * 8 < d4) o[c * 2] = make_float4(v[0], v[1], v[2], v[3]);
+      if (c * 8 + 4 < d4) o[c * 2 + 1] = make_float4(v[4], v[5], v[6], v[7]);
+    }
   }
-  nrm[r] = s;
-  if (fin) atomicMax(nrm_max, __float_as_uint(s));
-  else atomicExch(nonfinite, 1);
+  part[warp][lane] = s;
+  if (__any_sync(kFull, !fin) && lane == 0) atomicExch(&status[kStBad], 1u);
+  __syncthreads();
+  if (warp == 0) {
+    float t = 0.0f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t = __fadd_rn(t, part[w][lane]);
+    cn[pos] = row < 0 ? INFINITY : (inner ? 0.0f : t);
+    qn[pos] = row < 0 ? -1.0f : t;
+    // finite sums only: an infinite one is caught by the range check
+    const unsigned m = __reduce_max_sync(kFull, row < 0 || !(t >= 0.0f) ? 0u : __float_as_uint(t));
+    if (lane == 0) atomicMax(&status[kStNorm], m);
+  }
 }
+
+// The tiles of a query tile, in the order they are visited.  All candidate
+// tiles but a contiguous range [skip, skip + skipn) (its own fold), starting
+// at the query's own block (without a skip) or after the range, in steps of a
+// stride coprime to their number: near rows are often near in memory, so the
+// thresholds fall at once, and no slow order of the data is followed.
+struct TileOrder {
+  int ntiles, skip, skipn, count, first, stride;
+  __device__ __forceinline__ TileOrder(int ntiles_, int own, int skip_, int skipn_)
+      : ntiles(ntiles_), skip(skip_), skipn(skipn_) {
+    count = ntiles - skipn;
+    first = skipn > 0 ? 0 : own;
+    stride = count > 0 ? 1000003 % count : 0;
+    if (stride == 0) stride = 1;
+  }
+  __device__ __forceinline__ int at(int k) const {
+    int t = static_cast<int>((first + static_cast<long long>(k) * stride) % count);
+    if (skipn > 0) {
+      t += skip + skipn;
+      if (t >= ntiles) t -= ntiles;
+    }
+    return t;
+  }
+};
+
+struct SearchArgs {
+  const uint16_t* xh;      // blocks of [chunk][256 rows][8]
+  const uint16_t* xl;
+  const float* cn;
+  const float* qn;
+  unsigned* status;
+  int chunks, kg, stages;  // 8-coordinate chunks of a row / per stage; stages
+  int ntiles, qtiles;
+  int Kq;                  // values a list has to keep: K, plus the query itself
+  int cap;                 // entries per list
+  float scale, crel;       // a = cn + scale * acc
+  int inner;
+  // stream-K split: the (query tile, candidate tile) pairs of all query tiles
+  // in a row, `per` of them per CTA.  off: first pair of every query tile
+  // (nullptr: q * ntiles), skip: the tile range a query tile leaves out
+  const int* off;
+  const int2* skip;
+  int pairs, per, segs;
+  float2* list;            // [query position][segment][group][cap] (a, position)
+  int* cnt;                // [query position][segment][group], -1 = overflow
+  float* tau;
+};
+
+__device__ __forceinline__ float delta_of(float A, float nq, float nmax, float crel, int inner) {
+  if (inner) return crel * sqrtf(nq) * sqrtf(nmax) * 1.00001f + kDeltaFloor;
+  const float dmax = crel * (nq + nmax) + kDeltaFloor;
+  const float r2 = fmaxf(0.0f, A + nq + 2.0f * dmax) * 1.0001f + 1e-6f * nq;
+  const float cm = fminf(sqrtf(nmax), sqrtf(nq) + sqrtf(r2)) * 1.00001f;
+  return fminf(dmax, crel * (nq + cm * cm) + kDeltaFloor);
+}
+
+// order-preserving image of a float as an unsigned
+__device__ __forceinline__ unsigned ord_float(float v) {
+  const unsigned u = __float_as_uint(v);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float from_ord(unsigned o) {
+  return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
+}
+
+// An upper bound of the Kq-th smallest of the warp's values (v[t] of lane l,
+// +inf = none; at least Kq of them finite): bisection between their extremes
+// until at most Kq + slack values lie below the bound.
+template <int P>
+__device__ __forceinline__ float kth_bound(const float (&v)[P], int Kq, int slack, int rounds) {
+  float lo = INFINITY, hi = -INFINITY;
+#pragma unroll
+  for (int t = 0; t < P; ++t) {
+    lo = fminf(lo, v[t]);
+    if (v[t] < INFINITY) hi = fmaxf(hi, v[t]);
+  }
+  lo = from_ord(__reduce_min_sync(kFull, ord_float(lo)));
+  hi = from_ord(__reduce_max_sync(kFull, ord_float(hi)));
+  for (int it = 0; it < rounds; ++it) {
+    const float mid = 0.5f * lo + 0.5f * hi;
+    if (!(mid > lo) || !(mid < hi)) break;
+    int c = 0;
+#pragma unroll
+    for (int t = 0; t < P; ++t) c += v[t] <= mid;
+    c = __reduce_add_sync(kFull, c);
+    if (c >= Kq) {
+      hi = mid;
+      if (c <= Kq + slack) break;
+    } else {
+      lo = mid;
+    }
+  }
+  return hi;
+}
+
+// Cuts the list of lane `src`'s row (m entries, P * 32 = cap) back to the
+// values below its new threshold; returns the entries left.
+template <int P>
+__device__ __forceinline__ int cut_list(float2* list, int m, int Kq, float nq, float nmax, float crel, int inner,
+                                        float* tau, int lane) {
+  float2 e[P];
+  float v[P];
+#pragma unroll
+  for (int t = 0; t < P; ++t) {
+    const int i = lane + 32 * t;
+    e[t] = i < m ? list[i] : make_float2(INFINITY, 0.0f);
+    v[t] = e[t].x;
+  }
+  const float A = kth_bound<P>(v, Kq, Kq >> 4, 14);
+  const float lim = fminf(*tau, A + 2.0f * delta_of(A, nq, nmax, crel, inner));
+  int left = 0;
+  __syncwarp();
+#pragma unroll
+  for (int t = 0; t < P; ++t) {
+    const bool keep = v[t] < lim;
+    const unsigned b = __ballot_sync(kFull, keep);
+    if (keep) list[left + __popc(b & ((1u << lane) - 1u))] = e[t];
+    left += __popc(b);
+  }
+  __syncwarp();
+  *tau = lim;
+  return left;
+}
+
+struct SearchShared {
+  uint64_t full[kMaxStages], empty[kMaxStages];
+  uint64_t afull[2], aempty[2], qfull, qempty;
+  uint32_t tmem;
+  int stop;
+  unsigned long long tau[2][kQRows];  // (query tile, threshold) of every row, per group
+};
+
+constexpr size_t kSharedRoom = 2304;  // static shared memory of candidates_kernel
+static_assert(sizeof(SearchShared) <= kSharedRoom, "static shared memory");
+
+// What bounds it: the epilogue's issue slots (about 4 per value) and the list
+// cuts; the tensor pipe needs 12 instructions of 128 cycles for a 128 x 256
+// tile of 64 padded coordinates.  N = 256 is the widest instruction; two
+// accumulators (all 512 TMEM columns) let one group of four warps work on a
+// tile while the tensor core fills the other.  Against the mma.sync kernel with
+// per-lane heaps that this replaces, and its brute-force fallback rows:
+// 100000 x 50, K = 30: 24.8 + 9.7 -> 7.1 ms; against the brute force, which
+// took K > 96, inner products and the fold-wise searches: 20011 x 50, K = 100
+// 62.9 -> 1.0 ms; 12000 x 100 cosine, K = 30 38.3 -> 0.35 ms; 10000 x 50,
+// 10 folds, K = 10 1.5 -> 0.17 ms.
+template <int P>
+__global__ void __launch_bounds__(kThreads, 1) candidates_kernel(SearchArgs A) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ SearchShared sh;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int first_pair = blockIdx.x * A.per, last_pair = min(A.pairs, first_pair + A.per);
+  const uint32_t qbytes = static_cast<uint32_t>(A.chunks) * kQRows * 16;       // one of hi / lo
+  const uint32_t sbytes = static_cast<uint32_t>(A.kg) * kBlockRows * 16;       // one of hi / lo of a stage
+  const uint32_t qs = tc5::smem_u32(smem), ss = qs + 2 * qbytes;
+  volatile int* stop = &sh.stop;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < A.stages; ++s) {
+      tc5::mbar_init(tc5::smem_u32(&sh.full[s]), 1);
+      tc5::mbar_init(tc5::smem_u32(&sh.empty[s]), 1);
+    }
+    for (int g = 0; g < 2; ++g) {
+      tc5::mbar_init(tc5::smem_u32(&sh.afull[g]), 1);
+      tc5::mbar_init(tc5::smem_u32(&sh.aempty[g]), 4);
+    }
+    tc5::mbar_init(tc5::smem_u32(&sh.qfull), 1);
+    tc5::mbar_init(tc5::smem_u32(&sh.qempty), 1);
+    tc5::mbar_fence_init();
+    sh.stop = 0;
+  }
+  if (threadIdx.x < 2 * kQRows) sh.tau[threadIdx.x / kQRows][threadIdx.x % kQRows] = ~0ull;
+  if (warp == 9) tc5::tmem_alloc(tc5::smem_u32(&sh.tmem), 512);
+  tc5::fence_before();
+  __syncthreads();
+  tc5::fence_after();
+  const uint32_t tmem = sh.tmem;
+
+  // first query tile of the range
+  int q = 0;
+  if (A.off == nullptr) {
+    q = first_pair / A.ntiles;
+  } else {
+    int lo = 0, hi = A.qtiles - 1;  // last q with off[q] <= first_pair
+    while (lo < hi) {
+      const int m = (lo + hi + 1) >> 1;
+      if (A.off[m] <= first_pair) lo = m;
+      else hi = m - 1;
+    }
+    q = lo;
+  }
+
+  // every role walks the same (query tile, candidate tile) sequence
+  if (warp == 8) {
+    if (lane == 0) {
+      int stage = 0, qn = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      int issued = 0;
+      for (int pair = first_pair, qt = q; ok && pair < last_pair; ++qt) {
+        const int o = A.off != nullptr ? A.off[qt] : qt * A.ntiles;
+        const int2 sk = A.skip != nullptr ? A.skip[qt] : make_int2(0, 0);
+        const TileOrder ord(A.ntiles, qt * kQRows / kBlockRows, sk.x, sk.y);
+        const int end = min(last_pair, o + ord.count);
+        if (pair >= end) continue;
+        // the query tile: half of a block, 2 KB of every chunk
+        if (qn > 0) ok = tc5::mbar_wait(tc5::smem_u32(&sh.qempty), (qn - 1) & 1, stop);
+        if (!ok) break;
+        ++qn;
+        const uint32_t qb = tc5::smem_u32(&sh.qfull);
+        tc5::mbar_expect(qb, 2 * qbytes);
+        const size_t src0 = (static_cast<size_t>(qt / 2) * A.chunks * kBlockRows + (qt & 1) * kQRows) * 8;
+        for (int c = 0; c < A.chunks; ++c) {
+          const size_t src = src0 + static_cast<size_t>(c) * kBlockRows * 8;
+          tc5::bulk_load(qs + c * kQRows * 16, A.xh + src, kQRows * 16, qb);
+          tc5::bulk_load(qs + qbytes + c * kQRows * 16, A.xl + src, kQRows * 16, qb);
+        }
+        for (; ok && pair < end; ++pair) {
+          const int tile = ord.at(pair - o);
+          for (int c0 = 0; c0 < A.chunks; c0 += A.kg) {
+            ok = tc5::mbar_wait(tc5::smem_u32(&sh.empty[stage]), phase ^ 1u, stop);
+            if (!ok) break;
+            const int nc = min(A.kg, A.chunks - c0);
+            const uint32_t bytes = static_cast<uint32_t>(nc) * kBlockRows * 16;
+            const uint32_t bar = tc5::smem_u32(&sh.full[stage]), dst = ss + stage * 2 * sbytes;
+            const size_t src = (static_cast<size_t>(tile) * A.chunks + c0) * kBlockRows * 8;
+            tc5::mbar_expect(bar, 2 * bytes);
+            tc5::bulk_load(dst, A.xh + src, bytes, bar);
+            tc5::bulk_load(dst + sbytes, A.xl + src, bytes, bar);
+            ++issued;
+            if (++stage == A.stages) {
+              stage = 0;
+              phase ^= 1u;
+            }
+          }
+        }
+      }
+      if (!ok) {
+        // the copies in flight land before the block's memory is given up
+        int zero = 0;
+        for (int b = 1; b <= min(issued, A.stages); ++b) {
+          const int s = (stage - b + A.stages) % A.stages;
+          tc5::mbar_wait(tc5::smem_u32(&sh.full[s]), s < stage ? phase : phase ^ 1u, &zero);
+        }
+        if (qn > 0) tc5::mbar_wait(tc5::smem_u32(&sh.qfull), (qn - 1) & 1, &zero);
+      }
+    }
+  } else if (warp == 9) {
+    if (lane == 0) {
+      const uint32_t idesc = tc5::idesc_bf16(kQRows, kBlockRows);
+      int stage = 0, qn = 0, it = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int pair = first_pair, qt = q; ok && pair < last_pair; ++qt) {
+        const int o = A.off != nullptr ? A.off[qt] : qt * A.ntiles;
+        const int2 sk = A.skip != nullptr ? A.skip[qt] : make_int2(0, 0);
+        const int end = min(last_pair, o + A.ntiles - sk.y);
+        if (pair >= end) continue;
+        ok = tc5::mbar_wait(tc5::smem_u32(&sh.qfull), qn & 1, stop);
+        ++qn;
+        for (; ok && pair < end; ++pair, ++it) {
+          const int buf = it & 1;
+          ok = tc5::mbar_wait(tc5::smem_u32(&sh.aempty[buf]), ((it >> 1) & 1) ^ 1, stop);
+          if (!ok) break;
+          tc5::fence_after();
+          const uint32_t dcol = tmem + buf * kBlockRows;
+          for (int c0 = 0; c0 < A.chunks; c0 += A.kg) {
+            ok = tc5::mbar_wait(tc5::smem_u32(&sh.full[stage]), phase, stop);
+            if (!ok) break;
+            tc5::fence_after();
+            const uint32_t bs = ss + stage * 2 * sbytes;
+            const int k1 = min(A.kg, A.chunks - c0) / 2;
+            for (int k = 0; k < k1; ++k) {
+              const uint32_t ao = static_cast<uint32_t>(c0 + 2 * k) * kQRows * 16;
+              const uint32_t bo = static_cast<uint32_t>(2 * k) * kBlockRows * 16;
+              const uint64_t ah = tc5::operand(qs + ao, kQRows), al = tc5::operand(qs + qbytes + ao, kQRows);
+              const uint64_t bh = tc5::operand(bs + bo, kBlockRows), bl = tc5::operand(bs + sbytes + bo, kBlockRows);
+              tc5::mma(dcol, ah, bh, idesc, c0 + k > 0);
+              tc5::mma(dcol, ah, bl, idesc, true);
+              tc5::mma(dcol, al, bh, idesc, true);
+            }
+            tc5::commit(tc5::smem_u32(&sh.empty[stage]));
+            if (++stage == A.stages) {
+              stage = 0;
+              phase ^= 1u;
+            }
+          }
+          if (ok) tc5::commit(tc5::smem_u32(&sh.afull[buf]));
+        }
+        if (ok) tc5::commit(tc5::smem_u32(&sh.qempty));
+      }
+      // on an early end the instructions still queued finish first
+      if (!ok) {
+        int zero = 0;
+        tc5::commit(tc5::smem_u32(&sh.qempty));
+        tc5::mbar_wait(tc5::smem_u32(&sh.qempty), qn > 0 ? (qn - 1) & 1 : 0, &zero);
+      }
+    }
+  } else {
+    const int g = warp >> 2;                 // this warp's accumulator / tile parity
+    const int r = (warp & 3) * 32 + lane;    // its row of the query tile
+    const uint32_t acc = tmem + g * kBlockRows + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    const float nmax = __uint_as_float(A.status[kStNorm]);
+    const int trig0 = A.Kq + max(32, A.Kq / 2), room = A.cap - 32;
+    int it = 0;
+    bool ok = true;
+    for (int pair = first_pair, qt = q; ok && pair < last_pair; ++qt) {
+      const int o = A.off != nullptr ? A.off[qt] : qt * A.ntiles;
+      const int2 sk = A.skip != nullptr ? A.skip[qt] : make_int2(0, 0);
+      const TileOrder ord(A.ntiles, qt * kQRows / kBlockRows, sk.x, sk.y);
+      const int end = min(last_pair, o + ord.count);
+      if (pair >= end) continue;
+      const int seg = blockIdx.x - o / A.per;
+      const size_t qpos = static_cast<size_t>(qt) * kQRows + r;
+      const size_t slot = (qpos * A.segs + seg) * 2 + g;
+      float2* const list = A.list + slot * A.cap;
+      const float nq = A.qn[qpos];
+      float tau = nq < 0.0f ? -INFINITY : INFINITY;
+      int cnt = 0, trig = min(trig0, room);
+      bool fresh = true, failed = false;
+      for (; ok && pair < end; ++pair, ++it) {
+        if ((it & 1) != g) continue;
+        const int tile = ord.at(pair - o);
+        const float* cn = A.cn + static_cast<size_t>(tile) * kBlockRows;
+        ok = __all_sync(kFull, tc5::mbar_wait(tc5::smem_u32(&sh.afull[g]), (it >> 1) & 1, stop));
+        if (!ok) break;
+        tc5::fence_after();
+        if (fresh) {
+          // The list's first tile: bound the row's Kq-th smallest value of the
+          // tile by bisection on the accumulator, each thread for its own row,
+          // so that the list starts with about Kq values instead of 256.
+          fresh = false;
+          float lo = INFINITY, hi = -INFINITY;
+          int fin = 0;
+          for (int c = 0; c < kBlockRows; c += 32) {
+            float v[32];
+            tc5::load32(acc + c, v);
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+              const float4 n4 = __ldg(reinterpret_cast<const float4*>(cn + c + i));
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float a = __fmaf_rn(v[i + e], A.scale, e == 0 ? n4.x : e == 1 ? n4.y : e == 2 ? n4.z : n4.w);
+                lo = fminf(lo, a);
+                if (a < INFINITY) {
+                  hi = fmaxf(hi, a);
+                  ++fin;
+                }
+              }
+            }
+          }
+          bool active = fin >= A.Kq;
+          for (int round = 0; round < 10; ++round) {
+            if (!__any_sync(kFull, active)) break;
+            const float mid = 0.5f * lo + 0.5f * hi;
+            int below = 0;
+            for (int c = 0; c < kBlockRows; c += 32) {
+              float v[32];
+              tc5::load32(acc + c, v);
+#pragma unroll
+              for (int i = 0; i < 32; i += 4) {
+                const float4 n4 = __ldg(reinterpret_cast<const float4*>(cn + c + i));
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                  below += __fmaf_rn(v[i + e], A.scale, e == 0 ? n4.x : e == 1 ? n4.y : e == 2 ? n4.z : n4.w) <= mid;
+              }
+            }
+            if (active) {
+              if (below >= A.Kq) {
+                hi = mid;
+                if (below <= A.Kq + (A.Kq >> 3)) active = false;
+              } else {
+                lo = mid;
+              }
+            }
+          }
+          if (fin >= A.Kq && nq >= 0.0f) tau = hi + 2.0f * delta_of(hi, nq, nmax, A.crel, A.inner);
+        }
+        // the other group's threshold for the same query holds for this group
+        // too: it is at least the row's final limit
+        const unsigned long long other = *const_cast<volatile unsigned long long*>(&sh.tau[g ^ 1][r]);
+        if (!failed && static_cast<int>(other >> 32) == qt)
+          tau = fminf(tau, __uint_as_float(static_cast<unsigned>(other)));
+        const int pos0 = tile * kBlockRows;
+        for (int c = 0; c < kBlockRows; c += 32) {
+          float v[32];
+          tc5::load32(acc + c, v);
+          float m = INFINITY;
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) {
+            const float4 n4 = __ldg(reinterpret_cast<const float4*>(cn + c + i));
+            v[i] = __fmaf_rn(v[i], A.scale, n4.x);
+            v[i + 1] = __fmaf_rn(v[i + 1], A.scale, n4.y);
+            v[i + 2] = __fmaf_rn(v[i + 2], A.scale, n4.z);
+            v[i + 3] = __fmaf_rn(v[i + 3], A.scale, n4.w);
+            m = tc5::min3(m, v[i], v[i + 1]);
+            m = tc5::min3(m, v[i + 2], v[i + 3]);
+          }
+          if (!__any_sync(kFull, m < tau)) continue;
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            if (v[i] < tau) list[cnt++] = make_float2(v[i], __int_as_float(pos0 + c + i));
+          }
+          unsigned todo = __ballot_sync(kFull, cnt > trig);
+          while (todo != 0u) {
+            const int src = __ffs(todo) - 1;
+            todo &= todo - 1u;
+            __syncwarp();
+            float2* const l2 = reinterpret_cast<float2*>(
+                __shfl_sync(kFull, reinterpret_cast<unsigned long long>(list), src));
+            float t2 = __shfl_sync(kFull, tau, src);
+            const int left = cut_list<P>(l2, __shfl_sync(kFull, cnt, src), A.Kq, __shfl_sync(kFull, nq, src), nmax,
+                                         A.crel, A.inner, &t2, lane);
+            if (lane == src) {
+              cnt = left;
+              tau = t2;
+              trig = min(room, max(trig0, left + max(32, A.Kq / 2)));
+              if (left > room) {  // too many values within 2 delta: the row goes to the brute force
+                failed = true;
+                cnt = 0;
+                tau = -INFINITY;
+              } else {
+                *const_cast<volatile unsigned long long*>(&sh.tau[g][r]) =
+                    (static_cast<unsigned long long>(qt) << 32) | __float_as_uint(tau);
+              }
+            }
+          }
+        }
+        tc5::fence_before();
+        __syncwarp();
+        if (lane == 0) tc5::mbar_arrive(tc5::smem_u32(&sh.aempty[g]));
+      }
+      if (pair < end) pair = end;
+      A.cnt[slot] = failed ? -1 : cnt;
+      A.tau[slot] = failed ? -INFINITY : tau;
+    }
+  }
+  __syncwarp();
+  tc5::fence_before();
+  __syncthreads();
+  tc5::fence_after();
+  if (warp == 9) tc5::tmem_free(tmem, 512);
+  if (threadIdx.x == 0 && sh.stop != 0) atomicExch(&A.status[kStTimeout], 1u);
+}
+
+struct RerankArgs {
+  SearchArgs s;
+  const float* x;      // n x d4 floats, 16-byte aligned rows
+  int d, d4, K, npos, mode;
+  const int* perm;
+  int* idx;
+  float* dist;
+  int* fb_rows;
+};
+
+// One warp per query position.
+__global__ void __launch_bounds__(128) rerank_kernel(RerankArgs R) {
+  __shared__ float2 room[4][kSurvivors];
+  const SearchArgs& A = R.s;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int pos = blockIdx.x * 4 + warp;
+  if (pos >= R.npos) return;
+  const int row = R.perm != nullptr ? R.perm[pos] : pos;
+  const float nq = A.qn[pos];
+  if (nq < 0.0f) return;  // padding
+  const float nmax = __uint_as_float(A.status[kStNorm]);
+  const unsigned below = (1u << lane) - 1u;
+  float2* list = room[warp];
+  bool bad = A.status[kStBad] != 0u || A.status[kStTimeout] != 0u || !(nmax >= 1e-20f && nmax <= 1e36f);
+  int m = 0;
+  if (!bad) {
+    const int qt = pos / kQRows;
+    const int o = A.off != nullptr ? A.off[qt] : qt * A.ntiles;
+    const int count = A.ntiles - (A.skip != nullptr ? A.skip[qt].y : 0);
+    const int nl = count > 0 ? 2 * ((o + count - 1) / A.per - o / A.per + 1) : 0;  // this row's lists
+    const size_t slot = static_cast<size_t>(pos) * A.segs * 2;
+    float tau = INFINITY;
+    int low = 0;
+    for (int l = lane; l < nl; l += 32) {
+      tau = fminf(tau, A.tau[slot + l]);
+      low = min(low, A.cnt[slot + l]);
+    }
+    tau = from_ord(__reduce_min_sync(kFull, ord_float(tau)));
+    bad = __reduce_min_sync(kFull, low) < 0;
+    for (int l = 0; l < nl && !bad; ++l) {
+      const int c = A.cnt[slot + l];
+      const float2* src = A.list + (slot + l) * A.cap;
+      for (int e0 = 0; e0 < c; e0 += 32) {
+        const float2 v = e0 + lane < c ? src[e0 + lane] : make_float2(INFINITY, 0.0f);
+        const bool keep = v.x < tau;
+        const unsigned b = __ballot_sync(kFull, keep);
+        if (m + __popc(b) > kSurvivors) {
+          // many short segments each hold about Kq values: cut the joined list
+          __syncwarp();
+          m = cut_list<kSurvivors / 32>(list, m, A.Kq, nq, nmax, A.crel, A.inner, &tau, lane);
+          if (m + __popc(b) > kSurvivors) {
+            bad = true;
+            break;
+          }
+        }
+        if (keep) list[m + __popc(b & below)] = v;
+        m += __popc(b);
+      }
+    }
+    __syncwarp();
+    bad = bad || m < A.Kq;
+  }
+  if (bad) {
+    if (lane == 0) R.fb_rows[atomicAdd(&A.status[kStFallback], 1u)] = row;
+    return;
+  }
+  float v[kSurvivors / 32];
+#pragma unroll
+  for (int t = 0; t < kSurvivors / 32; ++t) v[t] = lane + 32 * t < m ? list[lane + 32 * t].x : INFINITY;
+  const float AK = kth_bound<kSurvivors / 32>(v, A.Kq, 0, 24);
+  const float lim = AK + 2.0f * delta_of(AK, nq, nmax, A.crel, A.inner);
+  // keep the values within the limit, except the query itself
+  int m2 = 0;
+#pragma unroll
+  for (int t = 0; t < kSurvivors / 32; ++t) {
+    if (32 * t >= m) break;
+    const int i = lane + 32 * t;
+    const float2 e = i < m ? list[i] : make_float2(INFINITY, 0.0f);
+    const int p = __float_as_int(e.y);
+    const bool keep = i < m && e.x <= lim && p != pos;
+    const unsigned b = __ballot_sync(kFull, keep);
+    __syncwarp();
+    if (keep) list[m2 + __popc(b & below)] = make_float2(0.0f, e.y);
+    __syncwarp();
+    m2 += __popc(b);
+  }
+  if (m2 < R.K) {
+    if (lane == 0) R.fb_rows[atomicAdd(&A.status[kStFallback], 1u)] = row;
+    return;
+  }
+  // canonical distances, a lane per candidate; the keys replace the entries
+  unsigned long long* key = reinterpret_cast<unsigned long long*>(list);
+  const float4* xq = reinterpret_cast<const float4*>(R.x + static_cast<size_t>(row) * R.d4);
+  const int full4 = R.d / 4, rest = R.d & 3;
+  for (int i = lane; i < m2; i += 32) {
+    const int p = __float_as_int(list[i].y);
+    const int j = R.perm != nullptr ? R.perm[p] : p;
+    const float4* xj = reinterpret_cast<const float4*>(R.x + static_cast<size_t>(j) * R.d4);
+    float a = 0.0f;
+    if (A.inner) {
+#pragma unroll 4
+      for (int k = 0; k < full4; ++k) {
+        const float4 u = xq[k], w = xj[k];
+        a = __fadd_rn(a, __fmul_rn(u.x, w.x));
+        a = __fadd_rn(a, __fmul_rn(u.y, w.y));
+        a = __fadd_rn(a, __fmul_rn(u.z, w.z));
+        a = __fadd_rn(a, __fmul_rn(u.w, w.w));
+      }
+      if (rest) {
+        const float4 u = xq[full4], w = xj[full4];
+        a = __fadd_rn(a, __fmul_rn(u.x, w.x));
+        if (rest > 1) a = __fadd_rn(a, __fmul_rn(u.y, w.y));
+        if (rest > 2) a = __fadd_rn(a, __fmul_rn(u.z, w.z));
+      }
+      a = __fsub_rn(0.0f, a);  // +0 for a zero product, so that equal values have equal keys
+    } else {
+#pragma unroll 4
+      for (int k = 0; k < full4; ++k) {
+        const float4 u = xq[k], w = xj[k];
+        float f = __fsub_rn(u.x, w.x);
+        a = __fadd_rn(a, __fmul_rn(f, f));
+        f = __fsub_rn(u.y, w.y);
+        a = __fadd_rn(a, __fmul_rn(f, f));
+        f = __fsub_rn(u.z, w.z);
+        a = __fadd_rn(a, __fmul_rn(f, f));
+        f = __fsub_rn(u.w, w.w);
+        a = __fadd_rn(a, __fmul_rn(f, f));
+      }
+      if (rest) {
+        const float4 u = xq[full4], w = xj[full4];
+        float f = __fsub_rn(u.x, w.x);
+        a = __fadd_rn(a, __fmul_rn(f, f));
+        if (rest > 1) {
+          f = __fsub_rn(u.y, w.y);
+          a = __fadd_rn(a, __fmul_rn(f, f));
+        }
+        if (rest > 2) {
+          f = __fsub_rn(u.z, w.z);
+          a = __fadd_rn(a, __fmul_rn(f, f));
+        }
+      }
+    }
+    key[i] = (static_cast<unsigned long long>(ord_float(a)) << 32) | static_cast<unsigned>(j);
+  }
+  __syncwarp();
+  // rank of every key; the first K are the row's neighbours
+  for (int i = lane; i < m2; i += 32) {
+    const unsigned long long mine = key[i];
+    int rank = 0;
+#pragma unroll 4
+    for (int e = 0; e < m2; ++e) rank += key[e] < mine;
+    if (rank < R.K) {
+      float a = from_ord(static_cast<unsigned>(mine >> 32));
+      // the brute force reports minus a float sum: a zero sum gives -0
+      if (A.inner && a == 0.0f) a = -0.0f;
+      const size_t out = static_cast<size_t>(row) * R.K + rank;
+      R.idx[out] = static_cast<int>(mine & 0xffffffffu);
+      R.dist[out] = knn_output_distance(a, R.mode);
+    }
+  }
+}
+
+}  // namespace
 
 __global__ void split_rows_kernel(const float* __restrict__ x, int n, int d, int dp, uint16_t* __restrict__ xh,
                                   uint16_t* __restrict__ xl) {
@@ -91,448 +745,6 @@ __global__ void split_rows_kernel(const float* __restrict__ x, int n, int d, int
   xl[o] = static_cast<uint16_t>(lb);
 }
 
-__device__ __forceinline__ void mma16816(float* c, const uint32_t* a, uint2 b) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};\n"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b.x), "r"(b.y));
-}
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
-}
-
-struct TcArgs {
-  const uint16_t* xh;   // n x dp, permuted 16-blocks
-  const uint16_t* xl;
-  const float* nrm;     // n
-  int n, dp, kp, segs;
-  int row_words;        // 32-bit words per candidate row in shared memory (= 8 mod 16)
-  int* cand;            // n x segs x 2 x kp candidate rows (-1 = none)
-  float* cand_a;        // their approximate distances
-  float* bound;         // n x segs: the smaller final heap threshold (+inf = nothing excluded)
-};
-
-constexpr int kMaxPer = 8;   // re-rank candidates per lane (segs x 2 x kp <= 256)
-
-// Shared memory: 2 x (hi, lo) candidate tiles, 2 x tile norms, per warp a
-// 16 x kTileStride distance tile, 16 x 4 flag masks, 32 thresholds and 32
-// lane-interleaved max-heaps of kp (distance, row) entries; above kTcRegKs
-// k-steps also the warp's 16 lo query rows (row stride row_words, the
-// candidate tiles' conflict-free stride).
-size_t tc_smem_bytes(int row_words, int kp, int dp) {
-  const size_t lo_rows = dp > 16 * kTcRegKs ? kTcWarps * 16 * static_cast<size_t>(row_words) * 4 : 0;
-  return 2 * 2 * static_cast<size_t>(kTcN) * row_words * 4 + 2 * kTcN * 4 +
-         kTcWarps * (16 * kTileStride * 4 + 64 * 4 + 32 * 4 + 32 * static_cast<size_t>(kp) * 8) + lo_rows;
-}
-
-// KS: k-steps of 16 coordinates in the query fragments (dp <= 16 KS).  Up to
-// kTcRegKs every thread keeps its 2 KS 16-byte chunks of a candidate tile
-// (kTcN x dp / 8 / 128) in registers; above it the chunks are recomputed per
-// tile and the lo query fragments are read from shared memory per k-step.
-template <int KS>
-__global__ void __launch_bounds__(32 * kTcWarps, 2) tc_candidates_kernel(TcArgs A) {
-  constexpr bool kLoShared = KS > kTcRegKs;
-  constexpr int kMaxLoads = kLoShared ? 1 : 2 * KS;
-  constexpr int kRegLo = kLoShared ? 1 : KS;
-  extern __shared__ __align__(16) unsigned char smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
-  const int n = A.n, dp = A.dp, kp = A.kp, rw = A.row_words, ksn = dp >> 4;
-  const int seg = blockIdx.y, segs = A.segs;
-  uint32_t* cbuf = reinterpret_cast<uint32_t*>(smem);  // [buf][hi/lo][kTcN][rw]
-  float* cnb = reinterpret_cast<float*>(cbuf + 2 * 2 * kTcN * rw);  // [buf][kTcN]
-  float* dt = cnb + 2 * kTcN + warp * (16 * kTileStride + 64 + 32 + 32 * kp * 2);  // [16][kTileStride]
-  unsigned* fmask = reinterpret_cast<unsigned*>(dt + 16 * kTileStride);            // [16][4]
-  float* htau = reinterpret_cast<float*>(fmask + 64);                              // [32] per heap
-  float* hv = htau + 32;                                                           // [kp][32]
-  int* hj = reinterpret_cast<int*>(hv + 32 * kp);                                  // [kp][32]
-  htau[lane] = INFINITY;
-
-  const int q0 = blockIdx.x * kTcQ + warp * 16;
-  // the warp's 16 lo query rows in shared memory (only above kTcRegKs)
-  uint32_t* qlo = reinterpret_cast<uint32_t*>(cnb + 2 * kTcN + kTcWarps * (16 * kTileStride + 64 + 32 + 32 * kp * 2)) +
-                  warp * 16 * rw;
-  if (kLoShared) {
-    const int hw = dp >> 1;  // 32-bit words per row
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(A.xl);
-    for (int w = lane; w < 16 * hw; w += 32) {
-      const int rr = w / hw, c = w - rr * hw;
-      qlo[rr * rw + c] = src[static_cast<size_t>(min(q0 + rr, n - 1)) * hw + c];
-    }
-    __syncwarp();
-  }
-  // query fragments: rows g and g + 8 of the warp's 16 queries
-  uint32_t ah[KS][4], al[kRegLo][4];
-  {
-    const int ra = min(q0 + g, n - 1), rb = min(q0 + g + 8, n - 1);
-#pragma unroll
-    for (int ks = 0; ks < KS; ++ks) {
-      uint2 pa = make_uint2(0u, 0u), pb = pa, qa = pa, qb = pa;
-      if (ks < ksn) {
-        pa = *reinterpret_cast<const uint2*>(A.xh + static_cast<size_t>(ra) * dp + ks * 16 + 4 * tig);
-        pb = *reinterpret_cast<const uint2*>(A.xh + static_cast<size_t>(rb) * dp + ks * 16 + 4 * tig);
-        if (!kLoShared) {
-          qa = *reinterpret_cast<const uint2*>(A.xl + static_cast<size_t>(ra) * dp + ks * 16 + 4 * tig);
-          qb = *reinterpret_cast<const uint2*>(A.xl + static_cast<size_t>(rb) * dp + ks * 16 + 4 * tig);
-        }
-      }
-      ah[ks][0] = pa.x; ah[ks][2] = pa.y; ah[ks][1] = pb.x; ah[ks][3] = pb.y;
-      if (!kLoShared) {
-        al[ks][0] = qa.x; al[ks][2] = qa.y; al[ks][1] = qb.x; al[ks][3] = qb.y;
-      }
-    }
-  }
-  const int qa_row = q0 + g, qb_row = q0 + g + 8;
-  const float nq_g = A.nrm[min(qa_row, n - 1)], nq_g8 = A.nrm[min(qb_row, n - 1)];
-  // the heap this lane owns: query row r, the columns of quad lanes 2 h, 2 h + 1
-  const int r = lane & 15, h = lane >> 4, myq = q0 + r;
-  // the heaps whose thresholds this lane's fragment values are filtered by
-  const int heap_a = g + 16 * (tig >> 1), heap_b = heap_a + 8;
-  int cnt = 0;
-  float tau = INFINITY;
-
-  // this thread's 16-byte chunks of a tile (the same every tile): smem word
-  // offset of the hi chunk and element offset inside the tile's rows
-  const int chunks = dp >> 3;
-  int ld_smem[kMaxLoads], ld_row[kMaxLoads], ld_col[kMaxLoads], nld = 0;
-#pragma unroll
-  for (int t = 0; t < kMaxLoads; ++t) {
-    const int e = threadIdx.x + t * 32 * kTcWarps;
-    ld_row[t] = 0;
-    ld_col[t] = 0;
-    ld_smem[t] = 0;
-    if (!kLoShared && e < kTcN * chunks) {
-      const int c = e / chunks, ch = e - c * chunks;
-      ld_row[t] = c;
-      ld_col[t] = ch * 8;
-      ld_smem[t] = c * rw + ch * 4;
-      nld = t + 1;
-    }
-  }
-  __syncwarp();
-
-  // scattered tile order: the tile at step k is (first + k * stride) mod ntiles,
-  // stride coprime to ntiles (1000003 is a prime above any tile count); this
-  // segment takes the steps seg, seg + segs, ...
-  const int ntiles = (n + kTcN - 1) / kTcN;
-  const int stride = static_cast<int>(1000003ull % static_cast<unsigned long long>(ntiles));
-  const int jump = static_cast<int>((static_cast<unsigned long long>(stride) * segs) % ntiles);
-  const int first = static_cast<int>((static_cast<unsigned long long>(blockIdx.x) * 7919ull +
-                                      static_cast<unsigned long long>(seg) * stride) % ntiles);
-  const int nsteps = ntiles > seg ? (ntiles - seg + segs - 1) / segs : 0;
-
-  auto load_tile = [&](int buf, int tile) {
-    const int base = tile * kTcN;
-    uint32_t* dh = cbuf + (buf * 2 + 0) * kTcN * rw;
-    uint32_t* dl = cbuf + (buf * 2 + 1) * kTcN * rw;
-    if (kLoShared) {
-      for (int e = threadIdx.x; e < kTcN * chunks; e += 32 * kTcWarps) {
-        const int c = e / chunks, ch = e - c * chunks;
-        const int so = c * rw + ch * 4;
-        if (base + c < n) {
-          const size_t src = static_cast<size_t>(base + c) * dp + ch * 8;
-          cp_async16(dh + so, A.xh + src);
-          cp_async16(dl + so, A.xl + src);
-        } else {
-          *reinterpret_cast<uint4*>(dh + so) = make_uint4(0u, 0u, 0u, 0u);
-          *reinterpret_cast<uint4*>(dl + so) = make_uint4(0u, 0u, 0u, 0u);
-        }
-      }
-    }
-#pragma unroll
-    for (int t = 0; t < kMaxLoads; ++t) {
-      if (!kLoShared && t < nld) {
-        const int row = base + ld_row[t];
-        if (row < n) {
-          const size_t src = static_cast<size_t>(row) * dp + ld_col[t];
-          cp_async16(dh + ld_smem[t], A.xh + src);
-          cp_async16(dl + ld_smem[t], A.xl + src);
-        } else {
-          *reinterpret_cast<uint4*>(dh + ld_smem[t]) = make_uint4(0u, 0u, 0u, 0u);
-          *reinterpret_cast<uint4*>(dl + ld_smem[t]) = make_uint4(0u, 0u, 0u, 0u);
-        }
-      }
-    }
-    for (int c = threadIdx.x; c < kTcN; c += 32 * kTcWarps) cnb[buf * kTcN + c] = base + c < n ? A.nrm[base + c] : 0.0f;
-    cp_async_commit();
-  };
-
-  int tile = first;
-  if (nsteps > 0) load_tile(0, tile);
-  for (int step = 0; step < nsteps; ++step) {
-    const int buf = step & 1;
-    const int t0 = tile * kTcN;
-    int next = tile + jump;
-    if (next >= ntiles) next -= ntiles;
-    if (step + 1 < nsteps) {
-      load_tile(buf ^ 1, next);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-    const uint32_t* th = cbuf + (buf * 2 + 0) * kTcN * rw;
-    const uint32_t* tl = cbuf + (buf * 2 + 1) * kTcN * rw;
-    const float* cn = cnb + buf * kTcN;
-    // only the last tile and the tiles holding this warp's queries need the
-    // column checks (past the end, the query itself)
-    const bool edge = t0 + kTcN > n || (t0 < q0 + 16 && q0 < t0 + kTcN) || q0 + 16 > n;
-    const float tau_a = htau[heap_a], tau_b = htau[heap_b];
-    unsigned fa = 0u, fb = 0u;  // bit 2 nt + c: column nt * 8 + 2 tig + c of rows g / g + 8
-    // eight independent accumulator chains (one per n-tile) hide the mma latency
-    float accs[8][4];
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) accs[nt][0] = accs[nt][1] = accs[nt][2] = accs[nt][3] = 0.0f;
-#pragma unroll
-    for (int ks = 0; ks < KS; ++ks) {
-      if (ks < ksn) {
-        uint32_t lo[4];
-        if (kLoShared) {
-          const uint2 la = *reinterpret_cast<const uint2*>(qlo + g * rw + ks * 8 + 2 * tig);
-          const uint2 lb = *reinterpret_cast<const uint2*>(qlo + (g + 8) * rw + ks * 8 + 2 * tig);
-          lo[0] = la.x; lo[2] = la.y; lo[1] = lb.x; lo[3] = lb.y;
-        } else {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) lo[i] = al[kLoShared ? 0 : ks][i];
-        }
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-          const int off = (nt * 8 + g) * rw + ks * 8 + 2 * tig;
-          const uint2 bh = *reinterpret_cast<const uint2*>(th + off);
-          const uint2 bl = *reinterpret_cast<const uint2*>(tl + off);
-          mma16816(accs[nt], ah[ks], bh);
-          mma16816(accs[nt], ah[ks], bl);
-          mma16816(accs[nt], lo, bh);
-        }
-      }
-    }
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      const float* acc = accs[nt];
-      const int col = nt * 8 + 2 * tig;
-      const float c0 = cn[col], c1 = cn[col + 1];
-      const float v0 = nq_g + c0 - 2.0f * acc[0], v1 = nq_g + c1 - 2.0f * acc[1];
-      const float v2 = nq_g8 + c0 - 2.0f * acc[2], v3 = nq_g8 + c1 - 2.0f * acc[3];
-      bool f0 = v0 < tau_a, f1 = v1 < tau_a, f2 = v2 < tau_b, f3 = v3 < tau_b;
-      if (edge) {
-        const int j0 = t0 + col, j1 = j0 + 1;
-        f0 = f0 && j0 < n && j0 != qa_row && qa_row < n;
-        f1 = f1 && j1 < n && j1 != qa_row && qa_row < n;
-        f2 = f2 && j0 < n && j0 != qb_row && qb_row < n;
-        f3 = f3 && j1 < n && j1 != qb_row && qb_row < n;
-      }
-      fa |= (static_cast<unsigned>(f0) | (static_cast<unsigned>(f1) << 1)) << (2 * nt);
-      fb |= (static_cast<unsigned>(f2) | (static_cast<unsigned>(f3) << 1)) << (2 * nt);
-      if (f0 | f1) *reinterpret_cast<float2*>(dt + g * kTileStride + col) = make_float2(v0, v1);
-      if (f2 | f3) *reinterpret_cast<float2*>(dt + (g + 8) * kTileStride + col) = make_float2(v2, v3);
-    }
-    fmask[g * 4 + tig] = fa;
-    fmask[(g + 8) * 4 + tig] = fb;
-    __syncwarp();
-    // the owner of each heap inserts its flagged values: 16 bits per quad lane,
-    // quad lanes 2 h and 2 h + 1 feed heap (r, h)
-    unsigned m = fmask[r * 4 + 2 * h] | (fmask[r * 4 + 2 * h + 1] << 16);
-    while (m != 0u) {
-      const int b = __ffs(m) - 1;
-      m &= m - 1u;
-      const int qt = 2 * h + (b >> 4), bb = b & 15;
-      const int col = (bb >> 1) * 8 + 2 * qt + (bb & 1);
-      const float v = dt[r * kTileStride + col];
-      if (!(v < tau)) continue;
-      const int j = t0 + col;
-      if (cnt < kp) {
-        // push: sift up
-        int c = cnt++;
-        while (c > 0) {
-          const int p = (c - 1) >> 1;
-          const float pv = hv[p * 32 + lane];
-          if (!(pv < v)) break;
-          hv[c * 32 + lane] = pv;
-          hj[c * 32 + lane] = hj[p * 32 + lane];
-          c = p;
-        }
-        hv[c * 32 + lane] = v;
-        hj[c * 32 + lane] = j;
-        if (cnt == kp) tau = hv[lane];
-      } else {
-        // replace the maximum: sift down
-        int c = 0;
-        for (;;) {
-          const int l = 2 * c + 1;
-          if (l >= kp) break;
-          int big = l;
-          float bv = hv[l * 32 + lane];
-          if (l + 1 < kp) {
-            const float rv = hv[(l + 1) * 32 + lane];
-            if (rv > bv) {
-              big = l + 1;
-              bv = rv;
-            }
-          }
-          if (!(bv > v)) break;
-          hv[c * 32 + lane] = bv;
-          hj[c * 32 + lane] = hj[big * 32 + lane];
-          c = big;
-        }
-        hv[c * 32 + lane] = v;
-        hj[c * 32 + lane] = j;
-        tau = hv[lane];
-      }
-    }
-    htau[lane] = tau;
-    tile = next;
-    __syncthreads();
-  }
-  // heaps out; the bound is the smaller final threshold of the row's two heaps
-  const float mine = cnt == kp ? tau : INFINITY;
-  const float other = __shfl_xor_sync(0xffffffffu, mine, 16);
-  if (myq < n) {
-    const size_t base = ((static_cast<size_t>(myq) * segs + seg) * 2 + h) * kp;
-    for (int e = 0; e < kp; ++e) {
-      A.cand[base + e] = e < cnt ? hj[e * 32 + lane] : -1;
-      A.cand_a[base + e] = e < cnt ? hv[e * 32 + lane] : INFINITY;
-    }
-    if (h == 0) A.bound[static_cast<size_t>(myq) * segs + seg] = fminf(mine, other);
-  }
-}
-
-// order-preserving image of a float as an unsigned
-__device__ __forceinline__ unsigned ord_float(float v) {
-  const unsigned u = __float_as_uint(v);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-
-// One warp per query: A_K (the K-th smallest approximate distance of its
-// m = segs x 2 x kp candidates), canonical distances of the candidates with
-// a <= A_K + 2 delta, the K smallest of those by (distance, index), and the
-// certificate B > A_K + 2 delta (every row goes to the fallback list when the
-// data hold a non-finite value).
-__global__ void tc_rerank_kernel(const float* __restrict__ x, int n, int d, int K, int m, int segs,
-                                 const int* __restrict__ cand, const float* __restrict__ cand_a,
-                                 const float* __restrict__ bound, const float* __restrict__ nrm,
-                                 const unsigned* __restrict__ nrm_max, const int* __restrict__ nonfinite,
-                                 float crel, int* __restrict__ idx, float* __restrict__ dist,
-                                 int* __restrict__ fb_rows, int* __restrict__ fb_count) {
-  const int lane = threadIdx.x & 31;
-  const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (q >= n) return;
-  if (*nonfinite) {
-    if (lane == 0) fb_rows[atomicAdd(fb_count, 1)] = q;
-    return;
-  }
-  float av[kMaxPer];
-  int jv[kMaxPer];
-  unsigned long long key[kMaxPer];
-#pragma unroll
-  for (int t = 0; t < kMaxPer; ++t) {
-    const int e = lane + 32 * t;
-    av[t] = INFINITY;
-    jv[t] = -1;
-    if (e < m) {
-      const int j = cand[static_cast<size_t>(q) * m + e];
-      if (j >= 0) {
-        jv[t] = j;
-        av[t] = cand_a[static_cast<size_t>(q) * m + e];
-      }
-    }
-  }
-  float thr = INFINITY;
-  {
-    // A_K: the approximate distance of the K-th smallest (a, row) key
-    unsigned long long k2[kMaxPer];
-#pragma unroll
-    for (int t = 0; t < kMaxPer; ++t)
-      k2[t] = jv[t] >= 0 ? (static_cast<unsigned long long>(ord_float(av[t])) << 32) | static_cast<unsigned>(jv[t])
-                         : ~0ull;
-    unsigned long long kth = ~0ull;
-    for (int o = 0; o < K; ++o) {
-      unsigned long long best = k2[0];
-#pragma unroll
-      for (int t = 1; t < kMaxPer; ++t) best = k2[t] < best ? k2[t] : best;
-#pragma unroll
-      for (int s = 16; s > 0; s >>= 1) {
-        const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, s);
-        best = other < best ? other : best;
-      }
-      kth = best;
-      if (best == ~0ull) break;
-#pragma unroll
-      for (int t = 0; t < kMaxPer; ++t)
-        if (k2[t] == best) k2[t] = ~0ull;
-    }
-    if (kth != ~0ull) {
-      const unsigned o = static_cast<unsigned>(kth >> 32);
-      thr = __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
-    }
-  }
-  const float delta = (nrm[q] + __uint_as_float(*nrm_max)) * crel;
-  const float limit = thr + 2.0f * delta;
-  const float* xq = x + static_cast<size_t>(q) * d;
-  // canonical distances of the candidates within the limit
-#pragma unroll
-  for (int t = 0; t < kMaxPer; ++t) {
-    key[t] = ~0ull;
-    if (jv[t] >= 0 && av[t] <= limit) {
-      const float* xj = x + static_cast<size_t>(jv[t]) * d;
-      float a = 0.0f;
-      for (int k = 0; k < d; ++k) {
-        const float diff = __fsub_rn(xq[k], xj[k]);
-        a = __fadd_rn(a, __fmul_rn(diff, diff));
-      }
-      // canonical distances are >= 0: their bit patterns order like the values
-      key[t] = (static_cast<unsigned long long>(__float_as_uint(a)) << 32) | static_cast<unsigned>(jv[t]);
-    }
-  }
-  for (int o = 0; o < K; ++o) {
-    unsigned long long best = key[0];
-#pragma unroll
-    for (int t = 1; t < kMaxPer; ++t) best = key[t] < best ? key[t] : best;
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) {
-      const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, s);
-      best = other < best ? other : best;
-    }
-#pragma unroll
-    for (int t = 0; t < kMaxPer; ++t)
-      if (key[t] == best) key[t] = ~0ull;
-    if (lane == 0) {
-      const size_t out = static_cast<size_t>(q) * K + o;
-      if (best == ~0ull) {
-        idx[out] = -1;
-        dist[out] = INFINITY;
-      } else {
-        idx[out] = static_cast<int>(best & 0xffffffffu);
-        dist[out] = __fsqrt_rn(__uint_as_float(static_cast<unsigned>(best >> 32)));
-      }
-    }
-  }
-  if (lane == 0) {
-    float B = INFINITY;
-    for (int s = 0; s < segs; ++s) B = fminf(B, bound[static_cast<size_t>(q) * segs + s]);
-    if (!(B > limit)) fb_rows[atomicAdd(fb_count, 1)] = q;
-  }
-}
-
-}  // namespace
-
-// Segments and heap size: the K nearest rows spread over segs x 2 heaps,
-// each heap holding about twice its expected share plus a margin.
-void tc_shape(int K, int* segs, int* kp) {
-  *segs = K <= 40 ? 8 : 4;
-  const int share = (K + 2 * *segs - 1) / (2 * *segs);
-  int k = (2 * share + 8 + 7) / 8 * 8;
-  k = k < 16 ? 16 : k;
-  const int cap = kMaxPer * 32 / (2 * *segs);
-  *kp = k > cap ? cap : k;
-}
-
 int bf16_split_rows(const float* x, int n, int d, int dp, uint16_t* xh, uint16_t* xl, cudaStream_t st) {
   const size_t total = static_cast<size_t>(n) * dp;
   if (total == 0) return 0;
@@ -541,109 +753,200 @@ int bf16_split_rows(const float* x, int n, int d, int dp, uint16_t* xh, uint16_t
   return static_cast<int>(cudaGetLastError());
 }
 
-bool knn_tc_supported(int n, int d, int K) {
-  int segs = 0, kp = 0;
-  tc_shape(K, &segs, &kp);
-  if (!(d >= 1 && d <= 16 * kTcMaxKs && K >= 1 && K <= 96 && n > 2 * kp + kTcN)) return false;
-  const int dp = (d + 15) / 16 * 16, half = dp / 2;
-  const int rw = (half % 16 == 8) ? half : half + 8;
-  return tc_smem_bytes(rw, kp, dp) <= kTcSmemLimit;
-}
-
 namespace {
 
+// From one candidate tile on: whole calls at 256 rows x 10, K = 10 take 144 us
+// here and 150 us by the brute force, at K = 100 159 and 491 us, at 1000 rows x
+// 50, K = 100 196 and 1922 us.  Up to 223 neighbours: lists of 512 entries.
+constexpr int kMinRows = 256;
+
 struct TcLayout {
-  int dp, kp, segs, rw;
-  size_t o_xh, o_xl, o_nrm, o_flags, o_cand, o_canda, o_bound, o_fb, o_brute, total;
+  int dp, chunks, kg, stages, npos, ntiles, qtiles, cap, Kq, pairs, per, segs, d4, ctas;
+  size_t smem;
+  size_t o_xh, o_xl, o_cn, o_qn, o_status, o_xp, o_cnt, o_tau, o_list, o_fb, o_brute, total;
 };
 
-TcLayout tc_layout(int n, int d, int K, int segments) {
+int list_entries(int Kq) { return Kq <= 36 ? 128 : Kq <= 112 ? 256 : 512; }
+
+// The operand blocks, the stream-K split over `sms` CTAs and the scratch
+// offsets.  fp: the fold-wise search's row order, or null.
+TcLayout tc_layout(int n, int d, int K, int segments, int sms, const KnnFoldPlan* fp) {
   TcLayout L{};
   L.dp = (d + 15) / 16 * 16;
-  tc_shape(K, &L.segs, &L.kp);
-  const int half = L.dp / 2;
-  L.rw = (half % 16 == 8) ? half : half + 8;
-  const size_t m = static_cast<size_t>(L.segs) * 2 * L.kp;
+  L.chunks = L.dp / 8;
+  L.d4 = (d + 3) / 4 * 4;
+  L.Kq = fp != nullptr ? K : K + 1;
+  L.cap = list_entries(L.Kq);
+  L.ntiles = fp != nullptr ? fp->tiles : (n + kBlockRows - 1) / kBlockRows;
+  L.qtiles = fp != nullptr ? 2 * fp->tiles : (n + kQRows - 1) / kQRows;
+  L.pairs = fp != nullptr ? fp->pairs : L.ntiles * L.qtiles;
+  L.npos = L.ntiles * kBlockRows;
+  L.ctas = L.pairs < sms ? (L.pairs > 0 ? L.pairs : 1) : sms;
+  L.per = (L.pairs + L.ctas - 1) / L.ctas;
+  if (L.per < 1) L.per = 1;
+  L.segs = (L.ntiles - 1) / L.per + 2;
+  // stages of 32 coordinates (32 KB), four where the query tile (up to 128 KB)
+  // leaves the room; never less than half an SM's shared memory, so that one
+  // CTA owns the SM's TMEM
+  L.kg = L.chunks < 4 ? L.chunks : 4;
+  const size_t query = static_cast<size_t>(2) * L.chunks * kQRows * 16;
+  const size_t stage = static_cast<size_t>(2) * L.kg * kBlockRows * 16;
+  L.stages = kMaxStages;
+  while (L.stages > 2 && query + L.stages * stage > kSmemLimit - kSharedRoom) --L.stages;
+  L.smem = query + L.stages * stage;
+  if (L.smem < 116 * 1024) L.smem = 116 * 1024;
   auto al = [](size_t v) { return (v + 255) / 256 * 256; };
   size_t o = 0;
-  L.o_xh = o; o = al(o + static_cast<size_t>(n) * L.dp * 2);
-  L.o_xl = o; o = al(o + static_cast<size_t>(n) * L.dp * 2);
-  L.o_nrm = o; o = al(o + static_cast<size_t>(n) * 4);
-  L.o_flags = o; o = al(o + 16);  // nrm_max, nonfinite, fb_count
-  L.o_cand = o; o = al(o + static_cast<size_t>(n) * m * 4);
-  L.o_canda = o; o = al(o + static_cast<size_t>(n) * m * 4);
-  L.o_bound = o; o = al(o + static_cast<size_t>(n) * L.segs * 4);
+  const size_t lists = static_cast<size_t>(L.qtiles) * kQRows * L.segs * 2;
+  L.o_xh = o; o = al(o + static_cast<size_t>(L.npos) * L.dp * 2);
+  L.o_xl = o; o = al(o + static_cast<size_t>(L.npos) * L.dp * 2);
+  L.o_cn = o; o = al(o + static_cast<size_t>(L.npos) * 4);
+  L.o_qn = o; o = al(o + static_cast<size_t>(L.npos) * 4);
+  L.o_status = o; o = al(o + 16);
+  L.o_xp = o; o = al(o + static_cast<size_t>(n) * L.d4 * 4);
+  L.o_cnt = o; o = al(o + lists * 4);
+  L.o_tau = o; o = al(o + lists * 4);
+  L.o_list = o; o = al(o + lists * L.cap * sizeof(float2));
   L.o_fb = o; o = al(o + static_cast<size_t>(n) * 4);
   L.o_brute = o; o = al(o + knn_bruteforce_scratch(n, K, segments));
   L.total = o;
   return L;
 }
 
-}  // namespace
+template <int P>
+cudaError_t launch_candidates(const SearchArgs& S, const TcLayout& L, cudaStream_t st) {
+  const cudaError_t e = cudaFuncSetAttribute(candidates_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             static_cast<int>(L.smem));
+  if (e != cudaSuccess) return e;
+  candidates_kernel<P><<<L.ctas, kThreads, L.smem, st>>>(S);
+  return cudaGetLastError();
+}
 
-size_t knn_tc_scratch(int n, int d, int K, int segments) { return tc_layout(n, d, K, segments).total; }
-
-int knn_tc_graph(const float* x, int n, int d, int K, int segments, void* scratch, int* idx, float* dist,
-                 cudaStream_t st) {
-  const TcLayout L = tc_layout(n, d, K, segments);
-  unsigned char* b = static_cast<unsigned char*>(scratch);
+int tc_search(const TcLayout& L, const float* x, int n, int d, int K, bool inner, int mode, const int* d_folds,
+              const int* perm, const int* off, const int2* skip, int segments, unsigned char* b, int* idx,
+              float* dist, cudaStream_t st) {
+  unsigned* status = reinterpret_cast<unsigned*>(b + L.o_status);
+  cudaError_t e = cudaMemsetAsync(status, 0, 16, st);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  // rows the re-rank can load as 16-byte vectors, or a padded copy of them
+  const bool in_place = d % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+  float* xp = in_place ? nullptr : reinterpret_cast<float*>(b + L.o_xp);
   uint16_t* xh = reinterpret_cast<uint16_t*>(b + L.o_xh);
   uint16_t* xl = reinterpret_cast<uint16_t*>(b + L.o_xl);
-  float* nrm = reinterpret_cast<float*>(b + L.o_nrm);
-  unsigned* flags = reinterpret_cast<unsigned*>(b + L.o_flags);  // [0] nrm_max bits, [1] nonfinite, [2] fallback count
-  int* cand = reinterpret_cast<int*>(b + L.o_cand);
-  float* cand_a = reinterpret_cast<float*>(b + L.o_canda);
-  float* bound = reinterpret_cast<float*>(b + L.o_bound);
+  float* cn = reinterpret_cast<float*>(b + L.o_cn);
+  float* qn = reinterpret_cast<float*>(b + L.o_qn);
   int* fb = reinterpret_cast<int*>(b + L.o_fb);
-  cudaError_t e = cudaMemsetAsync(flags, 0, 16, st);
+  prep_kernel<<<L.npos / 32, 256, 0, st>>>(x, n, d, L.chunks, L.npos, perm, inner ? 1 : 0, xh, xl, cn, qn, xp, L.d4,
+                                          status);
+  SearchArgs S{};
+  S.xh = xh;
+  S.xl = xl;
+  S.cn = cn;
+  S.qn = qn;
+  S.status = status;
+  S.chunks = L.chunks;
+  S.kg = L.kg;
+  S.stages = L.stages;
+  S.ntiles = L.ntiles;
+  S.qtiles = L.qtiles;
+  S.Kq = L.Kq;
+  S.cap = L.cap;
+  S.scale = inner ? -1.0f : -2.0f;
+  S.crel = 1.5e-5f + 1e-6f * static_cast<float>(L.dp);
+  S.inner = inner ? 1 : 0;
+  S.off = off;
+  S.skip = skip;
+  S.pairs = L.pairs;
+  S.per = L.per;
+  S.segs = L.segs;
+  S.list = reinterpret_cast<float2*>(b + L.o_list);
+  S.cnt = reinterpret_cast<int*>(b + L.o_cnt);
+  S.tau = reinterpret_cast<float*>(b + L.o_tau);
+  e = L.cap == 128   ? launch_candidates<4>(S, L, st)
+      : L.cap == 256 ? launch_candidates<8>(S, L, st)
+                     : launch_candidates<16>(S, L, st);
   if (e != cudaSuccess) return static_cast<int>(e);
-  tc_prep_kernel<<<(n + 127) / 128, 128, 0, st>>>(x, n, d, L.dp, xh, xl, nrm, flags,
-                                                 reinterpret_cast<int*>(flags + 1));
-  TcArgs A{};
-  A.xh = xh;
-  A.xl = xl;
-  A.nrm = nrm;
-  A.n = n;
-  A.dp = L.dp;
-  A.kp = L.kp;
-  A.segs = L.segs;
-  A.row_words = L.rw;
-  A.cand = cand;
-  A.cand_a = cand_a;
-  A.bound = bound;
-  const size_t smem = tc_smem_bytes(L.rw, L.kp, L.dp);
-  const dim3 grid((n + kTcQ - 1) / kTcQ, L.segs);
-  if (L.dp <= 64) {
-    e = cudaFuncSetAttribute(tc_candidates_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem));
-    if (e != cudaSuccess) return static_cast<int>(e);
-    tc_candidates_kernel<4><<<grid, 32 * kTcWarps, smem, st>>>(A);
-  } else if (L.dp <= 16 * kTcRegKs) {
-    e = cudaFuncSetAttribute(tc_candidates_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem));
-    if (e != cudaSuccess) return static_cast<int>(e);
-    tc_candidates_kernel<8><<<grid, 32 * kTcWarps, smem, st>>>(A);
-  } else {
-    e = cudaFuncSetAttribute(tc_candidates_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem));
-    if (e != cudaSuccess) return static_cast<int>(e);
-    tc_candidates_kernel<16><<<grid, 32 * kTcWarps, smem, st>>>(A);
-  }
-  const float crel = 1e-4f + 2e-6f * static_cast<float>(L.dp);
-  tc_rerank_kernel<<<(n + 3) / 4, 128, 0, st>>>(x, n, d, K, L.segs * 2 * L.kp, L.segs, cand, cand_a, bound, nrm,
-                                                 flags, reinterpret_cast<const int*>(flags + 1), crel, idx, dist, fb,
-                                                 reinterpret_cast<int*>(flags + 2));
+  RerankArgs R{};
+  R.s = S;
+  R.x = in_place ? x : xp;
+  R.d = d;
+  R.d4 = L.d4;
+  R.K = K;
+  R.npos = perm != nullptr ? L.npos : n;
+  R.mode = mode;
+  R.perm = perm;
+  R.idx = idx;
+  R.dist = dist;
+  R.fb_rows = fb;
+  rerank_kernel<<<(R.npos + 3) / 4, 128, 0, st>>>(R);
   count_launch(3);
   e = cudaGetLastError();
   if (e != cudaSuccess) return static_cast<int>(e);
-  return knn_bruteforce_rows(x, n, d, K, segments, fb, reinterpret_cast<const int*>(flags + 2), b + L.o_brute, idx,
-                             dist, st);
+  return knn_bruteforce_rows(x, n, d, K, inner, d_folds, mode, segments, fb,
+                             reinterpret_cast<const int*>(status + kStFallback), b + L.o_brute, idx, dist, st);
 }
 
-int knn_tc_fallback_count(const void* scratch, int n, int d, int K, int segments, int* out, cudaStream_t st) {
-  const TcLayout L = tc_layout(n, d, K, segments);
+}  // namespace
+
+bool knn_tc_supported(int n, int d, int K) {
+  return d >= 1 && d <= kMaxDp && K >= 1 && K + 1 <= 224 && n >= kMinRows && n > K;
+}
+
+bool knn_tc_explicit(int n, int d, int K) {
+  const int heaps = 2 * (K <= 40 ? 8 : 4);
+  int kp = (2 * ((K + heaps - 1) / heaps) + 15) / 8 * 8;
+  kp = kp < 16 ? 16 : kp;
+  return d >= 1 && d <= kMaxDp && K >= 1 && K <= 96 && n > 2 * kp + 64;
+}
+
+size_t knn_tc_scratch(int n, int d, int K, int segments, int sms, const KnnFoldPlan* fp) {
+  return tc_layout(n, d, K, segments, sms, fp).total;
+}
+
+int knn_tc_graph(const float* x, int n, int d, int K, int metric, int segments, int sms, void* scratch, int* idx,
+                 float* dist, cudaStream_t st) {
+  const TcLayout L = tc_layout(n, d, K, segments, sms, nullptr);
+  const int mode = metric == 2 ? kKnnOutSqrt : metric == 0 ? kKnnOutCosine : kKnnOutInner;
+  return tc_search(L, x, n, d, K, metric != 2, mode, nullptr, nullptr, nullptr, nullptr, segments,
+                   static_cast<unsigned char*>(scratch), idx, dist, st);
+}
+
+int knn_tc_fallback_count(const void* scratch, int n, int d, int K, int segments, int sms, int* out,
+                          cudaStream_t st) {
+  const TcLayout L = tc_layout(n, d, K, segments, sms, nullptr);
   const unsigned char* b = static_cast<const unsigned char*>(scratch);
-  return static_cast<int>(cudaMemcpyAsync(out, b + L.o_flags + 8, sizeof(int), cudaMemcpyDeviceToHost, st));
+  return static_cast<int>(
+      cudaMemcpyAsync(out, b + L.o_status + 4 * kStFallback, sizeof(int), cudaMemcpyDeviceToHost, st));
+}
+
+KnnFoldPlan knn_fold_plan(const std::vector<int>& folds) {
+  KnnFoldPlan p;
+  const int n = static_cast<int>(folds.size());
+  std::map<int, std::vector<int>> members;
+  for (int i = 0; i < n; ++i) members[folds[i]].push_back(i);
+  for (const auto& kv : members) p.tiles += static_cast<int>((kv.second.size() + kBlockRows - 1) / kBlockRows);
+  for (const auto& kv : members) {
+    const int size = static_cast<int>(kv.second.size());
+    const int first = static_cast<int>(p.perm.size()) / kBlockRows, own = (size + kBlockRows - 1) / kBlockRows;
+    p.perm.insert(p.perm.end(), kv.second.begin(), kv.second.end());
+    p.perm.resize(static_cast<size_t>(first + own) * kBlockRows, -1);
+    for (int q = 0; q < 2 * own; ++q) {
+      const bool rows = q * kQRows < size;  // a query tile of padding alone has no pairs
+      p.off.push_back(p.pairs);
+      p.skip.push_back(rows ? first : 0);
+      p.skip.push_back(rows ? own : p.tiles);
+      if (rows) p.pairs += p.tiles - own;
+    }
+  }
+  return p;
+}
+
+int knn_tc_fold_search(const float* x, int n, int d, int K, bool inner, const int* d_folds, const KnnFoldPlan& fp,
+                       const int* d_perm, const int* d_off, const int* d_skip, int segments, int sms, void* scratch,
+                       int* idx, float* dist, cudaStream_t st) {
+  const TcLayout L = tc_layout(n, d, K, segments, sms, &fp);
+  return tc_search(L, x, n, d, K, inner, kKnnOutRaw, d_folds, d_perm, d_off, reinterpret_cast<const int2*>(d_skip),
+                   segments, static_cast<unsigned char*>(scratch), idx, dist, st);
 }
 
 }  // namespace kgb
