@@ -6,7 +6,7 @@
 // the rows of other folds:
 //
 //  1. prep: every row is split once into bfloat16 hi + lo parts
-//     (x = hi + lo + r, |r| <= 2^-18 |x|), stored in blocks of 256 rows as
+//     (x = hi + lo + r, |r| <= 2^-16 |x|), stored in blocks of 256 rows as
 //     [chunk of 8 coordinates][row], the layout the tensor core reads, so that
 //     a tile is one contiguous copy;
 //  2. candidates: a persistent CTA per SM multiplies 128 queries with tiles of
@@ -27,12 +27,12 @@
 // values, or lie outside the value range below go to the brute force.
 //
 // Error bound (u = 2^-24), N = |q|^2 + |c|^2: the split drops at most
-// 3.01 * 2^-18 sum|q_i c_i|; 3 dp accumulated products, allowed two ulps each,
+// 3.1 * 2^-16 sum|q_i c_i|; 3 dp accumulated products, allowed two ulps each,
 // add 3 dp 2^-22 sum|q_i c_i|; twice their sum is at most N times that for L2
 // (sum|q_i c_i| <= |q||c|), and |q||c| times that for inner products.  The
 // canonical chain adds 2 (d + 4) u N, the float norms and the last fma
-// (d + 4) u N.  delta = N crel, crel = 1.5e-5 + 1e-6 dp, covers the sum
-// (1.2e-5 + 7.2e-7 dp + 1.8e-7 (d + 4)).  The rows that matter lie within
+// (d + 4) u N.  delta = N crel, crel = 5e-5 + 1e-6 dp, covers the sum
+// (4.8e-5 + 7.2e-7 dp + 1.8e-7 (d + 4)).  The rows that matter lie within
 // R = sqrt(A + |q|^2 + 2 delta_max) of the query, so |c| <= |q| + R replaces
 // the largest norm of the data there; delta falls with A, so an earlier
 // threshold is never below a later one.  Norms outside [1e-20, 1e36] (or
@@ -852,7 +852,7 @@ int tc_search(const TcLayout& L, const float* x, int n, int d, int K, bool inner
   S.Kq = L.Kq;
   S.cap = L.cap;
   S.scale = inner ? -1.0f : -2.0f;
-  S.crel = 1.5e-5f + 1e-6f * static_cast<float>(L.dp);
+  S.crel = 5e-5f + 1e-6f * static_cast<float>(L.dp);
   S.inner = inner ? 1 : 0;
   S.off = off;
   S.skip = skip;
