@@ -438,12 +438,17 @@ void constrained_majority(int* labels, const int* groups, size_t n) {
   for (size_t i = 0; i < n; ++i) labels[i] = lab[groups[i]];
 }
 
-// Status word of the device landmark planning (plan.cu): non-zero when the
-// atlas labels or the quota allocation were inconsistent.
+// Status word of the device k-means and landmark planning: 2 when a wait of the
+// k-means ran out (kmeans.cu), else non-zero when the atlas labels or the quota
+// allocation were inconsistent (plan.cu).
+void check_plan_status_value(int v) {
+  if (v == 2) fail(KGB_ETIMEOUT, "a wait inside the k-means kernel ran out");
+  if (v != 0) fail(KGB_EINTERNAL, "Landmark quota allocation produced the wrong sample size.");
+}
 void check_plan_status(const int* d_status) {
   int v = 0;
   ck(cudaMemcpy(&v, d_status, sizeof(int), cudaMemcpyDeviceToHost), "D2H");
-  if (v != 0) fail(KGB_EINTERNAL, "Landmark quota allocation produced the wrong sample size.");
+  check_plan_status_value(v);
 }
 
 int host_threads(int requested) {
@@ -1057,8 +1062,9 @@ void tc_kmeans_inputs(Ctx& ctx, kgb::KMeansBatch& B, const float* d_x, int n, in
   B.xh = split.xh;
   B.xl = split.xl;
   B.dp = split.dp;
-  B.ch = ctx.alloc<uint16_t>(static_cast<size_t>(B.problems) * B.k * split.dp);
-  B.cl = ctx.alloc<uint16_t>(static_cast<size_t>(B.problems) * B.k * split.dp);
+  const size_t rows = static_cast<size_t>(B.problems) * B.n;
+  B.multi = ctx.alloc<int4>(rows);
+  B.multi_mask = ctx.alloc<uint32_t>(rows * kgb::kmeans_mask_words(B.k) + 16);
 }
 
 // Host side of one KODAMA.matrix call between its enqueue and its finalize:
@@ -1133,6 +1139,8 @@ void matrix_from_device_graph(Ctx& ctx, const float* d_x, int n, int d, int* d_g
   const std::vector<float> split_u = kgb::split_uniforms(kmax);
   float* d_split = ctx.upload(split_u.data(), split_u.size());
   int* d_atlas_labels = ctx.alloc<int>(n);
+  int* d_plan_status = ctx.alloc<int>(1);
+  ck(cudaMemsetAsync(d_plan_status, 0, sizeof(int), st), "memset");
   {
     kgb::KMeansBatch B{};
     B.problems = 1;
@@ -1155,6 +1163,7 @@ void matrix_from_device_graph(Ctx& ctx, const float* d_x, int n, int d, int* d_g
     B.members = ctx.alloc<int>(n);
     B.offsets = ctx.alloc<int>(ck_atlas + 1);
     B.fscratch = ctx.alloc<float>(3 * ck_atlas + 1);
+    B.status = d_plan_status;
     tc_kmeans_inputs(ctx, B, d_x, n, d, tc_split);
     ck_launch(kgb::kmeans_run(B, st), "atlas k-means");
   }
@@ -1177,10 +1186,8 @@ void matrix_from_device_graph(Ctx& ctx, const float* d_x, int n, int d, int* d_g
   int* d_nonland = pls && n > L ? ctx.alloc<int>(static_cast<size_t>(M) * (n - L)) : nullptr;
   int* d_plan_init = ctx.alloc<int>(static_cast<size_t>(M) * kk);
   uint64_t* d_land_hash = ctx.alloc<uint64_t>(M);
-  int* d_plan_status = ctx.alloc<int>(1);
   int* d_km_assign = nullptr;
   {
-    ck(cudaMemsetAsync(d_plan_status, 0, sizeof(int), st), "memset");
     kgb::PlanArgs pa;
     pa.n = n;
     pa.strata = coarse_k;
@@ -1263,6 +1270,7 @@ void matrix_from_device_graph(Ctx& ctx, const float* d_x, int n, int d, int* d_g
     B.members = ctx.alloc<int>(static_cast<size_t>(M) * L);
     B.offsets = ctx.alloc<int>(static_cast<size_t>(M) * (kk + 1));
     B.fscratch = ctx.alloc<float>(static_cast<size_t>(M) * (3 * kk + 1));
+    B.status = d_plan_status;
     tc_kmeans_inputs(ctx, B, d_x, n, d, tc_split);
     ck_launch(kgb::kmeans_run(B, st), "landmark k-means");
   }
@@ -1651,7 +1659,7 @@ void matrix_from_device_graph(Ctx& ctx, const float* d_x, int n, int d, int* d_g
 // Fills kgb_matrix_result from a completed call's tail (ctx null: no stage
 // timings, as for a captured batch).
 void matrix_finalize(Ctx* ctx, MatrixTail& t, kgb_matrix_result* out, Clock& clk) {
-  if (t.plan_status != 0) fail(KGB_EINTERNAL, "Landmark quota allocation produced the wrong sample size.");
+  check_plan_status_value(t.plan_status);
   for (size_t i = 0; i < t.pls_status.status.size(); ++i) pls_status_check(t.pls_status.status[i], t.pls_status.present[i]);
   const int M = t.M, T = t.T, n = t.n, K = t.K, L = t.L;
   if (t.res_stage != nullptr) std::memcpy(out->res, t.res_stage, t.res_bytes);

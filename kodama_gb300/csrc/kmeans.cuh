@@ -28,20 +28,23 @@ struct KMeansBatch {
   int* offsets;             // problems x (k+1) scratch: cluster offsets in members
   float* fscratch;          // problems x (3k+1) scratch for empty-cluster splitting
   // tensor-core assignment (kmeans_tc_supported): x split into bf16 hi / lo
-  // (bf16_split_rows, dp columns), scratch for the centroids' split; xh null =
-  // every distance computed exactly
+  // rows (bf16_split_rows, dp columns), room for the rows that need exact
+  // distances and their candidate masks; xh null = every distance computed
+  // exactly
   const uint16_t* xh;
   const uint16_t* xl;
   int dp;
-  uint16_t* ch;             // problems x k x dp
-  uint16_t* cl;
-  int tc_blocks;            // set by kmeans_run: 64-row blocks per CTA
+  int4* multi;              // problems x n
+  uint32_t* multi_mask;     // problems x n x kmeans_mask_words(k)
+  int* status;              // set to 2 when a bounded wait ran out
+  int tc_blocks;            // set by kmeans_run: 128-row tiles per CTA
   float tc_crel;            // set by kmeans_run: the error bound's factor
-  int tc_cent_smem;         // set by kmeans_run: fp32 centroids staged in shared memory (else read from L2)
 };
 
-// The tensor-core assignment applies (d <= 64, k <= 128).
+// The tensor-core assignment applies: d <= 256, k <= 512 and the centroids'
+// operand fits in shared memory beside the row ring.
 bool kmeans_tc_supported(int d, int k);
+size_t kmeans_mask_words(int k);
 
 size_t kmeans_sort_smem(int k);
 int kmeans_row_norms(const float* x, int n, int d, float* out, cudaStream_t st);

@@ -68,8 +68,7 @@ int knn_tc_fold_search(const float* x, int n, int d, int K, bool inner, const in
                        int* idx, float* dist, cudaStream_t st);
 
 // Rows of x (n x d) split into bfloat16 hi + lo parts (x = hi + lo + r,
-// |r| <= 2^-16 |x|), dp = d rounded up to 16, coordinates permuted inside
-// each 16-block so one lane's m16n8k16 fragment values are contiguous.
+// |r| <= 2^-16 |x|), n x dp each, dp = d rounded up to 16 with zeros.
 int bf16_split_rows(const float* x, int n, int d, int dp, uint16_t* xh, uint16_t* xl, cudaStream_t st);
 
 // Fold-wise search: for each row the K nearest rows of other folds (folds[n]),

@@ -60,6 +60,7 @@ constexpr int kQRows = 128;       // queries per tile (mma M = TMEM lanes)
 constexpr int kMaxDp = 256;
 constexpr int kThreads = 320;     // 8 epilogue warps, the copy warp, the mma warp
 constexpr int kMaxStages = 4;
+constexpr int kNormSlots = 8;     // candidate tiles whose additive terms are staged
 constexpr size_t kSmemLimit = 227 * 1024;
 constexpr float kDeltaFloor = 2e-35f;
 constexpr int kSurvivors = 512;   // joined list entries of a query in the re-rank
@@ -233,7 +234,8 @@ __device__ __forceinline__ int cut_list(float2* list, int m, int Kq, float nq, f
     e[t] = i < m ? list[i] : make_float2(INFINITY, 0.0f);
     v[t] = e[t].x;
   }
-  const float A = kth_bound<P>(v, Kq, Kq >> 4, 14);
+  // a quarter more than Kq values may stay: every bisection round is a reduction
+  const float A = kth_bound<P>(v, Kq, Kq >> 2, 14);
   const float lim = fminf(*tau, A + 2.0f * delta_of(A, nq, nmax, crel, inner));
   int left = 0;
   __syncwarp();
@@ -251,13 +253,13 @@ __device__ __forceinline__ int cut_list(float2* list, int m, int Kq, float nq, f
 
 struct SearchShared {
   uint64_t full[kMaxStages], empty[kMaxStages];
-  uint64_t afull[2], aempty[2], qfull, qempty;
+  uint64_t afull[2], aempty[2], qfull, qempty, nfull[kNormSlots];
   uint32_t tmem;
   int stop;
   unsigned long long tau[2][kQRows];  // (query tile, threshold) of every row, per group
 };
 
-constexpr size_t kSharedRoom = 2304;  // static shared memory of candidates_kernel
+constexpr size_t kSharedRoom = 2432;  // static shared memory of candidates_kernel
 static_assert(sizeof(SearchShared) <= kSharedRoom, "static shared memory");
 
 // What bounds it: the epilogue's issue slots (about 4 per value) and the list
@@ -266,19 +268,20 @@ static_assert(sizeof(SearchShared) <= kSharedRoom, "static shared memory");
 // accumulators (all 512 TMEM columns) let one group of four warps work on a
 // tile while the tensor core fills the other.  Against the mma.sync kernel with
 // per-lane heaps that this replaces, and its brute-force fallback rows:
-// 100000 x 50, K = 30: 24.8 + 9.7 -> 7.1 ms; against the brute force, which
+// 100000 x 50, K = 30: 24.8 + 9.7 -> 6.1 ms; against the brute force, which
 // took K > 96, inner products and the fold-wise searches: 20011 x 50, K = 100
-// 62.9 -> 1.0 ms; 12000 x 100 cosine, K = 30 38.3 -> 0.35 ms; 10000 x 50,
-// 10 folds, K = 10 1.5 -> 0.17 ms.
+// 62.9 -> 0.89 ms; 12000 x 100 cosine, K = 30 38.3 -> 0.3 ms; 10000 x 50,
+// 10 folds, K = 10 1.5 -> 0.16 ms.
 template <int P>
 __global__ void __launch_bounds__(kThreads, 1) candidates_kernel(SearchArgs A) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ SearchShared sh;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = tc5::warp_index(), lane = threadIdx.x & 31;
   const int first_pair = blockIdx.x * A.per, last_pair = min(A.pairs, first_pair + A.per);
   const uint32_t qbytes = static_cast<uint32_t>(A.chunks) * kQRows * 16;       // one of hi / lo
   const uint32_t sbytes = static_cast<uint32_t>(A.kg) * kBlockRows * 16;       // one of hi / lo of a stage
-  const uint32_t qs = tc5::smem_u32(smem), ss = qs + 2 * qbytes;
+  float* const norms = reinterpret_cast<float*>(smem);  // [slot][256]
+  const uint32_t qs = tc5::smem_u32(smem) + kNormSlots * kBlockRows * 4, ss = qs + 2 * qbytes;
   volatile int* stop = &sh.stop;
   if (threadIdx.x == 0) {
     for (int s = 0; s < A.stages; ++s) {
@@ -289,6 +292,7 @@ __global__ void __launch_bounds__(kThreads, 1) candidates_kernel(SearchArgs A) {
       tc5::mbar_init(tc5::smem_u32(&sh.afull[g]), 1);
       tc5::mbar_init(tc5::smem_u32(&sh.aempty[g]), 4);
     }
+    for (int g = 0; g < kNormSlots; ++g) tc5::mbar_init(tc5::smem_u32(&sh.nfull[g]), 1);
     tc5::mbar_init(tc5::smem_u32(&sh.qfull), 1);
     tc5::mbar_init(tc5::smem_u32(&sh.qempty), 1);
     tc5::mbar_fence_init();
@@ -299,7 +303,7 @@ __global__ void __launch_bounds__(kThreads, 1) candidates_kernel(SearchArgs A) {
   tc5::fence_before();
   __syncthreads();
   tc5::fence_after();
-  const uint32_t tmem = sh.tmem;
+  const uint32_t tmem = __shfl_sync(kFull, sh.tmem, 0);
 
   // first query tile of the range
   int q = 0;
@@ -321,7 +325,7 @@ __global__ void __launch_bounds__(kThreads, 1) candidates_kernel(SearchArgs A) {
       int stage = 0, qn = 0;
       uint32_t phase = 0;
       bool ok = true;
-      int issued = 0;
+      int issued = 0, it = 0;
       for (int pair = first_pair, qt = q; ok && pair < last_pair; ++qt) {
         const int o = A.off != nullptr ? A.off[qt] : qt * A.ntiles;
         const int2 sk = A.skip != nullptr ? A.skip[qt] : make_int2(0, 0);
@@ -345,6 +349,17 @@ __global__ void __launch_bounds__(kThreads, 1) candidates_kernel(SearchArgs A) {
           for (int c0 = 0; c0 < A.chunks; c0 += A.kg) {
             ok = tc5::mbar_wait(tc5::smem_u32(&sh.empty[stage]), phase ^ 1u, stop);
             if (!ok) break;
+            if (c0 == 0) {
+              // the tile's additive terms.  At most kMaxStages tiles are
+              // multiplied after the one whose stage was just freed, and a
+              // tile is multiplied once the tile two before it is read out, so
+              // the tile kNormSlots before this one is done with its slot
+              const uint32_t nb = tc5::smem_u32(&sh.nfull[it % kNormSlots]);
+              tc5::mbar_expect(nb, kBlockRows * 4);
+              tc5::bulk_load(tc5::smem_u32(norms + (it % kNormSlots) * kBlockRows),
+                             A.cn + static_cast<size_t>(tile) * kBlockRows, kBlockRows * 4, nb);
+              ++it;
+            }
             const int nc = min(A.kg, A.chunks - c0);
             const uint32_t bytes = static_cast<uint32_t>(nc) * kBlockRows * 16;
             const uint32_t bar = tc5::smem_u32(&sh.full[stage]), dst = ss + stage * 2 * sbytes;
@@ -368,58 +383,63 @@ __global__ void __launch_bounds__(kThreads, 1) candidates_kernel(SearchArgs A) {
           tc5::mbar_wait(tc5::smem_u32(&sh.full[s]), s < stage ? phase : phase ^ 1u, &zero);
         }
         if (qn > 0) tc5::mbar_wait(tc5::smem_u32(&sh.qfull), (qn - 1) & 1, &zero);
+        for (int i = it - min(it, kNormSlots); i < it; ++i)
+          tc5::mbar_wait(tc5::smem_u32(&sh.nfull[i % kNormSlots]), (i / kNormSlots) & 1, &zero);
       }
     }
   } else if (warp == 9) {
-    if (lane == 0) {
-      const uint32_t idesc = tc5::idesc_bf16(kQRows, kBlockRows);
-      int stage = 0, qn = 0, it = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int pair = first_pair, qt = q; ok && pair < last_pair; ++qt) {
-        const int o = A.off != nullptr ? A.off[qt] : qt * A.ntiles;
-        const int2 sk = A.skip != nullptr ? A.skip[qt] : make_int2(0, 0);
-        const int end = min(last_pair, o + A.ntiles - sk.y);
-        if (pair >= end) continue;
-        ok = tc5::mbar_wait(tc5::smem_u32(&sh.qfull), qn & 1, stop);
-        ++qn;
-        for (; ok && pair < end; ++pair, ++it) {
-          const int buf = it & 1;
-          ok = tc5::mbar_wait(tc5::smem_u32(&sh.aempty[buf]), ((it >> 1) & 1) ^ 1, stop);
+    const uint32_t idesc = tc5::idesc_bf16(kQRows, kBlockRows);
+    int stage = 0, qn = 0, it = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int pair = first_pair, qt = q; ok && pair < last_pair; ++qt) {
+      const int o = A.off != nullptr ? A.off[qt] : qt * A.ntiles;
+      const int2 sk = A.skip != nullptr ? A.skip[qt] : make_int2(0, 0);
+      const int end = min(last_pair, o + A.ntiles - sk.y);
+      if (pair >= end) continue;
+      ok = __all_sync(kFull, tc5::mbar_wait(tc5::smem_u32(&sh.qfull), qn & 1, stop));
+      ++qn;
+      for (; ok && pair < end; ++pair, ++it) {
+        const int buf = it & 1;
+        ok = __all_sync(kFull, tc5::mbar_wait(tc5::smem_u32(&sh.aempty[buf]), ((it >> 1) & 1) ^ 1, stop));
+        if (!ok) break;
+        tc5::fence_after();
+        const uint32_t dcol = tmem + buf * kBlockRows;
+        for (int c0 = 0; c0 < A.chunks; c0 += A.kg) {
+          ok = __all_sync(kFull, tc5::mbar_wait(tc5::smem_u32(&sh.full[stage]), phase, stop));
           if (!ok) break;
           tc5::fence_after();
-          const uint32_t dcol = tmem + buf * kBlockRows;
-          for (int c0 = 0; c0 < A.chunks; c0 += A.kg) {
-            ok = tc5::mbar_wait(tc5::smem_u32(&sh.full[stage]), phase, stop);
-            if (!ok) break;
-            tc5::fence_after();
-            const uint32_t bs = ss + stage * 2 * sbytes;
-            const int k1 = min(A.kg, A.chunks - c0) / 2;
-            for (int k = 0; k < k1; ++k) {
-              const uint32_t ao = static_cast<uint32_t>(c0 + 2 * k) * kQRows * 16;
-              const uint32_t bo = static_cast<uint32_t>(2 * k) * kBlockRows * 16;
-              const uint64_t ah = tc5::operand(qs + ao, kQRows), al = tc5::operand(qs + qbytes + ao, kQRows);
-              const uint64_t bh = tc5::operand(bs + bo, kBlockRows), bl = tc5::operand(bs + sbytes + bo, kBlockRows);
-              tc5::mma(dcol, ah, bh, idesc, c0 + k > 0);
-              tc5::mma(dcol, ah, bl, idesc, true);
-              tc5::mma(dcol, al, bh, idesc, true);
-            }
-            tc5::commit(tc5::smem_u32(&sh.empty[stage]));
-            if (++stage == A.stages) {
-              stage = 0;
-              phase ^= 1u;
-            }
+          // descriptors advance by whole 16-coordinate steps (their address
+          // field counts 16 bytes)
+          const uint32_t bs = ss + stage * 2 * sbytes, ao = static_cast<uint32_t>(c0) * kQRows * 16;
+          uint64_t ah = tc5::operand(qs + ao, kQRows), al = tc5::operand(qs + qbytes + ao, kQRows);
+          uint64_t bh = tc5::operand(bs, kBlockRows), bl = tc5::operand(bs + sbytes, kBlockRows);
+          const int k1 = min(A.kg, A.chunks - c0) / 2;
+#pragma unroll 2
+          for (int k = 0; k < k1; ++k) {
+            tc5::mma(dcol, ah, bh, idesc, c0 + k > 0);
+            tc5::mma(dcol, ah, bl, idesc, true);
+            tc5::mma(dcol, al, bh, idesc, true);
+            ah += 2 * kQRows;
+            al += 2 * kQRows;
+            bh += 2 * kBlockRows;
+            bl += 2 * kBlockRows;
           }
-          if (ok) tc5::commit(tc5::smem_u32(&sh.afull[buf]));
+          tc5::commit(tc5::smem_u32(&sh.empty[stage]));
+          if (++stage == A.stages) {
+            stage = 0;
+            phase ^= 1u;
+          }
         }
-        if (ok) tc5::commit(tc5::smem_u32(&sh.qempty));
+        if (ok) tc5::commit(tc5::smem_u32(&sh.afull[buf]));
       }
-      // on an early end the instructions still queued finish first
-      if (!ok) {
-        int zero = 0;
-        tc5::commit(tc5::smem_u32(&sh.qempty));
-        tc5::mbar_wait(tc5::smem_u32(&sh.qempty), qn > 0 ? (qn - 1) & 1 : 0, &zero);
-      }
+      if (ok) tc5::commit(tc5::smem_u32(&sh.qempty));
+    }
+    // on an early end the instructions still queued finish first
+    if (!ok) {
+      int zero = 0;
+      tc5::commit(tc5::smem_u32(&sh.qempty));
+      tc5::mbar_wait(tc5::smem_u32(&sh.qempty), qn > 0 ? (qn - 1) & 1 : 0, &zero);
     }
   } else {
     const int g = warp >> 2;                 // this warp's accumulator / tile parity
@@ -446,8 +466,9 @@ __global__ void __launch_bounds__(kThreads, 1) candidates_kernel(SearchArgs A) {
       for (; ok && pair < end; ++pair, ++it) {
         if ((it & 1) != g) continue;
         const int tile = ord.at(pair - o);
-        const float* cn = A.cn + static_cast<size_t>(tile) * kBlockRows;
-        ok = __all_sync(kFull, tc5::mbar_wait(tc5::smem_u32(&sh.afull[g]), (it >> 1) & 1, stop));
+        const float* cn = norms + (it % kNormSlots) * kBlockRows;
+        ok = tc5::mbar_wait(tc5::smem_u32(&sh.nfull[it % kNormSlots]), (it / kNormSlots) & 1, stop);
+        ok = __all_sync(kFull, ok && tc5::mbar_wait(tc5::smem_u32(&sh.afull[g]), (it >> 1) & 1, stop));
         if (!ok) break;
         tc5::fence_after();
         if (fresh) {
@@ -462,7 +483,7 @@ __global__ void __launch_bounds__(kThreads, 1) candidates_kernel(SearchArgs A) {
             tc5::load32(acc + c, v);
 #pragma unroll
             for (int i = 0; i < 32; i += 4) {
-              const float4 n4 = __ldg(reinterpret_cast<const float4*>(cn + c + i));
+              const float4 n4 = *reinterpret_cast<const float4*>(cn + c + i);
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
                 const float a = __fmaf_rn(v[i + e], A.scale, e == 0 ? n4.x : e == 1 ? n4.y : e == 2 ? n4.z : n4.w);
@@ -484,7 +505,7 @@ __global__ void __launch_bounds__(kThreads, 1) candidates_kernel(SearchArgs A) {
               tc5::load32(acc + c, v);
 #pragma unroll
               for (int i = 0; i < 32; i += 4) {
-                const float4 n4 = __ldg(reinterpret_cast<const float4*>(cn + c + i));
+                const float4 n4 = *reinterpret_cast<const float4*>(cn + c + i);
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
                   below += __fmaf_rn(v[i + e], A.scale, e == 0 ? n4.x : e == 1 ? n4.y : e == 2 ? n4.z : n4.w) <= mid;
@@ -513,7 +534,7 @@ __global__ void __launch_bounds__(kThreads, 1) candidates_kernel(SearchArgs A) {
           float m = INFINITY;
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
-            const float4 n4 = __ldg(reinterpret_cast<const float4*>(cn + c + i));
+            const float4 n4 = *reinterpret_cast<const float4*>(cn + c + i);
             v[i] = __fmaf_rn(v[i], A.scale, n4.x);
             v[i + 1] = __fmaf_rn(v[i + 1], A.scale, n4.y);
             v[i + 2] = __fmaf_rn(v[i + 2], A.scale, n4.z);
@@ -732,23 +753,36 @@ __global__ void __launch_bounds__(128) rerank_kernel(RerankArgs R) {
 
 }  // namespace
 
-__global__ void split_rows_kernel(const float* __restrict__ x, int n, int d, int dp, uint16_t* __restrict__ xh,
-                                  uint16_t* __restrict__ xl) {
+// a 16-byte chunk (8 coordinates) of a row per thread
+__global__ void split_rows_kernel(const float* __restrict__ x, int n, int d, int chunks, uint4* __restrict__ xh,
+                                  uint4* __restrict__ xl) {
   const size_t e = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e >= static_cast<size_t>(n) * dp) return;
-  const int r = static_cast<int>(e / dp), k = static_cast<int>(e % dp);
-  const float v = k < d ? x[static_cast<size_t>(r) * d + k] : 0.0f;
-  const uint32_t hb = bf16_bits(v);
-  const uint32_t lb = bf16_bits(__fsub_rn(v, __uint_as_float(hb << 16)));
-  const size_t o = static_cast<size_t>(r) * dp + perm16(k);
-  xh[o] = static_cast<uint16_t>(hb);
-  xl[o] = static_cast<uint16_t>(lb);
+  if (e >= static_cast<size_t>(n) * chunks) return;
+  const size_t r = e / chunks;
+  const int c = static_cast<int>(e % chunks);
+  uint32_t h[4], l[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint32_t hb[2], lb[2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const int k = 8 * c + 2 * q + s;
+      const float v = k < d ? x[r * d + k] : 0.0f;
+      hb[s] = bf16_bits(v);
+      lb[s] = bf16_bits(__fsub_rn(v, __uint_as_float(hb[s] << 16)));
+    }
+    h[q] = hb[0] | (hb[1] << 16);
+    l[q] = lb[0] | (lb[1] << 16);
+  }
+  xh[e] = make_uint4(h[0], h[1], h[2], h[3]);
+  xl[e] = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
 int bf16_split_rows(const float* x, int n, int d, int dp, uint16_t* xh, uint16_t* xl, cudaStream_t st) {
-  const size_t total = static_cast<size_t>(n) * dp;
+  const size_t total = static_cast<size_t>(n) * (dp / 8);
   if (total == 0) return 0;
-  split_rows_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, st>>>(x, n, d, dp, xh, xl);
+  split_rows_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, st>>>(
+      x, n, d, dp / 8, reinterpret_cast<uint4*>(xh), reinterpret_cast<uint4*>(xl));
   count_launch();
   return static_cast<int>(cudaGetLastError());
 }
@@ -789,7 +823,7 @@ TcLayout tc_layout(int n, int d, int K, int segments, int sms, const KnnFoldPlan
   // leaves the room; never less than half an SM's shared memory, so that one
   // CTA owns the SM's TMEM
   L.kg = L.chunks < 4 ? L.chunks : 4;
-  const size_t query = static_cast<size_t>(2) * L.chunks * kQRows * 16;
+  const size_t query = static_cast<size_t>(2) * L.chunks * kQRows * 16 + kNormSlots * kBlockRows * 4;
   const size_t stage = static_cast<size_t>(2) * L.kg * kBlockRows * 16;
   L.stages = kMaxStages;
   while (L.stages > 2 && query + L.stages * stage > kSmemLimit - kSharedRoom) --L.stages;

@@ -2,11 +2,17 @@
 // untiled bulk copies that stage their operands and the mbarriers between
 // them, shared by the distance kernels.
 //
-// Operand tiles sit in shared memory in the canonical K-major layout without
-// swizzle: 16-byte chunks of 8 bf16 coordinates, [chunk][row][8].  Eight rows
-// of one chunk are a 128-byte core matrix, so the descriptor's stride byte
-// offset (next 8 rows) is 128 and its leading byte offset (next chunk) is
-// rows x 16.  One instruction multiplies 16 coordinates = two chunks.
+// Operand tiles sit in shared memory in one of two K-major layouts; one
+// instruction multiplies 16 coordinates = two 16-byte chunks of 8 bf16.
+//   operand: no swizzle, [chunk][row][8].  Eight rows of one chunk are a
+//     128-byte core matrix, so the descriptor's stride byte offset (next 8
+//     rows) is 128 and its leading byte offset (next chunk) is rows x 16.  For
+//     tiles that arrive in this order (blocks prepared in memory, computed
+//     operands).
+//   operand128: 128-byte swizzle, [row][64 coordinates], chunk c of row r at
+//     (c ^ (r & 7)).  For gathered rows: the eight lanes that copy a row read
+//     one whole line and write all 32 banks.
+// Both feed an instruction at its full rate (128 x 256 x 16: 128 cycles).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -82,39 +88,70 @@ __device__ __forceinline__ uint64_t operand(uint32_t addr, uint32_t rows) {
          (static_cast<uint64_t>(128 >> 4) << 32) | (1ull << 46);
 }
 
+// ... of rows of 64 coordinates with the 128-byte swizzle; addr = the tile's
+// 1024-byte aligned start plus 32 bytes per 16 coordinates.
+__device__ __forceinline__ uint64_t operand128(uint32_t addr) {
+  return static_cast<uint64_t>((addr & 0x3ffffu) >> 4) | (1ull << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) |
+         (1ull << 46) | (2ull << 61);
+}
+
 // Instruction descriptor: bf16 x bf16 -> f32, both operands K-major.
 __device__ __forceinline__ constexpr uint32_t idesc_bf16(int m, int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) |
          (static_cast<uint32_t>(m >> 4) << 24);
 }
 
-// D (+)= A B^T over 16 coordinates; one thread issues it.
+// The warp's number as a value the compiler knows to be the same in all lanes.
+__device__ __forceinline__ int warp_index() {
+  return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
+}
+
+// D (+)= A B^T over 16 coordinates.  The whole warp calls it and one elected
+// lane issues: in warp-uniform code the descriptors stay in uniform registers,
+// while code of a single lane moves every operand into them, about 150 cycles a
+// product (128 x 64 x 16 takes 69).
 __device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate) {
   asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+      "{\n.reg .pred p, q;\nsetp.ne.b32 p, %4, 0;\nelect.sync _|q, 0xffffffff;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
       "l"(a), "l"(b), "r"(idesc), "r"(accumulate ? 1u : 0u)
       : "memory");
 }
-// The barrier is arrived at once every mma issued by this thread so far is done.
+// The barrier is arrived at once every product issued by this warp so far is
+// done (called by the whole warp, like mma).
 __device__ __forceinline__ void commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+  asm volatile(
+      "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar)
+      : "memory");
 }
 
-// 32 accumulator columns of the warp's 32 lanes (lane = row), one per register.
-__device__ __forceinline__ void load32(uint32_t addr, float (&v)[32]) {
-  uint32_t r[32];
+// 32 accumulator columns of the warp's 32 lanes (lane = row), one per register:
+// load32_start issues the load, load32_wait waits for every load issued so far.
+__device__ __forceinline__ void load32_start(uint32_t addr, float (&v)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
       "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,"
-      "%29,%30,%31}, [%32];\ntcgen05.wait::ld.sync.aligned;\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      "%29,%30,%31}, [%32];\n"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]),
+        "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(v[16]),
+        "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]), "=f"(v[24]),
+        "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
       : "r"(addr)
       : "memory");
-#pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void load32_wait(float (&v)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n"
+      : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]), "+f"(v[8]),
+        "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15]), "+f"(v[16]),
+        "+f"(v[17]), "+f"(v[18]), "+f"(v[19]), "+f"(v[20]), "+f"(v[21]), "+f"(v[22]), "+f"(v[23]), "+f"(v[24]),
+        "+f"(v[25]), "+f"(v[26]), "+f"(v[27]), "+f"(v[28]), "+f"(v[29]), "+f"(v[30]), "+f"(v[31])
+      :
+      : "memory");
+}
+__device__ __forceinline__ void load32(uint32_t addr, float (&v)[32]) {
+  load32_start(addr, v);
+  load32_wait(v);
 }
 
 __device__ __forceinline__ float min3(float a, float b, float c) {
