@@ -769,12 +769,13 @@ PlsBuffers pls_buffers(Ctx& ctx, const float* d_X, int R, int L, int p, const Pl
   a.train_idx = d_tidx;
   a.mean = ctx.alloc<float>(static_cast<size_t>(S) * p);
   a.sdev = ctx.alloc<float>(static_cast<size_t>(S) * p);
-  a.Z = ctx.alloc<float>(static_cast<size_t>(S) * L * p);
+  a.zp = (p + 7) / 8 * 8;
+  a.Z = ctx.alloc<float>(static_cast<size_t>(S) * L * a.zp);
   a.xsum = ctx.alloc<float>(static_cast<size_t>(S) * p);
   a.zexp = ctx.alloc<int>(static_cast<size_t>(S) * p);
   a.Xv = d_Xv;
   a.NV = NV;
-  a.Zv = d_Xv != nullptr ? ctx.alloc<float>(static_cast<size_t>(R) * NV * p) : nullptr;
+  a.Zv = d_Xv != nullptr ? ctx.alloc<float>(static_cast<size_t>(R) * NV * a.zp) : nullptr;
   a.gram = nullptr;
   ck_launch(kgb::pls_prepare(a, st), "PLS fold preparation");
 
@@ -789,6 +790,7 @@ PlsBuffers pls_buffers(Ctx& ctx, const float* d_X, int R, int L, int p, const Pl
   e.predict_mode = d_Xv != nullptr;
   e.s_in_smem = s_in_smem ? 1 : 0;
   e.tiles_after_s = 1;  // no fold Gram yet: every slice computes scores in the fit
+  e.zp = a.zp;
   e.Z = a.Z;
   e.xsum = a.xsum;
   e.zexp = a.zexp;
@@ -812,11 +814,13 @@ PlsBuffers pls_buffers(Ctx& ctx, const float* d_X, int R, int L, int p, const Pl
   e.pred = ctx.alloc<uint16_t>(static_cast<size_t>(R) * (e.predict_mode ? NV : L));
   e.eval_comp = ctx.alloc<int>(S);
   e.status = ctx.alloc<int>(S);
+  e.s_raw = ctx.alloc<float>(static_cast<size_t>(S) * p * C0max);
   e.s_scr = ctx.alloc<float>(static_cast<size_t>(S) * p * C0max);
-  e.W = ctx.alloc<float>(static_cast<size_t>(S) * p * max_components);
-  e.V = ctx.alloc<float>(static_cast<size_t>(S) * p * max_components);
   e.T = ctx.alloc<float>(static_cast<size_t>(S) * L * requested);
   e.Tt = ctx.alloc<float>(static_cast<size_t>(S) * L * requested);
+  e.Tv = e.predict_mode ? nullptr : ctx.alloc<float>(static_cast<size_t>(S) * L * requested);
+  e.Tp = e.predict_mode ? ctx.alloc<float>(static_cast<size_t>(R) * NV * requested) : nullptr;
+  e.tpos = ctx.alloc<uint16_t>(static_cast<size_t>(S) * L);
   e.pos = ctx.alloc<uint16_t>(static_cast<size_t>(S) * L);
   e.posok = ctx.alloc<uint8_t>(static_cast<size_t>(S) * L);
   e.sc = ctx.alloc<float>(static_cast<size_t>(S) * L);

@@ -27,6 +27,9 @@
 #include <float.h>
 #include <math.h>
 
+#include <algorithm>
+#include <type_traits>
+
 namespace kgb {
 
 namespace {
@@ -39,48 +42,74 @@ constexpr int kEvalWarps = kEvalThreads / 32;
 // Preparation (label independent)
 // ---------------------------------------------------------------------------
 
-// train_center_scale_float: one thread per (slice, column).
-__global__ void stats_kernel(PlsPrepArgs a) {
-  const int s = blockIdx.x, r = s / a.F;
-  const int j = blockIdx.y * blockDim.x + threadIdx.x;
-  if (j >= a.p) return;
+// The values of one column down the rows idx[0..n) of a row-major matrix
+// (stride ld), in order: each lane's column, 32 rows' loads in flight while the
+// 32 before them are taken.  A column is a serial float chain, so its time is
+// the loads' latency: with 8 loads in flight per thread and nothing overlapped
+// a chain over 1800 rows took about 150 us, here about 20.  Warp-collective;
+// lanes with !in read column 0.
+template <class Take>
+__device__ __forceinline__ void column_walk(const float* __restrict__ X, int ld, const int* __restrict__ idx, int n,
+                                            int j, bool in, int lane, Take&& take) {
+  if (n <= 0) return;
+  const float* xj = X + (in ? j : 0);
+  float va[32], vb[32];
+  auto rows = [&](int t) { return idx[min(t + lane, n - 1)]; };
+  auto fetch = [&](float (&v)[32], int ids) {
+#pragma unroll
+    for (int q = 0; q < 32; ++q) v[q] = xj[static_cast<size_t>(__shfl_sync(kFull, ids, q)) * ld];
+  };
+  auto use = [&](const float (&v)[32], int left) {
+    if (left >= 32) {
+#pragma unroll
+      for (int q = 0; q < 32; ++q) take(v[q]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 32; ++q)
+        if (q < left) take(v[q]);
+    }
+  };
+  int ids = rows(0);
+  fetch(va, ids);
+  ids = rows(32);
+  for (int t = 0; t < n; t += 64) {
+    const int id2 = rows(t + 64);
+    if (t + 32 < n) fetch(vb, ids);
+    use(va, n - t);
+    ids = rows(t + 96);
+    if (t + 64 < n) fetch(va, id2);
+    if (t + 32 < n) use(vb, n - t - 32);
+  }
+}
+
+// train_center_scale_float: a lane per (slice, column).
+__global__ void __launch_bounds__(64) stats_kernel(PlsPrepArgs a) {
+  const int s = blockIdx.x, r = s / a.F, lane = threadIdx.x & 31;
+  const int j = (blockIdx.y * 2 + (threadIdx.x >> 5)) * 32 + lane;
+  const bool in = j < a.p;
   const float* X = a.X + static_cast<size_t>(r) * a.L * a.p;
-  const int b = a.train_off[s], e = a.train_off[s + 1], nt = e - b;
-  const int* rows = a.train_idx;
+  const int b = a.train_off[s], nt = a.train_off[s + 1] - b;
+  const int* rows = a.train_idx + b;
   float m = 0.0f;
   if (a.center) {
-    for (int t = b; t < e; t += 8) {
-      float v[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) v[q] = t + q < e ? X[static_cast<size_t>(rows[t + q]) * a.p + j] : 0.0f;
-#pragma unroll
-      for (int q = 0; q < 8; ++q)
-        if (t + q < e) m = __fadd_rn(m, v[q]);
-    }
+    column_walk(X, a.p, rows, nt, j, in, lane, [&](float v) { m = __fadd_rn(m, v); });
     const float inv = nt == 0 ? 0.0f : __fdiv_rn(1.0f, static_cast<float>(nt));
     m = __fmul_rn(m, inv);
   }
   float sd = 1.0f;
   if (a.scale) {
     float acc = 1.0f;  // the reference's scale vector starts at 1
-    for (int t = b; t < e; t += 8) {
-      float v[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) v[q] = t + q < e ? X[static_cast<size_t>(rows[t + q]) * a.p + j] : 0.0f;
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        if (t + q < e) {
-          const float d = __fsub_rn(v[q], m);
-          acc = __fadd_rn(acc, __fmul_rn(d, d));
-        }
-      }
-    }
+    column_walk(X, a.p, rows, nt, j, in, lane, [&](float v) {
+      const float d = __fsub_rn(v, m);
+      acc = __fadd_rn(acc, __fmul_rn(d, d));
+    });
     // std::max(1.0f, float(rows.size() - 1)) with size_t arithmetic
     const float den1 = static_cast<float>(static_cast<unsigned long long>(nt) - 1ull);
     const float den = 1.0f < den1 ? den1 : 1.0f;
     const float q = __fsqrt_rn(__fdiv_rn(acc, den));
     sd = (q > 0.0f && isfinite(q)) ? q : 1.0f;
   }
+  if (!in) return;
   a.mean[static_cast<size_t>(s) * a.p + j] = m;
   a.sdev[static_cast<size_t>(s) * a.p + j] = sd;
 }
@@ -93,21 +122,21 @@ __global__ void standardize_kernel(PlsPrepArgs a) {
   const int S = a.problems * a.F, p = a.p;
   for (int s = blockIdx.y; s < S; s += gridDim.y) {
     const float* X = a.X + static_cast<size_t>(s / a.F) * a.L * p;
-    float* Z = a.Z + static_cast<size_t>(s) * a.L * p;
+    float* Z = a.Z + static_cast<size_t>(s) * a.L * a.zp;
     const float* mu = a.mean + static_cast<size_t>(s) * p;
     const float* sd = a.sdev + static_cast<size_t>(s) * p;
     for (int i = blockIdx.x; i < a.L; i += gridDim.x)
       for (int j = threadIdx.x; j < p; j += blockDim.x)
-        Z[static_cast<size_t>(i) * p + j] = __fdiv_rn(__fsub_rn(X[static_cast<size_t>(i) * p + j], mu[j]), sd[j]);
+        Z[static_cast<size_t>(i) * a.zp + j] = __fdiv_rn(__fsub_rn(X[static_cast<size_t>(i) * p + j], mu[j]), sd[j]);
   }
   if (a.Xv == nullptr) return;
   for (int r = blockIdx.y; r < a.problems; r += gridDim.y) {
     const size_t s = static_cast<size_t>(r) * a.F;
     const float* Xv = a.Xv + static_cast<size_t>(r) * a.NV * p;
-    float* Zv = a.Zv + static_cast<size_t>(r) * a.NV * p;
+    float* Zv = a.Zv + static_cast<size_t>(r) * a.NV * a.zp;
     for (int i = blockIdx.x; i < a.NV; i += gridDim.x)
       for (int j = threadIdx.x; j < p; j += blockDim.x)
-        Zv[static_cast<size_t>(i) * p + j] =
+        Zv[static_cast<size_t>(i) * a.zp + j] =
             __fdiv_rn(__fsub_rn(Xv[static_cast<size_t>(i) * p + j], a.mean[s * p + j]), a.sdev[s * p + j]);
   }
 }
@@ -119,25 +148,18 @@ __device__ __forceinline__ int biased_exp1(float v) {
 // Column sums of the standardised training rows in row order (the x_sum of
 // the cross-product, label independent), and each column's largest biased
 // exponent over those rows (the fixed-point bound of block_loading).
-__global__ void xsum_kernel(PlsPrepArgs a) {
-  const int s = blockIdx.x;
-  const int j = blockIdx.y * blockDim.x + threadIdx.x;
-  if (j >= a.p) return;
-  const float* Zs = a.Z + static_cast<size_t>(s) * a.L * a.p;
+__global__ void __launch_bounds__(64) xsum_kernel(PlsPrepArgs a) {
+  const int s = blockIdx.x, lane = threadIdx.x & 31;
+  const int j = (blockIdx.y * 2 + (threadIdx.x >> 5)) * 32 + lane;
+  const bool in = j < a.p;
   const int b = a.train_off[s], e = a.train_off[s + 1];
   float acc = 0.0f;
   int ze = 1;
-  for (int t = b; t < e; t += 8) {
-    float v[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) v[q] = t + q < e ? Zs[static_cast<size_t>(a.train_idx[t + q]) * a.p + j] : 0.0f;
-#pragma unroll
-    for (int q = 0; q < 8; ++q)
-      if (t + q < e) {
-        acc = __fadd_rn(acc, v[q]);
-        ze = max(ze, biased_exp1(v[q]));
-      }
-  }
+  column_walk(a.Z + static_cast<size_t>(s) * a.L * a.zp, a.zp, a.train_idx + b, e - b, j, in, lane, [&](float v) {
+    acc = __fadd_rn(acc, v);
+    ze = max(ze, biased_exp1(v));
+  });
+  if (!in) return;
   a.xsum[static_cast<size_t>(s) * a.p + j] = acc;
   a.zexp[static_cast<size_t>(s) * a.p + j] = ze;
 }
@@ -161,7 +183,7 @@ __global__ void __launch_bounds__(256) gram_kernel(PlsPrepArgs a, const uint8_t*
   __shared__ __align__(16) float zj[kGramR][kGramT];
   __shared__ __align__(16) float zk[kGramR][kGramT];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const float* Zs = a.Z + static_cast<size_t>(s) * a.L * a.p;
+  const float* Zs = a.Z + static_cast<size_t>(s) * a.L * a.zp;
   const int b = a.train_off[s], e = a.train_off[s + 1];
   float acc[4][4];
 #pragma unroll
@@ -173,8 +195,8 @@ __global__ void __launch_bounds__(256) gram_kernel(PlsPrepArgs a, const uint8_t*
       const int q = i / kGramT, c = i - q * kGramT;
       const int row = t0 + q < e ? a.train_idx[t0 + q] : -1;
       const int cj = jb * kGramT + c, ck = kb * kGramT + c;
-      zj[q][c] = (row >= 0 && cj < a.p) ? Zs[static_cast<size_t>(row) * a.p + cj] : 0.0f;
-      zk[q][c] = (row >= 0 && ck < a.p) ? Zs[static_cast<size_t>(row) * a.p + ck] : 0.0f;
+      zj[q][c] = (row >= 0 && cj < a.p) ? Zs[static_cast<size_t>(row) * a.zp + cj] : 0.0f;
+      zk[q][c] = (row >= 0 && ck < a.p) ? Zs[static_cast<size_t>(row) * a.zp + ck] : 0.0f;
     }
     __syncthreads();
     // rows of the tile past the last column hold no entry (warp-uniform: a
@@ -212,10 +234,11 @@ __global__ void __launch_bounds__(256) gram_kernel(PlsPrepArgs a, const uint8_t*
 
 constexpr int kMaxNC = 8;      // components per register pass over the rows
 constexpr int kMaxComp = 64;   // components of a fit held per row (local array)
-constexpr int kTile = 32 * 33; // per-warp transposing tile (floats)
+constexpr uint16_t kNoPos = 0xffffu;  // tpos of a validation row
+constexpr int kTile = 2 * 32 * 16;  // per-warp score tiles: two stages of 32 rows x 16 columns (floats)
 
 struct EvalShared {
-  int m, nt, stop, best, lab, fail;
+  int m, nt, stop, best, lab, fail, queue;
   float rn, inv;
 };
 
@@ -451,6 +474,75 @@ __device__ float warp_power_norm(const float* v, int n, int lane) {
   return power_norm2(warp_fma_chain(n, t, lane));
 }
 
+// One term of a two-float sum: the product and its fma remainder, Knuth's
+// two-sum, the remainders into lo; A: upper bound of the sum of magnitudes.
+__device__ __forceinline__ void two_float_add(float x, float y, float& hi, float& lo, float& A) {
+  const float q = __fmul_rn(x, y);
+  const float e = __fmaf_rn(x, y, -q);
+  const float t = __fadd_rn(hi, q);
+  const float z = __fsub_rn(t, hi);
+  const float r = __fadd_rn(__fsub_rn(hi, __fsub_rn(t, z)), __fsub_rn(q, z));
+  lo = __fadd_rn(lo, __fadd_rn(r, e));
+  A = __fadd_ru(A, fabsf(q));
+  hi = t;
+}
+
+// float(S_seq) for many dots at once: groups of eight lanes form a dot each,
+// dot it over terms 0..n-1.  S is formed in two floats by error-free steps
+// (product: x y and its fma remainder; sum: Knuth's two-sum), s + c with c the
+// rounded sum of the remainders.  With A an upper bound of sum |x y|, c holds
+// at most (2 nl + 6) roundings of values below u A (nl + 4), nl the terms of a
+// lane plus the three joins, and S_seq lies within n 2^-52 A of S (above);
+// remainders lost to underflow add n 2^-148.  If both ends of that interval
+// round to the same float, float(S_seq) is that float; else the warp forms the
+// dot as warp_seq_dot does.  About 12 instructions a term in one pass, where
+// the fixed-point form takes 37 in two, and three joins instead of five.
+template <class Load, class Put>
+__device__ __forceinline__ void group_seq_dots(int dots, int n, int lane, int warp, Load&& load, Put&& put) {
+  const int gl = lane & 7, g = lane >> 3;
+  const float nl = static_cast<float>((n + 7) / 8 + 3);
+  const float unit = 3.5527137e-15f;  // 2^-48
+  const float K = (2.0f * nl + 6.0f) * (nl + 4.0f) * 1.1f + static_cast<float>(n) * 0.0625f + 1.0f;
+  for (int d0 = warp * 4; d0 < dots; d0 += kEvalWarps * 4) {
+    const int d = d0 + g;
+    float s = 0.0f, c = 0.0f, A = 0.0f;
+    if (d < dots) {
+#pragma unroll 4
+      for (int k = gl; k < n; k += 8) {
+        float x, y;
+        load(d, k, x, y);
+        two_float_add(x, y, s, c, A);
+      }
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+      const float q = __shfl_xor_sync(kFull, s, o);
+      const float t = __fadd_rn(s, q);
+      // the two lanes join the same pair in either order: two-sum is exact, so
+      // both hold the same value
+      const float z = __fsub_rn(t, s);
+      const float r = __fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(q, z));
+      c = __fadd_rn(__fadd_rn(c, __shfl_xor_sync(kFull, c, o)), r);
+      A = __fadd_ru(A, __shfl_xor_sync(kFull, A, o));
+      s = t;
+    }
+    const float f = __fadd_rn(s, c);
+    const float z = __fsub_rn(f, s);
+    const float r = __fadd_rn(__fsub_rn(s, __fsub_rn(f, z)), __fsub_rn(c, z));
+    const float err = __fadd_ru(__fmul_ru(__fmul_ru(A, 1.0001f), __fmul_ru(K, unit)),
+                                __fmul_ru(static_cast<float>(n), 2.8e-45f));
+    const bool ok = A > 0.0f && __fadd_rn(f, __fadd_ru(r, err)) == f && __fadd_rn(f, __fadd_rd(r, -err)) == f;
+    if (d < dots && gl == 0 && ok) put(d, f);
+    unsigned left = __ballot_sync(kFull, d < dots && gl == 0 && !ok);
+    while (left != 0u) {
+      const int df = d0 + ((__ffs(left) - 1) >> 3);
+      left &= left - 1u;
+      const float v = warp_seq_dot(n, [&](int k, float& x, float& y) { load(df, k, x, y); }, lane);
+      if (lane == 0) put(df, v);
+    }
+  }
+}
+
 // loading[j] = float(S_seq) of sum over training rows k (ascending) of
 // double(Z[tix[k]][j]) * double(sc[k]), for every column j: t_mat_vec_float
 // of the scores path (plscv.cpp:884).  A thread per column and row group, so
@@ -466,12 +558,69 @@ __device__ float warp_power_norm(const float* v, int n, int lane) {
 // 4 * kEvalThreads + 2 * kLoadChunk words plus 8 bytes of alignment; every
 // thread of the block calls this.
 constexpr int kLoadChunk = 1024;
-__device__ void block_loading(const float* __restrict__ Zs, int p, const int* __restrict__ tix, int nt,
+
+// v as a multiple of 2^LSB (truncated below it)
+__device__ __forceinline__ long long exact_fixed_value(float v, int LSB) {
+  const unsigned u = __float_as_uint(v), b = (u >> 23) & 0xffu;
+  const long long m = (u & 0x7fffffu) | (b ? 0x800000u : 0u);
+  const int sh = (b ? static_cast<int>(b) - 150 : -149) - LSB;
+  const long long f = sh >= 0 ? (sh < 63 ? m << sh : 0ll) : (sh > -64 ? m >> -sh : 0ll);
+  return (u >> 31) ? -f : f;
+}
+
+// float(S_seq) of sum sc[t]^2 over t < n, by the whole block: the sums of
+// eight terms as above.  `red` holds 2 kEvalWarps words plus alignment.
+__device__ float block_norm2(const float* __restrict__ sc, int n, void* scratch, int lane, int warp) {
+  long long* vred = reinterpret_cast<long long*>((reinterpret_cast<uintptr_t>(scratch) + 7) & ~uintptr_t(7));
+  float* ared = reinterpret_cast<float*>(vred + kEvalWarps);
+  int* mred = reinterpret_cast<int*>(ared + kEvalWarps);
+  int mx = 1;
+  for (int t = threadIdx.x; t < n; t += kEvalThreads) mx = max(mx, biased_exp1(sc[t]));
+  mx = __reduce_max_sync(kFull, mx);
+  if (lane == 0) mred[warp] = mx;
+  __syncthreads();
+  mx = __reduce_max_sync(kFull, mred[lane & (kEvalWarps - 1)]);
+  const int LSB = 2 * mx - 252 + clog2i(n) - 62;
+  long long acc = 0;
+  float A = 0.0f;
+  for (int t0 = threadIdx.x; t0 < n; t0 += 8 * kEvalThreads) {
+    float v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = t0 + q * kEvalThreads < n ? sc[t0 + q * kEvalThreads] : 0.0f;
+    float hi = 0.0f, lo = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) two_float_add(v[q], v[q], hi, lo, A);
+    acc += exact_fixed_value(hi, LSB) + exact_fixed_value(lo, LSB);
+  }
+  acc = warp_sum_i64(acc);
+  A = warp_sum_ru(A);
+  if (lane == 0) {
+    vred[warp] = acc;
+    ared[warp] = A;
+  }
+  __syncthreads();
+  acc = 0;
+  A = 0.0f;
+  for (int q = 0; q < kEvalWarps; ++q) {
+    acc += vred[q];
+    A = __fadd_ru(A, ared[q]);
+  }
+  float out = 0.0f;
+  if (!(A > 0.0f && A < 1e37f && round_check(acc, LSB, __fmul_ru(A, 1.0001f), n + 2880, out)))
+    out = warp_seq_dot(n, [&](int k, float& x, float& y) {
+      x = sc[k];
+      y = sc[k];
+    }, lane);
+  __syncthreads();
+  return out;
+}
+
+__device__ void block_loading(const float* __restrict__ Zs, int zp, int p, const int* __restrict__ tix, int nt,
                               const float* __restrict__ sc, const int* __restrict__ zexp, float* ld, float* scratch,
                               int lane, int warp) {
   long long* pacc = reinterpret_cast<long long*>((reinterpret_cast<uintptr_t>(scratch) + 7) & ~uintptr_t(7));
   float* pA = reinterpret_cast<float*>(pacc + kEvalThreads);
-  int* pflag = reinterpret_cast<int*>(pA + kEvalThreads);  // bit 0: non-finite, bit 1: a nonzero term
+  int* pflag = reinterpret_cast<int*>(pA + kEvalThreads);  // non-zero values seen
   int* srow = pflag + kEvalThreads;
   float* ssc = reinterpret_cast<float*>(srow + kLoadChunk);
   int* flist = reinterpret_cast<int*>(pacc);  // undecided columns (after the partials are read)
@@ -494,7 +643,7 @@ __device__ void block_loading(const float* __restrict__ Zs, int p, const int* __
     const int LSB = (on ? zexp[j] : 1) + se - 252 + lg - 62;
     long long acc = 0;
     float A = 0.0f;
-    int bad = 0, nz = 0;
+    unsigned nz = 0u;
     for (int k0 = 0; k0 < nt; k0 += kLoadChunk) {
       const int cn = min(kLoadChunk, nt - k0);
       for (int i = t; i < cn; i += kEvalThreads) {
@@ -503,14 +652,31 @@ __device__ void block_loading(const float* __restrict__ Zs, int p, const int* __
       }
       __syncthreads();
       if (on) {
-#pragma unroll 8
-        for (int i = g; i < cn; i += G) {
-          const float x = Zs[static_cast<size_t>(srow[i]) * p + j], y = ssc[i];
-          const unsigned ux = __float_as_uint(x), uy = __float_as_uint(y);
-          bad |= (((ux >> 23) & 0xffu) == 0xffu) | (((uy >> 23) & 0xffu) == 0xffu);
-          nz |= ((ux << 1) != 0u) & ((uy << 1) != 0u);
-          A = __fadd_ru(A, __fmul_ru(fabsf(x), fabsf(y)));
-          acc += exact_fixed_term(x, y, LSB);
+        // the next eight rows' values load while these eight are added
+        float nx[8];
+        auto fetch = [&](int i0) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const int i = i0 + q * G;
+            nx[q] = i < cn ? Zs[static_cast<size_t>(srow[i]) * zp + j] : 0.0f;
+          }
+        };
+        fetch(g);
+        for (int i0 = g; i0 < cn; i0 += 8 * G) {
+          float v[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) v[q] = nx[q];
+          fetch(i0 + 8 * G);
+          // eight terms in two floats (group_seq_dots), then as fixed point
+          float hi = 0.0f, lo = 0.0f;
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const int i = i0 + q * G;
+            const float y = i < cn ? ssc[i] : 0.0f;
+            two_float_add(v[q], y, hi, lo, A);
+            nz |= __float_as_uint(v[q]);
+          }
+          acc += exact_fixed_value(hi, LSB) + exact_fixed_value(lo, LSB);
         }
       }
       __syncthreads();
@@ -518,7 +684,7 @@ __device__ void block_loading(const float* __restrict__ Zs, int p, const int* __
     if (on) {
       pacc[t] = acc;
       pA[t] = A;
-      pflag[t] = bad | (nz << 1);
+      pflag[t] = static_cast<int>(nz << 1);
     }
     __syncthreads();
     float out = 0.0f;
@@ -530,7 +696,11 @@ __device__ void block_loading(const float* __restrict__ Zs, int p, const int* __
         A = __fadd_ru(A, pA[t + q * PB]);
         fl |= pflag[t + q * PB];
       }
-      if (!(fl & 1)) ok = (fl & 2) ? round_check(acc, LSB, A, nt, out) : (out = 0.0f, true);
+      // a column of zeros; else the check, which counts the roundings of the
+      // eight-term sums (below 180 u^2 A) as 16 x 180 terms more; A is not
+      // finite where a value is not, and zero where products were lost
+      if (fl == 0) ok = true;
+      else if (A > 0.0f && A < 1e37f) ok = round_check(acc, LSB, __fmul_ru(A, 1.0001f), nt + 2880, out);
     }
     if (t == 0) fcount = 0;
     __syncthreads();
@@ -543,7 +713,7 @@ __device__ void block_loading(const float* __restrict__ Zs, int p, const int* __
     for (int f = warp; f < nf; f += kEvalWarps) {
       const int jf = flist[f];
       const double s = warp_fma_chain(nt, [&](int k, float& x, float& y) {
-        x = Zs[static_cast<size_t>(tix[k]) * p + jf];
+        x = Zs[static_cast<size_t>(tix[k]) * zp + jf];
         y = sc[k];
       }, lane);
       if (lane == 0) ld[jf] = __double2float_rn(s);
@@ -552,32 +722,143 @@ __device__ void block_loading(const float* __restrict__ Zs, int p, const int* __
   }
 }
 
-// Scores of 32 rows (one per lane; row < 0 = none) for components
-// q0 .. q0+nq-1 (nq <= kMaxNC): acc[q] = sum over features in order of
-// z(row, j) * W(j, q0+q).  The rows come in through the warp's transposing
-// tile with 128-byte loads.
-__device__ __forceinline__ void warp_scores(const float* __restrict__ base, int p, int myrow, const float* W, int ldw,
-                                            int q0, int nq, float* tile, int lane, float* acc) {
+__device__ __forceinline__ void cp_async16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                   static_cast<unsigned>(__cvta_generic_to_shared(dst))),
+               "l"(src));
+}
+
+// Scores of all rows of a row-major matrix (zp floats apart, zp a multiple of
+// 4, 16-byte aligned) for components q0 .. q0 + NQ - 1: out(row, acc) with
+// acc[q] = sum over features in order of z(row, j) * W(j, q0 + q), every product
+// and sum rounded on its own.  A warp takes 32 rows, a lane each; 16 columns at
+// a time come in with cp.async, the next 16 while these are used.  The rows
+// are read in memory order, validation rows too: their scores are needed for
+// the predictions anyway, and no row waits for an index.  Column chunks sit at
+// (chunk ^ (row / 2 & 3)), so the lanes' 16-byte reads hit all banks.
+// With 128-byte loads of 32 indexed rows into a padded transposing tile, eight
+// in flight, this phase was 42% of an evaluation at 6750 x 200 rows, 5
+// components (3.4 M cycles a slice; here 0.7 M).
+// The batches are dealt to the first `warps` warps; tick() follows every batch of
+// a warp.
+template <int NQ, class Out, class Tick>
+__device__ __forceinline__ void stream_scores(const float* __restrict__ base, int zp, int p, int nrows, const float* W,
+                                              int ldw, int q0, float* tile, int lane, int warp, int warps, Out&& out,
+                                              Tick&& tick) {
+  const int nblk = (p + 15) / 16, nb = (nrows + 31) / 32;
+  const int mine = warp < nb ? (nb - warp + warps - 1) / warps : 0;
+  const int steps = mine * nblk;
+  int lb = warp, lk = 0;  // batch and column block of the next load
+  auto load = [&](int step) {
+    if (step < steps) {
 #pragma unroll
-  for (int q = 0; q < kMaxNC; ++q) acc[q] = 0.0f;
-  for (int j0 = 0; j0 < p; j0 += 32) {
-    const int jl = j0 + lane;
-#pragma unroll 8
-    for (int i = 0; i < 32; ++i) {
-      const int ri = __shfl_sync(kFull, myrow, i);
-      tile[i * 33 + lane] = (ri >= 0 && jl < p) ? base[static_cast<size_t>(ri) * p + jl] : 0.0f;
+      for (int i = 0; i < 4; ++i) {
+        const int r = i * 8 + (lane >> 2), c = lane & 3, col = lk * 16 + 4 * c;
+        const int row = min(lb * 32 + r, nrows - 1);
+        if (col < zp)
+          cp_async16(tile + (step & 1) * 512 + r * 16 + ((c ^ ((r >> 1) & 3)) << 2),
+                     base + static_cast<size_t>(row) * zp + col);
+      }
+      if (++lk == nblk) {
+        lk = 0;
+        lb += warps;
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+  };
+  float acc[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) acc[q] = 0.0f;
+  load(0);
+  int b = warp, k = 0;
+  for (int step = 0; step < steps; ++step) {
+    load(step + 1);
+    asm volatile("cp.async.wait_group 1;\n" ::);
+    __syncwarp();
+    const float* t = tile + (step & 1) * 512 + lane * 16;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int j0 = k * 16 + 4 * c;
+      if (j0 >= p) break;
+      const float4 v4 = *reinterpret_cast<const float4*>(t + ((c ^ ((lane >> 1) & 3)) << 2));
+      const float v[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (j0 + e < p) {
+          const float* w = W + static_cast<size_t>(j0 + e) * ldw + q0;
+          float wq[NQ];
+          if (NQ >= 4 && ldw % 4 == 0) {
+#pragma unroll
+            for (int q = 0; q < NQ; q += 4) {
+              const float4 w4 = *reinterpret_cast<const float4*>(w + q);
+              wq[q] = w4.x;
+              if (q + 1 < NQ) wq[q + 1] = w4.y;
+              if (q + 2 < NQ) wq[q + 2] = w4.z;
+              if (q + 3 < NQ) wq[q + 3] = w4.w;
+            }
+          } else {
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) wq[q] = w[q];
+          }
+          // (packed f32x2 operations are no use here: the assembler contracts
+          // a packed product and sum into one rounding)
+#pragma unroll
+          for (int q = 0; q < NQ; ++q) acc[q] = __fadd_rn(acc[q], __fmul_rn(v[e], wq[q]));
+        }
+      }
     }
     __syncwarp();
-    const int jn = min(32, p - j0);
-    for (int jj = 0; jj < jn; ++jj) {
-      const float v = tile[lane * 33 + jj];
-      const float* wr = W + static_cast<size_t>(j0 + jj) * ldw + q0;
+    if (++k == nblk) {
+      if (b * 32 + lane < nrows) out(b * 32 + lane, acc);
 #pragma unroll
-      for (int q = 0; q < kMaxNC; ++q)
-        if (q < nq) acc[q] = __fadd_rn(acc[q], __fmul_rn(v, wr[q]));
+      for (int q = 0; q < NQ; ++q) acc[q] = 0.0f;
+      k = 0;
+      b += warps;
+      tick();
     }
-    __syncwarp();
   }
+  asm volatile("cp.async.wait_group 0;\n" ::);
+}
+
+// out(row, q, score) for every component q of nc, kMaxNC at a time.
+template <class Out, class Tick>
+__device__ __forceinline__ void stream_all_scores(const float* __restrict__ base, int zp, int p, int nrows,
+                                                  const float* W, int ldw, int nc, float* tile, int lane, int warp,
+                                                  int warps, Out&& out, Tick&& tick) {
+  for (int q0 = 0; q0 < nc; q0 += kMaxNC) {
+    auto go = [&](auto nq) {
+      constexpr int NQ = decltype(nq)::value;
+      stream_scores<NQ>(base, zp, p, nrows, W, ldw, q0, tile, lane, warp, warps, [&](int row, const float (&acc)[NQ]) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) out(row, q0 + q, acc[q]);
+      }, tick);
+    };
+    const int nq = min(kMaxNC, nc - q0);
+    switch (nq) {
+      case 1: go(std::integral_constant<int, 1>{}); break;
+      case 2: go(std::integral_constant<int, 2>{}); break;
+      case 3: go(std::integral_constant<int, 3>{}); break;
+      case 4: go(std::integral_constant<int, 4>{}); break;
+      case 5: go(std::integral_constant<int, 5>{}); break;
+      case 6: go(std::integral_constant<int, 6>{}); break;
+      case 7: go(std::integral_constant<int, 7>{}); break;
+      default: go(std::integral_constant<int, 8>{}); break;
+    }
+  }
+}
+
+// acc plus the lanes' 32 values in lane order, the same in every lane.  The
+// shuffles are issued together, so the chain runs at the speed of its adds; with
+// a condition around each add it ran at shuffle latency, 40 cycles a value.
+// Values to leave out are passed as +0: a sum that starts at +0 is never -0, so
+// adding +0 changes nothing.
+__device__ __forceinline__ float warp_add32(float acc, float v) {
+  float t[32];
+#pragma unroll
+  for (int q = 0; q < 32; ++q) t[q] = __shfl_sync(kFull, v, q);
+#pragma unroll
+  for (int q = 0; q < 32; ++q) acc = __fadd_rn(acc, t[q]);
+  return acc;
 }
 
 // Sequential float chain over positions b..e-1 of a row-major matrix
@@ -588,72 +869,281 @@ template <int D>
 __device__ float warp_masked_chain(const float* __restrict__ m, int ld, int c, const uint8_t* __restrict__ ok, int b,
                                    int e, int lane) {
   float acc = 0.0f;
+  if (b >= e) return acc;
   float v[D];
-  bool f[D];
+  // flag and value are loaded side by side: a load behind a test of the flag
+  // would wait for it
+  auto fetch = [&](int i) {
+    const int k = min(i, e - 1);
+    const float x = m[static_cast<size_t>(k) * ld + c];
+    const bool take = ok[k] != 0;
+    return i < e && take ? x : 0.0f;
+  };
 #pragma unroll
-  for (int g = 0; g < D; ++g) {
-    const int i = b + g * 32 + lane;
-    v[g] = i < e ? m[static_cast<size_t>(i) * ld + c] : 0.0f;
-    f[g] = i < e && ok[i] != 0;
-  }
+  for (int g = 0; g < D; ++g) v[g] = fetch(b + g * 32 + lane);
   for (int base = b; base < e; base += 32 * D) {
 #pragma unroll
     for (int g = 0; g < D; ++g) {
       const int gb = base + g * 32;
       if (gb >= e) break;
-      const unsigned msk = __ballot_sync(kFull, f[g]);
       const float cur = v[g];
-      const int i = gb + D * 32 + lane;
-      v[g] = i < e ? m[static_cast<size_t>(i) * ld + c] : 0.0f;
-      f[g] = i < e && ok[i] != 0;
-#pragma unroll 8
-      for (int q = 0; q < 32; ++q) {
-        const float t = __shfl_sync(kFull, cur, q);
-        if ((msk >> q) & 1u) acc = __fadd_rn(acc, t);
-      }
+      v[g] = fetch(gb + D * 32 + lane);
+      acc = warp_add32(acc, cur);
     }
   }
   return acc;
 }
 
-// Sequential float chain sum_i a_i * b_i over i = 0..n-1 (rows of a
-// row-major matrix with stride ld, columns ca and cb), warp-cooperative like
-// warp_chain; each 32-row group's operands are loaded D groups ahead of its
-// products and adds, so nothing waits on a fresh load.
-template <int D>
-__device__ float warp_product_chain(const float* __restrict__ m, int n, int ld, int ca, int cb, int lane) {
-  float acc = 0.0f;
-  float va[D], vb[D];
+// Per lane, acc and the sequential float chain sum_i t(i, ca) * t(i, cb) over the
+// n rows of a row-major matrix of nc columns.  Batches of 256 / nc rows come into
+// a ring of four in `buf` (kTile floats), three ahead; the products of the next
+// eight rows are formed while those of the last eight are added (+0 past the
+// end, as in warp_add32).
+__device__ float warp_score_products(float acc, const float* t, int n, int nc, int ca, int cb, float* buf, int lane) {
+  static_assert(kTile >= 4 * 256, "batch ring");
+  const int rows = 256 / nc;  // nc <= 64: at least 4 rows
+  const int nb = (n + rows - 1) / rows;
+  auto fetch = [&](int b) {
+    if (b < nb) {
+      const int total = min(rows, n - b * rows) * nc;
+      const float* src = t + static_cast<size_t>(b) * rows * nc;
+      float* dst = buf + (b & 3) * 256;
 #pragma unroll
-  for (int g = 0; g < D; ++g) {
-    const int i = g * 32 + lane;
-    va[g] = i < n ? m[static_cast<size_t>(i) * ld + ca] : 0.0f;
-    vb[g] = i < n ? m[static_cast<size_t>(i) * ld + cb] : 0.0f;
+      for (int u = 0; u < 8; ++u)
+        if (u * 32 + lane < total)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(
+                           static_cast<unsigned>(__cvta_generic_to_shared(dst + u * 32 + lane))),
+                       "l"(src + u * 32 + lane));
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+  };
+  for (int b = 0; b < 3; ++b) fetch(b);
+  for (int b = 0; b < nb; ++b) {
+    asm volatile("cp.async.wait_group 2;\n" ::);
+    __syncwarp();
+    fetch(b + 3);  // into the slot whose rows were added before the barrier
+    const float* r = buf + (b & 3) * 256;
+    const int cn = min(rows, n - b * rows);
+    float pr[8];
+    auto form = [&](int i0) {
+      if (i0 + 8 <= cn) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) pr[q] = __fmul_rn(r[(i0 + q) * nc + ca], r[(i0 + q) * nc + cb]);
+      } else {
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          pr[q] = i0 + q < cn ? __fmul_rn(r[(i0 + q) * nc + ca], r[(i0 + q) * nc + cb]) : 0.0f;
+      }
+    };
+    form(0);
+    for (int i0 = 0; i0 < cn; i0 += 8) {
+      float cur[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) cur[q] = pr[q];
+      form(i0 + 8);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc = __fadd_rn(acc, cur[q]);
+    }
+    __syncwarp();
   }
-  for (int base = 0; base < n; base += 32 * D) {
+  asm volatile("cp.async.wait_group 0;\n" ::);
+  return acc;
+}
+
+// Label cross-product of every slice: column `code` of s_raw is the sum of the
+// class's standardised training rows (ascending) less its share of the column
+// sums (centered_label_crossprod, plscv.cpp:700-731).
+//
+// cross_stream_kernel: a CTA per (slice, 32 features) streams the rows in memory
+// order through a ring of 64-row tiles (cp.async, three ahead) and adds each row
+// to its class's sums in shared memory.  Warp w owns the codes c & 7 == w, so a
+// class's rows are added by one warp in ascending order.  All features of a row
+// are read by neighbouring CTAs at about the same time, so the launch runs at
+// memory speed (500 slices of 7500 x 200: 3 GB).  The classes' own row lists
+// (cross_kernel) read the same lines in random order behind two index loads:
+// 2.6 to 2.9 ms a launch there, 0.95 ms here; inside the evaluation kernel
+// the lists cost 2.1 M cycles a slice, 60% of it.  The lists remain for more
+// classes than shared memory holds sums for.
+constexpr int kStreamThreads = 256;
+constexpr int kStreamRows = 64;
+constexpr int kStreamSlots = 4;
+
+size_t cross_stream_smem(int C) {
+  return sizeof(float) * (static_cast<size_t>(C) * 32 + kStreamSlots * kStreamRows * 32) + sizeof(int) * C;
+}
+
+__global__ void __launch_bounds__(kStreamThreads) cross_stream_kernel(PlsEvalArgs a) {
+  extern __shared__ __align__(16) float xsm[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, p = a.p, C = a.C0max, L = a.L;
+  const int j0 = blockIdx.x * 32, j = j0 + lane;
+  float* ring = xsm;                                          // [slot][row][32]
+  float* acc = ring + kStreamSlots * kStreamRows * 32;        // [code][32]
+  int* cnt = reinterpret_cast<int*>(acc + static_cast<size_t>(C) * 32);
+  const int ntiles = (L + kStreamRows - 1) / kStreamRows;
+  for (int s = blockIdx.y; s < a.problems * a.F; s += gridDim.y) {
+    const int r = s / a.F, f = s % a.F;
+    const int* coff = a.class_off + static_cast<size_t>(r) * (C + 1);
+    const uint16_t* lab = a.labels + static_cast<size_t>(r) * L;
+    const uint8_t* fold = a.predict_mode ? nullptr : a.folds + static_cast<size_t>(r) * L;
+    const float* Zs = a.Z + static_cast<size_t>(s) * L * a.zp;
+    auto load = [&](int t) {
+      if (t < ntiles) {
+        float* dst = ring + (t & (kStreamSlots - 1)) * kStreamRows * 32;
 #pragma unroll
-    for (int g = 0; g < D; ++g) {
-      const int gb = base + g * 32;
-      if (gb >= n) break;
-      const float prod = __fmul_rn(va[g], vb[g]);
-      const int i = gb + D * 32 + lane;
-      va[g] = i < n ? m[static_cast<size_t>(i) * ld + ca] : 0.0f;
-      vb[g] = i < n ? m[static_cast<size_t>(i) * ld + cb] : 0.0f;
-      const int cnt = min(32, n - gb);
-#pragma unroll 8
-      for (int q = 0; q < 32; ++q) {
-        const float t = __shfl_sync(kFull, prod, q);
-        if (q < cnt) acc = __fadd_rn(acc, t);
+        for (int i = 0; i < kStreamRows / 32; ++i) {
+          const int rr = i * 32 + (threadIdx.x >> 3), c = 4 * (threadIdx.x & 7);
+          const int row = min(t * kStreamRows + rr, L - 1);
+          if (j0 + c < a.zp) cp_async16(dst + rr * 32 + c, Zs + static_cast<size_t>(row) * a.zp + j0 + c);
+        }
+      }
+      asm volatile("cp.async.commit_group;\n" ::);
+    };
+    // the codes and folds of a tile's rows, a lane each: fetched two tiles
+    // ahead, and looked at only when their tile is added
+    constexpr int H = kStreamRows / 32;
+    struct RowInfo {
+      uint16_t code[H];
+      uint8_t fold[H];
+    };
+    auto fetch_rows = [&](int t, RowInfo& ri) {
+#pragma unroll
+      for (int h = 0; h < H; ++h) {
+        const int row = min(t * kStreamRows + h * 32 + lane, L - 1);
+        ri.code[h] = lab[row];
+        ri.fold[h] = fold != nullptr ? fold[row] : 0;
+      }
+    };
+    for (int t = 0; t < kStreamSlots - 1; ++t) load(t);
+    for (int e = threadIdx.x; e < C * 32; e += kStreamThreads) acc[e] = 0.0f;
+    for (int c = threadIdx.x; c < C; c += kStreamThreads) cnt[c] = coff[c + 1] - coff[c];
+    __syncthreads();
+    if (!a.predict_mode) {
+      const int* vidx = a.val_idx + a.val_off[s];
+      const int nv = a.val_off[s + 1] - a.val_off[s];
+      for (int v = threadIdx.x; v < nv; v += kStreamThreads) atomicSub(&cnt[lab[vidx[v]]], 1);
+    }
+    RowInfo n1, n2;
+    fetch_rows(0, n1);
+    fetch_rows(1, n2);
+    for (int t = 0; t < ntiles; ++t) {
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(kStreamSlots - 2));
+      __syncthreads();  // tile t has landed for every thread; tile t - 1 is done with
+      load(t + kStreamSlots - 1);
+      // this lane's rows: the code if it trains the slice and belongs to this
+      // warp, else -1
+      int code[H];
+#pragma unroll
+      for (int h = 0; h < H; ++h) {
+        const int row = t * kStreamRows + h * 32 + lane;
+        const bool mine = row < L && (n1.code[h] & 7) == warp && (fold == nullptr || n1.fold[h] != f);
+        code[h] = mine ? n1.code[h] : -1;
+      }
+      n1 = n2;
+      fetch_rows(t + 2, n2);
+      const float* tile = ring + (t & (kStreamSlots - 1)) * kStreamRows * 32 + lane;
+#pragma unroll
+      for (int h = 0; h < H; ++h) {
+        unsigned m = __ballot_sync(kFull, code[h] >= 0);
+        while (m != 0u) {
+          // two rows at a time, so that one's loads cover the other's add
+          const int q1 = __ffs(m) - 1;
+          m &= m - 1u;
+          const bool two = m != 0u;
+          const int q2 = two ? __ffs(m) - 1 : q1;
+          m &= m - 1u;
+          const int k1 = __shfl_sync(kFull, code[h], q1), k2 = __shfl_sync(kFull, code[h], q2);
+          const float v1 = tile[(h * 32 + q1) * 32], v2 = tile[(h * 32 + q2) * 32];
+          float a1 = acc[k1 * 32 + lane], a2 = acc[k2 * 32 + lane];
+          a1 = __fadd_rn(a1, v1);
+          if (two && k1 == k2) {
+            a1 = __fadd_rn(a1, v2);
+          } else if (two) {
+            a2 = __fadd_rn(a2, v2);
+            acc[k2 * 32 + lane] = a2;
+          }
+          acc[k1 * 32 + lane] = a1;
+        }
+      }
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::);
+    __syncthreads();
+    const int nt = a.train_off[s + 1] - a.train_off[s];
+    const float inv_n = nt > 0 ? __fdiv_rn(1.0f, static_cast<float>(nt)) : 0.0f;
+    const float xs = j < p ? a.xsum[static_cast<size_t>(s) * p + j] : 0.0f;
+    for (int c = warp; c < C; c += kStreamThreads / 32) {
+      const float y_mean = __fmul_rn(static_cast<float>(cnt[c]), inv_n);
+      if (j < p && cnt[c] > 0)
+        a.s_raw[(static_cast<size_t>(s) * C + c) * p + j] = __fsub_rn(acc[c * 32 + lane], __fmul_rn(y_mean, xs));
+    }
+    __syncthreads();
+  }
+}
+
+// The same from the classes' row lists: a warp per (class, 32 features) with the
+// chain in a register and 32 to 64 rows' loads in flight.
+constexpr int kCrossThreads = 256;
+__global__ void __launch_bounds__(kCrossThreads, 2) cross_kernel(PlsEvalArgs a) {
+  const int lane = threadIdx.x & 31, p = a.p, C = a.C0max, JB = (p + 31) / 32;
+  for (int s = blockIdx.y; s < a.problems * a.F; s += gridDim.y) {
+    const int r = s / a.F, f = s % a.F;
+    const int* coff = a.class_off + static_cast<size_t>(r) * (C + 1);
+    const uint16_t* crow = a.class_rows + static_cast<size_t>(r) * a.L;
+    const uint8_t* fold = a.predict_mode ? nullptr : a.folds + static_cast<size_t>(r) * a.L;
+    const float* Zs = a.Z + static_cast<size_t>(s) * a.L * a.zp;
+    const int nt = a.train_off[s + 1] - a.train_off[s];
+    const float inv_n = nt > 0 ? __fdiv_rn(1.0f, static_cast<float>(nt)) : 0.0f;
+    const int warps = gridDim.x * (kCrossThreads / 32);
+    for (int item = blockIdx.x * (kCrossThreads / 32) + (threadIdx.x >> 5); item < C * JB; item += warps) {
+      const int code = item / JB, j = (item - code * JB) * 32 + lane;
+      const int b = coff[code], n = coff[code + 1] - b;
+      if (n == 0) continue;
+      const float* zj = Zs + (j < p ? j : 0);
+      float acc = 0.0f, va[32], vb[32];
+      int count = 0;
+      // rows t .. t + 31 of the class, -1 = past the end or in this fold
+      auto rows = [&](int t) {
+        int row = t + lane < n ? static_cast<int>(crow[b + t + lane]) : -1;
+        if (row >= 0 && fold != nullptr && fold[row] == f) row = -1;
+        return row;
+      };
+      auto fetch = [&](float (&v)[32], int ids) {
+  #pragma unroll
+        for (int q = 0; q < 32; ++q) {
+          const int row = __shfl_sync(kFull, ids, q);
+          v[q] = row >= 0 ? zj[static_cast<size_t>(row) * a.zp] : 0.0f;
+        }
+      };
+      auto use = [&](const float (&v)[32], int ids) {
+        const unsigned msk = __ballot_sync(kFull, ids >= 0);
+        count += __popc(msk);
+  #pragma unroll
+        for (int q = 0; q < 32; ++q)
+          if ((msk >> q) & 1u) acc = __fadd_rn(acc, v[q]);
+      };
+      int ia = rows(0), ib = rows(32);
+      fetch(va, ia);
+      for (int t = 0; t < n; t += 64) {
+        if (t + 32 < n) fetch(vb, ib);
+        const int ic = rows(t + 64), id = rows(t + 96);
+        use(va, ia);
+        if (t + 64 < n) fetch(va, ic);
+        if (t + 32 < n) use(vb, ib);
+        ia = ic;
+        ib = id;
+      }
+      if (j < p) {
+        const float y_mean = __fmul_rn(static_cast<float>(count), inv_n);
+        a.s_raw[(static_cast<size_t>(s) * C + code) * p + j] =
+            __fsub_rn(acc, __fmul_rn(y_mean, a.xsum[static_cast<size_t>(s) * p + j]));
       }
     }
   }
-  return acc;
 }
 
 __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int s = blockIdx.x, r = s / a.F, f = s % a.F;
-  const int p = a.p, L = a.L, C = a.C0max, NCm = a.requested, ldw = a.max_components;
+  const int p = a.p, zp = a.zp, L = a.L, C = a.C0max, NCm = a.requested, ldw = a.ldw;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   EvalShared& sh = *reinterpret_cast<EvalShared*>(smem);
   size_t off = 64;
@@ -682,18 +1172,19 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
   // which overlap it unless a slice of the launch computes scores during the
   // fit (no fold Gram)
   float* region = reinterpret_cast<float*>(carve(0));
-  float* tiles = (a.s_in_smem && a.tiles_after_s) ? region + static_cast<size_t>(p) * C : region;
+  // (16-byte copies land in the tiles)
+  float* tiles = (a.s_in_smem && a.tiles_after_s) ? region + (static_cast<size_t>(p) * C + 3) / 4 * 4 : region;
 
   const uint16_t* lab = a.labels + static_cast<size_t>(r) * L;
   const int* coff = a.class_off + static_cast<size_t>(r) * (C + 1);
   const uint16_t* crow = a.class_rows + static_cast<size_t>(r) * L;
   const uint8_t* fold = a.predict_mode ? nullptr : a.folds + static_cast<size_t>(r) * L;
-  const float* Zs = a.Z + static_cast<size_t>(s) * L * p;
+  const float* Zs = a.Z + static_cast<size_t>(s) * L * zp;
   const int tb = a.train_off[s], te = a.train_off[s + 1];
   const int nv = a.predict_mode ? a.NV : a.val_off[s + 1] - a.val_off[s];
   const int* vidx = a.predict_mode ? nullptr : a.val_idx + a.val_off[s];
   uint16_t* pred = a.pred + static_cast<size_t>(r) * (a.predict_mode ? a.NV : L);
-  const float* vbase = a.predict_mode ? a.Zv + static_cast<size_t>(r) * a.NV * p : Zs;
+  const float* vbase = a.predict_mode ? a.Zv + static_cast<size_t>(r) * a.NV * zp : Zs;
 
   // --- fold classes: codes with training rows, ascending -------------------
   for (int c = threadIdx.x; c < C; c += kEvalThreads) cnt[c] = coff[c + 1] - coff[c];
@@ -707,9 +1198,11 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
       if (cnt[c] > 0) klist[m++] = c;
     sh.m = m;
     sh.nt = te - tb;
+    sh.queue = 0;
     a.status[s] = 0;
   }
-  // class-list position of every row, and whether that position trains the slice
+  // class-list position of every row, whether that position trains the slice,
+  // and every row's position among the training rows
   uint16_t* posof = a.pos + static_cast<size_t>(s) * L;
   uint8_t* posok = a.posok + static_cast<size_t>(s) * L;
   for (int i = threadIdx.x; i < L; i += kEvalThreads) {
@@ -717,47 +1210,29 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
     posof[row] = static_cast<uint16_t>(i);
     posok[i] = (fold == nullptr || fold[row] != f) ? 1 : 0;
   }
+  uint16_t* tpos = a.tpos + static_cast<size_t>(s) * L;
+  if (fold != nullptr)
+    for (int i = threadIdx.x; i < nv; i += kEvalThreads) tpos[vidx[i]] = kNoPos;
+  for (int t = threadIdx.x; t < te - tb; t += kEvalThreads) tpos[a.train_idx[tb + t]] = static_cast<uint16_t>(t);
   __syncthreads();
   const int m = sh.m, nt = sh.nt;
-  if (m <= 1) {
-    // one training class: it is every prediction (labels.front() without one)
-    const int only = m == 1 ? klist[0] : lab[0];
+  if (m <= 1 || nt == 0) {
+    // one training class: it is every prediction (labels.front() without one);
+    // a slice without training rows but with classes is padding, with nothing
+    // to predict
+    const int only = m >= 1 ? klist[0] : lab[0];
     for (int v = threadIdx.x; v < nv; v += kEvalThreads)
       pred[a.predict_mode ? v : vidx[v]] = static_cast<uint16_t>(only);
     if (threadIdx.x == 0) a.eval_comp[s] = 1;
     return;
   }
 
-  // --- label cross-product S (p x m), column k = fold class k -------------
+  // --- label cross-product S (p x m), column k = fold class k, formed by
+  // cross_kernel for every code
   float* S = a.s_in_smem ? region : a.s_scr + static_cast<size_t>(s) * p * C;
-  {
-    const int JB = (p + 31) / 32;
-    const float inv_n = nt > 0 ? __fdiv_rn(1.0f, static_cast<float>(nt)) : 0.0f;
-    for (int it = warp; it < m * JB; it += kEvalWarps) {
-      const int k = it / JB, j = (it % JB) * 32 + lane;
-      const int code = klist[k];
-      const int b = coff[code], e = coff[code + 1];
-      float acc = 0.0f;
-      for (int base = b; base < e; base += 32) {
-        const int row = base + lane < e ? crow[base + lane] : -1;
-        const bool ok = row >= 0 && (fold == nullptr || fold[row] != f);
-        const unsigned msk = __ballot_sync(kFull, ok);
-        float v[32];
-#pragma unroll
-        for (int q = 0; q < 32; ++q) {
-          const int rq = __shfl_sync(kFull, row, q);
-          v[q] = (((msk >> q) & 1u) && j < p) ? Zs[static_cast<size_t>(rq) * p + j] : 0.0f;
-        }
-#pragma unroll
-        for (int q = 0; q < 32; ++q)
-          if ((msk >> q) & 1u) acc = __fadd_rn(acc, v[q]);
-      }
-      if (j < p) {
-        const float y_mean = __fmul_rn(static_cast<float>(cnt[code]), inv_n);
-        S[j + static_cast<size_t>(k) * p] =
-            __fsub_rn(acc, __fmul_rn(y_mean, a.xsum[static_cast<size_t>(s) * p + j]));
-      }
-    }
+  for (int k = warp; k < m; k += kEvalWarps) {
+    const float* src = a.s_raw + (static_cast<size_t>(s) * C + klist[k]) * p;
+    for (int j = lane; j < p; j += 32) S[j + static_cast<size_t>(k) * p] = src[j];
   }
   __syncthreads();
 
@@ -774,22 +1249,15 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
     // two power iterations (a second pass only for the strongest-column retry)
     for (int pass = 0; pass < 2; ++pass) {
       for (int it = 0; it < 2; ++it) {
-        for (int c = warp; c < m; c += kEvalWarps) {
-          const float* col = S + static_cast<size_t>(c) * p;
-          const float v = warp_seq_dot(p, [&](int k, float& x, float& y) {
-            x = col[k];
-            y = w[k];
-          }, lane);
-          if (lane == 0) tv[c] = v;
-        }
+        group_seq_dots(m, p, lane, warp, [&](int c, int k, float& x, float& y) {
+          x = S[k + static_cast<size_t>(c) * p];
+          y = w[k];
+        }, [&](int c, float v) { tv[c] = v; });
         __syncthreads();
-        for (int j = warp; j < p; j += kEvalWarps) {
-          const float v = warp_seq_dot(m, [&](int k, float& x, float& y) {
-            x = S[j + static_cast<size_t>(k) * p];
-            y = tv[k];
-          }, lane);
-          if (lane == 0) w[j] = v;
-        }
+        group_seq_dots(p, m, lane, warp, [&](int j, int k, float& x, float& y) {
+          x = S[j + static_cast<size_t>(k) * p];
+          y = tv[k];
+        }, [&](int j, float v) { w[j] = v; });
         __syncthreads();
       }
       if (warp == 0) {
@@ -827,14 +1295,10 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
     for (int j = threadIdx.x; j < p; j += kEvalThreads) w[j] = __fdiv_rn(w[j], rn);
     __syncthreads();
     if (gram) {
-      for (int i = warp; i < p; i += kEvalWarps) {
-        const float* gi = G + static_cast<size_t>(i) * p;
-        const float v = warp_seq_dot(p, [&](int k, float& x, float& y) {
-          x = gi[k];
-          y = w[k];
-        }, lane);
-        if (lane == 0) ld[i] = v;
-      }
+      group_seq_dots(p, p, lane, warp, [&](int i, int k, float& x, float& y) {
+        x = G[static_cast<size_t>(i) * p + k];
+        y = w[k];
+      }, [&](int i, float v) { ld[i] = v; });
       __syncthreads();
       if (warp == 0) {
         const float sns = warp_seq_dot(p, [&](int k, float& x, float& y) {
@@ -856,25 +1320,17 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
       __syncthreads();
     } else {
       // scores of the training rows, their norm, loading = X^T scores
-      float* tile = tiles + warp * kTile;
-      for (int b0 = warp * 32; b0 < nt; b0 += kEvalWarps * 32) {
-        const int t = b0 + lane;
-        const int row = t < nt ? tix[t] : -1;
-        float acc[kMaxNC];
-        warp_scores(Zs, p, row, w, 1, 0, 1, tile, lane, acc);
-        if (t < nt) scv[t] = acc[0];
-      }
+      stream_scores<1>(Zs, zp, p, L, w, 1, 0, tiles + warp * kTile, lane, warp, kEvalWarps,
+                       [&](int row, const float (&v)[1]) {
+        const int t = tpos[row];
+        if (t != kNoPos) scv[t] = v[0];
+      }, []() {});
       __syncthreads();
-      if (warp == 0) {
-        const float d = warp_seq_dot(nt, [&](int k, float& x, float& y) {
-          x = scv[k];
-          y = scv[k];
-        }, lane);
-        if (lane == 0) {
-          const float sn = __fsqrt_rn(0.0f < d ? d : 0.0f);
-          sh.stop = !(isfinite(sn) && sn > 1.0e-10f);
-          sh.inv = sh.stop ? 0.0f : __fdiv_rn(1.0f, sn);
-        }
+      const float d = block_norm2(scv, nt, tiles, lane, warp);
+      if (threadIdx.x == 0) {
+        const float sn = __fsqrt_rn(0.0f < d ? d : 0.0f);
+        sh.stop = !(isfinite(sn) && sn > 1.0e-10f);
+        sh.inv = sh.stop ? 0.0f : __fdiv_rn(1.0f, sn);
       }
       __syncthreads();
       if (sh.stop) break;
@@ -882,15 +1338,21 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
       for (int t = threadIdx.x; t < nt; t += kEvalThreads) scv[t] = __fmul_rn(scv[t], inv);
       for (int j = threadIdx.x; j < p; j += kEvalThreads) w[j] = __fmul_rn(w[j], inv);
       __syncthreads();
-      block_loading(Zs, p, tix, nt, scv, a.zexp + static_cast<size_t>(s) * p, ld, tiles, lane, warp);
+      block_loading(Zs, zp, p, tix, nt, scv, a.zexp + static_cast<size_t>(s) * p, ld, tiles, lane, warp);
     }
     for (int j = threadIdx.x; j < p; j += kEvalThreads) pw[j] = w[j];
     // Gram-Schmidt against the previous loadings
     for (int q = 0; q < comp; ++q) {
-      if (threadIdx.x == 0) {
+      if (warp == 0) {
+        // one chain over the features: the lanes form 32 products, every lane
+        // adds them in order
         float proj = 0.0f;
-        for (int j = 0; j < p; ++j) proj = __fadd_rn(proj, __fmul_rn(Vsm[static_cast<size_t>(j) * ldw + q], ld[j]));
-        sh.inv = proj;
+        for (int j0 = 0; j0 < p; j0 += 32) {
+          const int j = j0 + lane;
+          const float pr = j < p ? __fmul_rn(Vsm[static_cast<size_t>(j) * ldw + q], ld[j]) : 0.0f;
+          proj = warp_add32(proj, pr);
+        }
+        if (lane == 0) sh.inv = proj;
       }
       __syncthreads();
       const float proj = sh.inv;
@@ -922,6 +1384,7 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
     for (int k = threadIdx.x; k < m; k += kEvalThreads) {
       float acc = 0.0f;
       const float* col = S + static_cast<size_t>(k) * p;
+#pragma unroll 8
       for (int j = 0; j < p; ++j) acc = __fadd_rn(acc, __fmul_rn(ld[j], col[j]));
       tv[k] = acc;
     }
@@ -961,37 +1424,78 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
   const int nc = a.predict_mode ? fitted : min(a.requested, fitted);
   float* Ts = a.T + static_cast<size_t>(s) * L * NCm;   // by class-list position: Ts[pos * nc + q]
   float* Tt = a.Tt + static_cast<size_t>(s) * L * NCm;  // by training position: Tt[t * nc + q]
-  {
-    float* tile = tiles + warp * kTile;
-    for (int b0 = warp * 32; b0 < nt; b0 += kEvalWarps * 32) {
-      const int t = b0 + lane;
-      const int row = t < nt ? tix[t] : -1;
-      for (int q0 = 0; q0 < nc; q0 += kMaxNC) {
-        const int nq = min(kMaxNC, nc - q0);
-        float acc[kMaxNC];
-        warp_scores(Zs, p, row, Wsm, ldw, q0, nq, tile, lane, acc);
-        if (row >= 0) {
-          const size_t ps = static_cast<size_t>(posof[row]) * nc;
-#pragma unroll
-          for (int q = 0; q < kMaxNC; ++q) {
-            if (q < nq) {
-              Ts[ps + q0 + q] = acc[q];
-              Tt[static_cast<size_t>(t) * nc + q0 + q] = acc[q];
-            }
-          }
+  float* Tv = a.Tv != nullptr ? a.Tv + static_cast<size_t>(s) * L * NCm : nullptr;  // by validation row: Tv[row * nc + q]
+  auto keep_score = [&](int row, int q, float v) {
+    const int t = tpos[row];
+    if (t != kNoPos) {
+      Ts[static_cast<size_t>(posof[row]) * nc + q] = v;
+      Tt[static_cast<size_t>(t) * nc + q] = v;
+    } else if (Tv != nullptr) {
+      Tv[static_cast<size_t>(row) * nc + q] = v;
+    }
+  };
+  // The score cross-products are serial chains over all training rows.  With up
+  // to seven components they fit the lanes of one warp, which follows the others
+  // a round of batches behind; after the scores they took as long as half of
+  // them again, one warp working.
+  const int ncp = nc * (nc + 1) / 2;
+  const bool follow = nc < kMaxNC && !a.da_mode;
+  int prr = 0, pcol = min(lane, ncp - 1);
+  while (pcol > prr) {
+    pcol -= prr + 1;
+    ++prr;
+  }
+  if (!follow) {
+    stream_all_scores(Zs, zp, p, L, Wsm, ldw, nc, tiles + warp * kTile, lane, warp, kEvalWarps, keep_score, []() {});
+  } else {
+    constexpr int kScorers = kEvalWarps - 1;
+    const int nb = (L + 31) / 32, rounds = (nb + kScorers - 1) / kScorers;
+    if (warp < kScorers) {
+      int done = 0;
+      stream_all_scores(Zs, zp, p, L, Wsm, ldw, nc, tiles + warp * kTile, lane, warp, kScorers, keep_score, [&]() {
+        ++done;
+        __syncthreads();
+      });
+      for (; done < rounds; ++done) __syncthreads();
+    } else {
+      float acc = 0.0f;
+      int t0 = 0;
+      for (int k = 0; k < rounds; ++k) {
+        __syncthreads();  // round k's scores are written
+        int cn = 0;
+        for (int i = 0; i < kScorers; ++i) {
+          const int row = (k * kScorers + i) * 32 + lane;
+          cn += __popc(__ballot_sync(kFull, row < L && tpos[min(row, L - 1)] != kNoPos));
         }
+        acc = warp_score_products(acc, Tt + static_cast<size_t>(t0) * nc, cn, nc, prr, pcol, tiles + warp * kTile, lane);
+        t0 += cn;
+      }
+      if (lane < ncp) {
+        cp[prr * nc + pcol] = acc;
+        cp[pcol * nc + prr] = acc;
       }
     }
   }
+  // the rows to predict: scored with the training rows, except the separate
+  // ones of predict mode
+  float* rowscores = a.predict_mode ? a.Tp + static_cast<size_t>(r) * a.NV * NCm : Tv;
+  auto score_rows = [&]() {
+    stream_all_scores(vbase, zp, p, nv, Wsm, ldw, nc, tiles + warp * kTile, lane, warp, kEvalWarps,
+                      [&](int row, int q, float v) { rowscores[static_cast<size_t>(row) * nc + q] = v; }, []() {});
+    __syncthreads();
+  };
   __syncthreads();
   // class sums (the training rows of each class in row order, i.e. the
   // flagged class-list positions in order): one warp per chain
-  const int ncs = m * nc, ncp = nc * (nc + 1) / 2;
-  for (int it = warp; it < ncs; it += kEvalWarps) {
+  const int ncs = m * nc;
+  auto class_sum = [&](int it) {
     const int k = it / nc, q = it % nc;
     const int code = klist[k];
-    const float acc = warp_masked_chain<2>(Ts, nc, q, posok, coff[code], coff[code + 1], lane);
+    const float acc = warp_masked_chain<4>(Ts, nc, q, posok, coff[code], coff[code + 1], lane);
     if (lane == 0) cs[k * nc + q] = acc;
+  };
+  if (a.da_mode) {
+    for (int it = warp; it < ncs; it += kEvalWarps) class_sum(it);
   }
   if (a.da_mode) {
     // --- PLS-DA (the PLS_DA branch of run_plscv_host, plscv.cpp:2428-2443) ---
@@ -1071,48 +1575,48 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
     __syncthreads();
     // predict_pls_da_labels_float (plscv.cpp:1267-1292): first maximum of
     // mean + scores x coefficients
-    float* tile = tiles + warp * kTile;
-    for (int b0 = warp * 32; b0 < nv; b0 += kEvalWarps * 32) {
-      const int v = b0 + lane;
-      const int row = v < nv ? (a.predict_mode ? v : vidx[v]) : -1;
+    if (a.predict_mode) score_rows();
+    for (int v = threadIdx.x; v < nv; v += kEvalThreads) {
+      const int row = a.predict_mode ? v : vidx[v];
+      const float* tr = rowscores + static_cast<size_t>(row) * nc;
       float sr[kMaxComp];
-      for (int q0 = 0; q0 < nc; q0 += kMaxNC) {
-        const int nq = min(kMaxNC, nc - q0);
-        float acc[kMaxNC];
-        warp_scores(vbase, p, row, Wsm, ldw, q0, nq, tile, lane, acc);
-#pragma unroll
-        for (int q = 0; q < kMaxNC; ++q)
-          if (q < nq) sr[q0 + q] = acc[q];
-      }
-      if (row >= 0) {
-        int best = 0;
-        float bs = -INFINITY;
-        for (int k = 0; k < m; ++k) {
-          float sc = cst[k];
-          for (int q = 0; q < nc; ++q) sc = __fadd_rn(sc, __fmul_rn(sr[q], sol[q * m + k]));
-          if (sc > bs) {
-            bs = sc;
-            best = k;
-          }
+      for (int q = 0; q < nc; ++q) sr[q] = tr[q];
+      int best = 0;
+      float bs = -INFINITY;
+      for (int k = 0; k < m; ++k) {
+        float sc = cst[k];
+        for (int q = 0; q < nc; ++q) sc = __fadd_rn(sc, __fmul_rn(sr[q], sol[q * m + k]));
+        if (sc > bs) {
+          bs = sc;
+          best = k;
         }
-        pred[row] = static_cast<uint16_t>(klist[best]);
       }
+      pred[row] = static_cast<uint16_t>(klist[best]);
     }
     return;
   }
-  // score cross-products (all training rows in order): one warp per chain
-  for (int it = warp; it < ncp; it += kEvalWarps) {
-    int pr = it, rr = 0;
+  // score cross-products (all training rows in order), where no warp followed
+  // the scores: a lane per chain
+  for (int c0 = warp * 32; !follow && c0 < ncp; c0 += kEvalWarps * 32) {
+    int pr = min(c0 + lane, ncp - 1), rr = 0;
     while (pr > rr) {
       pr -= rr + 1;
       ++rr;
     }
     const int col = pr;
-    const float acc = warp_product_chain<4>(Tt, nt, nc, rr, col, lane);
-    if (lane == 0) {
+    const float acc = warp_score_products(0.0f, Tt, nt, nc, rr, col, tiles + warp * kTile, lane);
+    if (c0 + lane < ncp) {
       cp[rr * nc + col] = acc;
       cp[col * nc + rr] = acc;
     }
+  }
+  // the class sums go to whichever warp is free
+  for (;;) {
+    int it = 0;
+    if (lane == 0) it = atomicAdd(&sh.queue, 1);
+    it = __shfl_sync(kFull, it, 0);
+    if (it >= ncs) break;
+    class_sum(it);
   }
   __syncthreads();
   // fit_lda_from_score_statistics_float, parallel where the reference's loops
@@ -1196,32 +1700,23 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
   __syncthreads();
   // --- predictions ---------------------------------------------------------
   {
-    float* tile = tiles + warp * kTile;
-    for (int b0 = warp * 32; b0 < nv; b0 += kEvalWarps * 32) {
-      const int v = b0 + lane;
-      const int row = v < nv ? (a.predict_mode ? v : vidx[v]) : -1;
+    if (a.predict_mode) score_rows();
+    for (int v = threadIdx.x; v < nv; v += kEvalThreads) {
+      const int row = a.predict_mode ? v : vidx[v];
+      const float* tr = rowscores + static_cast<size_t>(row) * nc;
       float sr[kMaxComp];
-      for (int q0 = 0; q0 < nc; q0 += kMaxNC) {
-        const int nq = min(kMaxNC, nc - q0);
-        float acc[kMaxNC];
-        warp_scores(vbase, p, row, Wsm, ldw, q0, nq, tile, lane, acc);
-#pragma unroll
-        for (int q = 0; q < kMaxNC; ++q)
-          if (q < nq) sr[q0 + q] = acc[q];
-      }
-      if (row >= 0) {
-        int best = 0;
-        float bs = -INFINITY;
-        for (int k = 0; k < m; ++k) {
-          float sc = cst[k];
-          for (int q = 0; q < nc; ++q) sc = __fadd_rn(sc, __fmul_rn(sr[q], lin[k * nc + q]));
-          if (sc > bs) {
-            bs = sc;
-            best = k;
-          }
+      for (int q = 0; q < nc; ++q) sr[q] = tr[q];
+      int best = 0;
+      float bs = -INFINITY;
+      for (int k = 0; k < m; ++k) {
+        float sc = cst[k];
+        for (int q = 0; q < nc; ++q) sc = __fadd_rn(sc, __fmul_rn(sr[q], lin[k * nc + q]));
+        if (sc > bs) {
+          bs = sc;
+          best = k;
         }
-        pred[row] = static_cast<uint16_t>(klist[best]);
       }
+      pred[row] = static_cast<uint16_t>(klist[best]);
     }
   }
 }
@@ -1272,8 +1767,8 @@ int pls_assemble_result(int problems, int n, int L, int NV, const int* land, con
 
 int pls_prepare(const PlsPrepArgs& a, cudaStream_t st) {
   const int S = a.problems * a.F;
-  dim3 g1(S, (a.p + 127) / 128);
-  stats_kernel<<<g1, 128, 0, st>>>(a);
+  dim3 g1(S, (a.p + 63) / 64);
+  stats_kernel<<<g1, 64, 0, st>>>(a);
   count_launch();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return static_cast<int>(e);
@@ -1285,7 +1780,7 @@ int pls_prepare(const PlsPrepArgs& a, cudaStream_t st) {
   count_launch();
   e = cudaGetLastError();
   if (e != cudaSuccess) return static_cast<int>(e);
-  xsum_kernel<<<g1, 128, 0, st>>>(a);
+  xsum_kernel<<<g1, 64, 0, st>>>(a);
   count_launch();
   return static_cast<int>(cudaGetLastError());
 }
@@ -1310,22 +1805,42 @@ size_t pls_eval_smem(int p, int C0max, int requested, int max_components, bool s
   b += al(sizeof(float) * C * N) + al(sizeof(float) * C) + al(sizeof(double) * N);
   const size_t cross = s_in_smem ? sizeof(float) * static_cast<size_t>(p) * C : 0;
   const size_t tiles = sizeof(float) * static_cast<size_t>(kEvalWarps) * kTile;
-  b += tiles_after_s ? cross + tiles : (cross > tiles ? cross : tiles);
+  b += tiles_after_s ? al(cross) + tiles : (cross > tiles ? cross : tiles);
   return b;
 }
 
 int pls_evaluate(const PlsEvalArgs& a, cudaStream_t st) {
   const int S = a.problems * a.F;
   if (a.requested > kMaxComp || a.max_components > kMaxComp) return static_cast<int>(cudaErrorInvalidValue);
-  const size_t smem =
-      pls_eval_smem(a.p, a.C0max, a.requested, a.max_components, a.s_in_smem != 0, a.tiles_after_s != 0);
+  // weight rows padded to whole 16-byte vectors, unless that would cost the
+  // second CTA of an SM (or not fit at all)
+  auto bytes = [&](int ldw) {
+    return pls_eval_smem(a.p, a.C0max, a.requested, ldw, a.s_in_smem != 0, a.tiles_after_s != 0);
+  };
+  const int padded = (a.max_components + 3) / 4 * 4;
+  const size_t two_ctas = 112 * 1024, most = 224 * 1024;
+  PlsEvalArgs b = a;
+  b.ldw = bytes(padded) <= (bytes(a.max_components) <= two_ctas ? two_ctas : most) ? padded : a.max_components;
+  const size_t smem = bytes(b.ldw);
   if (smem > 48 * 1024) {
     const cudaError_t e =
         cudaFuncSetAttribute(eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
   }
-  eval_kernel<<<S, kEvalThreads, smem, st>>>(a);
-  count_launch();
+  const size_t stream_smem = cross_stream_smem(a.C0max);
+  if (stream_smem <= most) {
+    if (stream_smem > 48 * 1024) {
+      const cudaError_t e = cudaFuncSetAttribute(cross_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 static_cast<int>(stream_smem));
+      if (e != cudaSuccess) return static_cast<int>(e);
+    }
+    cross_stream_kernel<<<dim3((a.p + 31) / 32, std::min(S, 65535)), kStreamThreads, stream_smem, st>>>(b);
+  } else {
+    const int items = a.C0max * ((a.p + 31) / 32), per = kCrossThreads / 32;
+    cross_kernel<<<dim3(std::min((items + per - 1) / per, 1024), std::min(S, 65535)), kCrossThreads, 0, st>>>(b);
+  }
+  eval_kernel<<<S, kEvalThreads, smem, st>>>(b);
+  count_launch(2);
   return static_cast<int>(cudaGetLastError());
 }
 

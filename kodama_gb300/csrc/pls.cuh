@@ -26,13 +26,14 @@ struct PlsPrepArgs {
   const int* train_idx;  // ascending training rows of each slice
   float* mean;           // S x p
   float* sdev;           // S x p
-  float* Z;              // S x L x p standardised rows (all L rows, with the slice's statistics)
+  int zp;                // floats per standardised row: p rounded up to 8 (padding never read as data)
+  float* Z;              // S x L x zp standardised rows (all L rows, with the slice's statistics)
   float* xsum;           // S x p
   int* zexp;             // S x p: largest biased exponent (at least 1) of each column over the training rows
   float* gram;           // S x p x p (only for build_gram)
   // predict mode: standardise NV extra rows per problem with the slice's statistics
   const float* Xv;       // R x NV x p, or nullptr
-  float* Zv;             // R x NV x p
+  float* Zv;             // R x NV x zp
   int NV;
 };
 
@@ -51,7 +52,8 @@ struct PlsEvalArgs {
   int da_mode;           // 1: PLS-DA (one-hot regression on the scores) instead of LDA
   int s_in_smem;         // 1: the label cross-product of a slice lives in shared memory
   int tiles_after_s;     // 1: some slice computes training scores during the fit (no fold Gram)
-  const float* Z;        // S x L x p
+  int zp;                // floats per row of Z and Zv
+  const float* Z;        // S x L x zp
   const float* xsum;     // S x p
   const int* zexp;       // S x p (PlsPrepArgs::zexp)
   const float* gram;     // S x p x p, or nullptr
@@ -61,7 +63,7 @@ struct PlsEvalArgs {
   const int* train_idx;  // ascending training rows of each slice
   const int* val_off;    // S + 1 (CV)
   const int* val_idx;    // ascending validation rows of each slice (CV)
-  const float* Zv;       // R x NV x p (predict mode)
+  const float* Zv;       // R x NV x zp (predict mode)
   int NV;
   const float* w0;       // p: the SIMPLS start vector (std::mt19937(1), normal_distribution<float>)
   const float* logprior; // logf(max(k / nt, FLT_MIN)) tables
@@ -73,14 +75,17 @@ struct PlsEvalArgs {
   int* eval_comp;        // S: components evaluated by the slice
   int* status;           // S: 0 ok, 1 no supervised direction (degenerate fit), 2 LDA factorisation failed
   // scratch
-  float* s_scr;          // S x p x C0max
-  float* W;              // S x p x max_components
-  float* V;              // S x p x max_components
+  float* s_raw;          // S x C0max x p: the cross-product by code
+  float* s_scr;          // S x p x C0max: by fold class, when not in shared memory
   float* T;              // S x L x requested (training-row scores, by class-list position)
   float* Tt;             // S x L x requested (the same scores in training order)
+  float* Tv;             // S x L x requested (CV: validation-row scores, by row), or nullptr
+  float* Tp;             // R x NV x requested (predict mode: scores of the rows to predict), or nullptr
+  uint16_t* tpos;        // S x L: position of each row among the slice's training rows, 0xffff = validation row
   uint16_t* pos;         // S x L: position of each row in the slice's class list
   uint8_t* posok;        // S x L: whether the row at a class-list position trains the slice
   float* sc;             // S x L (scores path of the fit)
+  int ldw;               // set by pls_evaluate: floats per row of the weights in shared memory
 };
 
 int pls_evaluate(const PlsEvalArgs& a, cudaStream_t st);
