@@ -37,6 +37,7 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kEvalThreads = 512;
 constexpr int kEvalWarps = kEvalThreads / 32;
+constexpr int kFollowRows = 8 * kEvalThreads;  // rows from which a warp follows the scores
 
 // ---------------------------------------------------------------------------
 // Preparation (label independent)
@@ -46,7 +47,7 @@ constexpr int kEvalWarps = kEvalThreads / 32;
 // (stride ld), in order: each lane's column, 32 rows' loads in flight while the
 // 32 before them are taken.  A column is a serial float chain, so its time is
 // the loads' latency: with 8 loads in flight per thread and nothing overlapped
-// a chain over 1800 rows took about 150 us, here about 20.  Warp-collective;
+// the two walks over 1800 rows took 287 and 300 us, here 62 each.  Warp-collective;
 // lanes with !in read column 0.
 template <class Take>
 __device__ __forceinline__ void column_walk(const float* __restrict__ X, int ld, const int* __restrict__ idx, int n,
@@ -1437,9 +1438,11 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
   // The score cross-products are serial chains over all training rows.  With up
   // to seven components they fit the lanes of one warp, which follows the others
   // a round of batches behind; after the scores they took as long as half of
-  // them again, one warp working.
+  // them again, one warp working.  A short stream is not worth the warp and
+  // the rounds' barriers: at 2000 x 50 rows (4 batches a warp) the scores went
+  // from 62k to 129k cycles and the evaluation from 0.42 to 0.44 ms.
   const int ncp = nc * (nc + 1) / 2;
-  const bool follow = nc < kMaxNC && !a.da_mode;
+  const bool follow = nc < kMaxNC && !a.da_mode && L >= kFollowRows;
   int prr = 0, pcol = min(lane, ncp - 1);
   while (pcol > prr) {
     pcol -= prr + 1;
