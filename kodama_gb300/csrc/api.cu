@@ -517,29 +517,17 @@ EvolveBuffers run_evolution(Ctx& ctx, kgb::EvolveParams P, int C0max) {
   P.best = b.best;
   P.status = b.status;
   P.C0max = C0max;
-  P.trans = ctx.alloc<int>(static_cast<size_t>(problems) * C0max * C0max);
-  P.foldcnt = ctx.alloc<int>(static_cast<size_t>(problems) * P.F * C0max);
+  P.foldcnt = ctx.alloc<int>(static_cast<size_t>(problems) * (P.F + 1) * C0max);
   const int grid = std::min(problems, ctx.sms());
+  P.empty_rows = ctx.alloc<uint16_t>(static_cast<size_t>(grid) * L);
   constexpr size_t kSmemBudget = 224 * 1024;
   const size_t Lp = (static_cast<size_t>(L) + 7) / 8 * 8;
-  // prefer (in order): rows, transitions in shared memory
-  bool placed = false;
   size_t smem = 0;
-  for (int option = 0; option < 4 && !placed; ++option) {
-    const bool rows = option < 2;
-    const bool trans = (option % 2) == 0;
-    smem = kgb::evolve_smem_bytes(L, C0max, rows, trans);
-    if (smem <= kSmemBudget) {
-      placed = true;
-      P.smem_rows = rows;
-      P.smem_trans = trans;
-    }
-  }
-  if (!placed) fail(KGB_EINVAL, "too many distinct labels for the evolution kernel");
+  if (!kgb::evolve_place(P, kSmemBudget, &smem))
+    fail(KGB_EINVAL, "too many distinct labels for the evolution kernel");
   P.rows_scratch = P.smem_rows ? nullptr
                                : ctx.alloc<uint16_t>(static_cast<size_t>(grid) * kgb::kEvolveRowArrays * Lp);
-  P.raw_scratch = ctx.alloc<uint64_t>(static_cast<size_t>(grid) * (L / 2 + 64));
-  if (P.smem_trans) P.trans = nullptr;
+  P.engine_save = ctx.alloc<uint64_t>(static_cast<size_t>(grid) * kgb::kEvolveEngineSave);
   {
     int* roff = ctx.alloc<int>(static_cast<size_t>(problems) * (L + 1));
     uint16_t* ridx = ctx.alloc<uint16_t>(static_cast<size_t>(problems) * L * P.w);
@@ -946,27 +934,15 @@ EvolveBuffers run_pls_evolution(Ctx& ctx, kgb::EvolveParams P, PlsBuffers& b, in
   P.status = eb.status;
   P.C0max = C0max;
   P.w = 1;
-  P.trans = ctx.alloc<int>(static_cast<size_t>(problems) * C0max * C0max);
   const int grid = problems;
   constexpr size_t kSmemBudget = 200 * 1024;
   const size_t Lp = (static_cast<size_t>(L) + 7) / 8 * 8;
-  bool placed = false;
   size_t smem = 0;
-  for (int option = 0; option < 4 && !placed; ++option) {
-    const bool rows = option < 2;
-    const bool trans = (option % 2) == 0;
-    smem = kgb::evolve_smem_bytes(L, C0max, rows, trans);
-    if (smem <= kSmemBudget) {
-      placed = true;
-      P.smem_rows = rows;
-      P.smem_trans = trans;
-    }
-  }
-  if (!placed) fail(KGB_EINVAL, "too many distinct labels for the evolution kernel");
+  if (!kgb::evolve_place(P, kSmemBudget, &smem))
+    fail(KGB_EINVAL, "too many distinct labels for the evolution kernel");
   P.rows_scratch = P.smem_rows ? nullptr
                                : ctx.alloc<uint16_t>(static_cast<size_t>(grid) * kgb::kEvolveRowArrays * Lp);
-  P.raw_scratch = ctx.alloc<uint64_t>(static_cast<size_t>(grid) * (L / 2 + 64));
-  if (P.smem_trans) P.trans = nullptr;
+  P.engine_save = ctx.alloc<uint64_t>(static_cast<size_t>(grid) * kgb::kEvolveEngineSave);
   {
     std::vector<double> psq(static_cast<size_t>(L) + 1);
     const double nd = static_cast<double>(L);

@@ -20,6 +20,13 @@
 // (no contraction), random draws follow rng.cuh, and the unordered_map
 // iteration order that fixes the summation order of the diversity term is
 // reproduced (reverse first-insertion order, bucket runs on collisions).
+//
+// What bounds it: a cycle is a chain of short phases in one CTA, 40k to 100k
+// cycles long, about half of them issuing (208k warp instructions a cycle at 10000
+// rows and 30 neighbours), the rest barriers and latency.  So per-row passes take
+// eight rows a thread, one thread's work is kept to what is serial, and double
+// arithmetic, 64 cycles a dependent operation and 512 for all 1024 threads, is
+// left to single warps.
 #include "evolve.cuh"
 #include "launch_count.cuh"
 #include "rng.cuh"
@@ -39,10 +46,21 @@ constexpr int kWarps = kThreads / 32;
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kRowArrays = 8;  // cl, cur, curpred, pred/perm, J, list, 2 x (32-bit scratch)
 
+// The run's scores and counters, kept by thread 0.
+struct RunState {
+  double accbest, scorebest, cur_acc, cur_score;
+  int nc_cur, nc_best;
+  int best_updates, accepts, st_att, st_acc, rejections, absorb_moves, tr_acc, success;
+};
+
 struct Fixed {
+  RunState run;
   Mt64State rng;
-  uint64_t mt_alt[kMtN];  // the engine state's second buffer (produce_outputs_group)
-  int first_reject;
+  union {
+    uint64_t mt_alt[kMtN];  // the engine state's second buffer (produce_outputs_group)
+    int sel_hist[256];      // digit counts of learned_flip; labels of vote_empty_rows
+  };
+  int rejected;
   int i0;
   int ns;
   int red_i[kWarps];
@@ -50,14 +68,16 @@ struct Fixed {
   int nc;          // distinct labels of the proposal
   int changed_cnt;  // dirty_rows_block: rows whose label changed
   int dirty_cnt;    // dirty_rows_block: rows listed for the vote
-  int moves_sel;
-  int n_empty;
+  int walk_cnt;    // groups whose final position is walked
+  int empty_cnt;   // rows without out-of-fold neighbours
+  unsigned empty_folds[8];  // the folds they are in
   int selected_target;
   int rev_total;   // this problem's reverse-neighbour entries (rev_off[L])
   double acc;
   double score;
+  double cooling[2];  // annealing factors of this and the next acceptance test, by cycle parity
+  int max_groups;  // largest size of the coming proposal
   int accept;
-  int improves;
   // this problem's groups and fixed flags (bind_groups)
   const int* goff;
   const int* gmem;
@@ -67,8 +87,10 @@ struct Fixed {
   int sel_count;
   int sel_digit;
   int sel_need;
-  int sel_hist[256];
 };
+// The room the struct is given, part of how many labels fit (evolve_place).
+constexpr size_t kFixedBytes = 8768;
+static_assert(sizeof(Fixed) <= kFixedBytes, "evolve_place's limit");
 
 struct Smem {
   Fixed* f;
@@ -80,8 +102,10 @@ struct Smem {
   uint16_t* jarr;    // swap target of every shuffle step
   uint16_t* list;    // shuffle steps bucketed by swap target
   int* scratch32;    // per-position counts / bucket offsets
-  int* trans;        // class x prediction counts (shared or global)
-  uint64_t* raw;     // engine outputs of one shuffle (global scratch)
+  int* hist;         // per warp: one counter per code, all zero between uses
+  int hist_stride;   // counters per warp
+  int hist_warps;    // warps that have counters
+  uint64_t* save;    // the engine's state before a shuffle (global scratch)
   int* cnt;          // per code: count in proposal
   int* firstpos;     // per code: first row
   int* movable;      // per code: non-fixed rows
@@ -95,22 +119,113 @@ struct Smem {
 
 __device__ __forceinline__ size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-__device__ int block_sum(int v, Fixed& f) {
+// Where the per-row arrays lie is a property of the kernel, and the struct is only
+// ever inlined, so that the accesses are known to be to shared memory.
+template <bool kRows>
+__device__ __forceinline__ Smem carve_smem(const EvolveParams& P) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Smem s;
+  size_t off = 0;
+  s.f = reinterpret_cast<Fixed*>(smem_raw);
+  off = kFixedBytes;
+  const int C = P.C0max;
+  s.cnt = reinterpret_cast<int*>(smem_raw + off); off += align_up(sizeof(int) * C, 16);
+  s.firstpos = reinterpret_cast<int*>(smem_raw + off); off += align_up(sizeof(int) * C, 16);
+  s.movable = reinterpret_cast<int*>(smem_raw + off); off += align_up(sizeof(int) * C, 16);
+  s.order = reinterpret_cast<int*>(smem_raw + off); off += align_up(sizeof(int) * (C + 1), 16);
+  s.bt = reinterpret_cast<int*>(smem_raw + off); off += align_up(sizeof(int) * C, 16);
+  s.aux = reinterpret_cast<int*>(smem_raw + off); off += align_up(sizeof(int) * C, 16);
+  s.bsur = reinterpret_cast<double*>(smem_raw + off); off += align_up(sizeof(double) * C, 16);
+  s.weight = reinterpret_cast<double*>(smem_raw + off); off += align_up(sizeof(double) * C, 16);
+  s.cp = reinterpret_cast<double*>(smem_raw + off); off += align_up(sizeof(double) * 2 * C, 16);
+  const size_t Lp = align_up(static_cast<size_t>(P.L), 8);
+  s.save = P.engine_save + static_cast<size_t>(blockIdx.x) * kEvolveEngineSave;
+  s.hist_stride = static_cast<int>(align_up(C, 4));
+  s.hist_warps = P.hist_warps;
+  s.hist = reinterpret_cast<int*>(smem_raw + off);
+  off += sizeof(int) * static_cast<size_t>(s.hist_stride) * s.hist_warps;
+  uint16_t* rows = kRows ? reinterpret_cast<uint16_t*>(smem_raw + off)
+                         : P.rows_scratch + static_cast<size_t>(blockIdx.x) * kRowArrays * Lp;
+  s.cl = rows;
+  s.cur = rows + Lp;
+  s.curpred = rows + 2 * Lp;
+  s.pred = rows + 3 * Lp;
+  s.perm = s.pred;
+  s.jarr = rows + 4 * Lp;
+  s.list = rows + 5 * Lp;
+  s.scratch32 = reinterpret_cast<int*>(rows + 6 * Lp);  // 2 * Lp u16 = Lp ints
+  return s;
+}
+
+// The same layout for the functions kept out of line, where the two are looked up
+// instead.
+__device__ Smem carve_smem_any(const EvolveParams& P) {
+  return P.smem_rows ? carve_smem<true>(P) : carve_smem<false>(P);
+}
+
+__device__ __forceinline__ int block_sum(int v, Fixed& f) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   v = __reduce_add_sync(kFull, v);
   if (lane == 0) f.red_i[warp] = v;
   __syncthreads();
-  int t = 0;
-  if (threadIdx.x < 32) {
-    t = f.red_i[threadIdx.x];
-    t = __reduce_add_sync(kFull, t);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) f.red_i[0] = t;
-  __syncthreads();
-  const int out = f.red_i[0];
+  const int out = __reduce_add_sync(kFull, f.red_i[lane]);
   __syncthreads();
   return out;
+}
+
+// The per-row arrays start on 16-byte boundaries and are padded to whole
+// 8-row vectors; row_code unpacks row e of a vector.
+__device__ __forceinline__ int row_vectors(int L) { return (L + 7) >> 3; }
+__device__ __forceinline__ int row_code(const uint4& v, int e) {
+  const unsigned w = e < 2 ? v.x : e < 4 ? v.y : e < 6 ? v.z : v.w;
+  return static_cast<int>((w >> (16 * (e & 1))) & 0xffffu);
+}
+__device__ __forceinline__ uint4 load_rows(const uint16_t* a, int i) { return reinterpret_cast<const uint4*>(a)[i]; }
+__device__ __forceinline__ void copy_rows(uint16_t* dst, const uint16_t* src, int L) {
+  for (int i = threadIdx.x; i < row_vectors(L); i += kThreads) reinterpret_cast<uint4*>(dst)[i] = load_rows(src, i);
+}
+
+// acc plus n doubles from shared memory in order.  The FP64 pipe takes 64 cycles
+// for a dependent sum, so the values are read eight ahead of the chain.
+__device__ __forceinline__ double chain_add(double acc, const double* v, int n) {
+  int i = 0;
+  for (; i + 8 <= n; i += 8) {
+    double t[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) t[q] = v[i + q];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) acc = __dadd_rn(acc, t[q]);
+  }
+  for (; i < n; ++i) acc = __dadd_rn(acc, v[i]);
+  return acc;
+}
+
+// std::discrete_distribution (discrete_serial) by one warp: the divisions run a
+// lane each, the two running sums stay in order.  w is overwritten.
+__device__ __forceinline__ int discrete_warp(Mt64State& g, double* w, int n, double* cp, int lane) {
+  if (n < 2) return 0;
+  const double sum = chain_add(0.0, w, n);
+  __syncwarp();
+  for (int i = lane; i < n; i += 32) w[i] = __ddiv_rn(w[i], sum);
+  __syncwarp();
+  int at = 0;
+  if (lane == 0) {
+    double acc = 0.0;
+    for (int q0 = 0; q0 < n; q0 += 8) {
+      double t[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) t[q] = q0 + q < n ? w[q0 + q] : 0.0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        if (q0 + q >= n) break;
+        acc = q0 + q == 0 ? t[q] : __dadd_rn(acc, t[q]);
+        cp[q0 + q] = acc;
+      }
+    }
+    cp[n - 1] = 1.0;
+    at = discrete_probe(cp, n, canonical_serial(g));
+  }
+  return __shfl_sync(kFull, at, 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -128,8 +243,8 @@ __device__ int block_sum(int v, Fixed& f) {
 // CTA computes all J[i] in parallel from the engine blocks, buckets the steps
 // by target, and walks each wanted position down this chain.
 // ---------------------------------------------------------------------------
-// Exclusive prefix sum of a[0..n) in place (block-wide).
-__device__ void block_exclusive_scan(int* a, int n, Fixed& f) {
+// Exclusive prefix sum of a[0..n) in place (block-wide); returns the total.
+__device__ __forceinline__ int block_exclusive_scan(int* a, int n, Fixed& f) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int chunk = (n + kThreads - 1) / kThreads;
   const int b = threadIdx.x * chunk, e = min(n, b + chunk);
@@ -157,94 +272,115 @@ __device__ void block_exclusive_scan(int* a, int n, Fixed& f) {
     a[i] = run;
     run += v;
   }
+  const int total = f.red_i[kWarps - 1];
   __syncthreads();
+  return total;
 }
 
 // Engine producer group: the first 160 threads (warps 0-4) synchronised by
 // named barrier 1.
 constexpr int kProducerThreads = 160;
 __device__ __forceinline__ void producer_sync() { asm volatile("bar.sync 1, 160;" ::: "memory"); }
+__device__ __forceinline__ void shuffle_step_sync() { asm volatile("bar.sync 2, 1024;" ::: "memory"); }
 
-// Copy the next `count` engine outputs into raw[start..] (producer group).
-// The outputs left in g.out are copied first; every whole block of 312 that
-// follows is regenerated with its tempered words written straight into raw
-// (g.out is only refreshed for the last block, whose tail later draws read).
-// A regeneration reads the old state words from one buffer and writes the new
-// ones to the other (g.mt and alt in turn), so one barrier separates
-// regenerations: thread t < 156 forms word t from old words t, t + 1, t + 156
-// and then word t + 156 from old words t + 156, t + 157 and its own new word t
-// (word 311 takes the new word 0, which thread 155 forms again itself).
-__device__ void produce_outputs_group(Mt64State& g, uint64_t* alt, uint64_t* raw, int start, int count, int t) {
+// Advances the CTA's engine by the next `count` outputs (producer group), with a
+// shuffle_step_sync after every regeneration (one in all if the outputs left
+// suffice).  The state and its position go to `save` first.
+// Thread t < 156 keeps words t and t + 156 of the state in registers: the new word
+// t takes old words t, t + 1 and t + 156, the new word t + 156 old words t + 156,
+// t + 157 and the new word t; word 311 takes the new word 0, which thread 156
+// forms for its neighbour.  Regeneration r goes to f.mt_alt for even r, f.rng.mt
+// for odd r, where the other warps read its words, still to be tempered, until
+// the next step; the last block's outputs are written once at the end.
+// Tempering every block here and writing it to global memory, the state's words
+// reloaded, took 860 cycles a regeneration; this takes 270, as a function of its
+// own with its own registers (640 within the kernel's).
+__device__ __noinline__ void produce_outputs_group(int count, uint64_t* save) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Fixed& f = *reinterpret_cast<Fixed*>(smem_raw);
+  Mt64State& g = f.rng;
+  const int t = threadIdx.x, h = t + kMtM;
   const int pos0 = g.pos;
   const int lead = min(kMtN - pos0, count);
-  for (int i = t; i < lead; i += kProducerThreads) raw[start + i] = g.out[pos0 + i];
-  int done = lead;
-  int pos = pos0 + lead;
+  const bool live = t < kMtM, spare = t == kMtM;
+  const int i0 = live ? t : 0;
+  uint64_t a = g.mt[i0], b = g.mt[i0 + kMtM];
+  if (live) {
+    save[t] = a;
+    save[h] = b;
+  }
+  if (t == 0) save[kMtN] = static_cast<uint64_t>(pos0);
+  int done = lead, pos = pos0 + lead;
   uint64_t* cur = g.mt;
-  uint64_t* nxt = alt;
+  uint64_t* nxt = f.mt_alt;
   while (done < count) {
-    const int take = min(kMtN, count - done);
-    if (t < kMtN - kMtM) {
-      const int h = t + kMtM;
-      const uint64_t lo = mt64_mix(cur[t], cur[t + 1], cur[h]);
-      const uint64_t hi = h < kMtN - 1 ? mt64_mix(cur[h], cur[h + 1], lo)
-                                       : mt64_mix(cur[h], mt64_mix(cur[0], cur[1], cur[kMtM]), lo);
+    const uint64_t an = cur[i0 + 1];
+    uint64_t bn = cur[min(i0 + kMtM + 1, kMtN - 1)];
+    const uint64_t lo = mt64_mix(a, an, b);
+    const uint64_t first = __shfl_down_sync(kFull, lo, 1);  // thread 156's word 0, for thread 155
+    if (t == kMtM - 1) bn = first;
+    const uint64_t hi = mt64_mix(b, bn, lo);
+    if (live) {
       nxt[t] = lo;
       nxt[h] = hi;
-      const uint64_t tl = mt64_temper(lo), th = mt64_temper(hi);
-      if (t < take) raw[start + done + t] = tl;
-      if (h < take) raw[start + done + h] = th;
-      if (take < kMtN) {
-        g.out[t] = tl;
-        g.out[h] = th;
-      }
     }
-    // the next regeneration reads what this one wrote and overwrites what it read
+    a = lo;
+    b = hi;
+    pos = min(kMtN, count - done);
+    done += pos;
+    // the next regeneration reads what this one wrote and overwrites what it
+    // read, and what the other warps read of the one before
     producer_sync();
+    if (spare) b = nxt[kMtM];  // thread 156 stands in for word 0 only
     uint64_t* const tmp = cur;
     cur = nxt;
     nxt = tmp;
-    done += take;
-    pos = take;
+    if (done < count) shuffle_step_sync();
   }
-  if (cur != g.mt) {
-    for (int k = t; k < kMtN; k += kProducerThreads) g.mt[k] = cur[k];
+  producer_sync();  // everyone has read g.pos
+  if (live && done > lead) {
+    if (cur != g.mt) {
+      g.mt[t] = a;
+      g.mt[h] = b;
+    }
+    g.out[t] = mt64_temper(a);
+    g.out[h] = mt64_temper(b);
   }
   if (t == 0) g.pos = pos;
-  producer_sync();
+  shuffle_step_sync();
 }
 
 // Swap targets J[i] of every step of the shuffle of G groups.  The producer
-// group streams the engine outputs the pair draws consume into `raw`; the whole CTA then
-// downscales them in parallel.  A rejected draw (Lemire resampling, about one
-// in 2^64/G^2) shifts every later pair by one output: the pairs from the
-// rejection on are redone with the next output appended.
-__device__ void shuffle_targets_block(Fixed& f, uint16_t* J, int G, uint64_t* raw) {
+// group runs the engine on by the outputs of the pair draws; the other warps
+// downscale each regeneration while the next is formed.  One after the other,
+// through global memory, the two took 16.2k cycles for 10000 groups.  A rejected
+// draw (Lemire resampling, about one in 2^64/G^2) shifts every later pair by one
+// output: the shuffle is then drawn again from the saved state, in order.
+__device__ __forceinline__ void shuffle_targets_block(Fixed& f, uint16_t* J, int G, uint64_t* save) {
   if (threadIdx.x == 0) {
     f.i0 = 1;
     if (G >= 2 && (G & 1) == 0) {
       J[1] = static_cast<uint16_t>(draw_below_serial(f.rng, 2));
       f.i0 = 2;
     }
+    f.rejected = 0;
   }
   __syncthreads();
   const int i0 = f.i0;
   const int npairs = (G - i0) >> 1;
   if (npairs <= 0) return;
-  if (threadIdx.x < kProducerThreads) produce_outputs_group(f.rng, f.mt_alt, raw, 0, npairs, threadIdx.x);
-  __syncthreads();
-  int from = 0, shift = 0;
-  for (;;) {
-    if (threadIdx.x == 0) f.first_reject = npairs;
-    __syncthreads();
-    for (int p = from + threadIdx.x; p < npairs; p += kThreads) {
+  if (threadIdx.x < kProducerThreads) {
+    produce_outputs_group(npairs, save);
+  } else {
+    const int t = threadIdx.x - kProducerThreads, pos0 = f.rng.pos, lead = min(kMtN - pos0, npairs);
+    auto place = [&](int p, uint64_t word) {
       const uint64_t b0 = static_cast<uint64_t>(i0 + 2 * p) + 1ull;
       const uint64_t b1 = b0 + 1ull;
       const uint64_t range = b0 * b1;
-      const uint64_t u = raw[p + shift];
+      const uint64_t u = mt64_temper(word);
       const uint64_t lo = u * range;
       if (lo < range && lo < (0ull - range) % range) {
-        atomicMin(&f.first_reject, p);
+        f.rejected = 1;
       } else {
         // x < (G-1)*G < 2^32 for G <= 65535: 32-bit quotient and remainder
         const uint32_t x = static_cast<uint32_t>(__umul64hi(u, range));
@@ -253,16 +389,38 @@ __device__ void shuffle_targets_block(Fixed& f, uint16_t* J, int G, uint64_t* ra
         J[i0 + 2 * p] = static_cast<uint16_t>(qv);
         J[i0 + 2 * p + 1] = static_cast<uint16_t>(x - qv * d1);
       }
+    };
+    // what is left of the old block, while the first regeneration is formed
+    if (t < lead) place(t, f.rng.mt[pos0 + t]);
+    const uint64_t* words = f.mt_alt;
+    const uint64_t* next = f.rng.mt;
+    for (int from = lead; from < npairs; from += kMtN) {
+      shuffle_step_sync();
+      if (t < kMtN && from + t < npairs) place(from + t, words[t]);
+      const uint64_t* const tmp = words;
+      words = next;
+      next = tmp;
     }
-    __syncthreads();
-    const int r = f.first_reject;
-    if (r >= npairs) break;
-    // the output at r + shift was rejected: pairs r.. use one output later
-    if (threadIdx.x < kProducerThreads) produce_outputs_group(f.rng, f.mt_alt, raw, npairs + shift, 1, threadIdx.x);
-    ++shift;
-    from = r;
-    __syncthreads();
+    if (lead == npairs) shuffle_step_sync();
   }
+  __syncthreads();
+  if (f.rejected == 0) return;
+  __syncthreads();
+  for (int k = threadIdx.x; k < kMtN; k += kThreads) {
+    f.rng.mt[k] = save[k];
+    f.rng.out[k] = mt64_temper(save[k]);
+  }
+  if (threadIdx.x == 0) f.rng.pos = static_cast<int>(save[kMtN]);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = i0; i < G; i += 2) {
+      const uint64_t b1 = static_cast<uint64_t>(i) + 2ull;
+      const uint64_t x = draw_below_serial(f.rng, (b1 - 1ull) * b1);
+      J[i] = static_cast<uint16_t>(x / b1);
+      J[i + 1] = static_cast<uint16_t>(x % b1);
+    }
+  }
+  __syncthreads();
 }
 
 // Bucket the steps by swap target, for the targets below lim (the used
@@ -270,27 +428,40 @@ __device__ void shuffle_targets_block(Fixed& f, uint16_t* J, int G, uint64_t* ra
 // the start of bucket q+1.  A group only moves to higher positions (a later
 // step targeting its position p sits at a position above p), so walks that
 // decide membership of [0, lim) never need a bucket at or above lim.
-__device__ void bucket_steps_block(const Smem& s, int G, int lim) {
+__device__ __forceinline__ void bucket_steps_block(const Smem& s, int G, int lim) {
   const uint16_t* J = s.jarr;
   int* cnt = s.scratch32;
   uint16_t* list = s.list;
   for (int q = threadIdx.x; q < lim; q += kThreads) cnt[q] = 0;
   __syncthreads();
-  for (int st = 1 + threadIdx.x; st < G; st += kThreads)
-    if (J[st] < lim) atomicAdd(&cnt[J[st]], 1);
+  for (int i = threadIdx.x; i < row_vectors(G); i += kThreads) {
+    const uint4 v = load_rows(J, i);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int st = 8 * i + e, j = row_code(v, e);
+      if (st >= 1 && st < G && j < lim) atomicAdd(&cnt[j], 1);
+    }
+  }
   __syncthreads();
   block_exclusive_scan(cnt, lim, *s.f);
-  for (int st = 1 + threadIdx.x; st < G; st += kThreads) {
-    if (J[st] >= lim) continue;
-    const int slot = atomicAdd(&cnt[J[st]], 1);
-    list[slot] = static_cast<uint16_t>(st);
+  for (int i = threadIdx.x; i < row_vectors(G); i += kThreads) {
+    const uint4 v = load_rows(J, i);
+    int slot[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int st = 8 * i + e, j = row_code(v, e);
+      slot[e] = st >= 1 && st < G && j < lim ? atomicAdd(&cnt[j], 1) : -1;
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      if (slot[e] >= 0) list[slot[e]] = static_cast<uint16_t>(8 * i + e);
   }
   __syncthreads();
 }
 
 // Group at final position p: last step > q targeting q, else what step q
 // pulled into q (see above).
-__device__ int occupant_of(const Smem& s, int G, int p) {
+__device__ __forceinline__ int occupant_of(const Smem& s, int G, int p) {
   const uint16_t* J = s.jarr;
   const int* cnt = s.scratch32;
   int q = p, t = G - 1;
@@ -315,7 +486,7 @@ __device__ int occupant_of(const Smem& s, int G, int p) {
 // own position.  Positions only grow, so once the position reaches lim (the
 // buckets' limit) the walk stops and returns that position, which is enough
 // for a `< lim` test.
-__device__ int final_position_of(const Smem& s, int e, int lim) {
+__device__ __forceinline__ int final_position_of(const Smem& s, int e, int lim) {
   const int* cnt = s.scratch32;
   int pos = e == 0 ? 0 : s.jarr[e];
   int time = e;
@@ -430,54 +601,78 @@ __device__ __forceinline__ void vote_rows_match(const uint16_t* lab, const uint1
     out[q] = mx[q] == 0 ? -1 : (__popc(tied[q]) == 1 ? best[q] : vote_tiebreak(c[q], tied[q], sc[q], w, lane));
 }
 
-// Rows with no out-of-fold neighbour take the majority label of their
-// training folds (ties to the smaller code); kept out of line, as it is rare.
-__device__ __noinline__ void vote_empty_rows(const EvolveParams& P, const Smem& s, int prob, const uint16_t* lab,
-                                             uint16_t* out, int C0) {
-  const int L = P.L, w = P.w;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint16_t* nbp = P.nb + static_cast<size_t>(prob) * L * w;
-  // per-fold training majority (codes in [0, C0)).  The fold x code counts
-  // sit in s.scratch32 (L ints, free during the vote) when they fit, else in
-  // global memory.
-  const int F = P.F;
-  const bool in_smem = static_cast<long long>(F) * C0 <= L;
-  int* fc = in_smem ? s.scratch32 : P.foldcnt + static_cast<size_t>(prob) * F * P.C0max;
-  const int stride = in_smem ? C0 : P.C0max;
-  for (int i = threadIdx.x; i < F * stride; i += kThreads) fc[i] = 0;
-  for (int c = threadIdx.x; c < C0; c += kThreads) s.aux[c] = 0;
+// Rows with no out-of-fold neighbour take the majority label of their training
+// folds (ties to the smaller code).  P.foldcnt holds the rows per code of every
+// fold and, after the last, of all of them, for the labels being voted on: it is
+// counted once (count_folds) and follows the rows whose label changes
+// (move_fold).  Counting every row again for each vote took 30k cycles of a
+// cycle at 10000 rows and 300 codes.
+__device__ __forceinline__ int* fold_counts(const EvolveParams& P, int prob) {
+  return P.foldcnt + static_cast<size_t>(prob) * (P.F + 1) * P.C0max;
+}
+
+__device__ __forceinline__ void move_fold(const EvolveParams& P, int prob, int row, int from, int to) {
+  int* fc = fold_counts(P, prob);
+  const size_t fold = static_cast<size_t>(P.folds[static_cast<size_t>(prob) * P.L + row]) * P.C0max;
+  const size_t all = static_cast<size_t>(P.F) * P.C0max;
+  atomicSub(&fc[fold + from], 1);
+  atomicAdd(&fc[fold + to], 1);
+  atomicSub(&fc[all + from], 1);
+  atomicAdd(&fc[all + to], 1);
+}
+
+// Lists the rows without neighbours in P.empty_rows (f.empty_cnt of them) and
+// counts the folds of s.cur.
+__device__ __noinline__ void count_folds(const EvolveParams& P, int prob, int C0) {
+  const Smem s = carve_smem_any(P);
+  Fixed& f = *s.f;
+  const uint16_t* nbp = P.nb + static_cast<size_t>(prob) * P.L * P.w;
+  const uint8_t* fo = P.folds + static_cast<size_t>(prob) * P.L;
+  uint16_t* list = P.empty_rows + static_cast<size_t>(blockIdx.x) * P.L;
+  int* fc = fold_counts(P, prob);
+  if (threadIdx.x == 0) f.empty_cnt = 0;
+  if (threadIdx.x < 8) f.empty_folds[threadIdx.x] = 0u;
+  for (int i = threadIdx.x; i < (P.F + 1) * P.C0max; i += kThreads) fc[i] = 0;
   __syncthreads();
-  const uint8_t* fo = P.folds + static_cast<size_t>(prob) * L;
-  for (int r = threadIdx.x; r < L; r += kThreads) {
-    atomicAdd(&fc[fo[r] * stride + lab[r]], 1);
-    atomicAdd(&s.aux[lab[r]], 1);
+  for (int r = threadIdx.x; r < P.L; r += kThreads) {
+    if (nbp[static_cast<size_t>(r) * P.w] == kNoRow) {
+      list[atomicAdd(&f.empty_cnt, 1)] = static_cast<uint16_t>(r);
+      atomicOr(&f.empty_folds[fo[r] >> 5], 1u << (fo[r] & 31));
+    }
+    atomicAdd(&fc[fo[r] * P.C0max + s.cur[r]], 1);
+    atomicAdd(&fc[P.F * P.C0max + s.cur[r]], 1);
   }
   __syncthreads();
+}
+
+__device__ __noinline__ void vote_empty_rows(const EvolveParams& P, int prob, uint16_t* out, int C0) {
+  const Smem s = carve_smem_any(P);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint8_t* fo = P.folds + static_cast<size_t>(prob) * P.L;
+  const uint16_t* list = P.empty_rows + static_cast<size_t>(blockIdx.x) * P.L;
+  const int* fc = fold_counts(P, prob);
+  const int* all = fc + P.F * P.C0max;
   // one warp per fold, its lanes over the codes: the largest training count,
   // ties to the smaller code (the reference scans the codes in ascending
   // order keeping strict improvements)
-  for (int fo_i = warp; fo_i < F; fo_i += kWarps) {
+  for (int fo_i = warp; fo_i < P.F; fo_i += kWarps) {
+    if (((s.f->empty_folds[fo_i >> 5] >> (fo_i & 31)) & 1u) == 0u) continue;
     int bl = 0x7fffffff, bcount = -1;
     for (int c = lane; c < C0; c += 32) {
-      const int cnt = s.aux[c] - fc[fo_i * stride + c];
+      const int cnt = __ldcg(&all[c]) - __ldcg(&fc[fo_i * P.C0max + c]);
       if (cnt > bcount) {
         bl = c;
         bcount = cnt;
       }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const int oc = __shfl_xor_sync(kFull, bcount, o), ol = __shfl_xor_sync(kFull, bl, o);
-      if (oc > bcount || (oc == bcount && ol < bl)) {
-        bcount = oc;
-        bl = ol;
-      }
-    }
-    if (lane == 0) s.order[fo_i] = bl;  // order[] is free here; F <= C0max guaranteed by host
+    const int top = __reduce_max_sync(kFull, bcount);
+    bl = __reduce_min_sync(kFull, bcount == top ? bl : 0x7fffffff);
+    if (lane == 0) s.f->sel_hist[fo_i] = bl;  // F <= 255
   }
   __syncthreads();
-  for (int r = threadIdx.x; r < L; r += kThreads) {
-    if (nbp[static_cast<size_t>(r) * w] == kNoRow) out[r] = static_cast<uint16_t>(s.order[fo[r]]);
+  for (int i = threadIdx.x; i < s.f->empty_cnt; i += kThreads) {
+    const int r = list[i];
+    out[r] = static_cast<uint16_t>(s.f->sel_hist[fo[r]]);
   }
 }
 
@@ -492,7 +687,7 @@ constexpr int kVoteRows = 4;
 // neighbour take the majority label of their training folds (ties to the
 // smaller label).  Neighbour ids are fetched 8 rows at a time per warp so the
 // memory latency is paid once per batch; scores only for tied rows.
-__device__ void vote_block(const EvolveParams& P, const Smem& s, int prob, const uint16_t* lab,
+__device__ __forceinline__ void vote_block(const EvolveParams& P, const Smem& s, int prob, const uint16_t* lab,
                            uint16_t* out, int C0, bool has_empty, const uint16_t* rows = nullptr,
                            int nrows = -1) {
   const int L = P.L, w = P.w;
@@ -531,7 +726,7 @@ __device__ void vote_block(const EvolveParams& P, const Smem& s, int prob, const
       }
     }
   }
-  if (has_empty) vote_empty_rows(P, s, prob, lab, out, C0);
+  if (has_empty) vote_empty_rows(P, prob, out, C0);
   __syncthreads();
 }
 
@@ -539,22 +734,20 @@ __device__ void vote_block(const EvolveParams& P, const Smem& s, int prob, const
 // the rows whose label changed.  Lists them in s.jarr (free after the
 // relabel) and returns how many, or returns -1 when so many rows changed that
 // a full vote is cheaper; either way s.pred starts as a copy of s.curpred.
-//   pass: each warp takes a contiguous range of rows, copies their
-//     predictions, clears their flags and appends its changed rows'
-//     reverse-list bounds to s.list (one shared-counter atomic per warp step
-//     that has any);
+//   pass: eight rows a thread, predictions copied and the changed rows'
+//     reverse-list bounds appended to s.list;
 //   gather: each warp takes four changed rows at a time, its lanes reading 32
-//     reverse entries of each per step (all four rows' loads in flight); the
-//     lane that sets a row's flag first (atomicOr on the flag's word) appends
-//     the row to the list.
+//     reverse entries of each per step (all four rows' loads in flight) and
+//     setting the entries' bits, which returns nothing and waits for nothing;
+//   list: a word of bits per thread, places from a scan over the warp.
 // The list is in no particular order: every listed row is voted on its own.
-__device__ int dirty_rows_block(const EvolveParams& P, const Smem& s, int prob) {
+// Testing each entry's flag and appending it at once made every 32 entries wait
+// for two atomics: 11.0k cycles at 132 changed of 10000 rows.
+__device__ __forceinline__ int dirty_rows_block(const EvolveParams& P, const Smem& s, int prob, bool has_empty) {
   Fixed& f = *s.f;
-  const int L = P.L;
+  const int L = P.L, words = (L + 31) >> 5;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned below = (1u << lane) - 1u;
-  uint8_t* flag = reinterpret_cast<uint8_t*>(s.scratch32);
-  unsigned* flagw = reinterpret_cast<unsigned*>(s.scratch32);
+  unsigned* mark = reinterpret_cast<unsigned*>(s.scratch32);
   int* bounds = reinterpret_cast<int*>(s.list);  // 2 ints per changed row, room for L / 4 rows
   uint16_t* dirty = s.jarr;
   const int cap = L / 4;
@@ -564,24 +757,18 @@ __device__ int dirty_rows_block(const EvolveParams& P, const Smem& s, int prob) 
     f.changed_cnt = 0;
     f.dirty_cnt = 0;
   }
+  for (int i = threadIdx.x; i < words; i += kThreads) mark[i] = 0u;
   __syncthreads();
-  const int chunk = ((L + kWarps - 1) / kWarps + 31) / 32 * 32;
-  const int beg = min(L, warp * chunk), end = min(L, beg + chunk);
-  for (int b = beg; b < end; b += 32) {
-    const int r = b + lane;
-    bool ch = false;
-    if (r < end) {
-      s.pred[r] = s.curpred[r];
-      flag[r] = 0;
-      ch = s.cl[r] != s.cur[r];
-    }
-    const unsigned bm = __ballot_sync(kFull, ch);
-    if (bm != 0u) {
-      int slot0 = 0;
-      if (lane == 0) slot0 = atomicAdd(&f.changed_cnt, __popc(bm));
-      slot0 = __shfl_sync(kFull, slot0, 0);
-      const int slot = slot0 + __popc(bm & below);
-      if (ch && slot < cap) {
+  for (int i = threadIdx.x; i < row_vectors(L); i += kThreads) {
+    reinterpret_cast<uint4*>(s.pred)[i] = load_rows(s.curpred, i);
+    const uint4 a = load_rows(s.cl, i), b = load_rows(s.cur, i);
+    if (a.x == b.x && a.y == b.y && a.z == b.z && a.w == b.w) continue;
+    for (int e = 0; e < 8; ++e) {
+      const int r = 8 * i + e;
+      if (r >= L || row_code(a, e) == row_code(b, e)) continue;
+      if (has_empty) move_fold(P, prob, r, row_code(b, e), row_code(a, e));
+      const int slot = atomicAdd(&f.changed_cnt, 1);
+      if (slot < cap) {
         bounds[2 * slot] = roff[r];
         bounds[2 * slot + 1] = roff[r + 1];
       }
@@ -612,48 +799,64 @@ __device__ int dirty_rows_block(const EvolveParams& P, const Smem& s, int prob) 
         v[q] = k < e[q] ? ridx[k] : kNoRow;
       }
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        bool first = false;
-        if (v[q] != kNoRow) {
-          const unsigned bit = 1u << (8 * (v[q] & 3u));
-          first = (atomicOr(&flagw[v[q] >> 2], bit) & bit) == 0u;
-        }
-        const unsigned fm = __ballot_sync(kFull, first);
-        if (fm != 0u) {
-          int slot0 = 0;
-          if (lane == 0) slot0 = atomicAdd(&f.dirty_cnt, __popc(fm));
-          slot0 = __shfl_sync(kFull, slot0, 0);
-          if (first) dirty[slot0 + __popc(fm & below)] = v[q];
-        }
-      }
+      for (int q = 0; q < 4; ++q)
+        if (v[q] != kNoRow) atomicOr(&mark[v[q] >> 5], 1u << (v[q] & 31u));
     }
+  }
+  __syncthreads();
+  for (int i0 = warp * 32; i0 < words; i0 += kThreads) {
+    unsigned bits = i0 + lane < words ? mark[i0 + lane] : 0u;
+    const int n = __popc(bits);
+    int incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(kFull, incl, o);
+      if (lane >= o) incl += v;
+    }
+    int at = 0;
+    if (lane == 31 && incl > 0) at = atomicAdd(&f.dirty_cnt, incl);
+    at = __shfl_sync(kFull, at, 31) + incl - n;
+    for (; bits != 0u; bits &= bits - 1) dirty[at++] = static_cast<uint16_t>((i0 + lane) * 32 + __ffs(bits) - 1);
   }
   __syncthreads();
   return f.dirty_cnt;
 }
 
 // Count labels of `lab` per code, first positions and distinct count.
-// have_cnt: s.cnt already holds the counts of `lab` (absorption_block counted
-// the same labels and left them unchanged).  A thread's rows come in
-// increasing order and a first position only decreases, so a row at or past
-// the current first position of its code needs no atomicMin: the plain read
-// filters nearly all of them after the first rows of each code.
+// have_cnt: s.cnt already holds the counts of `lab`.  The first kThreads rows
+// set the first positions; of the others, taken eight to a thread, only those
+// before their code's first position so far need an atomicMin: nearly none.
 // pred != nullptr: *ok also receives the count of rows with lab == pred
 // (both totals from one block reduction: ok + 2^16 nc, L and C0 < 2^15).
-__device__ int label_census(const EvolveParams& P, const Smem& s, const uint16_t* lab, int C0,
+__device__ __forceinline__ int label_census(const EvolveParams& P, const Smem& s, const uint16_t* lab, int C0,
                             bool have_cnt = false, const uint16_t* pred = nullptr, int* ok = nullptr) {
   for (int c = threadIdx.x; c < C0; c += kThreads) {
     if (!have_cnt) s.cnt[c] = 0;
     s.firstpos[c] = 0x7fffffff;
   }
   __syncthreads();
-  volatile int* fp = s.firstpos;
-  int hits = 0;
-  for (int r = threadIdx.x; r < P.L; r += kThreads) {
-    const int code = lab[r];
-    if (pred != nullptr) hits += code == pred[r];
+  if (threadIdx.x < P.L) {
+    const int r = threadIdx.x, code = lab[r];
     if (!have_cnt) atomicAdd(&s.cnt[code], 1);
-    if (r < fp[code]) atomicMin(&s.firstpos[code], r);
+    atomicMin(&s.firstpos[code], r);
+  }
+  __syncthreads();
+  int hits = 0;
+  for (int i = threadIdx.x; i < row_vectors(P.L); i += kThreads) {
+    const uint4 v = load_rows(lab, i);
+    const uint4 u = pred != nullptr ? load_rows(pred, i) : v;
+    int first[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) first[e] = 8 * i + e < P.L ? s.firstpos[row_code(v, e)] : 0;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int r = 8 * i + e;
+      if (r >= P.L) break;
+      const int code = row_code(v, e);
+      hits += code == row_code(u, e);
+      if (!have_cnt && r >= kThreads) atomicAdd(&s.cnt[code], 1);
+      if (r < first[e]) atomicMin(&s.firstpos[code], r);
+    }
   }
   __syncthreads();
   int local = 0;
@@ -666,17 +869,26 @@ __device__ int label_census(const EvolveParams& P, const Smem& s, const uint16_t
 
 // s.order[0..nc) = the codes of the census in the iteration order of
 // std::unordered_map<int,int> after reserve(L) and insertion in row order.
-__device__ __noinline__ void map_order(const EvolveParams& P, const Smem& s, int prob, int C0) {
+__device__ __forceinline__ void map_order(const EvolveParams& P, const Smem& s, int prob, int C0) {
   const bool nocollide = P.nocollide[prob] != 0;
   if (nocollide) {
     // every key has its own bucket: each new key goes to the list front, so
     // a key's rank counts the keys first seen after it (one warp per key)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int kHeld = 10;  // first positions a lane keeps in registers
+    int held[kHeld];
+#pragma unroll
+    for (int q = 0; q < kHeld; ++q) {
+      const int c = lane + 32 * q;
+      held[q] = c < C0 && s.cnt[c] > 0 ? s.firstpos[c] : -1;
+    }
     for (int c = warp; c < C0; c += kWarps) {
       if (s.cnt[c] == 0) continue;
       int rank = 0;
       const int fp = s.firstpos[c];
-      for (int c2 = lane; c2 < C0; c2 += 32) rank += (s.cnt[c2] > 0 && s.firstpos[c2] > fp);
+#pragma unroll
+      for (int q = 0; q < kHeld; ++q) rank += held[q] > fp;
+      for (int c2 = lane + 32 * kHeld; c2 < C0; c2 += 32) rank += (s.cnt[c2] > 0 && s.firstpos[c2] > fp);
       rank = __reduce_add_sync(kFull, rank);
       if (lane == 0) s.order[rank] = c;
     }
@@ -718,219 +930,306 @@ __device__ __noinline__ void map_order(const EvolveParams& P, const Smem& s, int
   __syncthreads();
 }
 
-// core_objective_score for the kNN classifier; census must be current.
-__device__ double objective(const EvolveParams& P, const Smem& s, int prob, double acc, int nc, int C0) {
+// Accuracy of `ok` hits and core_objective_score for the kNN classifier, in
+// f.acc and f.score; census must be current.  Double operations are left to
+// single warps: one of the whole block takes the FP64 pipe 512 cycles, a
+// division 4400.
+__device__ __forceinline__ void objective(const EvolveParams& P, const Smem& s, int prob, int ok, int nc, int C0) {
+  Fixed& f = *s.f;
   const bool use_div = P.guarded && P.pol_diversity;
   const bool reject1 = P.guarded && P.pol_reject1;
-  if (!use_div && !reject1) return acc;
-  if (reject1 && nc == 1) return -INFINITY;
-  if (!use_div) return acc;
-  map_order(P, s, prob, C0);
-  if (threadIdx.x < 32) {
-    // psq[c] = (c/L)*(c/L) rounded as the reference rounds each step; the
-    // warp loads the terms, lane 0 adds them in iteration order
-    for (int q = threadIdx.x; q < nc; q += 32) s.cp[q] = P.psq[s.cnt[s.order[q]]];
-    __syncwarp();
-    if (threadIdx.x == 0) {
-      double same = 0.0;
-      for (int q = 0; q < nc; ++q) same = __dadd_rn(same, s.cp[q]);
-      const double diff = __dsub_rn(1.0, same);
-      const double dlp = (0.0 < diff) ? diff : 0.0;
-      s.f->score = __dmul_rn(acc, __dsqrt_rn(dlp));
-    }
+  if (threadIdx.x == 32) f.acc = __ddiv_rn(static_cast<double>(ok), static_cast<double>(P.L));
+  const bool ranked = use_div && !(reject1 && nc == 1);
+  if (ranked) {
+    map_order(P, s, prob, C0);
+    // psq[c] = (c/L)*(c/L) rounded as the reference rounds each step
+    for (int q = threadIdx.x; q < nc; q += kThreads) s.cp[q] = P.psq[s.cnt[s.order[q]]];
   }
   __syncthreads();
-  const double out = s.f->score;
-  __syncthreads();
-  return out;
+  if (threadIdx.x < 32) {
+    const double acc = f.acc;
+    double score = reject1 && nc == 1 ? -INFINITY : acc;
+    if (ranked) {
+      const double diff = __dsub_rn(1.0, chain_add(0.0, s.cp, nc));
+      score = __dmul_rn(acc, __dsqrt_rn((0.0 < diff) ? diff : 0.0));
+    }
+    if (threadIdx.x == 0) f.score = score;
+  }
 }
 
-// propose_many_to_one_absorption on s.cl given proposal predictions pp.
-// Returns 1 if the labels changed.
-__device__ int absorption_block(const EvolveParams& P, const Smem& s, int prob, const uint16_t* pp, int C0) {
-  Fixed& f = *s.f;
-  int* tr = s.trans;
-  const int C = P.C0max;
-  for (int i = threadIdx.x; i < C0 * C; i += kThreads) tr[i] = 0;
+// Groups the rows of s.cl by code: s.cnt[c] rows of which s.movable[c] are not
+// fixed, their predictions pp at s.list[class_start(s, c)..], in no particular
+// order.  A row's place in its class is what the count's atomicAdd returned
+// (kept in s.jarr).  Returns the number of codes in use.
+__device__ __forceinline__ int class_start(const Smem& s, int c) { return s.aux[c] & 0xffff; }
+__device__ __forceinline__ int class_groups(const EvolveParams& P, const Smem& s, const uint16_t* pp, int C0) {
+  const bool any_fixed = s.f->fxd != nullptr;
   for (int c = threadIdx.x; c < C0; c += kThreads) {
     s.cnt[c] = 0;
     s.movable[c] = 0;
-    s.bt[c] = -1;
   }
   __syncthreads();
-  // one atomic per row into the table: with the table in shared memory the
-  // class sizes are its row sums; with it in global memory a second,
-  // shared-memory atomic per row counts them.  Without fixed rows every row
-  // is movable.
-  const bool any_fixed = s.f->fxd != nullptr;
-  const bool count_rows = !P.smem_trans;
-  for (int r = threadIdx.x; r < P.L; r += kThreads) {
-    const int a = s.cl[r];
-    atomicAdd(&tr[a * C + pp[r]], 1);
-    if (count_rows) atomicAdd(&s.cnt[a], 1);
-    if (any_fixed && s.f->fxd[r] != 1) atomicAdd(&s.movable[a], 1);
+  for (int i = threadIdx.x; i < row_vectors(P.L); i += kThreads) {
+    const uint4 v = load_rows(s.cl, i);
+    unsigned at[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int r = 8 * i + e;
+      at[e] = r < P.L ? atomicAdd(&s.cnt[row_code(v, e)], 1) : 0;
+      if (any_fixed && r < P.L && s.f->fxd[r] != 1) atomicAdd(&s.movable[row_code(v, e)], 1);
+    }
+    reinterpret_cast<uint4*>(s.jarr)[i] =
+        make_uint4(at[0] | at[1] << 16, at[2] | at[3] << 16, at[4] | at[5] << 16, at[6] | at[7] << 16);
   }
   __syncthreads();
+  // starts (below 2^16) and codes in use in one scan
+  for (int c = threadIdx.x; c < C0; c += kThreads) s.aux[c] = s.cnt[c] > 0 ? s.cnt[c] + 0x10000 : 0;
+  __syncthreads();
+  const int nc = static_cast<int>(static_cast<unsigned>(block_exclusive_scan(s.aux, C0, *s.f) - P.L) >> 16);
+  for (int i = threadIdx.x; i < row_vectors(P.L); i += kThreads) {
+    const uint4 v = load_rows(s.cl, i), u = load_rows(pp, i), at = load_rows(s.jarr, i);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      if (8 * i + e >= P.L) break;
+      s.list[class_start(s, row_code(v, e)) + row_code(at, e)] = static_cast<uint16_t>(row_code(u, e));
+    }
+  }
+  if (!any_fixed)
+    for (int c = threadIdx.x; c < C0; c += kThreads) s.movable[c] = s.cnt[c];
+  __syncthreads();
+  return nc;
+}
+
+// Calls use(src, n, items, each, h) for every code src in use with movable rows,
+// by one warp of those that have counters: n rows, h[c] of them predicted as c
+// (zero again afterwards).  each(i) for i < items runs over the codes
+// predicted, some of them repeatedly (a small class: its rows' predictions) or
+// not at all (a large one: all codes).
+template <class Use>
+__device__ __forceinline__ void for_each_source(const Smem& s, int C0, Use&& use) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int local = 0;
-  if (count_rows) {
-    for (int c = threadIdx.x; c < C0; c += kThreads) {
-      if (!any_fixed) s.movable[c] = s.cnt[c];
-      local += s.cnt[c] > 0;
+  if (warp >= s.hist_warps) return;
+  int* h = s.hist + static_cast<size_t>(warp) * s.hist_stride;
+  for (int src = warp; src < C0; src += s.hist_warps) {
+    const int n = s.cnt[src];
+    if (n == 0 || s.movable[src] <= 0) continue;
+    const uint16_t* seg = s.list + class_start(s, src);
+    int i = lane;
+    for (; i + 96 < n; i += 128) {
+      int c[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) c[q] = seg[i + 32 * q];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) atomicAdd(&h[c[q]], 1);
     }
-  } else {
-    // class sizes: one warp per class, its lanes over the predictions
-    for (int c = warp; c < C0; c += kWarps) {
-      int sz = 0;
-      for (int q = lane; q < C0; q += 32) sz += tr[c * C + q];
-      sz = __reduce_add_sync(kFull, sz);
-      if (lane == 0) {
-        s.cnt[c] = sz;
-        if (!any_fixed) s.movable[c] = sz;
-        local += sz > 0;
-      }
-    }
+    for (; i < n; i += 32) atomicAdd(&h[seg[i]], 1);
+    __syncwarp();
+    const bool members = n < C0;
+    const int items = members ? n : C0;
+    auto each = [&](int k) { return members ? static_cast<int>(seg[k]) : k; };
+    use(src, n, items, each, h);
+    __syncwarp();
+    for (int k = lane; k < items; k += 32) h[each(k)] = 0;
+    __syncwarp();
   }
-  const int nc = block_sum(local, f);  // its barriers also publish the sizes
+}
+
+// propose_many_to_one_absorption on s.cl given proposal predictions pp.
+// Returns 1 if the labels changed.  On return s.cnt holds the counts of s.cl.
+// The class x prediction counts are never laid out: a source only meets the
+// predictions of its own rows, which its warp counts and reads back.  With a
+// C0 x C0 table (in global memory past 200 codes), a scan of it, double
+// divisions in every warp and the choice in one thread this took 18.6k cycles
+// of a cycle at 10000 rows and 50 codes, 54k at 750 and 100, 138k at 10000 and 300.
+__device__ __forceinline__ int absorption_block(const EvolveParams& P, const Smem& s, int prob, const uint16_t* pp, int C0) {
+  Fixed& f = *s.f;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int c = threadIdx.x; c < C0; c += kThreads) s.bt[c] = -1;
+  const int nc = class_groups(P, s, pp, C0);
   if (nc <= 2) return 0;
   const double n = static_cast<double>(P.L);
   const double nmax = (1.0 < n) ? n : 1.0;  // std::max(1.0, n)
-  // one warp per source, its lanes over the destinations.  The reference
-  // scans the destinations in ascending order keeping the best by
+  // The reference scans the destinations in ascending order keeping the best by
   // (surplus, count, destination size, smaller destination), starting from
-  // (0, 0, source size, source): that is the lexicographic maximum of those
-  // keys, found here by a warp reduction.
-  for (int src = warp; src < C0; src += kWarps) {
-    const int ssize = s.cnt[src];
-    if (ssize == 0 || s.movable[src] <= 0) continue;
-    const int* row = tr + src * C;
-    const int stay = row[src];
-    // exact surplus x n = cnt*n - ssize*dsize; only the candidates at the
-    // exact maximum can win the double comparison chain (double rounding is
-    // far below the 1/n spacing of distinct exact surpluses)
-    long long kmax = -0x7fffffffffffffffll;
-#pragma unroll 4
-    for (int dst = lane; dst < C0; dst += 32) {
-      const int cntd = row[dst];
-      const int dsize = s.cnt[dst];
-      if (dst == src || cntd == 0 || dsize == 0) continue;
-      const long long kx = static_cast<long long>(cntd) * P.L - static_cast<long long>(ssize) * dsize;
-      if (kx > kmax) kmax = kx;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const long long other = __shfl_xor_sync(kFull, kmax, o);
-      if (other > kmax) kmax = other;
-    }
-    int bt = src, bcount = 0, bsize = ssize;
-    double bsur = 0.0;
-    bool cand = false;
-#pragma unroll 4
-    for (int dst = lane; dst < C0; dst += 32) {
-      const int cntd = row[dst];
-      const int dsize = s.cnt[dst];
-      if (dst == src || cntd == 0 || dsize == 0) continue;
-      if (static_cast<long long>(cntd) * P.L - static_cast<long long>(ssize) * dsize != kmax) continue;
-      cand = true;
-      const double expected = __ddiv_rn(__dmul_rn(static_cast<double>(ssize), static_cast<double>(dsize)), nmax);
-      const double sur = __dsub_rn(static_cast<double>(cntd), expected);
-      if (sur > bsur || (sur == bsur && cntd > bcount) || (sur == bsur && cntd == bcount && dsize > bsize) ||
-          (sur == bsur && cntd == bcount && dsize == bsize && dst < bt)) {
-        bt = dst;
-        bsize = dsize;
-        bcount = cntd;
-        bsur = sur;
+  // (0, 0, source size, source).  Exact surplus x n = cnt*n - ssize*dsize; only
+  // the candidates at the exact maximum can win the double comparison chain
+  // (double rounding is far below the 1/n spacing of distinct exact surpluses).
+  // Candidates there with one count have one size and one double surplus, so
+  // the smallest wins; with several counts (rare) the doubles are compared.
+  for_each_source(s, C0, [&](int src, int ssize, int items, auto&& each, const int* h) {
+    const int stay = h[src];
+    // both products are below 2^32, and a surplus of zero or less is no move
+    unsigned kmax = 0;
+    int kcnt = 0, kdst = 0x7fffffff;
+    bool mixed = false;
+    const unsigned size = static_cast<unsigned>(ssize), rows = static_cast<unsigned>(P.L);
+    for (int i = lane; i < items; i += 32) {
+      const int dst = each(i), cntd = h[dst], dsize = s.cnt[dst];
+      const unsigned a = cntd * rows, b = size * dsize;
+      if (dst == src || dsize == 0 || a <= b) continue;  // (a count of zero is never a surplus)
+      if (a - b > kmax) {
+        kmax = a - b;
+        kcnt = cntd;
+        kdst = dst;
+        mixed = false;
+      } else if (a - b == kmax) {
+        mixed |= cntd != kcnt;
+        kdst = min(kdst, dst);
       }
     }
-    const unsigned cands = __ballot_sync(kFull, cand);
-    if (cands == 0u) continue;
-    if ((cands & (cands - 1u)) == 0u) {
-      // one lane holds every candidate: its best is the warp's
-      const int ld = __ffs(cands) - 1;
-      bt = __shfl_sync(kFull, bt, ld);
-      bcount = __shfl_sync(kFull, bcount, ld);
-      bsur = __shfl_sync(kFull, bsur, ld);
-    } else {
+    const unsigned top = __reduce_max_sync(kFull, kmax);
+    if (top == 0u) return;
+    const bool cand = kmax == top;
+    const int bcount = __reduce_max_sync(kFull, cand ? kcnt : 0);
+    int bt = __reduce_min_sync(kFull, cand ? kdst : 0x7fffffff);
+    int count = bcount;
+    if (__any_sync(kFull, cand && (mixed || kcnt != bcount))) {
+      int bsize = ssize;
+      double bsur = 0.0;
+      bt = src;
+      count = 0;
+      for (int i = lane; i < items; i += 32) {
+        const int dst = each(i), cntd = h[dst], dsize = s.cnt[dst];
+        if (dst == src || dsize == 0) continue;
+        const unsigned a = cntd * rows, b = size * dsize;
+        if (a <= b || a - b != top) continue;
+        const double expected = __ddiv_rn(__dmul_rn(static_cast<double>(ssize), static_cast<double>(dsize)), nmax);
+        const double sur = __dsub_rn(static_cast<double>(cntd), expected);
+        if (sur > bsur || (sur == bsur && cntd > count) || (sur == bsur && cntd == count && dsize > bsize) ||
+            (sur == bsur && cntd == count && dsize == bsize && dst < bt)) {
+          bt = dst;
+          bsize = dsize;
+          count = cntd;
+          bsur = sur;
+        }
+      }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double osur = __shfl_xor_sync(kFull, bsur, o);
-      const int ocount = __shfl_xor_sync(kFull, bcount, o);
-      const int osize = __shfl_xor_sync(kFull, bsize, o);
-      const int obt = __shfl_xor_sync(kFull, bt, o);
-      if (osur > bsur || (osur == bsur && ocount > bcount) || (osur == bsur && ocount == bcount && osize > bsize) ||
-          (osur == bsur && ocount == bcount && osize == bsize && obt < bt)) {
-        bt = obt;
-        bsize = osize;
-        bcount = ocount;
-        bsur = osur;
+      for (int o = 16; o > 0; o >>= 1) {
+        const double osur = __shfl_xor_sync(kFull, bsur, o);
+        const int ocount = __shfl_xor_sync(kFull, count, o);
+        const int osize = __shfl_xor_sync(kFull, bsize, o);
+        const int obt = __shfl_xor_sync(kFull, bt, o);
+        if (osur > bsur || (osur == bsur && ocount > count) || (osur == bsur && ocount == count && osize > bsize) ||
+            (osur == bsur && ocount == count && osize == bsize && obt < bt)) {
+          bt = obt;
+          bsize = osize;
+          count = ocount;
+          bsur = osur;
+        }
       }
     }
-    }
-    if (lane == 0 && !(bt == src || bsur <= 0.0 || bcount <= stay)) {
+    if (lane == 0 && bt != src && count > stay) {
       s.bt[src] = bt;
-      s.bsur[src] = bsur;
+      s.order[src] = count;
+    }
+  });
+  __syncthreads();
+  // the surpluses, a thread per source; s.firstpos[t] becomes the last source of
+  // target t and s.aux[t] (whose class starts are not needed any more) how many
+  for (int c = threadIdx.x; c < C0; c += kThreads) {
+    s.aux[c] = 0;
+    s.firstpos[c] = 0;
+  }
+  __syncthreads();
+  for (int src = threadIdx.x; src < C0; src += kThreads) {
+    const int bt = s.bt[src];
+    if (bt < 0) continue;
+    const double expected =
+        __ddiv_rn(__dmul_rn(static_cast<double>(s.cnt[src]), static_cast<double>(s.cnt[bt])), nmax);
+    const double sur = __dsub_rn(static_cast<double>(s.order[src]), expected);
+    if (sur > 0.0) {
+      s.bsur[src] = sur;
+      atomicAdd(&s.aux[bt], 1);
+      atomicMax(&s.firstpos[bt], src);
+    } else {
+      s.bt[src] = -1;
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    // per-target weights accumulated in ascending source order
-    for (int c = 0; c < C0; ++c) {
-      s.aux[c] = 0;
-      s.weight[c] = 0.0;
+  // per-target weights accumulated in ascending source order, a warp per target
+  // of several sources
+  for (int t = warp; t < C0; t += kWarps) {
+    const int k = s.aux[t];
+    if (k == 0) continue;
+    if (k == 1) {
+      if (lane == 0) s.weight[t] = s.bsur[s.firstpos[t]];
+      continue;
     }
-    for (int src = 0; src < C0; ++src) {
-      const int t = s.bt[src];
-      if (t < 0) continue;
-      s.weight[t] = __dadd_rn(s.weight[t], s.bsur[src]);
-      s.aux[t] += 1;
+    double weight = 0.0;
+    for (int c0 = 0; c0 < C0; c0 += 32) {
+      const unsigned m = __ballot_sync(kFull, c0 + lane < C0 && s.bt[min(c0 + lane, C0 - 1)] == t);
+      if (m == 0u) continue;
+      const double mine = (m >> lane) & 1u ? s.bsur[c0 + lane] : 0.0;
+      for (unsigned rem = m; rem != 0u; rem &= rem - 1)
+        weight = __dadd_rn(weight, __shfl_sync(kFull, mine, __ffs(rem) - 1));
     }
-    int nmulti = 0, nsingle = 0;
-    for (int t = 0; t < C0; ++t) {
-      if (s.aux[t] > 1) ++nmulti;
-      else if (s.aux[t] == 1) ++nsingle;
-    }
-    int sel = -1;
-    if (nmulti + nsingle > 0) {
-      const int want_multi = nmulti > 0;
-      int k = 0;
-      for (int t = 0; t < C0; ++t) {
-        if (s.aux[t] == 0 || (s.aux[t] > 1) != (want_multi != 0)) continue;
-        s.order[k] = t;
-        s.cp[C0 + k] = s.weight[t] > DBL_MIN ? s.weight[t] : DBL_MIN;  // std::max(weight, DBL_MIN)
-        ++k;
+    if (lane == 0) s.weight[t] = weight;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    // the targets of several sources, or where there are none those of one
+    bool multi = false;
+    for (int c = lane; c < C0; c += 32) multi |= s.aux[c] > 1;
+    multi = __any_sync(kFull, multi);
+    int k = 0;
+    for (int c0 = 0; c0 < C0; c0 += 32) {
+      const int t = c0 + lane;
+      const int a = t < C0 ? s.aux[t] : 0;
+      const bool in = multi ? a > 1 : a == 1;
+      const unsigned m = __ballot_sync(kFull, in);
+      if (in) {
+        const int at = k + __popc(m & ((1u << lane) - 1u));
+        s.order[at] = t;
+        s.cp[C0 + at] = s.weight[t] > DBL_MIN ? s.weight[t] : DBL_MIN;  // std::max(weight, DBL_MIN)
       }
-      const int pick = discrete_serial(f.rng, s.cp + C0, k, s.cp);
-      sel = s.order[pick];
+      k += __popc(m);
     }
-    f.selected_target = sel;
-  }
-  __syncthreads();
-  const int sel = f.selected_target;
-  if (sel < 0) return 0;
-  // sizes after remapping every non-fixed row of the selected sources
-  if (threadIdx.x == 0) {
-    int moved = 0;
-    int after = 0;
-    for (int c = 0; c < C0; ++c) {
-      int size = s.cnt[c];
-      if (s.bt[c] == sel && c != sel) {
-        moved += s.movable[c];
-        size -= s.movable[c];
+    __syncwarp();
+    int sel = -1, apply = 0;
+    if (k > 0) {
+      sel = s.order[discrete_warp(f.rng, s.cp + C0, k, s.cp, lane)];
+      // sizes after remapping every non-fixed row of the selected sources
+      int moved = 0, after = 0;
+      for (int c = lane; c < C0; c += 32) {
+        int size = s.cnt[c];
+        if (s.bt[c] == sel && c != sel) {
+          moved += s.movable[c];
+          size -= s.movable[c];
+        }
+        s.aux[c] = size;
+        after += c != sel && size > 0;
       }
-      s.aux[c] = size;
+      moved = __reduce_add_sync(kFull, moved);
+      __syncwarp();
+      if (lane == 0) {
+        s.aux[sel] += moved;
+        after += s.aux[sel] > 0;
+      }
+      after = __reduce_add_sync(kFull, after);
+      apply = moved > 0 && after > 1 && after < nc;
     }
-    s.aux[sel] += moved;
-    for (int c = 0; c < C0; ++c) after += s.aux[c] > 0;
-    f.flag = (moved > 0 && after > 1 && after < nc) ? 1 : 0;
+    if (lane == 0) {
+      f.selected_target = sel;
+      f.flag = apply;
+    }
   }
   __syncthreads();
-  const int apply = f.flag;
+  const int sel = f.selected_target, apply = f.flag;
   if (apply) {
-    for (int r = threadIdx.x; r < P.L; r += kThreads) {
-      const int a = s.cl[r];
-      if (s.f->fxd != nullptr && s.f->fxd[r] == 1) continue;
-      if (a != sel && s.bt[a] == sel) s.cl[r] = static_cast<uint16_t>(sel);
+    for (int i = threadIdx.x; i < row_vectors(P.L); i += kThreads) {
+      const uint4 v = load_rows(s.cl, i);
+      int to[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) to[e] = 8 * i + e < P.L ? s.bt[row_code(v, e)] : -1;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int r = 8 * i + e;
+        if (to[e] != sel || row_code(v, e) == sel) continue;
+        if (s.f->fxd != nullptr && s.f->fxd[r] == 1) continue;
+        s.cl[r] = static_cast<uint16_t>(sel);
+      }
     }
+    for (int c = threadIdx.x; c < C0; c += kThreads) s.cnt[c] = s.aux[c];
   }
   __syncthreads();
   return apply;
@@ -938,7 +1237,8 @@ __device__ int absorption_block(const EvolveParams& P, const Smem& s, int prob, 
 
 // Relabel of sampled groups when draws are needed (groups of several rows, or
 // no prediction guidance).  Thread 0, in shuffled order.
-__device__ __noinline__ void relabel_serial(const EvolveParams& P, const Smem& s, const uint16_t* pp, int ns, int C0) {
+__device__ __noinline__ void relabel_serial(const EvolveParams& P, const uint16_t* pp, int ns, int C0) {
+  const Smem s = carve_smem_any(P);
   Fixed& f = *s.f;
   int* hist = s.aux;
   for (int c = 0; c < C0; ++c) hist[c] = 0;
@@ -1007,7 +1307,7 @@ __device__ __noinline__ void relabel_serial(const EvolveParams& P, const Smem& s
 // prediction and whose label equals their prediction; the sizes of its label
 // and prediction classes; the run's progress; the fraction of valid
 // neighbours.
-__device__ void proposal_features(const EvolveParams& P, const Smem& s, int prob, int row, const int* cnt_cur,
+__device__ __forceinline__ void proposal_features(const EvolveParams& P, const Smem& s, int prob, int row, const int* cnt_cur,
                                   float progress, float* f) {
   const uint16_t* nbr = P.nb + (static_cast<size_t>(prob) * P.L + row) * P.w;
   const int c = s.cur[row], q = s.curpred[row];
@@ -1035,7 +1335,7 @@ __device__ void proposal_features(const EvolveParams& P, const Smem& s, int prob
 }
 
 // Census of s.cur into s.aux (per code).
-__device__ void census_cur(const EvolveParams& P, const Smem& s, int C0) {
+__device__ __forceinline__ void census_cur(const EvolveParams& P, const Smem& s, int C0) {
   for (int c = threadIdx.x; c < C0; c += kThreads) s.aux[c] = 0;
   __syncthreads();
   for (int r = threadIdx.x; r < P.L; r += kThreads) atomicAdd(&s.aux[s.cur[r]], 1);
@@ -1062,7 +1362,8 @@ __device__ __forceinline__ float gumbel_noise(uint64_t seed, int cycle, int row)
 // replacement from the network's softmax over the candidates) above the row,
 // so all keys are distinct and ties go to the smaller row.  The take-th
 // largest key is found by a 4-pass radix select with 8-bit digits.
-__device__ __noinline__ void learned_flip(const EvolveParams& P, const Smem& s, int prob, int cycle, int take, int C0) {
+__device__ __noinline__ void learned_flip(const EvolveParams& P, int prob, int cycle, int take, int C0) {
+  const Smem s = carve_smem_any(P);
   Fixed& f = *s.f;
   if (take <= 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1161,7 +1462,8 @@ __device__ __noinline__ void learned_flip(const EvolveParams& P, const Smem& s, 
 
 // Training snapshot of the current state: features of every row and its
 // label / prediction codes.
-__device__ __noinline__ void snapshot_state(const EvolveParams& P, const Smem& s, int prob, int cycle, int C0) {
+__device__ __noinline__ void snapshot_state(const EvolveParams& P, int prob, int cycle, int C0) {
+  const Smem s = carve_smem_any(P);
   census_cur(P, s, C0);
   const float progress = static_cast<float>(cycle) / static_cast<float>(P.T > 0 ? P.T : 1);
   for (int r = threadIdx.x; r < P.L; r += kThreads) {
@@ -1178,7 +1480,7 @@ __device__ __noinline__ void snapshot_state(const EvolveParams& P, const Smem& s
 // Points the CTA at problem prob's groups and fixed flags: shared by all
 // problems, or one block per problem (per_problem_groups: goff stride L + 1,
 // gmem and fixed stride L, group count gcount[prob]).
-__device__ __noinline__ void bind_groups(const EvolveParams& P, const Smem& s, int prob) {
+__device__ __forceinline__ void bind_groups(const EvolveParams& P, const Smem& s, int prob) {
   if (threadIdx.x == 0) {
     const bool per = P.per_problem_groups != 0;
     s.f->goff = P.goff + (per ? static_cast<size_t>(prob) * (P.L + 1) : 0);
@@ -1189,12 +1491,61 @@ __device__ __noinline__ void bind_groups(const EvolveParams& P, const Smem& s, i
   __syncthreads();
 }
 
-__device__ void evolve_problem(const EvolveParams& P, const Smem& s, int prob) {
+// Each of the first ns groups of the shuffle takes its own CV prediction; only
+// groups whose prediction differs from their label can change, so just those
+// are listed (in s.perm) and walked forward to their final shuffled position:
+// walked as they were met, a few lanes of a warp at a time walked while the
+// others waited.
+__device__ __forceinline__ void flip_sampled(const Smem& s, int G, int ns) {
+  Fixed& f = *s.f;
+  const int lane = threadIdx.x & 31;
+  const int* gmem = f.gmem;
+  if (threadIdx.x == 0) f.walk_cnt = 0;
+  __syncthreads();
+  for (int g0 = threadIdx.x; g0 - lane < G; g0 += 4 * kThreads) {
+    int row[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) row[q] = g0 + q * kThreads < G ? gmem[g0 + q * kThreads] : -1;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const bool walk = row[q] >= 0 && s.curpred[row[q]] != s.cur[row[q]] && (f.fxd == nullptr || f.fxd[row[q]] != 1);
+      const unsigned m = __ballot_sync(kFull, walk);
+      if (m == 0u) continue;
+      int at = 0;
+      if (lane == 0) at = atomicAdd(&f.walk_cnt, __popc(m));
+      at = __shfl_sync(kFull, at, 0);
+      if (walk) s.perm[at + __popc(m & ((1u << lane) - 1u))] = static_cast<uint16_t>(g0 + q * kThreads);
+    }
+  }
+  __syncthreads();
+  const int count = f.walk_cnt;
+  for (int i = threadIdx.x; i < count; i += kThreads) {
+    const int g = s.perm[i], row = gmem[g];
+    if (final_position_of(s, g, ns) < ns) s.cl[row] = s.curpred[row];
+  }
+}
+
+// u < exp(delta / temperature), delta < 0: in floats where they leave no doubt
+// (their quotient is within 3e-7 of itself, so expf of one above -80 within
+// 3e-5 of the double), else in doubles, whose exp takes 2000 cycles.
+__device__ __forceinline__ int annealed(double u, double delta, double temperature) {
+  const float x = static_cast<float>(delta) / static_cast<float>(temperature);
+  const float v = static_cast<float>(u);
+  if (x > -80.0f) {
+    const float e = expf(x);
+    if (v > e * 1.0001f) return 0;
+    if (v < e * 0.9999f) return 1;
+  } else if (x <= -80.0f && v > 1e-30f) {
+    return 0;
+  }
+  return u < exp(__ddiv_rn(delta, temperature));
+}
+
+__device__ __forceinline__ void evolve_problem(const EvolveParams& P, const Smem& s, int prob) {
   Fixed& f = *s.f;
   bind_groups(P, s, prob);
   const int L = P.L, T = P.T, G = f.G;
   const int C0 = P.ncodes[prob];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint16_t* init = P.init + static_cast<size_t>(prob) * L;
   uint16_t* gbest = P.clbest + static_cast<size_t>(prob) * L;
   uint16_t* gbestpred = P.cvpredbest + static_cast<size_t>(prob) * L;
@@ -1217,6 +1568,8 @@ __device__ void evolve_problem(const EvolveParams& P, const Smem& s, int prob) {
   __syncthreads();
   const bool has_empty = block_sum(local_empty, f) > 0;
 
+  if (has_empty) count_folds(P, prob, C0);
+
   // initial evaluation
   vote_block(P, s, prob, s.cur, s.curpred, C0, has_empty);
   int ok = 0;
@@ -1226,41 +1579,43 @@ __device__ void evolve_problem(const EvolveParams& P, const Smem& s, int prob) {
     gbestpred[r] = s.curpred[r];
   }
   ok = block_sum(ok, f);
-  const double n = static_cast<double>(L);
-  double accbest = __ddiv_rn(static_cast<double>(ok), n);
-  int nc_cur = label_census(P, s, s.cur, C0);
-  double scorebest = objective(P, s, prob, accbest, nc_cur, C0);
-  double cur_acc = accbest, cur_score = scorebest;
-  int nc_best = nc_cur;
-  int proposals = 0, best_updates = 0, accepts = 0, st_att = 0, st_acc = 0, rejections = 0,
-      absorb_moves = 0, tr_att = 0, tr_acc = 0, success = 0;
+  const int nc0 = label_census(P, s, s.cur, C0);
+  objective(P, s, prob, ok, nc0, C0);
+  RunState& run = f.run;
+  if (threadIdx.x == 0) {
+    run = RunState{};
+    run.accbest = run.cur_acc = f.acc;
+    run.scorebest = run.cur_score = f.score;
+    run.nc_cur = run.nc_best = nc0;
+  }
+  // the size bound of proposal `cycle`
+  auto group_bound = [&](int cycle) {
+    if (!(P.adaptive && P.pol_adaptive) || T <= 1) return G;
+    double progress = __ddiv_rn(static_cast<double>(cycle + 1), static_cast<double>(T + 1));
+    progress = progress < 0.0 ? 0.0 : (progress > 1.0 ? 1.0 : progress);
+    const double smooth = __dmul_rn(__dmul_rn(progress, progress), __dsub_rn(3.0, __dmul_rn(2.0, progress)));
+    double temp = __dsub_rn(1.0, smooth);
+    temp = temp < 0.0 ? 0.0 : (temp > 1.0 ? 1.0 : temp);
+    const int mc = 1 + static_cast<int>(floor(__dmul_rn(static_cast<double>(G - 1), temp)));
+    return mc > 1 ? mc : 1;
+  };
+  auto cooling = [&](int cycle) {
+    return __dsub_rn(1.0, __ddiv_rn(static_cast<double>(cycle + 1), static_cast<double>(T > 1 ? T : 1)));
+  };
+  if (threadIdx.x == kThreads - 1) {
+    f.max_groups = group_bound(0);
+    f.cooling[0] = cooling(0);
+  }
+  // between cycles s.cl equals s.cur: the proposal starts from the current
+  // (evolutionary) or best (greedy) state, which s.cur holds
+  copy_rows(s.cl, s.cur, L);
+  __syncthreads();
 
   for (int cycle = 0; cycle < T; ++cycle) {
-    if (P.snap_feat != nullptr && cycle == P.snap_cycle) snapshot_state(P, s, prob, cycle, C0);
-    // proposal = current (evolutionary) or best (greedy) state; s.cur holds
-    // it.  Thread 0 draws the proposal size before its share of the copy.
-    {
-      if (threadIdx.x == 0) {
-        int ns;
-        if (G <= 1) {
-          ns = G > 0 ? G : 0;
-        } else if (!(P.adaptive && P.pol_adaptive) || T <= 1) {
-          ns = uniform_int_serial(f.rng, 1, G);
-        } else {
-          double progress = __ddiv_rn(static_cast<double>(cycle + 1), static_cast<double>(T + 1));
-          progress = progress < 0.0 ? 0.0 : (progress > 1.0 ? 1.0 : progress);
-          const double smooth = __dmul_rn(__dmul_rn(progress, progress), __dsub_rn(3.0, __dmul_rn(2.0, progress)));
-          double temp = __dsub_rn(1.0, smooth);
-          temp = temp < 0.0 ? 0.0 : (temp > 1.0 ? 1.0 : temp);
-          const int mc = 1 + static_cast<int>(floor(__dmul_rn(static_cast<double>(G - 1), temp)));
-          ns = uniform_int_serial(f.rng, 1, mc > 1 ? mc : 1);
-        }
-        f.ns = ns;
-      }
-      for (int r = threadIdx.x; r < L; r += kThreads) s.cl[r] = s.cur[r];
-    }
+    if (P.snap_feat != nullptr && cycle == P.snap_cycle) snapshot_state(P, prob, cycle, C0);
+    if (threadIdx.x == 0) f.ns = G <= 1 ? (G > 0 ? G : 0) : uniform_int_serial(f.rng, 1, f.max_groups);
     __syncthreads();
-    shuffle_targets_block(f, s.jarr, G, s.raw);
+    shuffle_targets_block(f, s.jarr, G, s.save);
     const int ns = f.ns;
     if (threadIdx.x == 0) psize[cycle] = ns;
     if (ns > 0) {
@@ -1276,41 +1631,29 @@ __device__ void evolve_problem(const EvolveParams& P, const Smem& s, int prob) {
           take += final_position_of(s, g, ns) < ns;
         }
         take = block_sum(take, f);
-        learned_flip(P, s, prob, cycle, take, C0);
+        learned_flip(P, prob, cycle, take, C0);
       } else if (P.singleton && P.pol_guidance) {
         // Each sampled group takes its own CV prediction; only groups whose
         // prediction differs from their label can change, so walk just those
         // forward to their final shuffled position.
-        for (int g = threadIdx.x; g < G; g += kThreads) {
-          const int row = s.f->gmem[g];
-          if (s.curpred[row] == s.cur[row]) continue;
-          if (s.f->fxd != nullptr && s.f->fxd[row] == 1) continue;
-          if (final_position_of(s, g, ns) < ns) s.cl[row] = s.curpred[row];
-        }
+        flip_sampled(s, G, ns);
       } else {
         for (int p = threadIdx.x; p < ns; p += kThreads) s.perm[p] = static_cast<uint16_t>(occupant_of(s, G, p));
         __syncthreads();
-        if (threadIdx.x == 0) relabel_serial(P, s, s.curpred, ns, C0);
+        if (threadIdx.x == 0) relabel_serial(P, s.curpred, ns, C0);
       }
     }
     __syncthreads();
 
     int absorbed = 0;
-    bool cnt_of_cl = false;  // s.cnt holds the counts of s.cl
     if (P.pol_transition && P.absorption) {
-      ++tr_att;
       absorbed = absorption_block(P, s, prob, s.curpred, C0);
-      absorb_moves += absorbed;
-      cnt_of_cl = absorbed == 0;
     }
 
+    const bool cnt_of_cl = P.pol_transition && P.absorption;  // s.cnt holds the counts of s.cl
     {
-      const int nd = dirty_rows_block(P, s, prob);  // s.pred = s.curpred on return
-      if (nd < 0) {
-        vote_block(P, s, prob, s.cl, s.pred, C0, has_empty);
-      } else {
-        vote_block(P, s, prob, s.cl, s.pred, C0, has_empty, s.jarr, nd);
-      }
+      const int nd = dirty_rows_block(P, s, prob, has_empty);  // s.pred = s.curpred on return
+      vote_block(P, s, prob, s.cl, s.pred, C0, has_empty, nd < 0 ? nullptr : s.jarr, nd);
     }
     const int nc = L < 32768 && C0 < 32768 ? label_census(P, s, s.cl, C0, cnt_of_cl, s.pred, &ok)
                                            : label_census(P, s, s.cl, C0, cnt_of_cl);
@@ -1319,150 +1662,119 @@ __device__ void evolve_problem(const EvolveParams& P, const Smem& s, int prob) {
       for (int r = threadIdx.x; r < L; r += kThreads) ok += s.cl[r] == s.pred[r];
       ok = block_sum(ok, f);
     }
-    const double acc = __ddiv_rn(static_cast<double>(ok), n);
-    const double score = objective(P, s, prob, acc, nc, C0);
-    ++proposals;
-
-    const bool improves = score > scorebest;
-    bool accepted = improves, improving = improves, stoch = false;
-    if (P.evolutionary) {
-      if (threadIdx.x == 0) {
-        const double cooling = __dsub_rn(1.0, __ddiv_rn(static_cast<double>(cycle + 1),
-                                                        static_cast<double>(T > 1 ? T : 1)));
-        const double one_minus = __dsub_rn(1.0, cur_acc);
-        const double clipped = (0.0 < one_minus) ? one_minus : 0.0;
-        const double t0 = __dmul_rn(__dmul_rn(0.10, clipped), cooling);
-        const double temperature = (1.0e-9 < t0) ? t0 : 1.0e-9;
-        int acc_cur = score >= cur_score;
-        int impr = acc_cur;
-        int st = 0;
-        if (!acc_cur && P.pol_stochastic && temperature > 1.0e-9) {
-          st = 2;  // attempted
-          const double u = canonical_serial(f.rng);
-          acc_cur = u < exp(__ddiv_rn(__dsub_rn(score, cur_score), temperature));
-          if (acc_cur) st = 3;
+    objective(P, s, prob, ok, nc, C0);
+    // while warp 0 scores: the next cycle's annealing factor and size bound
+    if (threadIdx.x == kThreads - 1) {
+      f.cooling[(cycle + 1) & 1] = cooling(cycle + 1);
+      f.max_groups = group_bound(cycle + 1);
+    }
+    if (threadIdx.x == 0) {
+      const double acc = f.acc, score = f.score;
+      const bool improves = score > run.scorebest;
+      int acc_cur = improves, impr = improves, st = 0;
+      if (P.evolutionary) {
+        acc_cur = score >= run.cur_score;
+        impr = acc_cur;
+        if (!acc_cur && P.pol_stochastic) {
+          const double one_minus = __dsub_rn(1.0, run.cur_acc);
+          const double clipped = (0.0 < one_minus) ? one_minus : 0.0;
+          const double t0 = __dmul_rn(__dmul_rn(0.10, clipped), f.cooling[cycle & 1]);
+          const double temperature = (1.0e-9 < t0) ? t0 : 1.0e-9;
+          if (temperature > 1.0e-9) {
+            st = 2;  // attempted
+            acc_cur = annealed(canonical_serial(f.rng), __dsub_rn(score, run.cur_score), temperature);
+            if (acc_cur) st = 3;
+          }
         }
-        f.accept = acc_cur | (impr << 1) | (st << 2);
       }
-      __syncthreads();
-      const int code = f.accept;
-      accepted = code & 1;
-      improving = (code >> 1) & 1;
-      const int st = code >> 2;
-      if (st >= 2) ++st_att;
-      stoch = st == 3;
+      if (improves) {
+        run.accbest = acc;
+        run.scorebest = score;
+        run.nc_best = nc;
+        ++run.best_updates;
+      }
+      if (P.evolutionary) {
+        if (acc_cur) {
+          run.cur_acc = acc;
+          run.cur_score = score;
+          run.nc_cur = nc;
+          ++run.accepts;
+        } else {
+          ++run.rejections;
+        }
+        if (st >= 2) ++run.st_att;
+        if (st == 3) ++run.st_acc;
+      }
+      run.absorb_moves += absorbed;
+      if (acc_cur && absorbed) ++run.tr_acc;
+      if (acc == 1.0 && isfinite(score)) run.success = 1;
+      fl[3 * cycle + 0] = acc_cur ? 1 : 0;
+      fl[3 * cycle + 1] = (acc_cur && impr) ? 1 : 0;
+      fl[3 * cycle + 2] = st == 3 ? 1 : 0;
+      act[cycle] = P.evolutionary ? run.nc_cur : run.nc_best;
+      vacc[cycle] = run.accbest;
+      vscore[cycle] = run.scorebest;
+      f.accept = acc_cur | (improves << 1);
     }
     __syncthreads();
+    const int code = f.accept;
+    const bool accepted = code & 1, improves = (code >> 1) & 1;
     if (improves) {
       for (int r = threadIdx.x; r < L; r += kThreads) {
         gbest[r] = s.cl[r];
         gbestpred[r] = s.pred[r];
       }
-      accbest = acc;
-      scorebest = score;
-      ++best_updates;
-      nc_best = nc;
     }
-    const bool take = P.evolutionary ? accepted : improves;
-    if (take) {
-      for (int r = threadIdx.x; r < L; r += kThreads) {
-        s.cur[r] = s.cl[r];
-        s.curpred[r] = s.pred[r];
+    if (P.evolutionary ? accepted : improves) {
+      copy_rows(s.cur, s.cl, L);
+      copy_rows(s.curpred, s.pred, L);
+    } else {
+      if (has_empty) {
+        for (int r = threadIdx.x; r < L; r += kThreads)
+          if (s.cl[r] != s.cur[r]) move_fold(P, prob, r, s.cl[r], s.cur[r]);
+        __syncthreads();
       }
+      copy_rows(s.cl, s.cur, L);
     }
-    if (P.evolutionary) {
-      if (accepted) {
-        cur_acc = acc;
-        cur_score = score;
-        nc_cur = nc;
-        ++accepts;
-        if (stoch) ++st_acc;
-      } else {
-        ++rejections;
-      }
-    }
-    if (accepted && absorbed) ++tr_acc;
-    if (threadIdx.x == 0) {
-      fl[3 * cycle + 0] = accepted ? 1 : 0;
-      fl[3 * cycle + 1] = (accepted && improving) ? 1 : 0;
-      fl[3 * cycle + 2] = stoch ? 1 : 0;
-      act[cycle] = P.evolutionary ? nc_cur : nc_best;
-      vacc[cycle] = accbest;
-      vscore[cycle] = scorebest;
-    }
-    if (acc == 1.0 && isfinite(score)) success = 1;
     __syncthreads();
   }
 
   if (threadIdx.x == 0) {
     int* c = P.counters + static_cast<size_t>(prob) * 16;
+    const int moves = P.pol_transition && P.absorption ? T : 0;  // transitions attempted
     c[0] = T;
-    c[1] = proposals;
-    c[2] = best_updates;
-    c[3] = accepts;
-    c[4] = st_att;
-    c[5] = st_acc;
-    c[6] = rejections;
+    c[1] = T;
+    c[2] = run.best_updates;
+    c[3] = run.accepts;
+    c[4] = run.st_att;
+    c[5] = run.st_acc;
+    c[6] = run.rejections;
     c[7] = 0;
-    c[8] = absorb_moves;
-    c[9] = tr_att;
-    c[10] = tr_acc;
-    c[11] = tr_att;
-    c[12] = tr_acc;
-    c[13] = proposals + 1;
-    c[14] = success;
+    c[8] = run.absorb_moves;
+    c[9] = moves;
+    c[10] = run.tr_acc;
+    c[11] = moves;
+    c[12] = run.tr_acc;
+    c[13] = T + 1;
+    c[14] = run.success;
     c[15] = 0;
-    P.best[2 * prob] = accbest;
-    P.best[2 * prob + 1] = scorebest;
+    P.best[2 * prob] = run.accbest;
+    P.best[2 * prob + 1] = run.scorebest;
     P.status[prob] = 0;
   }
   __syncthreads();
 }
 
-__device__ Smem carve_smem(const EvolveParams& P, unsigned char* smem_raw) {
-  Smem s;
-  size_t off = 0;
-  s.f = reinterpret_cast<Fixed*>(smem_raw);
-  off = align_up(sizeof(Fixed), 16);
-  const int C = P.C0max;
-  s.cnt = reinterpret_cast<int*>(smem_raw + off); off += align_up(sizeof(int) * C, 16);
-  s.firstpos = reinterpret_cast<int*>(smem_raw + off); off += align_up(sizeof(int) * C, 16);
-  s.movable = reinterpret_cast<int*>(smem_raw + off); off += align_up(sizeof(int) * C, 16);
-  s.order = reinterpret_cast<int*>(smem_raw + off); off += align_up(sizeof(int) * (C + 1), 16);
-  s.bt = reinterpret_cast<int*>(smem_raw + off); off += align_up(sizeof(int) * C, 16);
-  s.aux = reinterpret_cast<int*>(smem_raw + off); off += align_up(sizeof(int) * C, 16);
-  s.bsur = reinterpret_cast<double*>(smem_raw + off); off += align_up(sizeof(double) * C, 16);
-  s.weight = reinterpret_cast<double*>(smem_raw + off); off += align_up(sizeof(double) * C, 16);
-  s.cp = reinterpret_cast<double*>(smem_raw + off); off += align_up(sizeof(double) * 2 * C, 16);
-  const size_t Lp = align_up(static_cast<size_t>(P.L), 8);
-  s.raw = P.raw_scratch + static_cast<size_t>(blockIdx.x) * (P.L / 2 + 64);
-  if (P.smem_trans) {
-    s.trans = reinterpret_cast<int*>(smem_raw + off);
-    off += align_up(sizeof(int) * static_cast<size_t>(C) * C, 16);
-  } else {
-    s.trans = nullptr;
-  }
-  uint16_t* rows = P.smem_rows ? reinterpret_cast<uint16_t*>(smem_raw + off)
-                               : P.rows_scratch + static_cast<size_t>(blockIdx.x) * kRowArrays * Lp;
-  s.cl = rows;
-  s.cur = rows + Lp;
-  s.curpred = rows + 2 * Lp;
-  s.pred = rows + 3 * Lp;
-  s.perm = s.pred;
-  s.jarr = rows + 4 * Lp;
-  s.list = rows + 5 * Lp;
-  s.scratch32 = reinterpret_cast<int*>(rows + 6 * Lp);  // 2 * Lp u16 = Lp ints
-  return s;
+__device__ __forceinline__ void clear_counters(const Smem& s) {
+  for (int i = threadIdx.x; i < s.hist_stride * s.hist_warps; i += kThreads) s.hist[i] = 0;
+  __syncthreads();
 }
 
-__global__ void __launch_bounds__(kThreads, 1) evolve_kernel(EvolveParams P) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Smem s = carve_smem(P, smem_raw);
-  const int C = P.C0max;
-  for (int prob = blockIdx.x; prob < P.problems; prob += gridDim.x) {
-    if (!P.smem_trans) s.trans = P.trans + static_cast<size_t>(prob) * C * C;
-    evolve_problem(P, s, prob);
-  }
+template <bool kRows>
+__global__ void __launch_bounds__(kThreads, 1) evolve_kernel(const __grid_constant__ EvolveParams P) {
+  const Smem s = carve_smem<kRows>(P);
+  clear_counters(s);
+  for (int prob = blockIdx.x; prob < P.problems; prob += gridDim.x) evolve_problem(P, s, prob);
 }
 
 // ===========================================================================
@@ -1476,170 +1788,158 @@ __global__ void __launch_bounds__(kThreads, 1) evolve_kernel(EvolveParams P) {
 //   the fragmentation penalty       core.cpp:954-968
 // ===========================================================================
 
-// Serial std::shuffle of a[0..n) with the libstdc++ 64-bit-engine algorithm
-// (pair draws, see shuffle_targets_block); a holds (a0, a1) int pairs and a
-// double key, swapped together.
-__device__ void shuffle_triples_serial(Mt64State& g, int* a0, int* a1, double* key, int n) {
-  auto swap3 = [&](int i, int j) {
-    const int t0 = a0[i], t1 = a1[i];
-    const double tk = key[i];
-    a0[i] = a0[j];
-    a1[i] = a1[j];
-    key[i] = key[j];
-    a0[j] = t0;
-    a1[j] = t1;
-    key[j] = tk;
-  };
-  if (n <= 1) return;
-  int i = 1;
-  if ((n & 1) == 0) {
-    swap3(1, static_cast<int>(draw_below_serial(g, 2)));
-    i = 2;
-  }
-  while (i < n) {
-    const uint64_t b0 = static_cast<uint64_t>(i) + 1ull, b1 = b0 + 1ull;
-    const uint64_t x = draw_below_serial(g, b0 * b1);
-    swap3(i, static_cast<int>(x / b1));
-    swap3(i + 1, static_cast<int>(x % b1));
-    i += 2;
-  }
-}
-
-// Class sizes, movable sizes and class x prediction counts of s.cl against pp
-// (build_class_transition_stats, core.cpp:980-993).  Returns the class count.
-__device__ int transition_stats(const EvolveParams& P, const Smem& s, const uint16_t* pp, int C0) {
-  int* tr = s.trans;
-  const int C = P.C0max;
-  for (int i = threadIdx.x; i < C0 * C; i += kThreads) tr[i] = 0;
-  for (int c = threadIdx.x; c < C0; c += kThreads) {
-    s.cnt[c] = 0;
-    s.movable[c] = 0;
-  }
-  __syncthreads();
-  // one atomic per row: the class sizes are the rows of the class x
-  // prediction table, and without fixed rows every row is movable
-  const bool any_fixed = s.f->fxd != nullptr;
-  for (int r = threadIdx.x; r < P.L; r += kThreads) {
-    const int a = s.cl[r];
-    atomicAdd(&tr[a * C + pp[r]], 1);
-    if (any_fixed && s.f->fxd[r] != 1) atomicAdd(&s.movable[a], 1);
-  }
-  __syncthreads();
-  for (int c = threadIdx.x; c < C0; c += kThreads) {
-    int sz = 0;
-    for (int q = 0; q < C0; ++q) sz += tr[c * C + q];
-    s.cnt[c] = sz;
-    if (!any_fixed) s.movable[c] = sz;
-  }
-  __syncthreads();
-  int local = 0;
-  for (int c = threadIdx.x; c < C0; c += kThreads) local += s.cnt[c] > 0;
-  return block_sum(local, *s.f);
-}
-
 // propose_auto_class_coarsening on s.cl.  plogp[k] = (k/L) * log(k/L) as the
-// reference rounds it.  One thread per source class computes its transition
-// entropy, its destination and its candidate score; the transition entropy
-// is formed as log(s) - sum_c c log(c) / s from host tables of k log k and
-// log k: it only feeds ceil(temperature * redundant), which an ulp-level
-// difference cannot move unless that product lies within an ulp of an
-// integer.  Returns 1 if the labels changed.
-__device__ int coarsening_block(const EvolvePlsParams& Q, const Smem& s, int prob, const uint16_t* pp, int C0) {
+// reference rounds it.  The transition entropy is formed as
+// log(s) - sum_c c log(c) / s from host tables of k log k and log k: it only
+// feeds ceil(temperature * redundant), which an ulp-level difference cannot move
+// unless that product lies within an ulp of an integer.  Returns 1 if the labels
+// changed.
+// A warp per source counts its rows' predictions (for_each_source), takes the
+// destination and lists the c log c terms in order; a thread per source adds its
+// terms; the candidates are shuffled as the groups are and ranked by counting.
+// With a thread per source over the whole class x prediction table and the
+// shuffle and the sort in one thread this took 480k to 890k cycles at 7500 rows
+// and 100 codes.
+__device__ __forceinline__ int coarsening_block(const EvolvePlsParams& Q, const Smem& s, int prob, const uint16_t* pp, int C0) {
   const EvolveParams& P = Q.base;
   Fixed& f = *s.f;
-  const int nc = transition_stats(P, s, pp, C0);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nc = class_groups(P, s, pp, C0);
   if (nc <= 2) return 0;
-  const int C = P.C0max;
-  double* te_of = s.bsur;     // per source: transition entropy
-  int* dst_of = s.bt;         // per source: destination, -1 = not a candidate
-  double* score_of = s.cp;    // per source: candidate score
-  for (int src = threadIdx.x; src < C0; src += kThreads) {
-    const int ssize = s.cnt[src];
-    dst_of[src] = -1;
-    te_of[src] = 0.0;
-    if (ssize == 0 || s.movable[src] <= 0) continue;
-    const int* row = s.trans + src * C;
-    int dbest = src, dsize = ssize, bcount = 0;
-    double clc = 0.0;
-    for (int dst = 0; dst < C0; ++dst) {
-      const int cntd = row[dst];
-      if (cntd == 0) continue;
-      clc = __dadd_rn(clc, Q.klogk[cntd]);
-      const int sz = s.cnt[dst];
-      if (dst != src && sz > 0 &&
-          (cntd > bcount || (cntd == bcount && sz > dsize) || (cntd == bcount && sz == dsize && dst < dbest))) {
-        dbest = dst;
-        dsize = sz;
-        bcount = cntd;
+  int* dst_of = s.bt;          // per source: destination, -1 = not a candidate
+  int* stay_of = s.firstpos;   // per source: rows predicted as itself
+  int* terms_of = s.order;     // per source: number of terms
+  double* score_of = s.cp;     // per source: candidate score
+  double* share_of = s.cp + C0;  // per code: (k/L) log(k/L)
+  double* te_of = s.bsur;      // per source: its share of the transition entropy
+  // c log c of the counts above 1 (1 log 1 = 0) in ascending code order: a
+  // source of n rows has at most n / 2
+  double* terms = reinterpret_cast<double*>(s.scratch32);
+  for (int c = threadIdx.x; c < C0; c += kThreads) {
+    dst_of[c] = -1;
+    te_of[c] = 0.0;
+    share_of[c] = s.cnt[c] > 0 ? Q.plogp[s.cnt[c]] : 0.0;
+  }
+  __syncthreads();
+  for_each_source(s, C0, [&](int src, int ssize, int items, auto&& each, const int* h) {
+    // destination: largest (count, size), smaller code, of the other codes in use
+    unsigned key = 0u;
+    int dst = 0x7fffffff;
+    for (int i = lane; i < items; i += 32) {
+      const int d = each(i), size = s.cnt[d];
+      if (d == src || size == 0 || h[d] == 0) continue;
+      const unsigned k = static_cast<unsigned>(h[d]) << 16 | static_cast<unsigned>(size);
+      if (k > key || (k == key && d < dst)) {
+        key = k;
+        dst = d;
       }
     }
-    te_of[src] = __dsub_rn(Q.logk[ssize], __ddiv_rn(clc, static_cast<double>(ssize)));
-    if (dbest == src || bcount == 0) continue;
-    const double stay = __ddiv_rn(static_cast<double>(row[src]), static_cast<double>(ssize));
-    dst_of[src] = dbest;
+    const unsigned top = __reduce_max_sync(kFull, key);
+    dst = __reduce_min_sync(kFull, key == top ? dst : 0x7fffffff);
+    double* to = terms + (class_start(s, src) >> 1);
+    int k = 0;
+    for (int c0 = 0; c0 < C0; c0 += 32) {
+      const int v = c0 + lane < C0 ? h[c0 + lane] : 0;
+      const unsigned m = __ballot_sync(kFull, v > 1);
+      if (v > 1) to[k + __popc(m & ((1u << lane) - 1u))] = Q.klogk[v];
+      k += __popc(m);
+    }
+    if (lane == 0) {
+      dst_of[src] = top != 0u ? dst : -1;
+      stay_of[src] = h[src];
+      terms_of[src] = k;
+    }
+  });
+  __syncthreads();
+  for (int src = threadIdx.x; src < C0; src += kThreads) {
+    const int ssize = s.cnt[src];
+    if (ssize == 0 || s.movable[src] <= 0) continue;
+    const double size = static_cast<double>(ssize);
+    const double clc = chain_add(0.0, terms + (class_start(s, src) >> 1), terms_of[src]);
+    const double te = __dsub_rn(Q.logk[ssize], __ddiv_rn(clc, size));
+    te_of[src] = __dmul_rn(__ddiv_rn(size, static_cast<double>(P.L)), te);
+    if (dst_of[src] < 0) continue;
+    const double stay = __ddiv_rn(static_cast<double>(stay_of[src]), size);
     score_of[src] =
         __dmul_rn(__ddiv_rn(1.0, __dsqrt_rn(static_cast<double>(s.movable[src]))), __dsub_rn(1.0, stay));
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const double n = static_cast<double>(P.L);
-    double ce = 0.0;
-    for (int c = 0; c < C0; ++c)
-      if (s.cnt[c] > 0) ce = __dsub_rn(ce, Q.plogp[s.cnt[c]]);
+  if (warp == 0) {
+    // class entropy and mean transition entropy, in source order
+    double ce = 0.0, wte = 0.0;
+    for (int c0 = 0; c0 < C0; c0 += 8) {
+      double a[8], b[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        a[q] = c0 + q < C0 ? share_of[c0 + q] : 0.0;
+        b[q] = c0 + q < C0 ? te_of[c0 + q] : 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        ce = __dsub_rn(ce, a[q]);  // zero for a code not in use
+        wte = __dadd_rn(wte, b[q]);
+      }
+    }
     const double keff = cr_exp(ce);
     const double lr = cr_log(__ddiv_rn(static_cast<double>(nc), 1.0 < keff ? keff : 1.0));
     const double frag = 0.0 < lr ? lr : 0.0;
-    double wte = 0.0;
-    int K = 0;
-    int* csrc = s.order;   // candidates in ascending source order: source, destination, score
-    int* cdst = s.firstpos;
-    double* cscore = s.weight;
-    for (int src = 0; src < C0; ++src) {
-      if (s.cnt[src] == 0 || s.movable[src] <= 0) continue;
-      wte = __dadd_rn(wte, __dmul_rn(__ddiv_rn(static_cast<double>(s.cnt[src]), n), te_of[src]));
-      if (dst_of[src] < 0) continue;
-      csrc[K] = src;
-      cdst[K] = dst_of[src];
-      cscore[K] = score_of[src];
-      ++K;
+    const double temperature = __ddiv_rn(frag, __dadd_rn(__dadd_rn(frag, wte), 1.0));
+    const double rd = __dsub_rn(static_cast<double>(nc), keff);
+    const double redundant = 0.0 < rd ? rd : 0.0;
+    int budget = static_cast<int>(ceil(__dmul_rn(temperature, redundant)));
+    if (budget < 1 && frag > 0.0) budget = 1;
+    if (lane == 0) f.flag = min(budget, nc - 2);
+  } else if (warp == 1) {
+    // candidates in ascending source order
+    int k = 0;
+    for (int c0 = 0; c0 < C0; c0 += 32) {
+      const int src = c0 + lane;
+      const int d = src < C0 ? dst_of[src] : -1;
+      const unsigned m = __ballot_sync(kFull, d >= 0);
+      if (d >= 0) {
+        const int at = k + __popc(m & ((1u << lane) - 1u));
+        s.order[at] = src << 16 | d;
+        s.weight[at] = score_of[src];
+      }
+      k += __popc(m);
     }
-    int budget = 0;
-    if (K > 0) {
-      const double temperature = __ddiv_rn(frag, __dadd_rn(__dadd_rn(frag, wte), 1.0));
-      const double rd = __dsub_rn(static_cast<double>(nc), keff);
-      const double redundant = 0.0 < rd ? rd : 0.0;
-      budget = static_cast<int>(ceil(__dmul_rn(temperature, redundant)));
-      if (budget < 1 && frag > 0.0) budget = 1;
-      budget = min(budget, nc - 2);
-    }
+    if (lane == 0) f.walk_cnt = k;
+  }
+  __syncthreads();
+  const int K = f.walk_cnt, budget = f.flag;
+  if (K == 0 || budget <= 0) return 0;
+  __syncthreads();
+  shuffle_targets_block(f, s.jarr, K, s.save);
+  __syncthreads();
+  bucket_steps_block(s, K, K);
+  for (int q = threadIdx.x; q < K; q += kThreads) {
+    const int at = occupant_of(s, K, q);
+    s.firstpos[q] = s.order[at];
+    s.cp[q] = s.weight[at];
+  }
+  for (int c = threadIdx.x; c < C0; c += kThreads) s.aux[c] = c;
+  __syncthreads();
+  // stable order by score, descending; the scores are positive, so their bits
+  // compare as they do
+  const unsigned long long* bits = reinterpret_cast<const unsigned long long*>(s.cp);
+  for (int q = threadIdx.x; q < K; q += kThreads) {
+    const unsigned long long mine = bits[q];
+    int rank = 0;
+    for (int j = 0; j < K; ++j) rank += bits[j] > mine || (bits[j] == mine && j < q);
+    s.order[rank] = s.firstpos[q];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int* remap = s.aux;
     int merged = 0;
-    if (K > 0 && budget > 0) {
-      shuffle_triples_serial(f.rng, csrc, cdst, cscore, K);
-      for (int a = 1; a < K; ++a) {  // stable sort by score, descending
-        const int v0 = csrc[a], v1 = cdst[a];
-        const double vk = cscore[a];
-        int b = a - 1;
-        while (b >= 0 && vk > cscore[b]) {
-          csrc[b + 1] = csrc[b];
-          cdst[b + 1] = cdst[b];
-          cscore[b + 1] = cscore[b];
-          --b;
-        }
-        csrc[b + 1] = v0;
-        cdst[b + 1] = v1;
-        cscore[b + 1] = vk;
-      }
-      int* remap = s.aux;
-      for (int c = 0; c < C0; ++c) remap[c] = c;
-      for (int q = 0; q < K && merged < budget; ++q) {
-        const int src = csrc[q];
-        if (remap[src] != src) continue;
-        int d = cdst[q];
-        while (remap[d] != d) d = remap[d];
-        if (d == src) continue;
-        remap[src] = d;
-        ++merged;
-      }
+    for (int q = 0; q < K && merged < budget; ++q) {
+      const int src = static_cast<int>(static_cast<unsigned>(s.order[q]) >> 16);
+      if (remap[src] != src) continue;
+      int d = s.order[q] & 0xffff;
+      while (remap[d] != d) d = remap[d];
+      if (d == src) continue;
+      remap[src] = d;
+      ++merged;
     }
     f.flag = merged;
   }
@@ -1660,27 +1960,52 @@ __device__ int coarsening_block(const EvolvePlsParams& Q, const Smem& s, int pro
   return block_sum(changed, f) > 0 ? 1 : 0;
 }
 
-// core_objective_score with the PLS fragmentation penalty; census current.
-__device__ double objective_pls(const EvolvePlsParams& Q, const Smem& s, int prob, double acc, int nc, int C0) {
+// core_objective_score with the PLS fragmentation penalty, in f.acc and f.score
+// for thread 0; census current.
+__device__ __forceinline__ void objective_pls(const EvolvePlsParams& Q, const Smem& s, int prob, int ok, int nc, int C0) {
   const EvolveParams& P = Q.base;
+  Fixed& f = *s.f;
   const bool use_div = P.guarded && P.pol_diversity;
   const bool use_frag = Q.coarsening && Q.pol_frag;
   const bool reject1 = P.guarded && P.pol_reject1;
-  if (!use_div && !use_frag && !reject1) return acc;
-  if (reject1 && nc == 1) return -INFINITY;
-  if (!use_div && !(use_frag && nc > 1)) return acc;
-  map_order(P, s, prob, C0);
-  if (threadIdx.x == 0) {
-    double score = acc;
+  if (threadIdx.x == 32) f.acc = __ddiv_rn(static_cast<double>(ok), static_cast<double>(P.L));
+  const bool single = reject1 && nc == 1;
+  const bool ranked = !single && (use_div || (use_frag && nc > 1));
+  // both sums' terms, then the two chains side by side
+  double* sq = s.cp;
+  double* pl = s.cp + C0;
+  if (ranked) {
+    map_order(P, s, prob, C0);
+    for (int q = threadIdx.x; q < nc; q += kThreads) {
+      const int c = s.cnt[s.order[q]];
+      sq[q] = use_div ? P.psq[c] : 0.0;
+      pl[q] = use_frag ? Q.plogp[c] : 0.0;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  const double acc = f.acc;
+  double score = single ? -INFINITY : acc;
+  if (ranked) {
+    double same = 0.0, entropy = 0.0;
+    for (int q0 = 0; q0 < nc; q0 += 8) {
+      double a[8], b[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        a[q] = q0 + q < nc ? sq[q0 + q] : 0.0;
+        b[q] = q0 + q < nc ? pl[q0 + q] : 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        same = __dadd_rn(same, a[q]);
+        entropy = __dsub_rn(entropy, b[q]);
+      }
+    }
     if (use_div) {
-      double same = 0.0;
-      for (int q = 0; q < nc; ++q) same = __dadd_rn(same, P.psq[s.cnt[s.order[q]]]);
       const double diff = __dsub_rn(1.0, same);
       score = __dmul_rn(score, __dsqrt_rn(0.0 < diff ? diff : 0.0));
     }
     if (use_frag && nc > 1) {
-      double entropy = 0.0;
-      for (int q = 0; q < nc; ++q) entropy = __dsub_rn(entropy, Q.plogp[s.cnt[s.order[q]]]);
       const double mse = P.L > 1 ? Q.logn : 0.0;
       double code_cost = 0.0;
       if (mse > 0.0) {
@@ -1694,54 +2019,78 @@ __device__ double objective_pls(const EvolvePlsParams& Q, const Smem& s, int pro
       const double pc = code_cost < frag_cost ? frag_cost : code_cost;
       score = __dsub_rn(score, __dmul_rn(__dsub_rn(1.0, acc), pc));
     }
-    s.f->score = score;
   }
-  __syncthreads();
-  const double out = s.f->score;
-  __syncthreads();
-  return out;
+  if (threadIdx.x == 0) f.score = score;
+}
+
+// Lanes holding the same code (of `bits` bits) as this one, of those with `in`.
+__device__ __forceinline__ unsigned same_code(int code, bool in, int bits) {
+  unsigned m = __ballot_sync(kFull, in);
+  for (int b = 0; b < bits; ++b) {
+    const unsigned v = __ballot_sync(kFull, (code >> b) & 1);
+    m &= (code >> b) & 1 ? v : ~v;
+  }
+  return m;
 }
 
 // Rows of s.cl grouped by code, ascending rows within a code, for the
-// cross-product chains of the PLS predictor: one warp per code.
-__device__ void class_lists(const EvolvePlsParams& Q, const Smem& s, int prob, int C0) {
+// cross-product chains of the PLS predictor: a counting sort.  Each of nw warps
+// takes a run of rows and has a counter per code; a row's place is its warp's
+// first place for the code plus the rows before it.  A warp per code reading all
+// rows took 120k to 160k cycles at 7500 rows and 100 codes.
+__device__ __forceinline__ void class_lists(const EvolvePlsParams& Q, const Smem& s, int prob, int C0) {
   const int L = Q.base.L, C = Q.base.C0max;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int c = threadIdx.x; c < C0; c += kThreads) s.cnt[c] = 0;
+  const unsigned below = (1u << lane) - 1u;
+  uint16_t* table = reinterpret_cast<uint16_t*>(s.scratch32);  // nw x C0, of 2 x L rounded up to 8
+  const int nw = min(kWarps, 2 * 8 * row_vectors(L) / C0);     // at least 2: C0 <= L
+  const int bits = 32 - __clz(C0 - 1 | 1);
+  const int chunk = ((L + nw - 1) / nw + 31) / 32 * 32;
+  const int beg = warp < nw ? min(L, warp * chunk) : 0, end = warp < nw ? min(L, beg + chunk) : 0;
+  uint16_t* mine = table + min(warp, nw - 1) * C0;
+  for (int i = threadIdx.x; i < nw * C0; i += kThreads) table[i] = 0;
   __syncthreads();
-  for (int r = threadIdx.x; r < L; r += kThreads) atomicAdd(&s.cnt[s.cl[r]], 1);
-  __syncthreads();
-  int* coff = Q.class_off + static_cast<size_t>(prob) * (C + 1);
-  if (threadIdx.x == 0) {
-    int run = 0;
-    for (int c = 0; c < C; ++c) {
-      coff[c] = run;
-      s.aux[c] = run;
-      run += c < C0 ? s.cnt[c] : 0;
+  // place(r, at): the row and its place among its warp's rows of the code
+  auto walk = [&](auto&& place) {
+    for (int b = beg; b < end; b += 32) {
+      const bool in = b + lane < end;
+      const int code = in ? s.cl[b + lane] : 0;
+      const unsigned m = same_code(code, in, bits);
+      const int at = in ? mine[code] : 0;
+      if (in) place(b + lane, at + __popc(m & below));
+      __syncwarp();
+      if (in && (m & below) == 0u) mine[code] = static_cast<uint16_t>(at + __popc(m));
+      __syncwarp();
     }
-    coff[C] = run;
+  };
+  walk([](int, int) {});
+  __syncthreads();
+  for (int c = threadIdx.x; c < C0; c += kThreads) {
+    int run = 0;
+    for (int k = 0; k < nw; ++k) {
+      const int v = table[k * C0 + c];
+      table[k * C0 + c] = static_cast<uint16_t>(run);
+      run += v;
+    }
+    s.cnt[c] = run;
+    s.aux[c] = run;
   }
+  __syncthreads();
+  block_exclusive_scan(s.aux, C0, *s.f);
+  int* coff = Q.class_off + static_cast<size_t>(prob) * (C + 1);
+  for (int c = threadIdx.x; c <= C; c += kThreads) coff[c] = c < C0 ? s.aux[c] : L;
+  for (int i = threadIdx.x; i < nw * C0; i += kThreads) table[i] = static_cast<uint16_t>(table[i] + s.aux[i % C0]);
   __syncthreads();
   uint16_t* rows = Q.class_rows + static_cast<size_t>(prob) * L;
-  for (int c = warp; c < C0; c += kWarps) {
-    if (s.cnt[c] == 0) continue;
-    int pos = s.aux[c];
-    for (int base = 0; base < L; base += 32) {
-      const int r = base + lane;
-      const bool hit = r < L && s.cl[r] == c;
-      const unsigned m = __ballot_sync(kFull, hit);
-      if (hit) rows[pos + __popc(m & ((1u << lane) - 1u))] = static_cast<uint16_t>(r);
-      pos += __popc(m);
-    }
-  }
+  walk([&](int r, int at) { rows[at] = static_cast<uint16_t>(r); });
   __syncthreads();
 }
 
-__device__ void pls_propose(const EvolvePlsParams& Q, const Smem& s, int prob, int cycle, PlsRunState& st, int C0) {
+__device__ __forceinline__ void pls_propose(const EvolvePlsParams& Q, const Smem& s, int prob, int cycle, PlsRunState& st, int C0) {
   const EvolveParams& P = Q.base;
   Fixed& f = *s.f;
   const int L = P.L, T = P.T, G = f.G;
-  for (int r = threadIdx.x; r < L; r += kThreads) s.cl[r] = s.cur[r];
+  copy_rows(s.cl, s.cur, L);
   __syncthreads();
   if (threadIdx.x == 0) {
     int ns;
@@ -1762,21 +2111,16 @@ __device__ void pls_propose(const EvolvePlsParams& Q, const Smem& s, int prob, i
     P.proposal_size[static_cast<size_t>(prob) * T + cycle] = ns;
   }
   __syncthreads();
-  shuffle_targets_block(f, s.jarr, G, s.raw);
+  shuffle_targets_block(f, s.jarr, G, s.save);
   const int ns = f.ns;
   if (ns > 0) {
     bucket_steps_block(s, G, ns);
     if (P.singleton && P.pol_guidance) {
-      for (int g = threadIdx.x; g < G; g += kThreads) {
-        const int row = s.f->gmem[g];
-        if (s.curpred[row] == s.cur[row]) continue;
-        if (s.f->fxd != nullptr && s.f->fxd[row] == 1) continue;
-        if (final_position_of(s, g, ns) < ns) s.cl[row] = s.curpred[row];
-      }
+      flip_sampled(s, G, ns);
     } else {
       for (int q = threadIdx.x; q < ns; q += kThreads) s.perm[q] = static_cast<uint16_t>(occupant_of(s, G, q));
       __syncthreads();
-      if (threadIdx.x == 0) relabel_serial(P, s, s.curpred, ns, C0);
+      if (threadIdx.x == 0) relabel_serial(P, s.curpred, ns, C0);
     }
   }
   __syncthreads();
@@ -1802,7 +2146,7 @@ __device__ void pls_propose(const EvolvePlsParams& Q, const Smem& s, int prob, i
   class_lists(Q, s, prob, C0);
 }
 
-__device__ void pls_step(const EvolvePlsParams& Q, const Smem& s, int prob) {
+__device__ __forceinline__ void pls_step(const EvolvePlsParams& Q, const Smem& s, int prob) {
   const EvolveParams& P = Q.base;
   Fixed& f = *s.f;
   bind_groups(P, s, prob);
@@ -1833,12 +2177,26 @@ __device__ void pls_step(const EvolvePlsParams& Q, const Smem& s, int prob) {
       f.rng.pos = g.pos;
       st = gst;
     }
-    for (int r = threadIdx.x; r < L; r += kThreads) {
-      s.cl[r] = Q.cl[ro + r];
-      s.pred[r] = Q.pred[ro + r];
-      if (cycle > 0) {
-        s.cur[r] = Q.cur[ro + r];
-        s.curpred[r] = Q.curpred[ro + r];
+    // four rows of all four arrays in flight (before the first cycle the
+    // current state is not read any further)
+    for (int r0 = threadIdx.x; r0 < L; r0 += 4 * kThreads) {
+      uint16_t v[4][4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const size_t o = ro + min(r0 + q * kThreads, L - 1);
+        v[q][0] = Q.cl[o];
+        v[q][1] = Q.pred[o];
+        v[q][2] = cycle > 0 ? Q.cur[o] : 0;
+        v[q][3] = cycle > 0 ? Q.curpred[o] : 0;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int r = r0 + q * kThreads;
+        if (r >= L) break;
+        s.cl[r] = v[q][0];
+        s.pred[r] = v[q][1];
+        s.cur[r] = v[q][2];
+        s.curpred[r] = v[q][3];
       }
     }
     __syncthreads();
@@ -1847,9 +2205,8 @@ __device__ void pls_step(const EvolvePlsParams& Q, const Smem& s, int prob) {
     int ok = 0;
     for (int r = threadIdx.x; r < L; r += kThreads) ok += s.cl[r] == s.pred[r];
     ok = block_sum(ok, f);
-    const double acc = __ddiv_rn(static_cast<double>(ok), static_cast<double>(L));
     const int nc = label_census(P, s, s.cl, C0);
-    const double score = objective_pls(Q, s, prob, acc, nc, C0);
+    objective_pls(Q, s, prob, ok, nc, C0);
     if (cycle == 0) {
       for (int r = threadIdx.x; r < L; r += kThreads) {
         s.cur[r] = s.cl[r];
@@ -1858,13 +2215,16 @@ __device__ void pls_step(const EvolvePlsParams& Q, const Smem& s, int prob) {
         gbestpred[r] = s.pred[r];
       }
       if (threadIdx.x == 0) {
+        const double acc = f.acc, score = f.score;
         st.accbest = st.cur_acc = acc;
         st.scorebest = st.cur_score = score;
         st.nc_cur = st.nc_best = nc;
       }
+      __syncthreads();
     } else {
       const int c = cycle - 1;
       if (threadIdx.x == 0) {
+        const double acc = f.acc, score = f.score;
         ++st.proposals;
         const bool improves = score > st.scorebest;
         int accepted = improves, improving = improves, stoch = 0;
@@ -1879,7 +2239,7 @@ __device__ void pls_step(const EvolvePlsParams& Q, const Smem& s, int prob) {
           if (!acc_cur && P.pol_stochastic && temperature > 1.0e-9) {
             ++st.st_att;
             const double u = canonical_serial(f.rng);
-            acc_cur = u < exp(__ddiv_rn(__dsub_rn(score, st.cur_score), temperature));
+            acc_cur = annealed(u, __dsub_rn(score, st.cur_score), temperature);
             stoch = acc_cur;
           }
           accepted = acc_cur;
@@ -1927,10 +2287,8 @@ __device__ void pls_step(const EvolvePlsParams& Q, const Smem& s, int prob) {
         }
       }
       if (take) {
-        for (int r = threadIdx.x; r < L; r += kThreads) {
-          s.cur[r] = s.cl[r];
-          s.curpred[r] = s.pred[r];
-        }
+        copy_rows(s.cur, s.cl, L);
+        copy_rows(s.curpred, s.pred, L);
       }
       __syncthreads();
     }
@@ -1986,44 +2344,60 @@ __device__ void pls_step(const EvolvePlsParams& Q, const Smem& s, int prob) {
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(kThreads, 1) evolve_pls_kernel(EvolvePlsParams Q) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Smem s = carve_smem(Q.base, smem_raw);
-  const int C = Q.base.C0max;
-  for (int prob = blockIdx.x; prob < Q.base.problems; prob += gridDim.x) {
-    if (!Q.base.smem_trans) s.trans = Q.base.trans + static_cast<size_t>(prob) * C * C;
-    pls_step(Q, s, prob);
-  }
+template <bool kRows>
+__global__ void __launch_bounds__(kThreads, 1) evolve_pls_kernel(const __grid_constant__ EvolvePlsParams Q) {
+  const Smem s = carve_smem<kRows>(Q.base);
+  clear_counters(s);
+  for (int prob = blockIdx.x; prob < Q.base.problems; prob += gridDim.x) pls_step(Q, s, prob);
 }
 
 }  // namespace
 
-size_t evolve_smem_bytes(int L, int C0max, bool rows_in_smem, bool trans_in_smem) {
+size_t evolve_smem_bytes(int L, int C0max, bool rows_in_smem, int hist_warps) {
   auto al = [](size_t v) { return (v + 15) / 16 * 16; };
-  size_t b = al(sizeof(Fixed));
-  b += 6 * al(sizeof(int) * C0max) + al(sizeof(int) * (C0max + 1));
+  size_t b = kFixedBytes;
+  b += 5 * al(sizeof(int) * C0max) + al(sizeof(int) * (C0max + 1));
   b += 2 * al(sizeof(double) * C0max) + al(sizeof(double) * 2 * C0max);
-  if (trans_in_smem) b += al(sizeof(int) * static_cast<size_t>(C0max) * C0max);
+  b += al(sizeof(int) * C0max) * hist_warps;
   if (rows_in_smem) b += kRowArrays * ((static_cast<size_t>(L) + 7) / 8 * 8) * sizeof(uint16_t);
   return b;
 }
 
-int evolve_pls_launch(const EvolvePlsParams& q, int grid, size_t smem, void* stream) {
-  cudaError_t e = cudaFuncSetAttribute(evolve_pls_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem));
+bool evolve_place(EvolveParams& p, size_t budget, size_t* smem) {
+  // per-row arrays in shared memory first, then counters for as many warps as
+  // fit: a source more or less at a time is little beside rows' round trips to L2
+  for (const bool rows : {true, false}) {
+    for (const int warps : {32, 24, 16, 12, 8, 6, 4, 2, 1}) {
+      *smem = evolve_smem_bytes(p.L, p.C0max, rows, warps);
+      if (*smem > budget) continue;
+      p.smem_rows = rows;
+      p.hist_warps = warps;
+      return true;
+    }
+  }
+  return false;
+}
+
+namespace {
+
+template <class Params>
+int launch(void (*kernel)(Params), const Params& p, int grid, size_t smem, void* stream) {
+  const cudaError_t e =
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);
-  evolve_pls_kernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(q);
+  kernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(p);
   count_launch();
   return static_cast<int>(cudaGetLastError());
 }
 
+}  // namespace
+
+int evolve_pls_launch(const EvolvePlsParams& q, int grid, size_t smem, void* stream) {
+  return launch(q.base.smem_rows ? evolve_pls_kernel<true> : evolve_pls_kernel<false>, q, grid, smem, stream);
+}
+
 int evolve_launch(const EvolveParams& p, int grid, size_t smem, void* stream) {
-  cudaError_t e = cudaFuncSetAttribute(evolve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem));
-  if (e != cudaSuccess) return static_cast<int>(e);
-  evolve_kernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(p);
-  count_launch();
-  return static_cast<int>(cudaGetLastError());
+  return launch(p.smem_rows ? evolve_kernel<true> : evolve_kernel<false>, p, grid, smem, stream);
 }
 
 }  // namespace kgb

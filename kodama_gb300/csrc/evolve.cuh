@@ -24,7 +24,7 @@ struct EvolveParams {
   int pol_guidance, pol_adaptive, pol_transition, pol_stochastic, pol_diversity, pol_reject1;
   uint64_t bucket_count;   // libstdc++ bucket count after reserve(L)
   int smem_rows;           // 1 = per-row arrays in shared memory
-  int smem_trans;          // 1 = class x prediction counts in shared memory
+  int hist_warps;          // warps with per-code counters in shared memory
   // inputs
   const uint16_t* nb;      // problems x L x w local neighbour ids (kNoRow = none)
   const float* sc;         // problems x L x w scores -(d*d)
@@ -54,10 +54,10 @@ struct EvolveParams {
   double* best;            // problems x 2 (accbest, scorebest)
   int* status;             // problems
   // scratch
-  int* trans;              // problems x C0max x C0max
-  int* foldcnt;            // problems x F x C0max
+  int* foldcnt;            // problems x (F + 1) x C0max
+  uint16_t* empty_rows;    // grid x L
   uint16_t* rows_scratch;  // grid x 8 x L (when the per-row arrays do not fit in shared memory)
-  uint64_t* raw_scratch;   // grid x (L/2 + 64) engine outputs of one shuffle
+  uint64_t* engine_save;   // grid x kEvolveEngineSave: the engine's state before a shuffle
   // learned proposal (kNN singleton path): network packed by mlp_pack_params, or nullptr
   const uint32_t* mlp;
   int mlp_greedy;          // 1 = relabel the top-scored candidates; 0 = sample them (Gumbel top-k)
@@ -98,7 +98,11 @@ struct EvolvePlsParams {
 };
 
 constexpr int kEvolveRowArrays = 8;
-size_t evolve_smem_bytes(int L, int C0max, bool rows_in_smem, bool trans_in_smem);
+constexpr int kEvolveEngineSave = kMtN + 8;
+size_t evolve_smem_bytes(int L, int C0max, bool rows_in_smem, int hist_warps);
+// Sets smem_rows and hist_warps to what fits in `budget` bytes of shared memory
+// (*smem of them); false if nothing does.
+bool evolve_place(EvolveParams& p, size_t budget, size_t* smem);
 int evolve_launch(const EvolveParams& p, int grid, size_t smem, void* stream);
 int evolve_pls_launch(const EvolvePlsParams& q, int grid, size_t smem, void* stream);
 

@@ -143,22 +143,10 @@ __device__ inline double canonical_serial(Mt64State& s) {
   return r >= 1.0 ? 0x1.fffffffffffffp-1 : r;
 }
 
-// std::discrete_distribution<int>(w, w+n)(engine).  cp is scratch of n doubles.
-__device__ inline int discrete_serial(Mt64State& s, const double* w, int n, double* cp) {
-  if (n < 2) return 0;
-  double sum = 0.0;
-  for (int i = 0; i < n; ++i) sum = __dadd_rn(sum, w[i]);
-  double acc = 0.0;
-  for (int i = 0; i < n; ++i) {
-    const double p = __ddiv_rn(w[i], sum);
-    acc = i == 0 ? p : __dadd_rn(acc, p);
-    cp[i] = acc;
-  }
-  cp[n - 1] = 1.0;
-  const double u = canonical_serial(s);
-  // lower_bound with the standard halving probe sequence (the cumulative array
-  // can be non-monotone in its last entry after rounding, so the probe order
-  // must be the standard one, not any bisection).
+// lower_bound of u with the standard halving probe sequence (the cumulative
+// array can be non-monotone in its last entry after rounding, so the probe order
+// must be the standard one, not any bisection).
+__device__ inline int discrete_probe(const double* cp, int n, double u) {
   int first = 0, len = n;
   while (len > 0) {
     const int half = len >> 1;
@@ -173,4 +161,18 @@ __device__ inline int discrete_serial(Mt64State& s, const double* w, int n, doub
   return first;
 }
 
+// std::discrete_distribution<int>(w, w+n)(engine).  cp is scratch of n doubles.
+__device__ inline int discrete_serial(Mt64State& s, const double* w, int n, double* cp) {
+  if (n < 2) return 0;
+  double sum = 0.0;
+  for (int i = 0; i < n; ++i) sum = __dadd_rn(sum, w[i]);
+  double acc = 0.0;
+  for (int i = 0; i < n; ++i) {
+    const double p = __ddiv_rn(w[i], sum);
+    acc = i == 0 ? p : __dadd_rn(acc, p);
+    cp[i] = acc;
+  }
+  cp[n - 1] = 1.0;
+  return discrete_probe(cp, n, canonical_serial(s));
+}
 }  // namespace kgb
