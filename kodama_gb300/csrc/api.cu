@@ -1099,15 +1099,16 @@ void matrix_from_device_graph(Ctx& ctx, const float* d_x, int n, int d, int* d_g
   cudaStream_t st = ctx.stream();
 
   // Where the background graph starts.  Its CTAs, once resident, hold the SMs
-  // that the atlas k-means' many short launches wait for, so it starts after
-  // the atlas -- unless it is the longer branch: the candidate search grows as
-  // n^2 d and the atlas plus the landmark stage about as n, and from about
-  // n = 40000 at d = 64 (N=20000, d=50: graph 2 ms, atlas + landmarks 6.5 ms;
-  // N=100000: 55 ms against 25 ms) the graph starts with the call.
-  const bool graph_first = static_cast<double>(n) * n * d >= 1.0e11;
+  // that the atlas k-means' many short launches and the landmark k-means' CTAs (a
+  // whole SM each) wait for.  A short graph goes with the landmark k-means, on the
+  // SMs that leaves idle.  A long one goes between the two, beside the planning,
+  // whose CTAs fit on the same SMs.  The search grows as n^2 d: 60000 x 50 rows
+  // (1.8e11) take 16.3 ms beside the planning and 17.4 beside the k-means,
+  // 100000 x 50 22.4 and 24.0, but 60000 x 20 (7e10) 16.8 and 15.5, 30000 x 200
+  // (1.8e11) 12.1 and 11.9 (100 runs of 20 cycles).
+  const bool graph_early = static_cast<double>(n) * n * d >= 1.0e11;
   int ev_bg0 = -1, ev_bg1 = -1, ev_planned = -1;
-  bool graph_bg = static_cast<bool>(build_graph) && graph_first &&
-                  ctx.on_background([&]() { build_graph(); }, &ev_bg0, &ev_bg1);
+  bool graph_bg = false;
 
   // shared landmark atlas (kodama_matrix.cpp:3662-3734)
   float* d_pnorm = ctx.alloc<float>(n);
@@ -1185,6 +1186,8 @@ void matrix_from_device_graph(Ctx& ctx, const float* d_x, int n, int d, int* d_g
     pa.scratch = ctx.alloc<char>(kgb::plan_scratch_bytes(n, coarse_k, L, M));
     ctx.fork();  // after the atlas and the status reset
     ck_launch(kgb::plan_landmarks(pa, ctx.side()), "landmark planning");
+    if (static_cast<bool>(build_graph) && graph_early && !graph_here)
+      graph_bg = ctx.on_background([&]() { build_graph(); }, &ev_bg0, &ev_bg1, ev_atlas);
     // the landmark k-means' assignment scratch is cleared beside the
     // planning, so that the k-means launch is the first thing the main
     // stream runs once the planning ends
@@ -1257,7 +1260,7 @@ void matrix_from_device_graph(Ctx& ctx, const float* d_x, int n, int d, int* d_g
   // the background graph becomes ready with the landmark k-means and is
   // queued after it, so the k-means' CTAs (a whole SM each) are placed first
   // and the graph fills the SMs they leave
-  if (static_cast<bool>(build_graph) && !graph_first && !graph_here)
+  if (static_cast<bool>(build_graph) && !graph_early && !graph_here)
     graph_bg = ctx.on_background([&]() { build_graph(); }, &ev_bg0, &ev_bg1, ev_planned);
   // folds (and the PLS slices) were planned on the host while the device worked
   FoldWork fold_work = folds_future.get();

@@ -20,6 +20,8 @@
 #include "launch_count.cuh"
 
 #include <cuda_runtime.h>
+
+#include <algorithm>
 #include <math.h>
 #include <stdint.h>
 
@@ -200,27 +202,45 @@ __global__ void project_kernel(ProjectArgs a) {
 }
 
 // Reverse adjacency of each problem's vote table: rev_idx[rev_off[v] ..
-// rev_off[v+1]) lists the rows r whose table contains v.  One CTA per problem.
+// rev_off[v+1]) lists the rows r whose table contains v.  A CTA per problem and
+// range of v: it reads the whole table, counts its own range (and how many entries
+// lie below it, where its lists start) and places its own rows.
+// What bounds it is the placing, one scattered two-byte store per entry and SM at
+// a time, and the two passes' loads, eight a thread in flight: with one CTA for
+// all v and a load at a time a table of 5003 x 30 took 221 us.
 __global__ void reverse_table_kernel(ReverseArgs a) {
   extern __shared__ int deg[];
   __shared__ int wsum[32];
+  __shared__ int below;
   const int p = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nwarps = (blockDim.x + 31) / 32;
+  const int nwarps = (blockDim.x + 31) / 32, step = blockDim.x;
+  const int width = (a.L + gridDim.y - 1) / gridDim.y;
+  const int lo = min(a.L, static_cast<int>(blockIdx.y) * width), hi = min(a.L, lo + width);
   const uint16_t* nb = a.nb + static_cast<size_t>(p) * a.L * a.w;
   int* off = a.rev_off + static_cast<size_t>(p) * (a.L + 1);
   uint16_t* idx = a.rev_idx + static_cast<size_t>(p) * a.L * a.w;
-  for (int v = tid; v <= a.L; v += blockDim.x) deg[v] = 0;
+  for (int v = tid; v < hi - lo; v += step) deg[v] = 0;
+  if (tid == 0) below = 0;
   __syncthreads();
   const int total = a.L * a.w;  // < 2^22: L < 2^16, w <= 32
-  for (int e = tid; e < total; e += blockDim.x) {
-    const uint16_t v = nb[e];
-    if (v != 0xFFFFu) atomicAdd(&deg[v], 1);
+  int under = 0;
+  for (int e0 = tid; e0 < total; e0 += 8 * step) {
+    int v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = e0 + q * step < total ? nb[e0 + q * step] : 0xFFFF;  // 0xFFFF: none
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      under += v[q] < lo;
+      if (v[q] >= lo && v[q] < hi) atomicAdd(&deg[v[q] - lo], 1);
+    }
   }
+  under = __reduce_add_sync(0xffffffffu, under);
+  if (lane == 0) atomicAdd(&below, under);
   __syncthreads();
   // exclusive scan of the in-degrees: each thread a contiguous chunk, then
   // the warps' and the block's prefixes
-  const int chunk = (a.L + blockDim.x - 1) / blockDim.x;
-  const int b = min(a.L, tid * chunk), e = min(a.L, b + chunk);
+  const int chunk = (hi - lo + step - 1) / step;
+  const int b = min(hi - lo, tid * chunk), e = min(hi - lo, b + chunk);
   int local = 0;
   for (int v = b; v < e; ++v) local += deg[v];
   int incl = local;
@@ -241,20 +261,25 @@ __global__ void reverse_table_kernel(ReverseArgs a) {
     if (lane < nwarps) wsum[lane] = w;  // inclusive warp totals
   }
   __syncthreads();
-  int run = (warp > 0 ? wsum[warp - 1] : 0) + incl - local;
+  int run = below + (warp > 0 ? wsum[warp - 1] : 0) + incl - local;
   for (int v = b; v < e; ++v) {
     const int c = deg[v];
     deg[v] = run;
-    off[v] = run;
+    off[lo + v] = run;
     run += c;
   }
-  if (tid == blockDim.x - 1) off[a.L] = wsum[nwarps - 1];
+  if (hi == a.L && lo < hi && tid == 0) off[a.L] = below + wsum[nwarps - 1];
   __syncthreads();
-  for (int e2 = tid; e2 < total; e2 += blockDim.x) {
-    const uint16_t v = nb[e2];
-    if (v == 0xFFFFu) continue;
-    const int slot = atomicAdd(&deg[v], 1);
-    idx[slot] = static_cast<uint16_t>(static_cast<unsigned>(e2) / static_cast<unsigned>(a.w));
+  for (int e0 = tid; e0 < total; e0 += 8 * step) {
+    int v[8], slot[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = e0 + q * step < total ? nb[e0 + q * step] : 0xFFFF;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) slot[q] = v[q] >= lo && v[q] < hi ? atomicAdd(&deg[v[q] - lo], 1) : -1;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (slot[q] >= 0)
+        idx[slot[q]] = static_cast<uint16_t>(static_cast<unsigned>(e0 + q * step) / static_cast<unsigned>(a.w));
   }
 }
 
@@ -499,11 +524,13 @@ int build_vote_tables(const VoteTableArgs& a, cudaStream_t st) {
 }
 
 int build_reverse_tables(const ReverseArgs& a, cudaStream_t st) {
-  const size_t smem = sizeof(int) * (static_cast<size_t>(a.L) + 1);
+  // two CTAs an SM: ranges until the chip is full, up to 16 of them
+  const int parts = std::max(1, std::min(std::min(16, 2 * 152 / a.problems), a.L));
+  const size_t smem = sizeof(int) * (static_cast<size_t>(a.L) / parts + 2);
   if (smem > 48 * 1024) {
     cudaFuncSetAttribute(reverse_table_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   }
-  reverse_table_kernel<<<a.problems, 1024, smem, st>>>(a);
+  reverse_table_kernel<<<dim3(a.problems, parts), 1024, smem, st>>>(a);
   count_launch();
   return static_cast<int>(cudaGetLastError());
 }

@@ -1,8 +1,8 @@
 // Per-run landmark planning on the device.
 //
 //   strata_kernel (one CTA): index_strata (kodama_matrix.cpp:806-854): the
-//     rows of every atlas cluster in ascending row order (counting sort, the
-//     stable scatter done by one warp with __match_any_sync ranks), and the
+//     rows of every atlas cluster in ascending row order (counting sort by
+//     warps of consecutive rows, each with counters of its own), and the
 //     run-independent parts of the quota allocation
 //     (kodama_matrix.cpp:880-903): floor of target*count/n and its fractional
 //     part, both in x86 extended precision (ext80.h).
@@ -25,11 +25,16 @@
 #include "plan.cuh"
 #include "rng.cuh"
 
+#include <algorithm>
+
 namespace kgb {
 namespace {
 
 constexpr int kPlanThreads = 256;
-constexpr int kSharedStrata = 8192;  // cursor/histogram in shared memory up to this many strata
+constexpr int kCounterBytes = 128 * 1024;  // strata_kernel: warps' counters in shared memory
+// plan_runs_kernel: order, quotas and fractions in shared memory.  No more than
+// that, so that a CTA fits beside one of the exact graph's, which runs meanwhile.
+constexpr int kSharedStrata = 2048;
 constexpr int kRounded = 0x40000000;  // marks a stratum of the shuffled order that took a residual slot
 
 size_t align256(size_t b) { return (b + 255) / 256 * 256; }
@@ -71,87 +76,105 @@ PlanScratch carve(const PlanArgs& a) {
   return s;
 }
 
+// Lanes whose code equals this lane's, of those in `act`, by `bits` ballots:
+// __match_any_sync takes two cycles of the SM per distinct code.
+__device__ __forceinline__ unsigned same_code(int code, unsigned act, int bits) {
+  unsigned m = act;
+  for (int b = 0; b < bits; ++b) {
+    const unsigned v = __ballot_sync(0xffffffffu, (code >> b) & 1);
+    m &= (code >> b) & 1 ? v : ~v;
+  }
+  return m;
+}
+
+// Each of nw warps takes a run of rows and counts them per stratum; after a scan
+// over warps and strata it walks them again and places them, so the rows of a
+// stratum keep ascending order.  One warp placing all rows took 0.94 ms at
+// 100000 rows.  With too many strata for two warps' counters in shared memory, one
+// warp counts in global memory.
 __global__ void __launch_bounds__(1024) strata_kernel(PlanArgs a, PlanScratch s) {
-  __shared__ int sh_count[kSharedStrata];
+  extern __shared__ int counters[];  // nw x strata
   __shared__ int bad;
   __shared__ unsigned long long asum;
-  const int tid = threadIdx.x;
-  const bool in_shared = a.strata <= kSharedStrata;
-  int* count = in_shared ? sh_count : s.counts;
+  __shared__ int wsum[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int fit = kCounterBytes / static_cast<int>(sizeof(int)) / a.strata;
+  const int nw = fit >= 2 ? min(32, fit) : 1;
+  int* count = fit >= 2 ? counters : s.counts;
   if (tid == 0) {
     bad = 0;
     asum = 0;
   }
-  for (int t = tid; t < a.strata; t += blockDim.x) count[t] = 0;
+  for (int t = tid; t < nw * a.strata; t += blockDim.x) count[t] = 0;
   __syncthreads();
-  for (int r = tid; r < a.n; r += blockDim.x) {
-    const int l = a.atlas[r];
-    if (l < 1 || l > a.strata) {
-      bad = 1;
-      continue;
+  const int chunk = ((a.n + nw - 1) / nw + 31) / 32 * 32;
+  const int beg = warp < nw ? min(a.n, warp * chunk) : 0, end = warp < nw ? min(a.n, beg + chunk) : 0;
+  int* mine = count + min(warp, nw - 1) * a.strata;
+  // the labels of eight 32-row steps are loaded ahead of their step
+  auto walk = [&](auto&& use) {
+    for (int b0 = beg; b0 < end; b0 += 8 * 32) {
+      int lv[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int r = b0 + 32 * u + lane;
+        lv[u] = r < end ? a.atlas[r] - 1 : -1;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (b0 + 32 * u < end) use(b0 + 32 * u + lane, lv[u]);
     }
-    atomicAdd(&count[l - 1], 1);
-  }
+  };
+  walk([&](int r, int l) {
+    if (r >= end) return;
+    if (l < 0 || l >= a.strata) bad = 1;
+    else atomicAdd(&mine[l], 1);
+  });
   __syncthreads();
   if (bad) {
     if (tid == 0) atomicExch(a.status, 1);
     return;
   }
-  // exclusive scan of the counts (one warp); the cursor starts at the offsets
-  if (tid < 32) {
-    int carry = 0;
-    for (int b = 0; b < a.strata; b += 32) {
-      const int t = b + tid;
-      const int c = t < a.strata ? count[t] : 0;
-      int v = c;
+  // per stratum the warps' starts within it, then the strata's offsets: a run of
+  // consecutive strata per thread
+  const int per = (a.strata + static_cast<int>(blockDim.x) - 1) / static_cast<int>(blockDim.x);
+  const int t0 = min(a.strata, tid * per), t1 = min(a.strata, t0 + per);
+  int local = 0;
+  for (int t = t0; t < t1; ++t)
+    for (int w = 0; w < nw; ++w) local += count[w * a.strata + t];
+  int incl = local;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, v, o);
-        if (tid >= o) v += y;
-      }
-      if (t < a.strata) s.offsets[t] = carry + v - c;
-      carry += __shfl_sync(0xffffffffu, v, 31);
-    }
-    if (tid == 0) s.offsets[a.strata] = carry;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
   }
+  if (lane == 31) wsum[warp] = incl;
   __syncthreads();
-  for (int t = tid; t < a.strata; t += blockDim.x) count[t] = s.offsets[t];  // count becomes the cursor
-  __syncthreads();
-  // stable scatter: rows of one stratum keep ascending order (one warp; the
-  // labels of eight 32-row steps are loaded ahead of their step)
-  if (tid < 32) {
-    for (int b0 = 0; b0 < a.n; b0 += 8 * 32) {
-      int lv[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int r = b0 + 32 * u + tid;
-        lv[u] = r < a.n ? a.atlas[r] - 1 : -1;
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int r = b0 + 32 * u + tid;
-        const bool valid = r < a.n;
-        const unsigned act = __ballot_sync(0xffffffffu, valid);
-        if (valid) {
-          const int l = lv[u];
-          const unsigned m = __match_any_sync(act, l);
-          const int leader = __ffs(m) - 1;
-          const int rank = __popc(m & ((1u << tid) - 1u));
-          int pos = 0;
-          if (tid == leader) {
-            pos = count[l];
-            count[l] = pos + __popc(m);
-          }
-          pos = __shfl_sync(act, pos, leader);
-          s.rows[pos + rank] = r;
-        }
-        __syncwarp();
-      }
+  int run = incl - local;
+  for (int w = 0; w < warp; ++w) run += wsum[w];
+  for (int t = t0; t < t1; ++t) {
+    s.offsets[t] = run;
+    for (int w = 0; w < nw; ++w) {
+      const int c = count[w * a.strata + t];
+      count[w * a.strata + t] = run;
+      run += c;
     }
   }
+  if (tid == 0) s.offsets[a.strata] = a.n;
+  __syncthreads();
+  const int bits = 32 - __clz(a.strata);
+  walk([&](int r, int l) {
+    const bool in = r < end;
+    const unsigned m = same_code(in ? l : 0, __ballot_sync(0xffffffffu, in), bits);
+    const int at = in ? mine[l] : 0;
+    const unsigned before = m & ((1u << lane) - 1u);
+    if (in) s.rows[at + __popc(before)] = r;
+    __syncwarp();
+    if (in && before == 0u) mine[l] = at + __popc(m);
+    __syncwarp();
+  });
   // quota parts (run-independent)
   const Ext80 total = ext80_from_u64(static_cast<uint64_t>(a.n));
-  unsigned long long local = 0;
+  unsigned long long bases = 0;
   for (int t = tid; t < a.strata; t += blockDim.x) {
     const int c = s.offsets[t + 1] - s.offsets[t];
     int base = 0;
@@ -164,9 +187,9 @@ __global__ void __launch_bounds__(1024) strata_kernel(PlanArgs a, PlanScratch s)
     }
     s.base[t] = base;
     s.frac[t] = frac;
-    local += static_cast<unsigned long long>(base);
+    bases += static_cast<unsigned long long>(base);
   }
-  atomicAdd(&asum, local);
+  atomicAdd(&asum, bases);
   __syncthreads();
   if (tid == 0) *s.assigned = static_cast<int>(asum);
 }
@@ -225,215 +248,140 @@ __device__ uint64_t draw_below_warp(Mt64State& rng, uint64_t range, int lane) {
   }
 }
 
-// Shared state of one std::sample call run by the whole CTA.
-struct __align__(16) SampleShared {
-  uint32_t p1[kMtN];  // the two acceptance positions of each step of a batch
-  uint32_t p2[kMtN];
-  uint16_t sel[kMtN]; // the walk's decisions: bit 0 the first row of a step, bit 8 the second
-  long long uns, nq;  // rows not yet visited, rows still wanted
-  int i, taken;       // next row of the stratum, rows taken so far
-  int rej;            // first step of the batch whose draw Lemire's method rejects
-  int visited;        // rows the batch's walk visited
-  int redraw;         // the rejected step is next and is drawn one output at a time
-};
+// std::sample in strata (forward population), by one warp: selection sampling with
+// two acceptance positions per draw while two or more rows remain.  A step's
+// range depends only on how many rows remain, so the lanes draw the positions of
+// up to 32 steps at once (one engine output per step) and the acceptance
+// recursion -- a compare and a decrement per row -- runs over them in every lane
+// alike; a taken row's flag is set a batch later, when its number has come from
+// memory.  A draw that Lemire's method would reject (probability about
+// range / 2^64) ends the batch and is drawn one output at a time, as are the
+// single draws once fewer than two rows remain.
+// What bounds it is the recursion, some 20 cycles a step.  By the whole CTA, with
+// six barriers and a trip to memory per batch, 100 strata of 10 rows took 430k
+// cycles and 300 of 333 rows 3.8 M.
+struct Sampler {
+  Mt64State& rng;
+  const int* rows;
+  uint8_t* flags;
+  int lane;
+  int wait_a = -1, wait_b = -1;  // rows of the batch before whose flags are to be set
 
-// std::sample of q rows out of the size rows starting at position first of
-// the strata row list (forward population): selection sampling, two
-// acceptance positions per draw while two or more rows remain.  The whole CTA
-// in batches: a step's range depends only on how many rows remain, so the
-// threads draw the acceptance positions of up to the rest of the engine's
-// output block at once (one output per step); thread 0 then walks the
-// acceptance recursion over them in order -- a compare and a decrement per
-// row, the decisions stored as bytes -- and the CTA flags the taken rows.  A
-// draw that Lemire's method would reject (probability about range / 2^64)
-// ends the batch; warp 0 redraws that step one output at a time, as it does
-// the single draws once fewer than two rows remain.  Called by every thread;
-// the count of rows taken is returned to thread 0.
-__device__ int sample_cta(int first, int size, int q, const int* __restrict__ rows, uint8_t* __restrict__ flags,
-                          Mt64State& rng, SampleShared& ss, int tid) {
-  if (size <= 0) return 0;
-  const int lane = tid & 31;
-  if (tid == 0) {
-    ss.uns = size;
-    ss.nq = q < size ? q : size;
-    ss.i = 0;
-    ss.taken = 0;
+  __device__ void settle() {
+    if (wait_a >= 0) flags[wait_a] = 1;
+    if (wait_b >= 0) flags[wait_b] = 1;
+    wait_a = wait_b = -1;
   }
-  __syncthreads();
-  long long uns = 0, nq = 0;
-  for (;;) {
-    uns = ss.uns;
-    nq = ss.nq;
-    const int pos0 = rng.pos, i0 = ss.i;
-    __syncthreads();  // every thread has read the state before it changes
-    if (nq == 0 || uns < 2) break;
-    if (pos0 >= kMtN) {
-      if (tid < 32) mt64_refill_warp(rng, lane);
-      __syncthreads();
-    }
-    const int pos = pos0 >= kMtN ? 0 : pos0;
-    const long long steps_left = uns / 2;
-    const int batch = static_cast<int>(kMtN - pos < steps_left ? kMtN - pos : steps_left);
-    if (tid == 0) ss.rej = batch;
-    __syncthreads();
-    for (int j = tid; j < batch; j += kPlanThreads) {
-      const long long ul = uns - 2LL * j;
-      const uint64_t b1 = static_cast<uint64_t>(ul - 1);
-      const uint64_t range = static_cast<uint64_t>(ul) * b1;
-      const uint64_t u = rng.out[pos + j];
+
+  // min(q, size) of the size rows at position first of the strata's row list
+  __device__ int take(int first, int size, int q) {
+    int uns = size, nq = min(q, size), at = first;
+    const int wanted = nq;
+    while (nq != 0 && uns >= 2) {
+      if (rng.pos >= kMtN) mt64_refill_warp(rng, lane);
+      const int pos = rng.pos, batch = min(32, min(kMtN - pos, uns >> 1));
+      const bool in = lane < batch;
+      const int ra = in ? rows[at + 2 * lane] : -1, rb = in ? rows[at + 2 * lane + 1] : -1;
+      settle();
+      const uint64_t left = static_cast<uint64_t>(in ? uns - 2 * lane : 2), b1 = left - 1, range = left * b1;
+      const uint64_t u = in ? rng.out[pos + lane] : 0;
       const uint64_t lo = u * range;
-      if (lo < range && lo < (0ull - range) % range) atomicMin(&ss.rej, j);
-      uint64_t p1, p2;
-      divmod_u64(__umul64hi(u, range), b1, p1, p2);
-      ss.p1[j] = static_cast<uint32_t>(p1);
-      ss.p2[j] = static_cast<uint32_t>(p2);
-    }
-    __syncthreads();
-    if (tid == 0) {
-      // nq <= size < 2^31: 32-bit counters; after a step that ends the sample
-      // (nn == 0) nothing more is taken, and the step's second row counts as
-      // visited only if the first did not end it
-      const int usable = ss.rej;
-      uint32_t nn = static_cast<uint32_t>(nq), n1 = nn;
-      int l = 0;
-      bool done = false;
-      // eight steps per pass without branches: once nn reaches 0 every later
-      // compare fails and nn stays 0, so the pass runs to its end and the
-      // step that ended the sample (and its n1) is picked out afterwards;
-      // p1, p2 and sel start 16-byte aligned
-      for (; l + 8 <= usable; l += 8) {
-        const uint4 P0 = *reinterpret_cast<const uint4*>(ss.p1 + l);
-        const uint4 P1 = *reinterpret_cast<const uint4*>(ss.p1 + l + 4);
-        const uint4 Q0 = *reinterpret_cast<const uint4*>(ss.p2 + l);
-        const uint4 Q1 = *reinterpret_cast<const uint4*>(ss.p2 + l + 4);
-        const uint32_t a1[8] = {P0.x, P0.y, P0.z, P0.w, P1.x, P1.y, P1.z, P1.w};
-        const uint32_t a2[8] = {Q0.x, Q0.y, Q0.z, Q0.w, Q1.x, Q1.y, Q1.z, Q1.w};
-        uint32_t sel[8];
-        int stop = 8;
-        uint32_t stop_n1 = 0;
+      const unsigned bad = __ballot_sync(0xffffffffu, in && lo < range && lo < (0ull - range) % range);
+      const int usable = bad != 0u ? __ffs(bad) - 1 : batch;
+      uint64_t d1, d2;
+      divmod_u64(__umul64hi(u, range), b1, d1, d2);
+      // positions of steps past the usable ones take nothing
+      const unsigned p1 = lane < usable ? static_cast<unsigned>(d1) : 0xffffffffu;
+      const unsigned p2 = lane < usable ? static_cast<unsigned>(d2) : 0xffffffffu;
+      // once nn is 0 every later compare fails, so the last row taken ends it
+      unsigned nn = static_cast<unsigned>(nq), m1 = 0, m2 = 0;
+      for (int j = 0; j < usable && nn != 0u; j += 8) {
+        unsigned a1[8], a2[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          const uint32_t before = nn;
-          const uint32_t t1 = a1[e] < nn ? 1u : 0u;
-          const uint32_t m1 = nn - t1;
-          const uint32_t t2 = a2[e] < m1 ? 1u : 0u;
-          nn = m1 - t2;
-          sel[e] = t1 | (t2 << 8);
-          const bool hit = before != 0 && nn == 0;
-          stop = hit ? e : stop;
-          stop_n1 = hit ? m1 : stop_n1;
+          a1[e] = __shfl_sync(0xffffffffu, p1, j + e);
+          a2[e] = __shfl_sync(0xffffffffu, p2, j + e);
         }
-        *reinterpret_cast<uint4*>(ss.sel + l) =
-            make_uint4(sel[0] | (sel[1] << 16), sel[2] | (sel[3] << 16), sel[4] | (sel[5] << 16), sel[6] | (sel[7] << 16));
-        if (nn == 0) {
-          l += stop;  // the step that ended the sample
-          n1 = stop_n1;
-          done = true;
-          break;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const unsigned t1 = a1[e] < nn ? 1u : 0u;
+          nn -= t1;
+          const unsigned t2 = a2[e] < nn ? 1u : 0u;
+          nn -= t2;
+          m1 |= t1 << (j + e);
+          m2 |= t2 << (j + e);
         }
       }
-      for (; l < usable && !done; ++l) {
-        const uint32_t a1 = ss.p1[l], a2 = ss.p2[l];
-        const uint32_t t1 = a1 < nn ? 1u : 0u;
-        n1 = nn - t1;
-        const uint32_t t2 = a2 < n1 ? 1u : 0u;
-        nn = n1 - t2;
-        ss.sel[l] = static_cast<uint16_t>(t1 | (t2 << 8));
-        if (nn == 0) {
-          done = true;
-          break;
-        }
-      }
-      const int steps = done ? l + 1 : usable;
-      const int visited = done ? 2 * l + 1 + (n1 != 0 ? 1 : 0) : 2 * usable;
-      rng.pos = pos + steps;
-      ss.uns = uns - visited;
-      ss.nq = nn;
-      ss.i = i0 + visited;
-      ss.taken += static_cast<int>(nq - static_cast<long long>(nn));
-      ss.visited = visited;
-      ss.redraw = !done && usable < batch;
-    }
-    __syncthreads();
-    for (int k = tid; k < ss.visited; k += kPlanThreads)
-      if ((ss.sel[k >> 1] >> (8 * (k & 1))) & 1u) flags[rows[first + i0 + k]] = 1;
-    if (ss.redraw) {
-      // the rejected step, drawn one output at a time by warp 0
-      if (tid < 32) {
-        long long un = ss.uns, nn = ss.nq;
-        int i = ss.i, taken = ss.taken;
-        const uint64_t b1 = static_cast<uint64_t>(un - 1);
-        uint64_t a1, a2;
-        divmod_u64(draw_below_warp(rng, static_cast<uint64_t>(un) * b1, lane), b1, a1, a2);
-        --un;
-        if (static_cast<long long>(a1) < nn) {
-          if (tid == 0) flags[rows[first + i]] = 1;
-          --nn;
-          ++taken;
-        }
-        ++i;
-        if (nn != 0) {
-          --un;
-          if (static_cast<long long>(a2) < nn) {
-            if (tid == 0) flags[rows[first + i]] = 1;
-            --nn;
-            ++taken;
-          }
-          ++i;
-        }
-        __syncwarp();
-        if (tid == 0) {
-          ss.uns = un;
-          ss.nq = nn;
-          ss.i = i;
-          ss.taken = taken;
-        }
-      }
-    }
-    __syncthreads();
-  }
-  if (nq != 0) {
-    // fewer than two rows left: one draw per row (warp 0)
-    if (tid < 32) {
-      long long un = uns, nn = nq;
-      int i = ss.i, taken = ss.taken;
-      for (; nn != 0; ++i) {
-        --un;
-        if (static_cast<long long>(draw_below_warp(rng, static_cast<uint64_t>(un) + 1, lane)) < nn) {
-          if (tid == 0) flags[rows[first + i]] = 1;
-          --nn;
-          ++taken;
-        }
+      int steps = usable, visited = 2 * usable;
+      if (nn == 0u) {
+        const int last = 31 - __clz(m1 | m2);
+        steps = last + 1;
+        visited = 2 * last + 1 + static_cast<int>((m2 >> last) & 1u);
       }
       __syncwarp();
-      if (tid == 0) ss.taken = taken;
+      if (lane == 0) rng.pos = pos + steps;
+      __syncwarp();
+      wait_a = (m1 >> lane) & 1u ? ra : -1;
+      wait_b = (m2 >> lane) & 1u ? rb : -1;
+      uns -= visited;
+      at += visited;
+      nq = static_cast<int>(nn);
+      if (nq != 0 && usable < batch) {
+        // the rejected step, drawn one output at a time
+        const uint64_t c1 = static_cast<uint64_t>(uns) - 1;
+        divmod_u64(draw_below_warp(rng, static_cast<uint64_t>(uns) * c1, lane), c1, d1, d2);
+        for (const uint64_t d : {d1, d2}) {
+          if (nq == 0) break;
+          if (d < static_cast<uint64_t>(nq)) {
+            if (lane == 0) flags[rows[at]] = 1;
+            --nq;
+          }
+          --uns;
+          ++at;
+        }
+      }
     }
-    __syncthreads();
+    for (; nq != 0; ++at) {
+      --uns;
+      if (draw_below_warp(rng, static_cast<uint64_t>(uns) + 1, lane) < static_cast<uint64_t>(nq)) {
+        if (lane == 0) flags[rows[at]] = 1;
+        --nq;
+      }
+    }
+    return wanted;
   }
-  return tid == 0 ? ss.taken : 0;
-}
-
-// std::mt19937 (Matsumoto & Nishimura 1998: n=624, m=397), serial.
-struct Mt32State {
-  uint32_t mt[624];
-  int pos;
 };
 
-__device__ void mt32_seed(Mt32State& s, uint32_t seed) {
-  s.mt[0] = seed;
-  for (int i = 1; i < 624; ++i) s.mt[i] = 1812433253u * (s.mt[i - 1] ^ (s.mt[i - 1] >> 30)) + static_cast<uint32_t>(i);
-  s.pos = 624;
+// std::mt19937 (Matsumoto & Nishimura 1998: n=624, m=397) by the whole CTA:
+// seeding is a chain, a block of outputs is formed in three parts, each from words
+// that are ready.
+constexpr int kMt32N = 624, kMt32M = 397;
+
+__device__ void mt32_seed(uint32_t* mt, uint32_t seed) {
+  uint32_t p = seed;
+  mt[0] = p;
+  for (int i = 1; i < kMt32N; ++i) {
+    p = 1812433253u * (p ^ (p >> 30)) + static_cast<uint32_t>(i);
+    mt[i] = p;
+  }
 }
 
-__device__ uint32_t mt32_next(Mt32State& s) {
-  if (s.pos >= 624) {
-    for (int i = 0; i < 624; ++i) {
-      const uint32_t y = (s.mt[i] & 0x80000000u) | (s.mt[i + 1 < 624 ? i + 1 : 0] & 0x7fffffffu);
-      s.mt[i] = s.mt[i + 397 < 624 ? i + 397 : i + 397 - 624] ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
+__device__ void mt32_block(uint32_t* mt, int tid) {
+  for (int part = 0; part < kMt32N; part += kMt32N - kMt32M) {
+    const int i = part + tid;
+    const bool in = tid < kMt32N - kMt32M && i < kMt32N;
+    uint32_t v = 0;
+    if (in) {
+      const uint32_t y = (mt[i] & 0x80000000u) | (mt[i + 1 < kMt32N ? i + 1 : 0] & 0x7fffffffu);
+      v = mt[i + kMt32M < kMt32N ? i + kMt32M : i + kMt32M - kMt32N] ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
     }
-    s.pos = 0;
+    __syncthreads();
+    if (in) mt[i] = v;
+    __syncthreads();
   }
-  uint32_t y = s.mt[s.pos++];
+}
+
+__device__ __forceinline__ uint32_t mt32_temper(uint32_t y) {
   y ^= y >> 11;
   y ^= (y << 7) & 0x9d2c5680u;
   y ^= (y << 15) & 0xefc60000u;
@@ -441,134 +389,206 @@ __device__ uint32_t mt32_next(Mt32State& s) {
   return y;
 }
 
+// Bytes of shared memory for the strata's order, quotas and fractions.
+size_t plan_smem_bytes(int strata) {
+  return strata <= kSharedStrata ? static_cast<size_t>(strata) * (sizeof(Ext80) + 2 * sizeof(int)) : 0;
+}
+
+// The chains of dependent steps (the shuffle's swaps, the residual allocation,
+// each stratum's sample) run on one thread or warp, so what they read is brought
+// into shared memory first: from global memory each step waited for L2.
 __global__ void __launch_bounds__(kPlanThreads) plan_runs_kernel(PlanArgs a, PlanScratch s) {
+  extern __shared__ __align__(16) unsigned char plan_smem[];
   __shared__ Mt64State rng;
-  __shared__ Mt32State rng32;
-  __shared__ SampleShared ss;
-  __shared__ int sh_bad, sh_total;
+  __shared__ uint32_t mt32[kMt32N];
+  __shared__ uint32_t swap_to[kMt32N];
+  __shared__ int sh_bad, sh_strata;
   __shared__ uint32_t sh_kseed;
   __shared__ int sh_warp[kPlanThreads / 32];
   const int run = blockIdx.x, tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   uint8_t* flags = s.flags + static_cast<size_t>(run) * a.n;
-  int* quota = s.quota + static_cast<size_t>(run) * a.strata;
-  int* order = s.order + static_cast<size_t>(run) * a.strata;
+  const bool shared_strata = a.strata <= kSharedStrata;
+  Ext80* sh_frac = reinterpret_cast<Ext80*>(plan_smem);  // by position in the shuffled order
+  int* quota = shared_strata ? reinterpret_cast<int*>(sh_frac + a.strata) : s.quota + static_cast<size_t>(run) * a.strata;
+  int* order = shared_strata ? quota + a.strata : s.order + static_cast<size_t>(run) * a.strata;
   for (int r = tid; r < a.n; r += kPlanThreads) flags[r] = 0;
   for (int t = tid; t < a.strata; t += kPlanThreads) quota[t] = s.base[t];
+  if (tid == 0) mt64_seed(rng, a.seed + static_cast<uint64_t>(a.first_run + run));
+  if (warp == 1) {
+    // the non-empty strata in order
+    int S = 0;
+    for (int b = 0; b < a.strata; b += 32) {
+      const int t = b + lane;
+      const bool in = t < a.strata && s.offsets[t + 1] > s.offsets[t];
+      const unsigned m = __ballot_sync(0xffffffffu, in);
+      if (in) order[S + __popc(m & ((1u << lane) - 1u))] = t;
+      S += __popc(m);
+    }
+    if (lane == 0) sh_strata = S;
+  }
   __syncthreads();
-  {
-    if (tid == 0) {
-      int bad = 0;
-      mt64_seed(rng, a.seed + static_cast<uint64_t>(a.first_run + run));
-      (void)mt64_next_serial(rng);
-      int S = 0;
-      for (int t = 0; t < a.strata; ++t)
-        if (s.offsets[t + 1] > s.offsets[t]) order[S++] = t;
-      shuffle_serial(order, S, rng);
-      const int residual = a.target - *s.assigned;
-      if (residual > 0) {
-        const Ext80 offset = ext80_canonical(mt64_next_serial(rng));
-        Ext80 cumulative{0, 0};
-        int selected = 0;
-        for (int i = 0; i < S; ++i) {
+  if (warp == 0) mt64_refill_warp(rng, lane);
+  __syncthreads();
+  const int S = sh_strata;
+  if (tid == 0) {
+    (void)mt64_next_serial(rng);
+    shuffle_serial(order, S, rng);
+    sh_bad = 0;
+  }
+  __syncthreads();
+  if (shared_strata)
+    for (int i = tid; i < S; i += kPlanThreads) sh_frac[i] = s.frac[order[i]];
+  __syncthreads();
+  if (tid == 0) {
+    const int residual = a.target - *s.assigned;
+    if (residual > 0) {
+      auto frac = [&](int i) { return shared_strata ? sh_frac[i] : s.frac[order[i] & ~kRounded]; };
+      const Ext80 offset = ext80_canonical(mt64_next_serial(rng));
+      Ext80 cumulative{0, 0};
+      int selected = 0;
+      for (int i = 0; i < S; ++i) {
+        cumulative = ext80_add(cumulative, frac(i));
+        const Ext80 next = ext80_add(offset, ext80_from_u64(static_cast<uint64_t>(selected)));
+        if (selected < residual && ext80_lt(next, cumulative)) {
           const int t = order[i];
-          cumulative = ext80_add(cumulative, s.frac[t]);
-          const Ext80 next = ext80_add(offset, ext80_from_u64(static_cast<uint64_t>(selected)));
-          if (selected < residual && ext80_lt(next, cumulative)) {
-            ++quota[t];
-            order[i] = t | kRounded;
-            ++selected;
-          }
-        }
-        while (selected < residual) {
-          int best = -1, besti = -1;
-          Ext80 bestv{0, 0};
-          for (int i = 0; i < S; ++i) {
-            const int t = order[i];
-            if (t & kRounded) continue;
-            if (best < 0 || ext80_lt(bestv, s.frac[t])) {
-              bestv = s.frac[t];
-              best = t;
-              besti = i;
-            }
-          }
-          if (best < 0) {
-            bad = 2;
-            break;
-          }
-          ++quota[best];
-          order[besti] = best | kRounded;
+          ++quota[t];
+          order[i] = t | kRounded;
           ++selected;
         }
       }
-      sh_bad = bad;
-    }
-    __syncthreads();
-    if (sh_bad == 0) {
-      int total = 0;
-      for (int t = 0; t < a.strata; ++t) {
-        const int q = quota[t];
-        if (q <= 0) continue;
-        total += sample_cta(s.offsets[t], s.offsets[t + 1] - s.offsets[t], q, s.rows, flags, rng, ss, tid);
+      while (selected < residual) {
+        int besti = -1;
+        Ext80 bestv{0, 0};
+        for (int i = 0; i < S; ++i) {
+          if (order[i] & kRounded) continue;
+          if (besti < 0 || ext80_lt(bestv, frac(i))) {
+            bestv = frac(i);
+            besti = i;
+          }
+        }
+        if (besti < 0) {
+          sh_bad = 2;
+          break;
+        }
+        const int best = order[besti];
+        ++quota[best];
+        order[besti] = best | kRounded;
+        ++selected;
       }
-      if (tid == 0 && total != a.target) sh_bad = 3;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      sh_kseed = static_cast<uint32_t>((mt64_next_serial(rng) & 0x7fffffffull) + 1ull);
-      sh_total = 0;
     }
   }
+  __syncthreads();
+  if (warp == 0 && sh_bad == 0) {
+    Sampler sampler{rng, s.rows, flags, lane};
+    int total = 0;
+    for (int t0 = 0; t0 < a.strata; t0 += 32) {
+      // 32 strata's ranges and quotas at a time
+      const int t = min(t0 + lane, a.strata - 1);
+      const int first = s.offsets[t], size = s.offsets[t + 1] - first, q = t0 + lane < a.strata ? quota[t] : 0;
+      for (unsigned m = __ballot_sync(0xffffffffu, q > 0 && size > 0); m != 0u; m &= m - 1) {
+        const int l = __ffs(m) - 1;
+        total += sampler.take(__shfl_sync(0xffffffffu, first, l), __shfl_sync(0xffffffffu, size, l),
+                              __shfl_sync(0xffffffffu, q, l));
+      }
+    }
+    sampler.settle();
+    if (lane == 0 && total != a.target) sh_bad = 3;
+  }
+  __syncthreads();
+  if (tid == 0) sh_kseed = static_cast<uint32_t>((mt64_next_serial(rng) & 0x7fffffffull) + 1ull);
   __syncthreads();
   if (sh_bad) {
     if (tid == 0) atomicExch(a.status, sh_bad);
     return;
   }
-  // ascending compaction of the selected rows (and of the others)
-  int* land = a.land + static_cast<size_t>(run) * a.target;
-  int* nonland = a.nonland == nullptr ? nullptr : a.nonland + static_cast<size_t>(run) * (a.n - a.target);
-  for (int b = 0; b < a.n; b += kPlanThreads) {
-    const int r = b + tid;
-    const int f = r < a.n ? flags[r] : 0;
-    const unsigned bal = __ballot_sync(0xffffffffu, f != 0);
-    if (lane == 0) sh_warp[warp] = __popc(bal);
-    __syncthreads();
-    int pos = sh_total;
-    for (int i = 0; i < warp; ++i) pos += sh_warp[i];
-    pos += __popc(bal & ((1u << lane) - 1u));
-    if (r < a.n) {
-      if (f) {
-        land[pos] = r;
-      } else if (nonland != nullptr) {
-        nonland[r - pos] = r;
-      }
-    }
-    __syncthreads();
-    if (tid == 0) {
-      int t = 0;
-      for (int i = 0; i < kPlanThreads / 32; ++i) t += sh_warp[i];
-      sh_total += t;
-    }
-    __syncthreads();
-  }
-  // initial centroid rows: head of the permutation of 0..L-1
   const int L = a.target;
   const int k = max(1, min(a.init_k, L));
-  int* perm = s.perm + static_cast<size_t>(run) * L;
-  for (int i = tid; i < L; i += kPlanThreads) perm[i] = i;
-  __syncthreads();
-  if (tid == 0) {
-    mt32_seed(rng32, sh_kseed);
-    const int steps = min(k, L - 1);
-    for (int r = 0; r < steps; ++r) {
-      const uint32_t u = mt32_next(rng32);
-      const int other = r + static_cast<int>(u % static_cast<uint32_t>(L - r));
-      const int t = perm[r];
-      perm[r] = perm[other];
-      perm[other] = t;
+  // ascending compaction of the selected rows (and of the others): a run of rows
+  // per warp, eight 32-row steps' flags in flight; the last warp seeds the
+  // permutation's engine beside it
+  constexpr int kCompactWarps = kPlanThreads / 32 - 1;
+  int* land = a.land + static_cast<size_t>(run) * a.target;
+  int* nonland = a.nonland == nullptr ? nullptr : a.nonland + static_cast<size_t>(run) * (a.n - a.target);
+  const int chunk = ((a.n + kCompactWarps - 1) / kCompactWarps + 31) / 32 * 32;
+  const int beg = warp < kCompactWarps ? min(a.n, warp * chunk) : 0;
+  const int end = warp < kCompactWarps ? min(a.n, beg + chunk) : 0;
+  auto walk = [&](auto&& use) {
+    for (int b0 = beg; b0 < end; b0 += 8 * 32) {
+      unsigned f[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int r = b0 + 32 * u + lane;
+        f[u] = r < end ? flags[r] : 0u;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) use(b0 + 32 * u + lane, f[u] != 0u);
     }
-    int* out = a.init_rows + static_cast<size_t>(run) * a.init_k;
-    for (int r = 0; r < k; ++r) out[r] = perm[r];
+  };
+  int taken = 0;
+  walk([&](int, bool f) { taken += __popc(__ballot_sync(0xffffffffu, f)); });
+  if (lane == 0) sh_warp[warp] = taken;
+  if (tid == kPlanThreads - 32) mt32_seed(mt32, sh_kseed);
+  __syncthreads();
+  int pos0 = 0;
+  for (int w = 0; w < warp; ++w) pos0 += sh_warp[w];
+  walk([&](int r, bool f) {
+    const unsigned m = __ballot_sync(0xffffffffu, f);
+    const int pos = pos0 + __popc(m & ((1u << lane) - 1u));
+    if (r < end) {
+      if (f) land[pos] = r;
+      else if (nonland != nullptr) nonland[r - pos] = r;
+    }
+    pos0 += __popc(m);
+  });
+  __syncthreads();
+  // initial centroid rows: head of the permutation of 0..L-1.  Step i swaps
+  // positions i and to(i) >= i.  Position x holds x until a step j with to(j) == x
+  // moves there what was at j; so before its own step, position j holds the root
+  // of the chain j -> last i < j with to(i) == j, and entry r of the head is the
+  // root of the last j < r with to(j) == to(r), or to(r) itself.
+  const int steps = min(k, L - 1);
+  int* out = a.init_rows + static_cast<size_t>(run) * a.init_k;
+  if (steps <= kMt32N) {
+    mt32_block(mt32, tid);
+    for (int i = tid; i < steps; i += kPlanThreads)
+      swap_to[i] = static_cast<uint32_t>(i) + mt32_temper(mt32[i]) % static_cast<uint32_t>(L - i);
+    __syncthreads();
+    // the last step before `upto` that swaps with position x, or -1
+    auto last_to = [&](int x, int upto) {
+      int at = -1;
+      for (int j = 0; j < upto; ++j) at = swap_to[j] == static_cast<uint32_t>(x) ? j : at;
+      return at;
+    };
+    for (int j = tid; j < steps; j += kPlanThreads) mt32[j] = static_cast<uint32_t>(last_to(j, j));
+    __syncthreads();
+    for (int r = tid; r < k; r += kPlanThreads) {
+      // past the last step (k = L) the entry is what its position holds
+      const int x = r < steps ? static_cast<int>(swap_to[r]) : r;
+      int j = last_to(x, min(r, steps));
+      if (j >= 0)
+        for (int up = static_cast<int>(mt32[j]); up >= 0; up = static_cast<int>(mt32[j])) j = up;
+      out[r] = j >= 0 ? j : x;
+    }
+  } else {
+    int* perm = s.perm + static_cast<size_t>(run) * L;
+    for (int i = tid; i < L; i += kPlanThreads) perm[i] = i;
+    for (int r0 = 0; r0 < steps; r0 += kMt32N) {
+      mt32_block(mt32, tid);
+      const int m = min(kMt32N, steps - r0);
+      for (int i = tid; i < m; i += kPlanThreads)
+        swap_to[i] = static_cast<uint32_t>(r0 + i) + mt32_temper(mt32[i]) % static_cast<uint32_t>(L - r0 - i);
+      __syncthreads();
+      if (tid == 0) {
+        for (int i = 0; i < m; ++i) {
+          const int r = r0 + i, other = static_cast<int>(swap_to[i]), t = perm[r];
+          perm[r] = perm[other];
+          perm[other] = t;
+        }
+      }
+      __syncthreads();
+    }
+    for (int r = tid; r < k; r += kPlanThreads) out[r] = perm[r];
   }
 }
 
@@ -604,9 +624,16 @@ int plan_landmarks(const PlanArgs& a, cudaStream_t st) {
       a.init_k > a.target)
     return static_cast<int>(cudaErrorInvalidValue);
   const PlanScratch s = carve(a);
-  strata_kernel<<<1, 1024, 0, st>>>(a, s);
+  const int fit = kCounterBytes / static_cast<int>(sizeof(int)) / a.strata;
+  const int counter_bytes = fit >= 2 ? std::min(32, fit) * a.strata * static_cast<int>(sizeof(int)) : 0;
+  cudaError_t e = cudaFuncSetAttribute(strata_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCounterBytes);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  strata_kernel<<<1, 1024, counter_bytes, st>>>(a, s);
   count_launch();
-  plan_runs_kernel<<<a.runs, kPlanThreads, 0, st>>>(a, s);
+  const size_t smem = plan_smem_bytes(a.strata);
+  e = cudaFuncSetAttribute(plan_runs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  if (e != cudaSuccess) return static_cast<int>(e);
+  plan_runs_kernel<<<a.runs, kPlanThreads, smem, st>>>(a, s);
   count_launch();
   return static_cast<int>(cudaGetLastError());
 }

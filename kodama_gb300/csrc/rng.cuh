@@ -54,10 +54,11 @@ __device__ __forceinline__ uint64_t mt64_mix(uint64_t cur, uint64_t next, uint64
 
 // Serial seeding by one thread.
 __device__ inline void mt64_seed(Mt64State& s, uint64_t seed) {
-  s.mt[0] = seed;
+  uint64_t p = seed;
+  s.mt[0] = p;
   for (int i = 1; i < kMtN; ++i) {
-    const uint64_t p = s.mt[i - 1];
-    s.mt[i] = 6364136223846793005ull * (p ^ (p >> 62)) + static_cast<uint64_t>(i);
+    p = 6364136223846793005ull * (p ^ (p >> 62)) + static_cast<uint64_t>(i);
+    s.mt[i] = p;
   }
   s.pos = kMtN;
 }
