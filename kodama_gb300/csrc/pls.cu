@@ -508,7 +508,7 @@ __device__ __forceinline__ void group_seq_dots(int dots, int n, int lane, int wa
     const int d = d0 + g;
     float s = 0.0f, c = 0.0f, A = 0.0f;
     if (d < dots) {
-#pragma unroll 4
+#pragma unroll 8
       for (int k = gl; k < n; k += 8) {
         float x, y;
         load(d, k, x, y);
@@ -622,8 +622,8 @@ __device__ void block_loading(const float* __restrict__ Zs, int zp, int p, const
   long long* pacc = reinterpret_cast<long long*>((reinterpret_cast<uintptr_t>(scratch) + 7) & ~uintptr_t(7));
   float* pA = reinterpret_cast<float*>(pacc + kEvalThreads);
   int* pflag = reinterpret_cast<int*>(pA + kEvalThreads);  // non-zero values seen
-  int* srow = pflag + kEvalThreads;
-  float* ssc = reinterpret_cast<float*>(srow + kLoadChunk);
+  // a row's offset and score together
+  int2* srow = reinterpret_cast<int2*>((reinterpret_cast<uintptr_t>(pflag + kEvalThreads) + 7) & ~uintptr_t(7));
   int* flist = reinterpret_cast<int*>(pacc);  // undecided columns (after the partials are read)
   __shared__ int fcount, smax;
   const int t = threadIdx.x, lg = clog2i(nt);
@@ -648,36 +648,54 @@ __device__ void block_loading(const float* __restrict__ Zs, int zp, int p, const
     for (int k0 = 0; k0 < nt; k0 += kLoadChunk) {
       const int cn = min(kLoadChunk, nt - k0);
       for (int i = t; i < cn; i += kEvalThreads) {
-        srow[i] = tix[k0 + i];
-        ssc[i] = sc[k0 + i];
+        srow[i] = make_int2(tix[k0 + i] * zp, __float_as_int(sc[k0 + i]));
       }
       __syncthreads();
       if (on) {
-        // the next eight rows' values load while these eight are added
-        float nx[8];
-        auto fetch = [&](int i0) {
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const int i = i0 + q * G;
-            nx[q] = i < cn ? Zs[static_cast<size_t>(srow[i]) * zp + j] : 0.0f;
-          }
-        };
-        fetch(g);
-        for (int i0 = g; i0 < cn; i0 += 8 * G) {
-          float v[8];
-#pragma unroll
-          for (int q = 0; q < 8; ++q) v[q] = nx[q];
-          fetch(i0 + 8 * G);
-          // eight terms in two floats (group_seq_dots), then as fixed point
+        const float* zj = Zs + j;
+        // eight terms in two floats (group_seq_dots), then as fixed point
+        auto add = [&](const float (&v)[8], const float (&y)[8]) {
           float hi = 0.0f, lo = 0.0f;
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
-            const int i = i0 + q * G;
-            const float y = i < cn ? ssc[i] : 0.0f;
-            two_float_add(v[q], y, hi, lo, A);
+            two_float_add(v[q], y[q], hi, lo, A);
             nz |= __float_as_uint(v[q]);
           }
           acc += exact_fixed_value(hi, LSB) + exact_fixed_value(lo, LSB);
+        };
+        // the next eight rows' values load while these eight are added
+        float v[8], y[8], nv[8], ny[8];
+        auto fetch = [&](int i0) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const int2 r = srow[i0 + q * G];
+            nv[q] = zj[r.x];
+            ny[q] = __int_as_float(r.y);
+          }
+        };
+        int i0 = g;
+        if (i0 + 7 * G < cn) {
+          fetch(i0);
+          for (; i0 + 15 * G < cn; i0 += 8 * G) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              v[q] = nv[q];
+              y[q] = ny[q];
+            }
+            fetch(i0 + 8 * G);
+            add(v, y);
+          }
+          add(nv, ny);
+          i0 += 8 * G;
+        }
+        if (i0 < cn) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const int2 r = i0 + q * G < cn ? srow[i0 + q * G] : make_int2(0, 0);
+            v[q] = i0 + q * G < cn ? zj[r.x] : 0.0f;
+            y[q] = __int_as_float(r.y);
+          }
+          add(v, y);
         }
       }
       __syncthreads();
@@ -732,33 +750,44 @@ __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
 // Scores of all rows of a row-major matrix (zp floats apart, zp a multiple of
 // 4, 16-byte aligned) for components q0 .. q0 + NQ - 1: out(row, acc) with
 // acc[q] = sum over features in order of z(row, j) * W(j, q0 + q), every product
-// and sum rounded on its own.  A warp takes 32 rows, a lane each; 16 columns at
-// a time come in with cp.async, the next 16 while these are used.  The rows
-// are read in memory order, validation rows too: their scores are needed for
-// the predictions anyway, and no row waits for an index.  Column chunks sit at
-// (chunk ^ (row / 2 & 3)), so the lanes' 16-byte reads hit all banks.
+// and sum rounded on its own.  A warp takes 64 rows, two a lane, so that a weight
+// read from shared memory serves two rows; eight columns at a time come in with
+// cp.async, the next eight while these are used.  The rows are read in memory
+// order, validation rows too: their scores are needed for the predictions anyway,
+// and no row waits for an index.  A row's two column chunks swap places every four
+// rows, so the lanes' 16-byte reads hit all banks.
 // With 128-byte loads of 32 indexed rows into a padded transposing tile, eight
 // in flight, this phase was 42% of an evaluation at 6750 x 200 rows, 5
-// components (3.4 M cycles a slice; here 0.7 M).
+// components (3.4 M cycles a slice).
 // The batches are dealt to the first `warps` warps; tick() follows every batch of
 // a warp.
+// One component alone (the fit's) has little to do per step, so it takes 32 rows
+// and keeps three steps in flight instead.
+constexpr int kScoreRows = 64;
 template <int NQ, class Out, class Tick>
 __device__ __forceinline__ void stream_scores(const float* __restrict__ base, int zp, int p, int nrows, const float* W,
                                               int ldw, int q0, float* tile, int lane, int warp, int warps, Out&& out,
                                               Tick&& tick) {
-  const int nblk = (p + 15) / 16, nb = (nrows + 31) / 32;
+  constexpr int R = NQ == 1 ? 1 : 2, kRows = 32 * R, kStage = kRows * 8, kStages = kTile / kStage;
+  const int nblk = (p + 7) / 8, nb = (nrows + kRows - 1) / kRows;
   const int mine = warp < nb ? (nb - warp + warps - 1) / warps : 0;
   const int steps = mine * nblk;
-  int lb = warp, lk = 0;  // batch and column block of the next load
+  // the next load: its batch, column block and this lane's sources
+  int lb = warp, lk = 0;
+  int src[2 * R];
+  const int lr = lane >> 1, lc = (lane & 1) * 4;
+  float* const dst = tile + lr * 8 + (lc ^ (((lr >> 2) & 1) << 2));  // 16 rows apart, the swap repeats
   auto load = [&](int step) {
     if (step < steps) {
+      if (lk == 0) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = i * 8 + (lane >> 2), c = lane & 3, col = lk * 16 + 4 * c;
-        const int row = min(lb * 32 + r, nrows - 1);
-        if (col < zp)
-          cp_async16(tile + (step & 1) * 512 + r * 16 + ((c ^ ((r >> 1) & 3)) << 2),
-                     base + static_cast<size_t>(row) * zp + col);
+        for (int i = 0; i < 2 * R; ++i)
+          src[i] = min(lb * kRows + i * 16 + lr, nrows - 1) * zp + lc;
+      }
+      float* to = dst + (step & (kStages - 1)) * kStage;
+      if (lk * 8 + lc < zp) {
+#pragma unroll
+        for (int i = 0; i < 2 * R; ++i) cp_async16(to + i * 128, base + (src[i] + lk * 8));
       }
       if (++lk == nblk) {
         lk = 0;
@@ -767,52 +796,72 @@ __device__ __forceinline__ void stream_scores(const float* __restrict__ base, in
     }
     asm volatile("cp.async.commit_group;\n" ::);
   };
-  float acc[NQ];
+  float acc[R][NQ];
 #pragma unroll
-  for (int q = 0; q < NQ; ++q) acc[q] = 0.0f;
-  load(0);
+  for (int q = 0; q < NQ * R; ++q) acc[q / NQ][q % NQ] = 0.0f;
+#pragma unroll
+  for (int i = 0; i < kStages - 1; ++i) load(i);
+  const bool wide = NQ >= 4 && ldw % 4 == 0;  // whole vectors of weights
   int b = warp, k = 0;
   for (int step = 0; step < steps; ++step) {
-    load(step + 1);
-    asm volatile("cp.async.wait_group 1;\n" ::);
+    load(step + kStages - 1);
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kStages - 1));
     __syncwarp();
-    const float* t = tile + (step & 1) * 512 + lane * 16;
+    const float* t = tile + (step & (kStages - 1)) * kStage + lane * 8;
+    const int first = ((lane >> 2) & 1) << 2;
+    const float* w = W + static_cast<size_t>(k * 8) * ldw + q0;
+    float v[R][4];
+    auto column = [&](int e) {
+      float wq[NQ];
+      if (wide) {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int j0 = k * 16 + 4 * c;
-      if (j0 >= p) break;
-      const float4 v4 = *reinterpret_cast<const float4*>(t + ((c ^ ((lane >> 1) & 3)) << 2));
-      const float v[4] = {v4.x, v4.y, v4.z, v4.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        if (j0 + e < p) {
-          const float* w = W + static_cast<size_t>(j0 + e) * ldw + q0;
-          float wq[NQ];
-          if (NQ >= 4 && ldw % 4 == 0) {
-#pragma unroll
-            for (int q = 0; q < NQ; q += 4) {
-              const float4 w4 = *reinterpret_cast<const float4*>(w + q);
-              wq[q] = w4.x;
-              if (q + 1 < NQ) wq[q + 1] = w4.y;
-              if (q + 2 < NQ) wq[q + 2] = w4.z;
-              if (q + 3 < NQ) wq[q + 3] = w4.w;
-            }
-          } else {
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) wq[q] = w[q];
-          }
-          // (packed f32x2 operations are no use here: the assembler contracts
-          // a packed product and sum into one rounding)
-#pragma unroll
-          for (int q = 0; q < NQ; ++q) acc[q] = __fadd_rn(acc[q], __fmul_rn(v[e], wq[q]));
+        for (int q = 0; q < NQ; q += 4) {
+          const float4 w4 = *reinterpret_cast<const float4*>(w + q);
+          wq[q] = w4.x;
+          if (q + 1 < NQ) wq[q + 1] = w4.y;
+          if (q + 2 < NQ) wq[q + 2] = w4.z;
+          if (q + 3 < NQ) wq[q + 3] = w4.w;
         }
+      } else {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) wq[q] = w[q];
+      }
+      w += ldw;
+      // (packed f32x2 operations are no use here: the assembler contracts
+      // a packed product and sum into one rounding)
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+#pragma unroll
+        for (int h = 0; h < R; ++h) acc[h][q] = __fadd_rn(acc[h][q], __fmul_rn(v[h][e], wq[q]));
+      }
+    };
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+#pragma unroll
+      for (int h = 0; h < R; ++h) {
+        const float4 x = *reinterpret_cast<const float4*>(t + h * 256 + (first ^ (4 * c)));
+        v[h][0] = x.x;
+        v[h][1] = x.y;
+        v[h][2] = x.z;
+        v[h][3] = x.w;
+      }
+      const int left = p - k * 8 - 4 * c;
+      if (left >= 4) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) column(e);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 3; ++e)
+          if (e < left) column(e);
       }
     }
     __syncwarp();
     if (++k == nblk) {
-      if (b * 32 + lane < nrows) out(b * 32 + lane, acc);
 #pragma unroll
-      for (int q = 0; q < NQ; ++q) acc[q] = 0.0f;
+      for (int h = 0; h < R; ++h)
+        if (b * kRows + 32 * h + lane < nrows) out(b * kRows + 32 * h + lane, acc[h]);
+#pragma unroll
+      for (int q = 0; q < NQ * R; ++q) acc[q / NQ][q % NQ] = 0.0f;
       k = 0;
       b += warps;
       tick();
@@ -948,6 +997,145 @@ __device__ float warp_score_products(float acc, const float* t, int n, int nc, i
     __syncwarp();
   }
   asm volatile("cp.async.wait_group 0;\n" ::);
+  return acc;
+}
+
+// warp_score_products for up to eight components.  Batches of 32 rows come in by
+// columns (of 36 floats, so that the lanes' columns start in different banks) and
+// a lane reads eight rows of its two columns in four vectors; missing rows are
+// +0.  13 cycles a row, 4.6 of them the sum's chain; with rows of nc floats, a
+// length known at run time only and a load per value it was 40, and the scores
+// waited for it.
+template <int NC>
+__device__ __forceinline__ float warp_score_products_by_column(float acc, const float* t, int n, int ca, int cb,
+                                                               float* buf, int lane) {
+  constexpr int kPitch = 36, kSlot = NC * kPitch, kSlots = 4 * kSlot <= kTile ? 4 : 3;
+  static_assert(kSlots * kSlot <= kTile, "batch ring");
+  const int nb = (n + 31) / 32;
+  int in = 0, out = 0;  // slots
+  auto fetch = [&](int b) {
+    if (b < nb) {
+      const int total = min(32, n - b * 32) * NC;
+      const float* src = t + static_cast<size_t>(b) * (32 * NC);
+      float* dst = buf + in * kSlot;
+#pragma unroll
+      for (int u = 0; u < NC; ++u) {
+        const int i = u * 32 + lane;
+        float* to = dst + (i % NC) * kPitch + i / NC;
+        if (i < total)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(
+                           static_cast<unsigned>(__cvta_generic_to_shared(to))),
+                       "l"(src + i));
+        else
+          *to = 0.0f;
+      }
+      in = in + 1 < kSlots ? in + 1 : 0;
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+  };
+  for (int b = 0; b < kSlots - 1; ++b) fetch(b);
+  for (int b = 0; b < nb; ++b) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kSlots - 2));
+    __syncwarp();
+    fetch(b + kSlots - 1);  // into the slot whose rows were added before the barrier
+    const float4* x = reinterpret_cast<const float4*>(buf + out * kSlot + ca * kPitch);
+    const float4* y = reinterpret_cast<const float4*>(buf + out * kSlot + cb * kPitch);
+    out = out + 1 < kSlots ? out + 1 : 0;
+    float pr[8];
+    auto form = [&](int i) {
+      const float4 x0 = x[i], x1 = x[i + 1], y0 = y[i], y1 = y[i + 1];
+      pr[0] = __fmul_rn(x0.x, y0.x);
+      pr[1] = __fmul_rn(x0.y, y0.y);
+      pr[2] = __fmul_rn(x0.z, y0.z);
+      pr[3] = __fmul_rn(x0.w, y0.w);
+      pr[4] = __fmul_rn(x1.x, y1.x);
+      pr[5] = __fmul_rn(x1.y, y1.y);
+      pr[6] = __fmul_rn(x1.z, y1.z);
+      pr[7] = __fmul_rn(x1.w, y1.w);
+    };
+    form(0);
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+      float cur[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) cur[q] = pr[q];
+      if (i + 2 < 8) form(i + 2);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc = __fadd_rn(acc, cur[q]);
+    }
+    __syncwarp();
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::);
+  return acc;
+}
+
+// Calls go(std::integral_constant<int, nc>) for nc of 1 to 8.
+template <class Go>
+__device__ __forceinline__ void with_components(int nc, Go&& go) {
+  switch (nc) {
+    case 1: go(std::integral_constant<int, 1>{}); break;
+    case 2: go(std::integral_constant<int, 2>{}); break;
+    case 3: go(std::integral_constant<int, 3>{}); break;
+    case 4: go(std::integral_constant<int, 4>{}); break;
+    case 5: go(std::integral_constant<int, 5>{}); break;
+    case 6: go(std::integral_constant<int, 6>{}); break;
+    case 7: go(std::integral_constant<int, 7>{}); break;
+    default: go(std::integral_constant<int, 8>{}); break;
+  }
+}
+
+__device__ __forceinline__ float score_products(float acc, const float* t, int n, int nc, int ca, int cb, float* buf,
+                                                int lane) {
+  if (nc > kMaxNC) return warp_score_products(acc, t, n, nc, ca, cb, buf, lane);
+  with_components(nc, [&](auto c) {
+    acc = warp_score_products_by_column<decltype(c)::value>(acc, t, n, ca, cb, buf, lane);
+  });
+  return acc;
+}
+
+// The sums of positions b..e-1 of a row-major matrix of NC columns whose flag is
+// set, in order, every column a chain of its own: lane q < NC returns column q's.
+// The lanes bring in a row each (two groups ahead of the one being added) and
+// pass them by columns through `buf`; a row left out is +0 (warp_add32).  A
+// warp per class and column, and a shuffle a value, took 50 cycles a row and column.
+template <int NC>
+__device__ __forceinline__ float warp_masked_columns(const float* __restrict__ m, const uint8_t* __restrict__ ok,
+                                                     int b, int e, float* buf, int lane) {
+  constexpr int kPitch = 36;
+  float acc = 0.0f, next[2][NC];
+  // flag and values are loaded side by side: loads behind a test of the flag
+  // would wait for it
+  auto fetch = [&](int i, float (&to)[NC]) {
+    const int k = min(i, e - 1);
+    const bool take = i < e && ok[k] != 0;
+#pragma unroll
+    for (int q = 0; q < NC; ++q) {
+      const float x = m[static_cast<size_t>(k) * NC + q];
+      to[q] = take ? x : 0.0f;
+    }
+  };
+  if (b >= e) return acc;
+  fetch(b + lane, next[0]);
+  fetch(b + 32 + lane, next[1]);
+  const float4* mine = reinterpret_cast<const float4*>(buf + min(lane, NC - 1) * kPitch);
+  for (int g = b; g < e; g += 32) {
+#pragma unroll
+    for (int q = 0; q < NC; ++q) {
+      buf[q * kPitch + lane] = next[0][q];
+      next[0][q] = next[1][q];
+    }
+    __syncwarp();
+    if (g + 64 < e) fetch(g + 64 + lane, next[1]);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float4 v = mine[i];
+      acc = __fadd_rn(acc, v.x);
+      acc = __fadd_rn(acc, v.y);
+      acc = __fadd_rn(acc, v.z);
+      acc = __fadd_rn(acc, v.w);
+    }
+    __syncwarp();
+  }
   return acc;
 }
 
@@ -1141,7 +1329,11 @@ __global__ void __launch_bounds__(kCrossThreads, 2) cross_kernel(PlsEvalArgs a) 
   }
 }
 
-__global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
+// kCtas: CTAs an SM, the bound on registers: two hide each other's latencies
+// (64 registers, some spilled); where there are no more slices than SMs there is
+// only one, with 128.
+template <int kCtas>
+__global__ void __launch_bounds__(kEvalThreads, kCtas) eval_kernel(PlsEvalArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int s = blockIdx.x, r = s / a.F, f = s % a.F;
   const int p = a.p, zp = a.zp, L = a.L, C = a.C0max, NCm = a.requested, ldw = a.ldw;
@@ -1193,28 +1385,51 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
   if (!a.predict_mode)
     for (int v = threadIdx.x; v < nv; v += kEvalThreads) atomicSub(&cnt[lab[vidx[v]]], 1);
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (warp == kEvalWarps - 1) {
     int m = 0;
-    for (int c = 0; c < C; ++c)
-      if (cnt[c] > 0) klist[m++] = c;
-    sh.m = m;
-    sh.nt = te - tb;
-    sh.queue = 0;
-    a.status[s] = 0;
+    for (int c0 = 0; c0 < C; c0 += 32) {
+      const bool in = c0 + lane < C && cnt[c0 + lane] > 0;
+      const unsigned b = __ballot_sync(kFull, in);
+      if (in) klist[m + __popc(b & ((1u << lane) - 1u))] = c0 + lane;
+      m += __popc(b);
+    }
+    if (lane == 0) {
+      sh.m = m;
+      sh.nt = te - tb;
+      sh.queue = 0;
+      a.status[s] = 0;
+    }
   }
   // class-list position of every row, whether that position trains the slice,
   // and every row's position among the training rows
   uint16_t* posof = a.pos + static_cast<size_t>(s) * L;
   uint8_t* posok = a.posok + static_cast<size_t>(s) * L;
-  for (int i = threadIdx.x; i < L; i += kEvalThreads) {
-    const int row = crow[i];
-    posof[row] = static_cast<uint16_t>(i);
-    posok[i] = (fold == nullptr || fold[row] != f) ? 1 : 0;
+  for (int i0 = threadIdx.x; i0 < L; i0 += 4 * kEvalThreads) {
+    int row[4];
+    bool train[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) row[q] = crow[min(i0 + q * kEvalThreads, L - 1)];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) train[q] = fold == nullptr || fold[row[q]] != f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int i = i0 + q * kEvalThreads;
+      if (i >= L) break;
+      posof[row[q]] = static_cast<uint16_t>(i);
+      posok[i] = train[q] ? 1 : 0;
+    }
   }
   uint16_t* tpos = a.tpos + static_cast<size_t>(s) * L;
   if (fold != nullptr)
     for (int i = threadIdx.x; i < nv; i += kEvalThreads) tpos[vidx[i]] = kNoPos;
-  for (int t = threadIdx.x; t < te - tb; t += kEvalThreads) tpos[a.train_idx[tb + t]] = static_cast<uint16_t>(t);
+  for (int t0 = threadIdx.x; t0 < te - tb; t0 += 4 * kEvalThreads) {
+    int row[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) row[q] = a.train_idx[tb + min(t0 + q * kEvalThreads, te - tb - 1)];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (t0 + q * kEvalThreads < te - tb) tpos[row[q]] = static_cast<uint16_t>(t0 + q * kEvalThreads);
+  }
   __syncthreads();
   const int m = sh.m, nt = sh.nt;
   if (m <= 1 || nt == 0) {
@@ -1233,8 +1448,13 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
   float* S = a.s_in_smem ? region : a.s_scr + static_cast<size_t>(s) * p * C;
   for (int k = warp; k < m; k += kEvalWarps) {
     const float* src = a.s_raw + (static_cast<size_t>(s) * C + klist[k]) * p;
-    for (int j = lane; j < p; j += 32) S[j + static_cast<size_t>(k) * p] = src[j];
+    if (a.s_in_smem && p % 4 == 0) {
+      for (int j = 4 * lane; j < p; j += 128) cp_async16(S + j + static_cast<size_t>(k) * p, src + j);
+    } else {
+      for (int j = lane; j < p; j += 32) S[j + static_cast<size_t>(k) * p] = src[j];
+    }
   }
+  asm volatile("cp.async.wait_all;\n" ::);
   __syncthreads();
 
   // --- SIMPLS weights ------------------------------------------------------
@@ -1452,7 +1672,8 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
     stream_all_scores(Zs, zp, p, L, Wsm, ldw, nc, tiles + warp * kTile, lane, warp, kEvalWarps, keep_score, []() {});
   } else {
     constexpr int kScorers = kEvalWarps - 1;
-    const int nb = (L + 31) / 32, rounds = (nb + kScorers - 1) / kScorers;
+    const int brows = nc == 1 ? kScoreRows / 2 : kScoreRows;  // of stream_scores
+    const int nb = (L + brows - 1) / brows, rounds = (nb + kScorers - 1) / kScorers;
     if (warp < kScorers) {
       int done = 0;
       stream_all_scores(Zs, zp, p, L, Wsm, ldw, nc, tiles + warp * kTile, lane, warp, kScorers, keep_score, [&]() {
@@ -1466,11 +1687,11 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
       for (int k = 0; k < rounds; ++k) {
         __syncthreads();  // round k's scores are written
         int cn = 0;
-        for (int i = 0; i < kScorers; ++i) {
-          const int row = (k * kScorers + i) * 32 + lane;
+        for (int i = 0; i < kScorers * brows / 32; ++i) {
+          const int row = k * kScorers * brows + i * 32 + lane;
           cn += __popc(__ballot_sync(kFull, row < L && tpos[min(row, L - 1)] != kNoPos));
         }
-        acc = warp_score_products(acc, Tt + static_cast<size_t>(t0) * nc, cn, nc, prr, pcol, tiles + warp * kTile, lane);
+        acc = score_products(acc, Tt + static_cast<size_t>(t0) * nc, cn, nc, prr, pcol, tiles + warp * kTile, lane);
         t0 += cn;
       }
       if (lane < ncp) {
@@ -1491,6 +1712,29 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
   // class sums (the training rows of each class in row order, i.e. the
   // flagged class-list positions in order): one warp per chain
   const int ncs = m * nc;
+  // largest class first, so that no long chain is begun last
+  int* by_size = reinterpret_cast<int*>(cst);  // the constants come later
+  if (!a.da_mode) {
+    for (int k = threadIdx.x; k < m; k += kEvalThreads) {
+      const int mine = cnt[klist[k]];
+      int rank = 0;
+      for (int j = 0; j < m; ++j) {
+        const int other = cnt[klist[j]];
+        rank += other > mine || (other == mine && j < k);
+      }
+      by_size[rank] = k;
+    }
+    __syncthreads();
+  }
+  auto class_sums = [&](int at) {
+    const int k = by_size[at], code = klist[k];
+    with_components(nc, [&](auto c) {
+      constexpr int NC = decltype(c)::value;
+      const float acc =
+          warp_masked_columns<NC>(Ts, posok, coff[code], coff[code + 1], tiles + warp * kTile, lane);
+      if (lane < NC) cs[k * NC + lane] = acc;
+    });
+  };
   auto class_sum = [&](int it) {
     const int k = it / nc, q = it % nc;
     const int code = klist[k];
@@ -1607,19 +1851,21 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
       ++rr;
     }
     const int col = pr;
-    const float acc = warp_score_products(0.0f, Tt, nt, nc, rr, col, tiles + warp * kTile, lane);
+    const float acc = score_products(0.0f, Tt, nt, nc, rr, col, tiles + warp * kTile, lane);
     if (c0 + lane < ncp) {
       cp[rr * nc + col] = acc;
       cp[col * nc + rr] = acc;
     }
   }
   // the class sums go to whichever warp is free
+  const bool by_class = nc <= kMaxNC;
   for (;;) {
     int it = 0;
     if (lane == 0) it = atomicAdd(&sh.queue, 1);
     it = __shfl_sync(kFull, it, 0);
-    if (it >= ncs) break;
-    class_sum(it);
+    if (it >= (by_class ? m : ncs)) break;
+    if (by_class) class_sums(it);
+    else class_sum(it);
   }
   __syncthreads();
   // fit_lda_from_score_statistics_float, parallel where the reference's loops
@@ -1704,23 +1950,34 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval_kernel(PlsEvalArgs a) {
   // --- predictions ---------------------------------------------------------
   {
     if (a.predict_mode) score_rows();
-    for (int v = threadIdx.x; v < nv; v += kEvalThreads) {
-      const int row = a.predict_mode ? v : vidx[v];
-      const float* tr = rowscores + static_cast<size_t>(row) * nc;
-      float sr[kMaxComp];
-      for (int q = 0; q < nc; ++q) sr[q] = tr[q];
-      int best = 0;
-      float bs = -INFINITY;
-      for (int k = 0; k < m; ++k) {
-        float sc = cst[k];
-        for (int q = 0; q < nc; ++q) sc = __fadd_rn(sc, __fmul_rn(sr[q], lin[k * nc + q]));
-        if (sc > bs) {
-          bs = sc;
-          best = k;
+    // NC > 0: the components, in registers (an array of a length known at run
+    // time lies in local memory: 116k cycles for 750 rows and 98 classes); 0: nc
+    auto predict = [&](auto c) {
+      constexpr int NC = decltype(c)::value;
+      const int nq = NC > 0 ? NC : nc;
+      for (int v = threadIdx.x; v < nv; v += kEvalThreads) {
+        const int row = a.predict_mode ? v : vidx[v];
+        const float* tr = rowscores + static_cast<size_t>(row) * nq;
+        float sr[NC > 0 ? NC : kMaxComp];
+#pragma unroll
+        for (int q = 0; q < nq; ++q) sr[q] = tr[q];
+        int best = 0;
+        float bs = -INFINITY;
+#pragma unroll 4
+        for (int k = 0; k < m; ++k) {
+          float sc = cst[k];
+#pragma unroll
+          for (int q = 0; q < nq; ++q) sc = __fadd_rn(sc, __fmul_rn(sr[q], lin[k * nq + q]));
+          if (sc > bs) {
+            bs = sc;
+            best = k;
+          }
         }
+        pred[row] = static_cast<uint16_t>(klist[best]);
       }
-      pred[row] = static_cast<uint16_t>(klist[best]);
-    }
+    };
+    if (nc <= kMaxNC) with_components(nc, predict);
+    else predict(std::integral_constant<int, 0>{});
   }
 }
 
@@ -1825,9 +2082,10 @@ int pls_evaluate(const PlsEvalArgs& a, cudaStream_t st) {
   PlsEvalArgs b = a;
   b.ldw = bytes(padded) <= (bytes(a.max_components) <= two_ctas ? two_ctas : most) ? padded : a.max_components;
   const size_t smem = bytes(b.ldw);
+  auto* const eval = S <= 152 ? eval_kernel<1> : eval_kernel<2>;
   if (smem > 48 * 1024) {
     const cudaError_t e =
-        cudaFuncSetAttribute(eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        cudaFuncSetAttribute(eval, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
   }
   const size_t stream_smem = cross_stream_smem(a.C0max);
@@ -1842,7 +2100,7 @@ int pls_evaluate(const PlsEvalArgs& a, cudaStream_t st) {
     const int items = a.C0max * ((a.p + 31) / 32), per = kCrossThreads / 32;
     cross_kernel<<<dim3(std::min((items + per - 1) / per, 1024), std::min(S, 65535)), kCrossThreads, 0, st>>>(b);
   }
-  eval_kernel<<<S, kEvalThreads, smem, st>>>(b);
+  eval<<<S, kEvalThreads, smem, st>>>(b);
   count_launch(2);
   return static_cast<int>(cudaGetLastError());
 }
