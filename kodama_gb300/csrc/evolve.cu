@@ -2348,7 +2348,7 @@ template <bool kRows>
 __global__ void __launch_bounds__(kThreads, 1) evolve_pls_kernel(const __grid_constant__ EvolvePlsParams Q) {
   const Smem s = carve_smem<kRows>(Q.base);
   clear_counters(s);
-  for (int prob = blockIdx.x; prob < Q.base.problems; prob += gridDim.x) pls_step(Q, s, prob);
+  pls_step(Q, s, Q.first + blockIdx.x);
 }
 
 }  // namespace

@@ -93,6 +93,7 @@ struct EvolvePlsParams {
   double logn;             // log(L)
   int coarsening;          // auto_class_coarsening
   int pol_coarsen, pol_frag;
+  int first;               // first problem of the launch, one CTA each
   int phase;               // 0: initial labels; 1: accept cycle-1 / propose cycle
   int cycle;
 };

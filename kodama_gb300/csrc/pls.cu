@@ -1169,7 +1169,7 @@ __global__ void __launch_bounds__(kStreamThreads) cross_stream_kernel(PlsEvalArg
   float* acc = ring + kStreamSlots * kStreamRows * 32;        // [code][32]
   int* cnt = reinterpret_cast<int*>(acc + static_cast<size_t>(C) * 32);
   const int ntiles = (L + kStreamRows - 1) / kStreamRows;
-  for (int s = blockIdx.y; s < a.problems * a.F; s += gridDim.y) {
+  for (int s = a.first * a.F + blockIdx.y; s < (a.first + a.problems) * a.F; s += gridDim.y) {
     const int r = s / a.F, f = s % a.F;
     const int* coff = a.class_off + static_cast<size_t>(r) * (C + 1);
     const uint16_t* lab = a.labels + static_cast<size_t>(r) * L;
@@ -1273,7 +1273,7 @@ __global__ void __launch_bounds__(kStreamThreads) cross_stream_kernel(PlsEvalArg
 constexpr int kCrossThreads = 256;
 __global__ void __launch_bounds__(kCrossThreads, 2) cross_kernel(PlsEvalArgs a) {
   const int lane = threadIdx.x & 31, p = a.p, C = a.C0max, JB = (p + 31) / 32;
-  for (int s = blockIdx.y; s < a.problems * a.F; s += gridDim.y) {
+  for (int s = a.first * a.F + blockIdx.y; s < (a.first + a.problems) * a.F; s += gridDim.y) {
     const int r = s / a.F, f = s % a.F;
     const int* coff = a.class_off + static_cast<size_t>(r) * (C + 1);
     const uint16_t* crow = a.class_rows + static_cast<size_t>(r) * a.L;
@@ -1335,7 +1335,7 @@ __global__ void __launch_bounds__(kCrossThreads, 2) cross_kernel(PlsEvalArgs a) 
 template <int kCtas>
 __global__ void __launch_bounds__(kEvalThreads, kCtas) eval_kernel(PlsEvalArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int s = blockIdx.x, r = s / a.F, f = s % a.F;
+  const int s = a.first * a.F + blockIdx.x, r = s / a.F, f = s % a.F;
   const int p = a.p, zp = a.zp, L = a.L, C = a.C0max, NCm = a.requested, ldw = a.ldw;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   EvalShared& sh = *reinterpret_cast<EvalShared*>(smem);
@@ -2082,7 +2082,7 @@ int pls_evaluate(const PlsEvalArgs& a, cudaStream_t st) {
   PlsEvalArgs b = a;
   b.ldw = bytes(padded) <= (bytes(a.max_components) <= two_ctas ? two_ctas : most) ? padded : a.max_components;
   const size_t smem = bytes(b.ldw);
-  auto* const eval = S <= 152 ? eval_kernel<1> : eval_kernel<2>;
+  auto* const eval = std::max(S, a.live) <= 152 ? eval_kernel<1> : eval_kernel<2>;
   if (smem > 48 * 1024) {
     const cudaError_t e =
         cudaFuncSetAttribute(eval, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));

@@ -41,7 +41,9 @@ int pls_prepare(const PlsPrepArgs& a, cudaStream_t st);
 int pls_build_gram(const PlsPrepArgs& a, const uint8_t* want, cudaStream_t st);
 
 struct PlsEvalArgs {
-  int problems;          // R
+  int problems;          // R, or those of one launch
+  int first;             // of them the first (the arrays hold all problems)
+  int live;              // slices of all launches that run side by side (0: this one's)
   int F;                 // slices per problem
   int L;                 // rows per problem
   int p;                 // columns
