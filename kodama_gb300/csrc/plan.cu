@@ -288,8 +288,8 @@ struct Sampler {
       const uint64_t lo = u * range;
       const unsigned bad = __ballot_sync(0xffffffffu, in && lo < range && lo < (0ull - range) % range);
       const int usable = bad != 0u ? __ffs(bad) - 1 : batch;
-      uint64_t d1, d2;
-      divmod_u64(__umul64hi(u, range), b1, d1, d2);
+      // floor(u left b1 / 2^64) by b1: the quotient is floor(u left / 2^64)
+      uint64_t d1 = __umul64hi(u, left), d2 = __umul64hi(u, range) - d1 * b1;
       // positions of steps past the usable ones take nothing
       const unsigned p1 = lane < usable ? static_cast<unsigned>(d1) : 0xffffffffu;
       const unsigned p2 = lane < usable ? static_cast<unsigned>(d2) : 0xffffffffu;
