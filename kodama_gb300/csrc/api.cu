@@ -1096,9 +1096,8 @@ struct MatrixTail {
 
 // build_graph (may be empty): queues the kNN graph into d_gidx / d_gdist.  It
 // needs only x, so outside a captured batch it runs on the low-priority
-// background stream beside the landmark planning and the landmark k-means
-// (from the start of the call, beside the atlas k-means too, when it is the
-// longer branch), and is joined before anything reads the graph; in a
+// background stream beside the landmark planning (when it is long) or the
+// landmark k-means, and is joined before anything reads the graph; in a
 // captured batch it runs right after the atlas.  Queues
 // the whole call; the results are read by matrix_finalize once the device
 // work is done (no host wait on the plain path, so a batch can capture it).
