@@ -1005,76 +1005,99 @@ __global__ void __launch_bounds__(kSumThreads) sums_kernel(KMeansBatch B) {
 }
 
 // Update step, sort and sums in one (one CTA per cluster and problem, d up
-// to 4 x kScanThreads): the CTA scans the problem's assignments in chunks of
-// kScanChunk rows -- a ballot per 32 rows, prefix over the warps -- so the
-// cluster's members of a chunk land in shared memory in ascending row order;
-// thread j then adds columns j, j + 256, ... down them, up to 32 rows' loads
-// in flight.  The size goes to offsets[c] (finalize_kernel reads sizes).
-// Without the member lists and the one-CTA sort this replaces sort_kernel and
-// sums_kernel when each problem's assignments are read by its k CTAs anyway.
-constexpr int kScanThreads = 256;
-constexpr int kScanChunk = 4 * kScanThreads;
-constexpr int kScanCols = 4;  // columns per thread
-constexpr int kScanBatch = 16;  // member rows whose loads are issued together
+// to kScanCols x kScanThreads): the CTA scans the problem's assignments, a run
+// of rows per warp, first counting and then listing the cluster's members in
+// ascending row order in shared memory (kScanCap at a time); thread j then adds
+// columns j, j + 512 down them, 32 to 64 rows' loads in flight.  The size goes to
+// offsets[c] (finalize_kernel reads sizes).  Without the member lists and the
+// one-CTA sort this replaces sort_kernel and sums_kernel when each problem's
+// assignments are read by its k CTAs anyway.
+// What bounds it: the scan's and the rows' loads.  Scanning, listing and adding
+// 1024 rows at a time waited for memory in every chunk: 20000 x 50 rows and 50
+// clusters 80 -> 36 us, 100000 x 50 and 300 143 -> 81, 4999 x 37 and 100 19 -> 12
+// (1000 x 10, one chunk before: 4.6 and 5.0).
+constexpr int kScanThreads = 512;
+constexpr int kScanWarps = kScanThreads / 32;
+constexpr int kScanCols = 2;     // columns per thread
+constexpr int kScanCap = 8192;   // members listed at a time
 
 __global__ void __launch_bounds__(kScanThreads) scan_sums_kernel(KMeansBatch B) {
-  __shared__ int mem[kScanChunk];
-  __shared__ int wcount[kScanThreads / 32];
+  __shared__ int mem[kScanCap];
+  __shared__ int wcount[kScanWarps];
   const int c = blockIdx.x, p = blockIdx.y;
   if (!B.active[p]) return;
   const int n = B.n, d = B.d, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int* as = B.assign + static_cast<size_t>(p) * n;
   const int* rows = B.rows != nullptr ? B.rows + static_cast<size_t>(p) * n : nullptr;
+  const int per = ((n + kScanWarps - 1) / kScanWarps + 31) / 32 * 32;
+  const int beg = min(n, warp * per), end = min(n, beg + per);
+  // use(row, member, members of the 32 rows), eight steps' loads in flight
+  auto walk = [&](auto&& use) {
+    for (int b0 = beg; b0 < end; b0 += 8 * 32) {
+      int a[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int r = b0 + 32 * u + lane;
+        a[u] = r < end ? as[r] : -1;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const bool in = a[u] == c;
+        use(b0 + 32 * u + lane, in, __ballot_sync(kFull, in));
+      }
+    }
+  };
+  int mine = 0;
+  walk([&](int, bool, unsigned m) { mine += __popc(m); });
+  if (lane == 0) wcount[warp] = mine;
+  __syncthreads();
+  int off = 0, count = 0;
+#pragma unroll
+  for (int q = 0; q < kScanWarps; ++q) {
+    off += q < warp ? wcount[q] : 0;
+    count += wcount[q];
+  }
   float s[kScanCols];
 #pragma unroll
   for (int q = 0; q < kScanCols; ++q) s[q] = 0.0f;
-  int count = 0;
-  for (int base = 0; base < n; base += kScanChunk) {
-    // warp w scans rows base + 128 w .. + 127, 32 at a time
-    unsigned bal[4];
-    int cw = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = base + warp * 128 + i * 32 + lane;
-      bal[i] = __ballot_sync(kFull, r < n && as[r] == c);
-      cw += __popc(bal[i]);
-    }
-    if (lane == 0) wcount[warp] = cw;
+  for (int first = 0; first < count; first += kScanCap) {
+    int pos = off - first;
+    walk([&](int r, bool in, unsigned m) {
+      const int at = pos + __popc(m & ((1u << lane) - 1u));
+      if (in && at >= 0 && at < kScanCap) mem[at] = rows != nullptr ? rows[r] : r;
+      pos += __popc(m);
+    });
     __syncthreads();
-    int off = 0, total = 0;
+    const int total = min(kScanCap, count - first);
 #pragma unroll
-    for (int q = 0; q < kScanThreads / 32; ++q) {
-      const int v = wcount[q];
-      off += q < warp ? v : 0;
-      total += v;
-    }
+    for (int q = 0; q < kScanCols; ++q) {
+      const int j = tid + q * kScanThreads;
+      if (j >= d) continue;
+      const float* xj = B.x + j;
+      float va[32], vb[32];
+      auto fetch = [&](float (&v)[32], int m0) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if ((bal[i] >> lane) & 1u) {
-        const int r = base + warp * 128 + i * 32 + lane;
-        mem[off + __popc(bal[i] & ((1u << lane) - 1u))] = rows != nullptr ? rows[r] : r;
-      }
-      off += __popc(bal[i]);
-    }
-    __syncthreads();
-    for (int m0 = 0; m0 < total; m0 += kScanBatch) {
-      const int mb = min(kScanBatch, total - m0);
+        for (int u = 0; u < 32; ++u) v[u] = xj[static_cast<size_t>(mem[min(m0 + u, total - 1)]) * d];
+      };
+      auto add = [&](const float (&v)[32], int left) {
+        if (left >= 32) {
 #pragma unroll
-      for (int q = 0; q < kScanCols; ++q) {
-        const int j = tid + q * kScanThreads;
-        if (q * kScanThreads < d) {
-          float v[kScanBatch];
+          for (int u = 0; u < 32; ++u) s[q] = fadd(s[q], v[u]);
+        } else {
 #pragma unroll
-          for (int u = 0; u < kScanBatch; ++u)
-            v[u] = (u < mb && j < d) ? B.x[static_cast<size_t>(mem[m0 + u]) * d + j] : 0.0f;
-#pragma unroll
-          for (int u = 0; u < kScanBatch; ++u)
-            if (u < mb) s[q] = fadd(s[q], v[u]);
+          for (int u = 0; u < 32; ++u)
+            if (u < left) s[q] = fadd(s[q], v[u]);
         }
+      };
+      fetch(va, 0);
+      for (int m = 0; m < total; m += 64) {
+        if (m + 32 < total) fetch(vb, m + 32);
+        add(va, total - m);
+        if (m + 64 < total) fetch(va, m + 64);
+        if (m + 32 < total) add(vb, total - m - 32);
       }
     }
-    count += total;
-    __syncthreads();  // mem and wcount are rewritten by the next chunk
+    __syncthreads();  // mem is rewritten by the next part
   }
   const float inv = count != 0 ? __fdiv_rn(1.0f, static_cast<float>(count)) : 0.0f;
   float* cent = B.cent + (static_cast<size_t>(p) * B.k + c) * d;
