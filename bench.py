@@ -58,7 +58,7 @@ BATCH_KW = dict(runs=50, cycles=50, knn_k=10, components=5, graph_neighbors=30, 
 # DRAM bytes (read + write) of one evolution-kernel launch, scaled from the
 # ncu capture of the full bench-size launch (dram__bytes_read.sum +
 # dram__bytes_write.sum; None until captured).
-EVOLVE_TRAFFIC_BYTES = 598524416
+EVOLVE_TRAFFIC_BYTES = 388666368
 
 
 CONFIG_DESC = ("KODAMA.matrix kNN N=20000 d=50 (12-cluster Gaussian mixture), M=100 runs, "
