@@ -291,7 +291,10 @@ __device__ __forceinline__ void shuffle_step_sync() { asm volatile("bar.sync 2, 
 // t + 157 and the new word t; word 311 takes the new word 0, which thread 156
 // forms for its neighbour.  Regeneration r goes to f.mt_alt for even r, f.rng.mt
 // for odd r, where the other warps read its words, still to be tempered, until
-// the next step; the last block's outputs are written once at the end.
+// the next step; the last block's outputs and the state go to f.rng once at the
+// end, after the last step's barrier: until then the other warps read the old
+// position and, for an odd number of regenerations, the block before in f.rng.mt.
+// The caller's block barrier publishes them.
 // Tempering every block here and writing it to global memory, the state's words
 // reloaded, took 860 cycles a regeneration; this takes 270, as a function of its
 // own with its own registers (640 within the kernel's).
@@ -337,7 +340,9 @@ __device__ __noinline__ void produce_outputs_group(int count, uint64_t* save) {
     nxt = tmp;
     if (done < count) shuffle_step_sync();
   }
-  producer_sync();  // everyone has read g.pos
+  // the other warps' last reads of the state and its position lie before this
+  // barrier; of the last regeneration they read what is in `cur`
+  shuffle_step_sync();
   if (live && done > lead) {
     if (cur != g.mt) {
       g.mt[t] = a;
@@ -347,7 +352,6 @@ __device__ __noinline__ void produce_outputs_group(int count, uint64_t* save) {
     g.out[h] = mt64_temper(b);
   }
   if (t == 0) g.pos = pos;
-  shuffle_step_sync();
 }
 
 // Swap targets J[i] of every step of the shuffle of G groups.  The producer
