@@ -772,22 +772,25 @@ __device__ __forceinline__ void stream_scores(const float* __restrict__ base, in
   const int nblk = (p + 7) / 8, nb = (nrows + kRows - 1) / kRows;
   const int mine = warp < nb ? (nb - warp + warps - 1) / warps : 0;
   const int steps = mine * nblk;
-  // the next load: its batch, column block and this lane's sources
+  // the next load: its batch, column block, the batch's first row and this lane's
+  // offsets from there (the rows to predict have no limit that keeps row * zp below
+  // 2^31; a batch has)
   int lb = warp, lk = 0;
+  const float* from = base;
   int src[2 * R];
   const int lr = lane >> 1, lc = (lane & 1) * 4;
   float* const dst = tile + lr * 8 + (lc ^ (((lr >> 2) & 1) << 2));  // 16 rows apart, the swap repeats
   auto load = [&](int step) {
     if (step < steps) {
       if (lk == 0) {
+        from = base + static_cast<size_t>(lb * kRows) * zp;
 #pragma unroll
-        for (int i = 0; i < 2 * R; ++i)
-          src[i] = min(lb * kRows + i * 16 + lr, nrows - 1) * zp + lc;
+        for (int i = 0; i < 2 * R; ++i) src[i] = min(i * 16 + lr, nrows - 1 - lb * kRows) * zp + lc;
       }
       float* to = dst + (step & (kStages - 1)) * kStage;
       if (lk * 8 + lc < zp) {
 #pragma unroll
-        for (int i = 0; i < 2 * R; ++i) cp_async16(to + i * 128, base + (src[i] + lk * 8));
+        for (int i = 0; i < 2 * R; ++i) cp_async16(to + i * 128, from + (src[i] + lk * 8));
       }
       if (++lk == nblk) {
         lk = 0;
