@@ -2407,8 +2407,9 @@ void fold_search(Ctx& ctx, const float* xs, int n, int d, int K, int metric, con
                  const int* d_folds, int* d_idx, float* d_dist) {
   const int segments = 4;
   const bool inner = metric != KGB_METRIC_EUCLIDEAN;
-  if (kgb::knn_tc_supported(n, d, K)) {
-    const kgb::KnnFoldPlan fp = kgb::knn_fold_plan(folds);
+  kgb::KnnFoldPlan fp;
+  if (kgb::knn_tc_supported(n, d, K)) fp = kgb::knn_fold_plan(folds, d, K);
+  if (fp.tiles > 0) {
     const int* d_perm = ctx.upload(fp.perm.data(), fp.perm.size());
     const int* d_off = ctx.upload(fp.off.data(), fp.off.size());
     const int* d_skip = ctx.upload(fp.skip.data(), fp.skip.size());

@@ -55,12 +55,13 @@ int knn_tc_fallback_count(const void* scratch, int n, int d, int K, int segments
 // to whole candidate tiles, so that a query tile leaves out its own fold's
 // tiles.  perm: row of every position (-1 = padding); per query tile the first
 // (query tile, candidate tile) pair and the (first, count) of the tiles left
-// out.
+// out.  No tiles: the padding of many small folds costs more than the tensor
+// search saves, the brute force (knn_fold_search) is the way.
 struct KnnFoldPlan {
   int tiles = 0, pairs = 0;
   std::vector<int> perm, off, skip;
 };
-KnnFoldPlan knn_fold_plan(const std::vector<int>& folds);
+KnnFoldPlan knn_fold_plan(const std::vector<int>& folds, int d, int K);
 // knn_fold_search through the tensor-core candidate search; d_perm, d_off and
 // d_skip are the plan's arrays on the device.
 int knn_tc_fold_search(const float* x, int n, int d, int K, bool inner, const int* d_folds, const KnnFoldPlan& fp,
