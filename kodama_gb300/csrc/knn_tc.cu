@@ -169,7 +169,8 @@ struct SearchArgs {
   // (nullptr: q * ntiles), skip: the tile range a query tile leaves out
   const int* off;
   const int2* skip;
-  int pairs, per, segs;
+  long long pairs;         // past 2^31 from 8.4 million rows on; a CTA's own are counted
+  int per, segs;           // from its first, and so are the query tiles' starts there
   float2* list;            // [query position][segment][group][cap] (a, position)
   int* cnt;                // [query position][segment][group], -1 = overflow
   float* tau;
@@ -278,7 +279,12 @@ __global__ void __launch_bounds__(kThreads, 1) candidates_kernel(SearchArgs A) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ SearchShared sh;
   const int warp = tc5::warp_index(), lane = threadIdx.x & 31;
-  const int first_pair = blockIdx.x * A.per, last_pair = min(A.pairs, first_pair + A.per);
+  const long long first_pair = static_cast<long long>(blockIdx.x) * A.per;
+  const int span = static_cast<int>(min(A.pairs - first_pair, static_cast<long long>(A.per)));
+  // first pair of a query tile, counted from the CTA's first
+  auto start_of = [&](int qt) {
+    return static_cast<int>((A.off != nullptr ? A.off[qt] : static_cast<long long>(qt) * A.ntiles) - first_pair);
+  };
   const uint32_t qbytes = static_cast<uint32_t>(A.chunks) * kQRows * 16;       // one of hi / lo
   const uint32_t sbytes = static_cast<uint32_t>(A.kg) * kBlockRows * 16;       // one of hi / lo of a stage
   float* const norms = reinterpret_cast<float*>(smem);  // [slot][256]
@@ -309,7 +315,7 @@ __global__ void __launch_bounds__(kThreads, 1) candidates_kernel(SearchArgs A) {
   // first query tile of the range
   int q = 0;
   if (A.off == nullptr) {
-    q = first_pair / A.ntiles;
+    q = static_cast<int>(first_pair / A.ntiles);
   } else {
     int lo = 0, hi = A.qtiles - 1;  // last q with off[q] <= first_pair
     while (lo < hi) {
@@ -327,11 +333,11 @@ __global__ void __launch_bounds__(kThreads, 1) candidates_kernel(SearchArgs A) {
       uint32_t phase = 0;
       bool ok = true;
       int issued = 0, it = 0;
-      for (int pair = first_pair, qt = q; ok && pair < last_pair; ++qt) {
-        const int o = A.off != nullptr ? A.off[qt] : qt * A.ntiles;
+      for (int pair = 0, qt = q; ok && pair < span; ++qt) {
+        const int o = start_of(qt);
         const int2 sk = A.skip != nullptr ? A.skip[qt] : make_int2(0, 0);
         const TileOrder ord(A.ntiles, qt * kQRows / kBlockRows, sk.x, sk.y);
-        const int end = min(last_pair, o + ord.count);
+        const int end = min(span, o + ord.count);
         if (pair >= end) continue;
         // the query tile: half of a block, 2 KB of every chunk
         if (qn > 0) ok = tc5::mbar_wait(tc5::smem_u32(&sh.qempty), (qn - 1) & 1, stop);
@@ -393,10 +399,10 @@ __global__ void __launch_bounds__(kThreads, 1) candidates_kernel(SearchArgs A) {
     int stage = 0, qn = 0, it = 0;
     uint32_t phase = 0;
     bool ok = true;
-    for (int pair = first_pair, qt = q; ok && pair < last_pair; ++qt) {
-      const int o = A.off != nullptr ? A.off[qt] : qt * A.ntiles;
+    for (int pair = 0, qt = q; ok && pair < span; ++qt) {
+      const int o = start_of(qt);
       const int2 sk = A.skip != nullptr ? A.skip[qt] : make_int2(0, 0);
-      const int end = min(last_pair, o + A.ntiles - sk.y);
+      const int end = min(span, o + A.ntiles - sk.y);
       if (pair >= end) continue;
       ok = __all_sync(kFull, tc5::mbar_wait(tc5::smem_u32(&sh.qfull), qn & 1, stop));
       ++qn;
@@ -450,13 +456,13 @@ __global__ void __launch_bounds__(kThreads, 1) candidates_kernel(SearchArgs A) {
     const int trig0 = A.Kq + max(32, A.Kq / 2), room = A.cap - 32;
     int it = 0;
     bool ok = true;
-    for (int pair = first_pair, qt = q; ok && pair < last_pair; ++qt) {
-      const int o = A.off != nullptr ? A.off[qt] : qt * A.ntiles;
+    for (int pair = 0, qt = q; ok && pair < span; ++qt) {
+      const int o = start_of(qt);
       const int2 sk = A.skip != nullptr ? A.skip[qt] : make_int2(0, 0);
       const TileOrder ord(A.ntiles, qt * kQRows / kBlockRows, sk.x, sk.y);
-      const int end = min(last_pair, o + ord.count);
+      const int end = min(span, o + ord.count);
       if (pair >= end) continue;
-      const int seg = blockIdx.x - o / A.per;
+      const int seg = blockIdx.x - static_cast<int>((first_pair + o) / A.per);
       const size_t qpos = static_cast<size_t>(qt) * kQRows + r;
       const size_t slot = (qpos * A.segs + seg) * 2 + g;
       float2* const list = A.list + slot * A.cap;
@@ -617,9 +623,10 @@ __global__ void __launch_bounds__(128) rerank_kernel(RerankArgs R) {
   int m = 0;
   if (!bad) {
     const int qt = pos / kQRows;
-    const int o = A.off != nullptr ? A.off[qt] : qt * A.ntiles;
+    const long long o = A.off != nullptr ? A.off[qt] : static_cast<long long>(qt) * A.ntiles;
     const int count = A.ntiles - (A.skip != nullptr ? A.skip[qt].y : 0);
-    const int nl = count > 0 ? 2 * ((o + count - 1) / A.per - o / A.per + 1) : 0;  // this row's lists
+    // this row's lists
+    const int nl = count > 0 ? 2 * (static_cast<int>((o + count - 1) / A.per - o / A.per) + 1) : 0;
     const size_t slot = static_cast<size_t>(pos) * A.segs * 2;
     float tau = INFINITY;
     int low = 0;
@@ -792,11 +799,14 @@ namespace {
 
 // From one candidate tile on: whole calls at 256 rows x 10, K = 10 take 144 us
 // here and 150 us by the brute force, at K = 100 159 and 491 us, at 1000 rows x
-// 50, K = 100 196 and 1922 us.  Up to 223 neighbours: lists of 512 entries.
+// 50, K = 100 196 and 1922 us.  Up to 223 neighbours: lists of 512 entries.  Up to
+// 2^26 rows: their lists, 4 KB a row at least, take all of the memory.
 constexpr int kMinRows = 256;
+constexpr int kMaxRows = 1 << 26;
 
 struct TcLayout {
-  int dp, chunks, kg, stages, npos, ntiles, qtiles, cap, Kq, pairs, per, segs, d4, ctas;
+  int dp, chunks, kg, stages, npos, ntiles, qtiles, cap, Kq, per, segs, d4, ctas;
+  long long pairs;
   size_t smem;
   size_t o_xh, o_xl, o_cn, o_qn, o_status, o_xp, o_cnt, o_tau, o_list, o_fb, o_brute, total;
 };
@@ -814,10 +824,10 @@ TcLayout tc_layout(int n, int d, int K, int segments, int sms, const KnnFoldPlan
   L.cap = list_entries(L.Kq);
   L.ntiles = fp != nullptr ? fp->tiles : (n + kBlockRows - 1) / kBlockRows;
   L.qtiles = fp != nullptr ? 2 * fp->tiles : (n + kQRows - 1) / kQRows;
-  L.pairs = fp != nullptr ? fp->pairs : L.ntiles * L.qtiles;
+  L.pairs = fp != nullptr ? fp->pairs : static_cast<long long>(L.ntiles) * L.qtiles;
   L.npos = L.ntiles * kBlockRows;
-  L.ctas = L.pairs < sms ? (L.pairs > 0 ? L.pairs : 1) : sms;
-  L.per = (L.pairs + L.ctas - 1) / L.ctas;
+  L.ctas = L.pairs < sms ? (L.pairs > 0 ? static_cast<int>(L.pairs) : 1) : sms;
+  L.per = static_cast<int>((L.pairs + L.ctas - 1) / L.ctas);
   if (L.per < 1) L.per = 1;
   L.segs = (L.ntiles - 1) / L.per + 2;
   // stages of 32 coordinates (32 KB), four where the query tile (up to 128 KB)
@@ -924,14 +934,14 @@ int tc_search(const TcLayout& L, const float* x, int n, int d, int K, bool inner
 }  // namespace
 
 bool knn_tc_supported(int n, int d, int K) {
-  return d >= 1 && d <= kMaxDp && K >= 1 && K + 1 <= 224 && n >= kMinRows && n > K;
+  return d >= 1 && d <= kMaxDp && K >= 1 && K + 1 <= 224 && n >= kMinRows && n <= kMaxRows && n > K;
 }
 
 bool knn_tc_explicit(int n, int d, int K) {
   const int heaps = 2 * (K <= 40 ? 8 : 4);
   int kp = (2 * ((K + heaps - 1) / heaps) + 15) / 8 * 8;
   kp = kp < 16 ? 16 : kp;
-  return d >= 1 && d <= kMaxDp && K >= 1 && K <= 96 && n > 2 * kp + 64;
+  return d >= 1 && d <= kMaxDp && K >= 1 && K <= 96 && n > 2 * kp + 64 && n <= kMaxRows;
 }
 
 size_t knn_tc_scratch(int n, int d, int K, int segments, int sms, const KnnFoldPlan* fp) {
