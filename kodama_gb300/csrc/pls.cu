@@ -900,6 +900,11 @@ __device__ __forceinline__ void stream_all_scores(const float* __restrict__ base
   }
 }
 
+// A barrier of the whole evaluation block that the scoring warps and the one that
+// follows them meet at from different places of the code, which __syncthreads does
+// not allow.
+__device__ __forceinline__ void round_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kEvalThreads) : "memory"); }
+
 // acc plus the lanes' 32 values in lane order, the same in every lane.  The
 // shuffles are issued together, so the chain runs at the speed of its adds; with
 // a condition around each add it ran at shuffle latency, 40 cycles a value.
@@ -1681,14 +1686,14 @@ __global__ void __launch_bounds__(kEvalThreads, kCtas) eval_kernel(PlsEvalArgs a
       int done = 0;
       stream_all_scores(Zs, zp, p, L, Wsm, ldw, nc, tiles + warp * kTile, lane, warp, kScorers, keep_score, [&]() {
         ++done;
-        __syncthreads();
+        round_sync();
       });
-      for (; done < rounds; ++done) __syncthreads();
+      for (; done < rounds; ++done) round_sync();
     } else {
       float acc = 0.0f;
       int t0 = 0;
       for (int k = 0; k < rounds; ++k) {
-        __syncthreads();  // round k's scores are written
+        round_sync();  // round k's scores are written
         int cn = 0;
         for (int i = 0; i < kScorers * brows / 32; ++i) {
           const int row = k * kScorers * brows + i * 32 + lane;
