@@ -323,6 +323,10 @@ __device__ __forceinline__ void group_seq_dots(int dots, int n, int lane, int wa
 
 constexpr int kLoadChunk = 1024;  // rows of a block_loading chunk
 
+// Fixed points from which a product's remainder lost to underflow (at most 2^-150)
+// counts less than a quarter of a unit, within the units round_check is given.
+constexpr int kMinLsb = -148;
+
 // v as a multiple of 2^LSB (truncated below it)
 __device__ __forceinline__ long long exact_fixed_value(float v, int LSB) {
   const unsigned u = __float_as_uint(v), b = (u >> 23) & 0xffu;
@@ -370,7 +374,7 @@ __device__ float block_norm2(const float* __restrict__ sc, int n, void* scratch,
     A = __fadd_ru(A, ared[q]);
   }
   float out = 0.0f;
-  if (!(A > 0.0f && A < 1e37f && round_check(acc, LSB, __fmul_ru(A, 1.0001f), n + 2880, out)))
+  if (!(LSB >= kMinLsb && A > 0.0f && A < 1e37f && round_check(acc, LSB, __fmul_ru(A, 1.0001f), n + 2880, out)))
     out = warp_seq_dot(n, [&](int k, float& x, float& y) {
       x = sc[k];
       y = sc[k];
@@ -494,9 +498,11 @@ __device__ void block_loading(const float* __restrict__ Zs, int zp, int p, const
       }
       // a column of zeros; else the check, which counts the roundings of the
       // eight-term sums (below 180 u^2 A) as 16 x 180 terms more; A is not
-      // finite where a value is not, and zero where products were lost
+      // finite where a value is not, and zero where products were lost; a column
+      // so small that remainders were lost (kMinLsb) takes the chain
       if (fl == 0) ok = true;
-      else if (A > 0.0f && A < 1e37f) ok = round_check(acc, LSB, __fmul_ru(A, 1.0001f), nt + 2880, out);
+      else if (LSB >= kMinLsb && A > 0.0f && A < 1e37f)
+        ok = round_check(acc, LSB, __fmul_ru(A, 1.0001f), nt + 2880, out);
     }
     if (t == 0) fcount = 0;
     __syncthreads();
