@@ -29,6 +29,7 @@
 // left to single warps.
 #include "evolve.cuh"
 #include "launch_count.cuh"
+#include "smem_limit.cuh"
 #include "rng.cuh"
 #include "crmath.cuh"
 #include "mlp.cuh"
@@ -2386,8 +2387,7 @@ namespace {
 
 template <class Params>
 int launch(void (*kernel)(Params), const Params& p, int grid, size_t smem, void* stream) {
-  const cudaError_t e =
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  const cudaError_t e = allow_shared_memory(kernel);
   if (e != cudaSuccess) return static_cast<int>(e);
   kernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(p);
   count_launch();

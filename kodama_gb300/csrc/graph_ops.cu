@@ -18,6 +18,7 @@
 //     d' = (1 + d) / (same/valid)^2 or +inf, row stably sorted by (d', id).
 #include "graph_ops.cuh"
 #include "launch_count.cuh"
+#include "smem_limit.cuh"
 
 #include <cuda_runtime.h>
 
@@ -527,9 +528,7 @@ int build_reverse_tables(const ReverseArgs& a, cudaStream_t st) {
   // two CTAs an SM: ranges until the chip is full, up to 16 of them
   const int parts = std::max(1, std::min(std::min(16, 2 * 152 / a.problems), a.L));
   const size_t smem = sizeof(int) * (static_cast<size_t>(a.L) / parts + 2);
-  if (smem > 48 * 1024) {
-    cudaFuncSetAttribute(reverse_table_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  }
+  if (smem > 48 * 1024) allow_shared_memory(reverse_table_kernel);
   reverse_table_kernel<<<dim3(a.problems, parts), 1024, smem, st>>>(a);
   count_launch();
   return static_cast<int>(cudaGetLastError());
@@ -544,9 +543,7 @@ int project_labels(const ProjectArgs& a, cudaStream_t st) {
 
 int code_labels(const CodingArgs& a, cudaStream_t st) {
   const size_t smem = sizeof(int) * (static_cast<size_t>(a.k) + 1);
-  if (smem > 48 * 1024) {
-    cudaFuncSetAttribute(code_labels_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  }
+  if (smem > 48 * 1024) allow_shared_memory(code_labels_kernel);
   code_labels_kernel<<<a.problems, 1024, smem, st>>>(a);
   count_launch();
   return static_cast<int>(cudaGetLastError());
@@ -586,8 +583,7 @@ int dissimilarity(const DissimArgs& a, cudaStream_t st) {
   cfg.dynamicSmemBytes = static_cast<size_t>(wpb) * a.K * (sizeof(float) + sizeof(int));
   cfg.stream = st;
   if (cfg.dynamicSmemBytes > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               static_cast<int>(cfg.dynamicSmemBytes));
+    const cudaError_t e = allow_shared_memory(kernel);
     if (e != cudaSuccess) return static_cast<int>(e);
   }
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a);

@@ -17,6 +17,7 @@
 #include "kmeans.cuh"
 #include "knn.cuh"
 #include "launch_count.cuh"
+#include "smem_limit.cuh"
 #include "tcgen05.cuh"
 
 #include <cuda_runtime.h>
@@ -1386,8 +1387,7 @@ int kmeans_run(const KMeansBatch& B, cudaStream_t st) {
   const int nch = (B.k + 31) / 32;
   // kernels with room for 2, 4, 8 or 16 chunks of 32 centroids in registers
   auto go = [&](auto kern, dim3 grid, size_t bytes, auto... more) {
-    const cudaError_t err =
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+    const cudaError_t err = allow_shared_memory(kern);
     if (err != cudaSuccess) return err;
     kern<<<grid, kThreads5, bytes, st>>>(T, more...);
     return cudaGetLastError();
@@ -1437,12 +1437,14 @@ int kmeans_run(const KMeansBatch& B, cudaStream_t st) {
     else if (B.d <= 64) assign_kernel<4><<<agrid, 128, cs_bytes, st>>>(B, final_pass);
     else assign_kernel<0><<<agrid, 128, cs_bytes, st>>>(B, final_pass);
   };
-  cudaFuncSetAttribute(assign_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cs_bytes));
-  cudaFuncSetAttribute(assign_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cs_bytes));
-  cudaFuncSetAttribute(assign_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cs_bytes));
-  cudaFuncSetAttribute(assign_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cs_bytes));
-  cudaFuncSetAttribute(sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sort_bytes));
-  cudaFuncSetAttribute(sums_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sum_bytes));
+  if (!tc) {
+    allow_shared_memory(assign_kernel<1>);
+    allow_shared_memory(assign_kernel<2>);
+    allow_shared_memory(assign_kernel<4>);
+    allow_shared_memory(assign_kernel<0>);
+  }
+  allow_shared_memory(sort_kernel);
+  allow_shared_memory(sums_kernel);
   const int iters = B.max_iter > 1 ? B.max_iter : 1;
   const bool scan = B.d <= kScanCols * kScanThreads;
   for (int it = 0; it < iters; ++it) {

@@ -20,6 +20,7 @@
 #include "ext80.h"
 #include "knn.cuh"
 #include "launch_count.cuh"
+#include "smem_limit.cuh"
 
 #include <cuda_runtime.h>
 #include <math.h>
@@ -333,8 +334,7 @@ int launch_segments(const float* x, int n, int d, int K, int segments, const int
     knn_segment_kernel<4, IP, FOLD><<<grid, kQ, smem, st>>>(x, n, d, K, seg_len, folds, qrows, nq, pd, pi);
   } else {
     if (smem > 48 * 1024) {
-      const cudaError_t e = cudaFuncSetAttribute(knn_segment_generic_kernel<IP, FOLD>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+      const cudaError_t e = allow_shared_memory(knn_segment_generic_kernel<IP, FOLD>);
       if (e != cudaSuccess) return static_cast<int>(e);
     }
     knn_segment_generic_kernel<IP, FOLD><<<grid, kQ, smem, st>>>(x, n, d, K, seg_len, folds, qrows, nq, pd, pi);

@@ -40,6 +40,7 @@
 // products lost to underflow.
 #include "knn.cuh"
 #include "launch_count.cuh"
+#include "smem_limit.cuh"
 
 #include "bf16_split.cuh"
 #include "tcgen05.cuh"
@@ -860,8 +861,7 @@ TcLayout tc_layout(int n, int d, int K, int segments, int sms, const KnnFoldPlan
 
 template <int P>
 cudaError_t launch_candidates(const SearchArgs& S, const TcLayout& L, cudaStream_t st) {
-  const cudaError_t e = cudaFuncSetAttribute(candidates_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(L.smem));
+  const cudaError_t e = allow_shared_memory(candidates_kernel<P>);
   if (e != cudaSuccess) return e;
   candidates_kernel<P><<<L.ctas, kThreads, L.smem, st>>>(S);
   return cudaGetLastError();

@@ -22,6 +22,7 @@
 // Lemire's method (rng.cuh).
 #include "ext80.h"
 #include "launch_count.cuh"
+#include "smem_limit.cuh"
 #include "plan.cuh"
 #include "rng.cuh"
 
@@ -626,12 +627,12 @@ int plan_landmarks(const PlanArgs& a, cudaStream_t st) {
   const PlanScratch s = carve(a);
   const int fit = kCounterBytes / static_cast<int>(sizeof(int)) / a.strata;
   const int counter_bytes = fit >= 2 ? std::min(32, fit) * a.strata * static_cast<int>(sizeof(int)) : 0;
-  cudaError_t e = cudaFuncSetAttribute(strata_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCounterBytes);
+  cudaError_t e = allow_shared_memory(strata_kernel);
   if (e != cudaSuccess) return static_cast<int>(e);
   strata_kernel<<<1, 1024, counter_bytes, st>>>(a, s);
   count_launch();
   const size_t smem = plan_smem_bytes(a.strata);
-  e = cudaFuncSetAttribute(plan_runs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  e = allow_shared_memory(plan_runs_kernel);
   if (e != cudaSuccess) return static_cast<int>(e);
   plan_runs_kernel<<<a.runs, kPlanThreads, smem, st>>>(a, s);
   count_launch();

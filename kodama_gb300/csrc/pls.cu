@@ -24,6 +24,7 @@
 #include "pls.cuh"
 #include "exact_dot.cuh"
 #include "launch_count.cuh"
+#include "smem_limit.cuh"
 
 #include <float.h>
 #include <math.h>
@@ -1588,15 +1589,13 @@ int pls_evaluate(const PlsEvalArgs& a, cudaStream_t st) {
   const size_t smem = bytes(b.ldw);
   auto* const eval = std::max(S, a.live) <= 152 ? eval_kernel<1> : eval_kernel<2>;
   if (smem > 48 * 1024) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(eval, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    const cudaError_t e = allow_shared_memory(eval);
     if (e != cudaSuccess) return static_cast<int>(e);
   }
   const size_t stream_smem = cross_stream_smem(a.C0max);
   if (stream_smem <= most) {
     if (stream_smem > 48 * 1024) {
-      const cudaError_t e = cudaFuncSetAttribute(cross_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 static_cast<int>(stream_smem));
+      const cudaError_t e = allow_shared_memory(cross_stream_kernel);
       if (e != cudaSuccess) return static_cast<int>(e);
     }
     cross_stream_kernel<<<dim3((a.p + 31) / 32, std::min(S, 65535)), kStreamThreads, stream_smem, st>>>(b);
