@@ -535,6 +535,7 @@ EvolveBuffers run_evolution(Ctx& ctx, kgb::EvolveParams P, int C0max) {
     ra.problems = problems;
     ra.L = L;
     ra.w = P.w;
+    ra.sms = ctx.sms();
     ra.nb = P.nb;
     ra.rev_off = roff;
     ra.rev_idx = ridx;
@@ -777,6 +778,7 @@ PlsBuffers pls_buffers(Ctx& ctx, const float* d_X, int R, int L, int p, const Pl
   e.requested = requested;
   e.predict_mode = d_Xv != nullptr;
   e.s_in_smem = s_in_smem ? 1 : 0;
+  e.sms = ctx.sms();
   e.tiles_after_s = 1;  // no fold Gram yet: every slice computes scores in the fit
   e.zp = a.zp;
   e.Z = a.Z;

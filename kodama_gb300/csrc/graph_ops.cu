@@ -526,7 +526,7 @@ int build_vote_tables(const VoteTableArgs& a, cudaStream_t st) {
 
 int build_reverse_tables(const ReverseArgs& a, cudaStream_t st) {
   // two CTAs an SM: ranges until the chip is full, up to 16 of them
-  const int parts = std::max(1, std::min(std::min(16, 2 * 152 / a.problems), a.L));
+  const int parts = std::max(1, std::min(std::min(16, 2 * a.sms / a.problems), a.L));
   const size_t smem = sizeof(int) * (static_cast<size_t>(a.L) / parts + 2);
   if (smem > 48 * 1024) allow_shared_memory(reverse_table_kernel);
   reverse_table_kernel<<<dim3(a.problems, parts), 1024, smem, st>>>(a);

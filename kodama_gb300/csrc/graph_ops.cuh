@@ -23,6 +23,7 @@ struct VoteTableArgs {
 
 struct ReverseArgs {
   int problems, L, w;
+  int sms;                // the device's SM count
   const uint16_t* nb;     // problems x L x w
   int* rev_off;           // problems x (L+1)
   uint16_t* rev_idx;      // problems x L x w

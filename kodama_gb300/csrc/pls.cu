@@ -1587,7 +1587,7 @@ int pls_evaluate(const PlsEvalArgs& a, cudaStream_t st) {
   PlsEvalArgs b = a;
   b.ldw = bytes(padded) <= (bytes(a.max_components) <= two_ctas ? two_ctas : most) ? padded : a.max_components;
   const size_t smem = bytes(b.ldw);
-  auto* const eval = std::max(S, a.live) <= 152 ? eval_kernel<1> : eval_kernel<2>;
+  auto* const eval = std::max(S, a.live) <= a.sms ? eval_kernel<1> : eval_kernel<2>;
   if (smem > 48 * 1024) {
     const cudaError_t e = allow_shared_memory(eval);
     if (e != cudaSuccess) return static_cast<int>(e);

@@ -44,6 +44,7 @@ struct PlsEvalArgs {
   int problems;          // R, or those of one launch
   int first;             // of them the first (the arrays hold all problems)
   int live;              // slices of all launches that run side by side (0: this one's)
+  int sms;               // the device's SM count
   int F;                 // slices per problem
   int L;                 // rows per problem
   int p;                 // columns
