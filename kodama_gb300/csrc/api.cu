@@ -272,6 +272,19 @@ class Ctx {
     bufs_.push_back(p);
     return static_cast<T*>(p);
   }
+  // `bytes` of memory, or nullptr where there is not that much: for work that has a
+  // way with less.
+  void* try_alloc(size_t bytes) {
+    void* p = nullptr;
+    const cudaError_t e = cudaMallocAsync(&p, bytes, stream_);
+    if (e == cudaErrorMemoryAllocation) {
+      (void)cudaGetLastError();
+      return nullptr;
+    }
+    ck(e, "cudaMallocAsync");
+    bufs_.push_back(p);
+    return p;
+  }
   template <class T>
   T* upload(const T* host, size_t count) {
     T* d = alloc<T>(count);
@@ -1753,9 +1766,14 @@ void matrix_finalize(Ctx* ctx, MatrixTail& t, kgb_matrix_result* out, Clock& clk
 // (native_knn.cpp:1157-1164).  Euclidean: the tensor-core candidate search
 // with its certificate where it applies (knn_tc.cu), else the brute force.
 // Cosine (rows scaled as normalize_rows_for_cosine, kodama_matrix.cpp:155)
-// and inner product: the brute-force search on minus the inner product.
+// and inner product: the same searches on minus the inner product.
 // fallback_rows (host, may be null) receives how many rows the brute force
 // computed.
+// The tensor search keeps candidate lists, 4 KB a row up to 35 neighbours, 8 KB up to
+// 111 and 16 KB above (more segments of them below some 40000 rows), and 32 bytes a
+// neighbour and row for rows that go to the brute force: with the operands 0.56 GB
+// at 100000 x 50, K = 30, and 11.9 GB at a million rows, K = 100.  Where that is not to
+// be had the brute force takes the call with its part alone (0.1 and 3.2 GB).
 void exact_graph(Ctx& ctx, const float* d_x, int n, int d, int K, int method, int metric, int* d_idx, float* d_dist,
                  int* fallback_rows) {
   const int segments = 4;
@@ -1769,14 +1787,18 @@ void exact_graph(Ctx& ctx, const float* d_x, int n, int d, int K, int method, in
     ck_launch(kgb::normalize_rows(d_x, n, d, 2, xn, ctx.stream()), "cosine rows");
     xs = xn;
   }
-  const bool tc = method == KGB_KNN_TENSOR || (method == KGB_KNN_AUTO && kgb::knn_tc_supported(n, d, K));
-  if (tc) {
-    void* scratch = ctx.alloc<unsigned char>(kgb::knn_tc_scratch(n, d, K, segments, ctx.sms()));
-    ck_launch(kgb::knn_tc_graph(xs, n, d, K, metric, segments, ctx.sms(), scratch, d_idx, d_dist, ctx.stream()),
+  void* room = nullptr;
+  if (method == KGB_KNN_TENSOR) {
+    room = ctx.alloc<unsigned char>(kgb::knn_tc_scratch(n, d, K, segments, ctx.sms()));
+  } else if (method == KGB_KNN_AUTO && kgb::knn_tc_supported(n, d, K)) {
+    room = ctx.try_alloc(kgb::knn_tc_scratch(n, d, K, segments, ctx.sms()));
+  }
+  if (room != nullptr) {
+    ck_launch(kgb::knn_tc_graph(xs, n, d, K, metric, segments, ctx.sms(), room, d_idx, d_dist, ctx.stream()),
               "kNN graph");
     if (fallback_rows != nullptr) {
       int count = 0;
-      ck_launch(kgb::knn_tc_fallback_count(scratch, n, d, K, segments, ctx.sms(), &count, ctx.stream()), "kNN graph");
+      ck_launch(kgb::knn_tc_fallback_count(room, n, d, K, segments, ctx.sms(), &count, ctx.stream()), "kNN graph");
       ctx.sync();
       *fallback_rows = count;
     }
@@ -2411,13 +2433,14 @@ void fold_search(Ctx& ctx, const float* xs, int n, int d, int K, int metric, con
   const bool inner = metric != KGB_METRIC_EUCLIDEAN;
   kgb::KnnFoldPlan fp;
   if (kgb::knn_tc_supported(n, d, K)) fp = kgb::knn_fold_plan(folds, d, K);
-  if (fp.tiles > 0) {
+  void* const room =
+      fp.tiles > 0 ? ctx.try_alloc(kgb::knn_tc_scratch(n, d, K, segments, ctx.sms(), &fp)) : nullptr;
+  if (room != nullptr) {
     const int* d_perm = ctx.upload(fp.perm.data(), fp.perm.size());
     const int* d_off = ctx.upload(fp.off.data(), fp.off.size());
     const int* d_skip = ctx.upload(fp.skip.data(), fp.skip.size());
-    void* scratch = ctx.alloc<unsigned char>(kgb::knn_tc_scratch(n, d, K, segments, ctx.sms(), &fp));
     ck_launch(kgb::knn_tc_fold_search(xs, n, d, K, inner, d_folds, fp, d_perm, d_off, d_skip, segments, ctx.sms(),
-                                      scratch, d_idx, d_dist, ctx.stream()),
+                                      room, d_idx, d_dist, ctx.stream()),
               "fold-wise kNN");
     return;
   }
