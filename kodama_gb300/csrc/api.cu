@@ -1790,7 +1790,7 @@ void exact_graph(Ctx& ctx, const float* d_x, int n, int d, int K, int method, in
   void* room = nullptr;
   if (method == KGB_KNN_TENSOR) {
     room = ctx.alloc<unsigned char>(kgb::knn_tc_scratch(n, d, K, segments, ctx.sms()));
-  } else if (method == KGB_KNN_AUTO && kgb::knn_tc_supported(n, d, K)) {
+  } else if (method == KGB_KNN_AUTO && kgb::knn_tc_pays(n, d, K, metric)) {
     room = ctx.try_alloc(kgb::knn_tc_scratch(n, d, K, segments, ctx.sms()));
   }
   if (room != nullptr) {
@@ -2431,8 +2431,7 @@ void fold_search(Ctx& ctx, const float* xs, int n, int d, int K, int metric, con
                  const int* d_folds, int* d_idx, float* d_dist) {
   const int segments = 4;
   const bool inner = metric != KGB_METRIC_EUCLIDEAN;
-  kgb::KnnFoldPlan fp;
-  if (kgb::knn_tc_supported(n, d, K)) fp = kgb::knn_fold_plan(folds, d, K);
+  const kgb::KnnFoldPlan fp = kgb::knn_fold_plan(folds, d, K, metric);
   void* const room =
       fp.tiles > 0 ? ctx.try_alloc(kgb::knn_tc_scratch(n, d, K, segments, ctx.sms(), &fp)) : nullptr;
   if (room != nullptr) {

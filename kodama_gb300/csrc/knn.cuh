@@ -40,6 +40,8 @@ int knn_bruteforce_rows(const float* x, int n, int d, int K, bool inner, const i
 // re-rank and a per-row certificate (knn_tc.cu); rows whose certificate fails
 // are recomputed by knn_bruteforce_rows.  sms: the device's SM count.
 bool knn_tc_supported(int n, int d, int K);
+// ... and is the faster one for the graph
+bool knn_tc_pays(int n, int d, int K, int metric);
 // the sizes a caller may force the tensor search for (KGB_KNN_TENSOR)
 bool knn_tc_explicit(int n, int d, int K);
 struct KnnFoldPlan;
@@ -55,13 +57,13 @@ int knn_tc_fallback_count(const void* scratch, int n, int d, int K, int segments
 // to whole candidate tiles, so that a query tile leaves out its own fold's
 // tiles.  perm: row of every position (-1 = padding); per query tile the first
 // (query tile, candidate tile) pair and the (first, count) of the tiles left
-// out.  No tiles: the padding of many small folds costs more than the tensor
-// search saves, the brute force (knn_fold_search) is the way.
+// out.  No tiles: the sizes are out of its range, or the padding of many small folds
+// costs more than the tensor search saves; the brute force (knn_fold_search) is the way.
 struct KnnFoldPlan {
   int tiles = 0, pairs = 0;
   std::vector<int> perm, off, skip;
 };
-KnnFoldPlan knn_fold_plan(const std::vector<int>& folds, int d, int K);
+KnnFoldPlan knn_fold_plan(const std::vector<int>& folds, int d, int K, int metric);
 // knn_fold_search through the tensor-core candidate search; d_perm, d_off and
 // d_skip are the plan's arrays on the device.
 int knn_tc_fold_search(const float* x, int n, int d, int K, bool inner, const int* d_folds, const KnnFoldPlan& fp,

@@ -798,11 +798,9 @@ int bf16_split_rows(const float* x, int n, int d, int dp, uint16_t* xh, uint16_t
 
 namespace {
 
-// From one candidate tile on: whole calls at 256 rows x 10, K = 10 take 144 us
-// here and 150 us by the brute force, at K = 100 159 and 491 us, at 1000 rows x
-// 50, K = 100 196 and 1922 us.  Up to 223 neighbours: lists of 512 entries.  Up to
-// 2^26 rows: their lists, 4 KB a row at least, take all of the memory.
-constexpr int kMinRows = 256;
+// Up to 223 neighbours: lists of 512 entries.  Up to 2^26 rows: their lists, 4 KB a row
+// at least, take all of the memory.
+constexpr int kMinRows = 97;
 constexpr int kMaxRows = 1 << 26;
 
 struct TcLayout {
@@ -966,6 +964,28 @@ int knn_tc_fallback_count(const void* scratch, int n, int d, int K, int segments
 
 namespace {
 
+// The brute force's time in ns: its scan of the rows (another kernel above 64
+// coordinates; at few rows the latency of a row's chain over a segment) and the
+// insertions into the kept neighbours, which grow with their number.
+double brute_ns(int n, int d, int K) {
+  const double rows = n, k = K;
+  const double scan = d <= 64 ? std::max(2.2e-4 * rows * rows * (d + 1), 1.2 * rows * (d + 6))
+                              : std::max(7e-3 * rows * rows * d, 18.0 * rows * d);
+  return scan + std::max(450.0 * k * std::sqrt(rows), 0.4 * rows * k * std::min(k, 64.0));
+}
+
+// ... and that of a 128 x 256 tile's products and lists.
+double pair_ns(int d) { return 6.0 + 0.03 * d; }
+
+// Points on a line, or on a circle once scaled to length one: from some thousands of
+// rows on more of them lie within the products' error bound of a row than its list
+// holds, and nearly all rows would go on to the brute force as well.  30000 rows, line
+// and circle, K = 10: 1.2 and 1.0 of the brute force's time, K = 30 0.7 and 0.6; 100000
+// rows, K = 30 1.1, K = 90 0.7 and 1.0; 8000 rows, K = 1 1.3 and below 1.
+bool too_close(int n, int d, int K, int metric) {
+  return metric != 1 && d <= (metric == 0 ? 2 : 1) && K <= n / 3000;
+}
+
 // Whether the fold-wise search is the faster by tensor cores.  Every fold is padded
 // to whole tiles, so the products grow with the number of folds: leave-one-out of n
 // rows would take n (n - 1) tiles' products and 4 KB or more of lists for 256 n
@@ -974,25 +994,30 @@ namespace {
 // 0.2% behind the better side on average, 1.15x at worst up to 100 folds and 1.36x
 // beyond; always the tensor search 8.5% and 3.3x): 10000 x 50, K = 10, 300 folds take 2.45 ms here and
 // 2.51 by the brute force, 1000 folds 10.8 and 3.1; 1000 x 8, K = 10, 60 folds 0.45
-// and 0.47, 300 folds 1.20 and 0.66; 10000 x 128, 1000 folds 13.7 and 100.  The brute
-// force has another kernel above 64 coordinates, inserts more the more neighbours
-// are kept, and waits for its chains at few rows.
+// and 0.47, 300 folds 1.20 and 0.66; 10000 x 128, 1000 folds 13.7 and 100.
 bool fold_plan_pays(int n, int d, int K, long long tiles, long long pairs) {
   // room: lists of up to 16 KB a position; pairs and positions are counted in ints
   if (tiles * kBlockRows > std::max(131072ll, 16ll * n) || pairs > (1ll << 30)) return false;
-  const double rows = n, k = K;
-  const double tensor = 50e3 + 8.0 * rows + static_cast<double>(pairs) * (6.0 + 0.03 * d);
-  const double scan = d <= 64 ? std::max(2.2e-4 * rows * rows * (d + 1), 1.2 * rows * (d + 6))
-                              : std::max(7e-3 * rows * rows * d, 18.0 * rows * d);
-  const double keep = std::max(450.0 * k * std::sqrt(rows), 0.4 * rows * k * std::min(k, 64.0));
-  return tensor < scan + keep;
+  return 50e3 + 8.0 * n + static_cast<double>(pairs) * pair_ns(d) < brute_ns(n, d, K);
 }
 
 }  // namespace
 
-KnnFoldPlan knn_fold_plan(const std::vector<int>& folds, int d, int K) {
+// The graph's search, measured against the brute force over 97 to 100000 rows, 1 to 256
+// coordinates, 1 to 90 neighbours and the three metrics.  Its launches take some 65 us
+// more, which few neighbours of few rows do not earn: 256 x 8, K = 1 0.145 and 0.101 ms
+// a call, 512 x 8, K = 5 0.13 and 0.12, K = 10 0.18 and 0.23, 2000 x 8, K = 1 equal; 100 x
+// 100, K = 30 0.19 and 0.45.
+bool knn_tc_pays(int n, int d, int K, int metric) {
+  if (!knn_tc_supported(n, d, K) || too_close(n, d, K, metric)) return false;
+  const double pairs = static_cast<double>((n + kBlockRows - 1) / kBlockRows) * ((n + kQRows - 1) / kQRows);
+  return 65e3 + pairs * pair_ns(d) < brute_ns(n, d, K);
+}
+
+KnnFoldPlan knn_fold_plan(const std::vector<int>& folds, int d, int K, int metric) {
   KnnFoldPlan p;
   const int n = static_cast<int>(folds.size());
+  if (!knn_tc_supported(n, d, K) || too_close(n, d, K, metric) || n < 256) return p;
   // the rows by fold, ascending within one (fold numbers lie below n: make_folds)
   std::vector<int> size;
   for (int f : folds) {

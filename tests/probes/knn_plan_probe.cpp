@@ -11,9 +11,11 @@ long long probe_scratch(int n, int d, int K, int sms) {
 
 int probe_supported(int n, int d, int K) { return kgb::knn_tc_supported(n, d, K) ? 1 : 0; }
 
+int probe_pays(int n, int d, int K, int metric) { return kgb::knn_tc_pays(n, d, K, metric) ? 1 : 0; }
+
 // tiles of the fold plan (0: brute force); off, skip and perm copied where room is given
 int probe_fold_plan(const int* folds, int n, int d, int K, int* perm, int* off, int* skip, int* pairs) {
-  const kgb::KnnFoldPlan p = kgb::knn_fold_plan(std::vector<int>(folds, folds + n), d, K);
+  const kgb::KnnFoldPlan p = kgb::knn_fold_plan(std::vector<int>(folds, folds + n), d, K, 2);
   *pairs = p.pairs;
   if (perm != nullptr) std::copy(p.perm.begin(), p.perm.end(), perm);
   if (off != nullptr) std::copy(p.off.begin(), p.off.end(), off);

@@ -41,6 +41,13 @@ def test_row_limit(probe):
     assert not probe.probe_supported((1 << 26) + 1, 10, 10)
 
 
+@pytest.mark.parametrize("n,d,K,metric,tensor", [
+    (96, 100, 30, 2, False), (100, 100, 30, 2, True), (256, 8, 1, 0, False), (256, 8, 10, 0, True), (1 << 25, 50, 30, 2, True),
+    (30000, 1, 10, 2, False), (30000, 1, 11, 2, True), (30000, 2, 10, 0, False), (30000, 2, 10, 1, True), (1000, 257, 5, 2, False)])
+def test_graph_rule(probe, n, d, K, metric, tensor):
+    assert bool(probe.probe_pays(n, d, K, metric)) == tensor
+
+
 def _plan(probe, folds, d, K):
     n = len(folds)
     folds = np.ascontiguousarray(folds, np.int32)
