@@ -1144,8 +1144,10 @@ void matrix_from_device_graph(Ctx& ctx, const float* d_x, int n, int d, int* d_g
   // SMs that leaves idle.  A long one goes between the two, beside the planning,
   // whose CTAs fit on the same SMs.  The search grows as n^2 d: 60000 x 50 rows
   // (1.8e11) take 16.3 ms beside the planning and 17.4 beside the k-means,
-  // 100000 x 50 22.4 and 24.0, but 60000 x 20 (7e10) 16.8 and 15.5, 30000 x 200
-  // (1.8e11) 12.1 and 11.9 (100 runs of 20 cycles).
+  // 100000 x 50 22.4 and 24.0, but 60000 x 20 (7e10) 16.8 and 15.5 (100 runs of 20
+  // cycles).  The stages it runs beside grow with n too, so the line is not one of
+  // n^2 d alone: 30000 x 200 (1.8e11) falls on the wrong side of it by 2% (12.1 and
+  // 11.9).
   const bool graph_early = static_cast<double>(n) * n * d >= 1.0e11;
   int ev_bg0 = -1, ev_bg1 = -1, ev_planned = -1;
   bool graph_bg = false;

@@ -33,6 +33,7 @@
 #include "rng.cuh"
 #include "crmath.cuh"
 #include "mlp.cuh"
+#include "warp_match.cuh"
 
 #include <cuda_runtime.h>
 #include <float.h>
@@ -571,18 +572,6 @@ __device__ __noinline__ int vote_tiebreak(int code, unsigned tied, const float* 
   return bc;
 }
 
-// Lanes holding the same code (of `bits` bits) as this one, of those with `in`,
-// by a ballot a bit.  __match_any_sync takes two cycles of the whole SM per
-// distinct code, which suits a vote's few (by ballots 20000 x 50 rows took 13.1 ms
-// in place of 12.1) but not a sort's.
-__device__ __forceinline__ unsigned same_code(int code, bool in, int bits) {
-  unsigned m = __ballot_sync(kFull, in);
-  for (int b = 0; b < bits; ++b) {
-    const unsigned v = __ballot_sync(kFull, (code >> b) & 1);
-    m &= (code >> b) & 1 ? v : ~v;
-  }
-  return m;
-}
 __device__ __forceinline__ int code_bits(int C0) { return 32 - __clz((C0 - 1) | 1); }
 
 // Fold votes of R rows by one warp (lane j holds neighbour slot j of every
@@ -2060,7 +2049,7 @@ __device__ __forceinline__ void class_lists(const EvolvePlsParams& Q, const Smem
     for (int b = beg; b < end; b += 32) {
       const bool in = b + lane < end;
       const int code = in ? s.cl[b + lane] : 0;
-      const unsigned m = same_code(code, in, bits);
+      const unsigned m = same_code(code, __ballot_sync(kFull, in), bits);
       const int at = in ? mine[code] : 0;
       if (in) place(b + lane, at + __popc(m & below));
       __syncwarp();

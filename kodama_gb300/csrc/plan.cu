@@ -25,6 +25,7 @@
 #include "smem_limit.cuh"
 #include "plan.cuh"
 #include "rng.cuh"
+#include "warp_match.cuh"
 
 #include <algorithm>
 
@@ -75,17 +76,6 @@ PlanScratch carve(const PlanArgs& a) {
   s.flags = reinterpret_cast<uint8_t*>(take(static_cast<size_t>(a.n) * R));
   s.perm = reinterpret_cast<int*>(take(sizeof(int) * static_cast<size_t>(a.target) * R));
   return s;
-}
-
-// Lanes whose code equals this lane's, of those in `act`, by `bits` ballots:
-// __match_any_sync takes two cycles of the SM per distinct code.
-__device__ __forceinline__ unsigned same_code(int code, unsigned act, int bits) {
-  unsigned m = act;
-  for (int b = 0; b < bits; ++b) {
-    const unsigned v = __ballot_sync(0xffffffffu, (code >> b) & 1);
-    m &= (code >> b) & 1 ? v : ~v;
-  }
-  return m;
 }
 
 // Each of nw warps takes a run of rows and counts them per stratum; after a scan

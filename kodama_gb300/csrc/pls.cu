@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(256) gram_kernel(PlsPrepArgs a, const uint8_t*
 constexpr int kMaxNC = 8;      // components per register pass over the rows
 constexpr int kMaxComp = 64;   // components of a fit held per row (local array)
 constexpr uint16_t kNoPos = 0xffffu;  // tpos of a validation row
-constexpr int kTile = 2 * 32 * 16;  // per-warp score tiles: two stages of 32 rows x 16 columns (floats)
+constexpr int kTile = 1024;  // floats per warp: two stages of 64 rows x 8 columns, or four of 32 (stream_scores)
 
 struct EvalShared {
   int m, nt, stop, best, lab, fail, queue;
@@ -370,6 +370,21 @@ __device__ __forceinline__ void stream_scores(const float* __restrict__ base, in
   asm volatile("cp.async.wait_group 0;\n" ::);
 }
 
+// Calls go(std::integral_constant<int, nc>) for nc of 1 to 8.
+template <class Go>
+__device__ __forceinline__ void with_components(int nc, Go&& go) {
+  switch (nc) {
+    case 1: go(std::integral_constant<int, 1>{}); break;
+    case 2: go(std::integral_constant<int, 2>{}); break;
+    case 3: go(std::integral_constant<int, 3>{}); break;
+    case 4: go(std::integral_constant<int, 4>{}); break;
+    case 5: go(std::integral_constant<int, 5>{}); break;
+    case 6: go(std::integral_constant<int, 6>{}); break;
+    case 7: go(std::integral_constant<int, 7>{}); break;
+    default: go(std::integral_constant<int, 8>{}); break;
+  }
+}
+
 // out(row, q, score) for every component q of nc, kMaxNC at a time.
 template <class Out, class Tick>
 __device__ __forceinline__ void stream_all_scores(const float* __restrict__ base, int zp, int p, int nrows,
@@ -383,17 +398,7 @@ __device__ __forceinline__ void stream_all_scores(const float* __restrict__ base
         for (int q = 0; q < NQ; ++q) out(row, q0 + q, acc[q]);
       }, tick);
     };
-    const int nq = min(kMaxNC, nc - q0);
-    switch (nq) {
-      case 1: go(std::integral_constant<int, 1>{}); break;
-      case 2: go(std::integral_constant<int, 2>{}); break;
-      case 3: go(std::integral_constant<int, 3>{}); break;
-      case 4: go(std::integral_constant<int, 4>{}); break;
-      case 5: go(std::integral_constant<int, 5>{}); break;
-      case 6: go(std::integral_constant<int, 6>{}); break;
-      case 7: go(std::integral_constant<int, 7>{}); break;
-      default: go(std::integral_constant<int, 8>{}); break;
-    }
+    with_components(min(kMaxNC, nc - q0), go);
   }
 }
 
@@ -572,21 +577,6 @@ __device__ __forceinline__ float warp_score_products_by_column(float acc, const 
   }
   asm volatile("cp.async.wait_group 0;\n" ::);
   return acc;
-}
-
-// Calls go(std::integral_constant<int, nc>) for nc of 1 to 8.
-template <class Go>
-__device__ __forceinline__ void with_components(int nc, Go&& go) {
-  switch (nc) {
-    case 1: go(std::integral_constant<int, 1>{}); break;
-    case 2: go(std::integral_constant<int, 2>{}); break;
-    case 3: go(std::integral_constant<int, 3>{}); break;
-    case 4: go(std::integral_constant<int, 4>{}); break;
-    case 5: go(std::integral_constant<int, 5>{}); break;
-    case 6: go(std::integral_constant<int, 6>{}); break;
-    case 7: go(std::integral_constant<int, 7>{}); break;
-    default: go(std::integral_constant<int, 8>{}); break;
-  }
 }
 
 __device__ __forceinline__ float score_products(float acc, const float* t, int n, int nc, int ca, int cb, float* buf,
@@ -1162,10 +1152,10 @@ __global__ void __launch_bounds__(kEvalThreads, kCtas) eval_kernel(PlsEvalArgs a
   };
   // The score cross-products are serial chains over all training rows.  With up
   // to seven components they fit the lanes of one warp, which follows the others
-  // a round of batches behind; after the scores they took as long as half of
-  // them again, one warp working.  A short stream is not worth the warp and
-  // the rounds' barriers: at 2000 x 50 rows (4 batches a warp) the scores went
-  // from 62k to 129k cycles and the evaluation from 0.42 to 0.44 ms.
+  // a round of batches behind: 50 runs of 7500 x 200 rows, 10 folds, 50 cycles
+  // 151.6 -> 149.6 ms.  For 10 and 300 slices of 1500 to 8000 rows, 20 to 200
+  // columns and 2 to 7 components the two ways take the same time, so the line at
+  // kFollowRows only keeps the rounds' barriers out of short streams.
   const int ncp = nc * (nc + 1) / 2;
   const bool follow = nc < kMaxNC && !a.da_mode && L >= kFollowRows;
   int prr = 0, pcol = min(lane, ncp - 1);
