@@ -927,13 +927,15 @@ __global__ void __launch_bounds__(kEvalThreads, kCtas) eval_kernel(PlsEvalArgs a
   }
   __syncthreads();
   const int m = sh.m, nt = sh.nt;
+  auto predict_all = [&](int code) {
+    for (int v = threadIdx.x; v < nv; v += kEvalThreads)
+      pred[a.predict_mode ? v : vidx[v]] = static_cast<uint16_t>(code);
+  };
   if (m <= 1 || nt == 0) {
     // one training class: it is every prediction (labels.front() without one);
     // a slice without training rows but with classes is padding, with nothing
     // to predict
-    const int only = m >= 1 ? klist[0] : lab[0];
-    for (int v = threadIdx.x; v < nv; v += kEvalThreads)
-      pred[a.predict_mode ? v : vidx[v]] = static_cast<uint16_t>(only);
+    predict_all(m >= 1 ? klist[0] : lab[0]);
     if (threadIdx.x == 0) a.eval_comp[s] = 1;
     return;
   }
@@ -1115,7 +1117,10 @@ __global__ void __launch_bounds__(kEvalThreads, kCtas) eval_kernel(PlsEvalArgs a
 
   if (fitted < 1) {
     if (a.predict_mode) {
+      // the call ends in an error, but what was queued behind this launch still takes
+      // the predictions as codes of classes: they are never left unwritten
       if (threadIdx.x == 0) a.status[s] = 1;
+      predict_all(klist[0]);
       return;
     }
     // DegeneratePLSFit: the most frequent training class, smallest on ties
@@ -1131,8 +1136,7 @@ __global__ void __launch_bounds__(kEvalThreads, kCtas) eval_kernel(PlsEvalArgs a
       a.eval_comp[s] = 1;
     }
     __syncthreads();
-    for (int v = threadIdx.x; v < nv; v += kEvalThreads)
-      pred[a.predict_mode ? v : vidx[v]] = static_cast<uint16_t>(sh.lab);
+    predict_all(sh.lab);
     return;
   }
 
@@ -1420,7 +1424,10 @@ __global__ void __launch_bounds__(kEvalThreads, kCtas) eval_kernel(PlsEvalArgs a
     a.eval_comp[s] = nc;
   }
   __syncthreads();
-  if (sh.fail) return;
+  if (sh.fail) {
+    predict_all(klist[0]);  // valid codes, as above
+    return;
+  }
   const float* lp = a.logprior + a.lp_off[s];
   for (int k = threadIdx.x; k < m; k += kEvalThreads) {
     // forward and backward substitution for the right-hand side of class k
