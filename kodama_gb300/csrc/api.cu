@@ -817,6 +817,7 @@ PlsBuffers pls_buffers(Ctx& ctx, const float* d_X, int R, int L, int p, const Pl
   e.pred = ctx.alloc<uint16_t>(static_cast<size_t>(R) * (e.predict_mode ? NV : L));
   e.eval_comp = ctx.alloc<int>(S);
   e.status = ctx.alloc<int>(S);
+  ck(cudaMemsetAsync(e.status, 0, sizeof(int) * static_cast<size_t>(S), st), "memset");
   e.s_raw = ctx.alloc<float>(static_cast<size_t>(S) * p * C0max);
   e.s_scr = ctx.alloc<float>(static_cast<size_t>(S) * p * C0max);
   e.T = ctx.alloc<float>(static_cast<size_t>(S) * L * requested);
@@ -845,7 +846,8 @@ void pls_refresh_slices(Ctx& ctx, PlsBuffers& b, const PlsSliceRoom& room, const
   ctx.h2d(room.logprior, tables.data(), tables.size());
   ctx.h2d(room.lp_off, lp_off.data(), lp_off.size());
   b.ntrain = sl.ntrain;
-  b.present = sl.present;
+  // a slice that was present once may have failed then
+  for (size_t q = 0; q < b.present.size(); ++q) b.present[q] |= sl.present[q];
   b.prep.train_off = room.train_off;
   b.prep.train_idx = room.train_idx;
   b.ev.train_off = room.train_off;
@@ -889,7 +891,9 @@ void class_lists_host(const std::vector<uint16_t>& codes, int C0max, std::vector
 }
 
 // Status words of PLS-LDA fits read back after the call's work: with a sink
-// the check is deferred to pls_status_check (the captured batch path).
+// the check is deferred to pls_status_check (the captured batch path).  A status is
+// that of any evaluation since the buffers were made, as the reference's exception
+// ends its call at the first.
 struct PlsStatusSink {
   std::vector<std::vector<int>> status;
   std::vector<std::vector<uint8_t>> present;

@@ -892,7 +892,6 @@ __global__ void __launch_bounds__(kEvalThreads, kCtas) eval_kernel(PlsEvalArgs a
       sh.m = m;
       sh.nt = te - tb;
       sh.queue = 0;
-      a.status[s] = 0;
     }
   }
   // class-list position of every row, whether that position trains the slice,
@@ -1118,7 +1117,8 @@ __global__ void __launch_bounds__(kEvalThreads, kCtas) eval_kernel(PlsEvalArgs a
   if (fitted < 1) {
     if (a.predict_mode) {
       // the call ends in an error, but what was queued behind this launch still takes
-      // the predictions as codes of classes: they are never left unwritten
+      // the predictions as codes of classes: they are never left unwritten.  Nor is a
+      // status taken back by a later evaluation: the host reads it after the last
       if (threadIdx.x == 0) a.status[s] = 1;
       predict_all(klist[0]);
       return;

@@ -76,7 +76,8 @@ struct PlsEvalArgs {
   const uint16_t* class_rows; // R x L rows sorted by code, ascending within a code
   uint16_t* pred;        // CV: R x L predicted codes; predict: R x NV
   int* eval_comp;        // S: components evaluated by the slice
-  int* status;           // S: 0 ok, 1 no supervised direction (degenerate fit), 2 LDA factorisation failed
+  int* status;           // S, cleared by the caller: 1 no supervised direction (degenerate fit), 2 LDA factorisation
+                         // failed, in any of the evaluations; its predictions are then the slice's first class
   // scratch
   float* s_raw;          // S x C0max x p: the cross-product by code
   float* s_scr;          // S x p x C0max: by fold class, when not in shared memory

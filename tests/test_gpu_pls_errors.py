@@ -35,11 +35,23 @@ def test_singular_covariance(kg, orc, n, p, coarsening):
     with pytest.raises(RuntimeError, match="Cholesky"):
         orc.core_plslda(x, lab, components=p, guarded=True, absorption=True, coarsening=coarsening, **kw)
     for _ in range(3):
-        try:
+        with pytest.raises(RuntimeError, match="Cholesky"):
             kg.CorePLSLDA(x, lab, max_components=p, fixed_components=p, guarded_diversity=True,
                           many_to_one_absorption=True, auto_class_coarsening=coarsening, **kw)
-        except RuntimeError as e:
-            assert "Cholesky" in str(e)
+    _healthy(kg, orc)
+
+
+def test_an_early_failure_is_not_forgotten(kg, orc):
+    # the first evaluation fails; absorption and coarsening would mend the later ones
+    for n, p, c in ((120, 5, 3), (80, 4, 2)):
+        x, r = _clusters(n, p, c, n)
+        lab = (r.permutation(n) + 1).astype(np.int32)
+        kw = dict(cycles=30, folds=5, stratified=False, seed=3, cv_seed=4)
+        with pytest.raises(RuntimeError, match="Cholesky"):
+            orc.core_plslda(x, lab, components=p, guarded=True, absorption=True, coarsening=True, evolutionary=True, **kw)
+        with pytest.raises(RuntimeError, match="Cholesky"):
+            kg.CorePLSLDA(x, lab, max_components=p, fixed_components=p, guarded_diversity=True, evolutionary_search=True,
+                          many_to_one_absorption=True, auto_class_coarsening=True, **kw)
     _healthy(kg, orc)
 
 
@@ -47,11 +59,9 @@ def test_singular_covariance_in_a_matrix(kg, orc):
     x, r = _clusters(300, 10, 5, 1)
     start = (r.permutation(300) + 1).astype(np.int32)
     for _ in range(3):
-        try:
+        with pytest.raises(RuntimeError, match="Cholesky"):
             kg.KODAMA_matrix(x, runs=4, cycles=4, classifier="pls", components=10, graph_neighbors=10, knn_k=5, folds=5,
                              starting_labels=start)
-        except RuntimeError as e:
-            assert "Cholesky" in str(e)
     _healthy(kg, orc)
 
 
