@@ -519,10 +519,14 @@ __device__ __forceinline__ void assign_tiles(const KMeansBatch& B, const Layout5
     // ---- landed stages are handed to the tensor core by three threads in
     // turn: the proxy fence takes about 1000 cycles, in the copying threads it
     // would also wait for the copies of later stages, in the issuing thread it
-    // would stand between the products
-    if (lane == 0) {
+    // would stand between the products.  No more threads than stages: a wait tells
+    // a phase from the one after the next only, and a thread at stage s has seen
+    // stage s - relays land, which has to be its slot's last use, s - S, or a later
+    // one (three threads on a ring of two passed stages on before they had landed)
+    const int relays = min(3, S);
+    if (lane == 0 && warp - 13 < relays) {
       const int end = pg.stages + (t1 - t0) * groups;
-      for (int s = pg.stages + (warp - 13); s < end; s += 3) {
+      for (int s = pg.stages + (warp - 13); s < end; s += relays) {
         if (!tc5::mbar_wait(tc5::smem_u32(&sh.full[s % S]), (s / S) & 1, stop)) break;
         fence_async_proxy();
         tc5::mbar_arrive(tc5::smem_u32(&sh.ready[s % S]));
