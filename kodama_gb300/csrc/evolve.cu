@@ -563,7 +563,9 @@ __device__ __noinline__ int vote_tiebreak(int code, unsigned tied, const float* 
         const float st = __shfl_sync(kFull, my, t);
         if ((msk >> t) & 1u) sum = __dadd_rn(sum, static_cast<double>(st));
       }
-      if (sum > bsum || (sum == bsum && v < bc)) {
+      // (the first label stands until a larger sum: a sum that is not a number never is
+      // one, and the result is a label of the row all the same)
+      if (bc == 0x7fffffff || sum > bsum || (sum == bsum && v < bc)) {
         bsum = sum;
         bc = v;
       }
