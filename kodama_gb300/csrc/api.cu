@@ -452,7 +452,7 @@ void constrained_majority(int* labels, const int* groups, size_t n) {
 }
 
 // Status word of the device k-means and landmark planning: 2 when a wait of the
-// k-means ran out (kmeans.cu), else non-zero when the atlas labels or the quota
+// k-means ran out (kmeans.cu), 1, 3 or 4 when the atlas labels or the quota
 // allocation were inconsistent (plan.cu).
 void check_plan_status_value(int v) {
   if (v == 2) fail(KGB_ETIMEOUT, "a wait inside the k-means kernel ran out");

@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(kPlanThreads) plan_runs_kernel(PlanArgs a, Pla
           }
         }
         if (besti < 0) {
-          sh_bad = 2;
+          sh_bad = 4;
           break;
         }
         const int best = order[besti];
